@@ -1750,7 +1750,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   if (timing) EGB_CUDA(cudaEventRecord(ctx->ev[5], st));
 
   launch_combine(tasks_d, (const CombineJob*)dtab(tab_cjobs), (const int32_t*)dtab(tab_chunkjob),
-                 nchunks, ctx->psi_d, ctx->psi_len, (double*)(A + off_partial), zero_d, err_d, st);
+                 nchunks, ctx->psi_d, ctx->psi_len, (double*)(A + off_partial), zero_d, err_d,
+                 ctx->num_sms, st);
   EGB_CUDA(cudaGetLastError());
   if (nchunks)
     EGB_CUDA(cudaMemcpyAsync(H + pin_rb, A + off_partial, sizeof(double) * (size_t)nchunks,

@@ -466,7 +466,7 @@ void launch_emit_items(const JobDev* jobs_d, const ItemRun* runs_d, int nruns, c
                        int64_t nitems, WorkItem* items_d, cudaStream_t st);
 void launch_combine(const TaskDev* tasks_d, const CombineJob* jobs_d, const int32_t* chunk_job_d,
                     int nchunks, const double* psi_tab, int64_t psi_len, double* partial,
-                    uint32_t* zero_flags, uint32_t* err, cudaStream_t st);
+                    uint32_t* zero_flags, uint32_t* err, int num_sms, cudaStream_t st);
 
 // egb_sort.cu
 constexpr int SORT_TILE = 2048;

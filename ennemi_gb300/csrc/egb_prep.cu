@@ -21,6 +21,10 @@
 //                CSEMI  psi(nxz) + psi(nyz) - psi(nz)           (:247)
 //                ENT    log(eps)                                (:42)
 //              psi comes from an FP64 table indexed by the integer count.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
 #include "egb_internal.cuh"
 #include "ennemi_gb.h"
 
@@ -115,14 +119,49 @@ __device__ double pw_leaf(const double* a, const int32_t* inv, int len, bool sq,
   return res;
 }
 
+// The same leaf on eight lanes: lane r keeps the running sum r_r, three
+// exchanges combine them (addition commutes, so every lane holds the same
+// bits) and the remaining values follow in order.  Every lane of the warp
+// calls it (len 0 where a group has no leaf).
+__device__ double pw_leaf8(const double* a, const int32_t* inv, int len, int r, bool sq, double m) {
+  const int end = len >= 8 ? len - (len % 8) : 0;
+  double s = r < end ? pw_value(a, inv, r, sq, m) : 0.0;
+  int i = 8 + r;
+  for (; i + 24 < end; i += 32) {  // four loads in flight, added in order
+    const double v0 = pw_value(a, inv, i, sq, m), v1 = pw_value(a, inv, i + 8, sq, m);
+    const double v2 = pw_value(a, inv, i + 16, sq, m), v3 = pw_value(a, inv, i + 24, sq, m);
+    s = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(s, v0), v1), v2), v3);
+  }
+  for (; i < end; i += 8) s = __dadd_rn(s, pw_value(a, inv, i, sq, m));
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+  if (end == 0) s = 0.0;
+  for (i = end; i < len; ++i) s = __dadd_rn(s, pw_value(a, inv, i, sq, m));
+  return s;
+}
+
 // The block's pairwise sum of x[0, n) (sq: of (x - m)^2): leaves in parallel,
 // then one height at a time; node sums in ns (global, read back through L2).
+// LANES: a leaf on one lane (fewest FP64 operations: the form for more
+// columns than the GPU holds blocks) or on eight (the shortest chain).
+template <int LANES>
 __device__ double pw_sum(const double* x, const int32_t* inv, const PwTree& tr,
                          const int2* __restrict__ nodes, const int32_t* __restrict__ levels,
                          double* ns, bool sq, double m) {
-  for (int i = threadIdx.x; i < tr.nleaf; i += blockDim.x) {
-    const int2 L = nodes[tr.node0 + i];
-    ns[i] = inv ? pw_leaf(x, inv + L.x, L.y, sq, m) : pw_leaf(x + L.x, nullptr, L.y, sq, m);
+  if (LANES == 1) {
+    for (int i = threadIdx.x; i < tr.nleaf; i += blockDim.x) {
+      const int2 L = nodes[tr.node0 + i];
+      ns[i] = inv ? pw_leaf(x, inv + L.x, L.y, sq, m) : pw_leaf(x + L.x, nullptr, L.y, sq, m);
+    }
+  } else {
+    const int r = threadIdx.x & 7, ngroup = blockDim.x >> 3;
+    for (int i0 = 0; i0 < tr.nleaf; i0 += ngroup) {
+      const int i = i0 + (threadIdx.x >> 3);
+      const int2 L = i < tr.nleaf ? nodes[tr.node0 + i] : make_int2(0, 0);
+      const double s = inv ? pw_leaf8(x, inv + L.x, L.y, r, sq, m)
+                           : pw_leaf8(x + L.x, nullptr, L.y, r, sq, m);
+      if (r == 0 && i < tr.nleaf) ns[i] = s;
+    }
   }
   __syncthreads();
   for (int h = 0; h < tr.nlvl; ++h) {
@@ -136,31 +175,144 @@ __device__ double pw_sum(const double* x, const int32_t* inv, const PwTree& tr,
   return __ldcg(ns + tr.nnode - 1);
 }
 
+// s + x_0 + x_1 + ... in order, each addition rounded, for the 32 values of
+// the warp's lanes (the first cnt of them; lane i holds x_i).
+//
+// While the running sum stays inside one binade it is an integer multiple
+// M u of the binade's ulp u, and RN(M u + x) = u (M + rint(x / u)): rounding
+// to the grid u does not depend on M unless x / u lies exactly between two
+// integers (the tie goes to the even sum).  So the additions up to the first
+// one that ties or leaves the binade's interior are a sum of integers, exact
+// and order-free; that one addition is done in FP64, and the rest follow on
+// the new grid.  Integer instructions only, FP64 having few lanes here: a
+// chain of dependent FP64 additions takes 79 cycles each with the loads off
+// it (1.53 ms for two columns of 20,000 rows, mean and deviation).
+__device__ double ordered_add(double s, double x, int cnt) {
+  constexpr int64_t ONE = (int64_t)1 << 52;
+  const int lane = threadIdx.x & 31;
+  const uint64_t ux = (uint64_t)__double_as_longlong(x);
+  const int ex = (int)((ux >> 52) & 0x7ffu);
+  const uint64_t mx = (ux & (uint64_t)(ONE - 1)) | (ex ? (uint64_t)ONE : 0ull);
+  int i0 = 0;  // values before lane i0 are in s
+  while (i0 < cnt) {
+    const uint64_t us = (uint64_t)__double_as_longlong(s);
+    const int e = (int)((us >> 52) & 0x7ffu);
+    int f = i0;  // first value to add in FP64
+    if (e != 0 && e != 0x7ff) {
+      // q = rint(|x| / u): |x| = mx 2^(max(ex, 1) - 1075), u = 2^(e - 1075)
+      const bool mine = lane >= i0 && lane < cnt;
+      const int sh = e - max(ex, 1);
+      const int sr = min(max(sh, 1), 55);  // mx < 2^53: 0 and no tie from 54 on
+      const uint64_t half = 1ull << (sr - 1), rem = mx & ((half << 1) - 1ull);
+      uint64_t q = sh <= 0 ? mx : (mx >> sr) + (rem > half ? 1u : 0u);
+      const bool ok = sh >= 0 && !(sh > 0 && rem == half);  // x below s's binade's end, no tie
+      if (!mine || !ok) q = 0;
+      const bool neg = ((ux ^ us) >> 63) != 0;  // towards zero, with s as positive
+      const int64_t M = (int64_t)((us & (uint64_t)(ONE - 1)) | (uint64_t)ONE);
+      // all at once while |M| +- the sum of q stays inside (q < 2^54, split
+      // at bit 28 for 32-bit reductions)
+      const uint32_t top = __reduce_add_sync(0xffffffffu, (uint32_t)(q >> 28) + 1u);
+      const int64_t reach = (int64_t)top << 28;  // > the sum of q
+      const bool simple = !__any_sync(0xffffffffu, mine && !ok) && M - reach > ONE && M + reach < 2 * ONE;
+      int64_t am;
+      if (simple) {
+        const int hi = neg ? -(int)(q >> 28) : (int)(q >> 28);
+        const int lo = (int)(q & 0xfffffffull);
+        const int64_t shi = __reduce_add_sync(0xffffffffu, hi);
+        // 28 bits in two halves of 14: 32 of them stay within an int
+        const int64_t slo0 = __reduce_add_sync(0xffffffffu, neg ? -(lo & 0x3fff) : (lo & 0x3fff));
+        const int64_t slo1 = __reduce_add_sync(0xffffffffu, neg ? -(lo >> 14) : (lo >> 14));
+        am = M + shi * ((int64_t)1 << 28) + slo1 * ((int64_t)1 << 14) + slo0;
+        f = cnt;
+      } else {
+        int64_t p = neg ? -(int64_t)q : (int64_t)q;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int64_t y = __shfl_up_sync(0xffffffffu, p, o);
+          if (lane >= o) p += y;
+        }
+        const int64_t m = M + p;  // the magnitude after this lane's value, in u
+        const unsigned b = __ballot_sync(0xffffffffu, mine && !(ok && m > ONE && m < 2 * ONE));
+        f = b ? __ffs(b) - 1 : cnt;
+        am = __shfl_sync(0xffffffffu, m, f > i0 ? f - 1 : 0);
+      }
+      if (f > i0)  // ONE < am < 2 ONE: the mantissa of a double of exponent e
+        s = __longlong_as_double((long long)((us & 0xfff0000000000000ull) | ((uint64_t)am & (uint64_t)(ONE - 1))));
+    }
+    // the addition that leaves the grid; a sum that leaves it at once (values
+    // that cancel, subnormal sums) takes eight, so that such data costs no
+    // more than the plain chain
+    const int g = min(cnt, f == i0 ? f + 8 : f + 1);
+    for (; f < g; ++f) s = __dadd_rn(s, __shfl_sync(0xffffffffu, x, f));
+    i0 = g;
+  }
+  return s;
+}
+
+// Sum of x (sq: of (x - m)^2) row by row from the first row, as NumPy reduces
+// axis 0 of an (n, group) array.  The other warps stage the terms of the next
+// rows in shared memory while warp 0 adds.
+constexpr int ROW_STAGE = 1024;
+__device__ double row_sum(const double* x, const int32_t* inv, int n, double* sm, bool sq, double m) {
+  auto stage = [&](int c) {
+    double* d = sm + (c & 1) * ROW_STAGE;
+    const int i0 = c * ROW_STAGE, cnt = min(ROW_STAGE, n - i0);
+    for (int i = (int)threadIdx.x - 32; i < cnt; i += (int)blockDim.x - 32)
+      d[i] = pw_value(x, inv, i0 + i, sq, m);
+  };
+  const int nc = (n + ROW_STAGE - 1) / ROW_STAGE;
+  double s = 0.0;
+  if (threadIdx.x >= 32) stage(0);
+  __syncthreads();
+  for (int c = 0; c < nc; ++c) {
+    if (threadIdx.x >= 32) {
+      if (c + 1 < nc) stage(c + 1);
+    } else {
+      const double* d = sm + (c & 1) * ROW_STAGE;
+      const int cnt = min(ROW_STAGE, n - c * ROW_STAGE);
+      int i = 0;
+      if (c == 0) s = d[i++];
+      for (; i < cnt; i += 32) {
+        const int k = min(32, cnt - i);
+        s = ordered_add(s, (int)threadIdx.x < k ? d[i + threadIdx.x] : 0.0, k);
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) sm[0] = s;
+  __syncthreads();
+  s = sm[0];
+  __syncthreads();
+  return s;
+}
+
+// LANES: pw_sum's form.  8 for a handful of columns (two of 10,000 samples:
+// 24 -> 10 us); 1 for more: 785 columns of 180,000 are FP64-bound (1.42 ms
+// against 1.65 on eight lanes), and a call of 44 columns of 1,000 measured
+// 1.40 ms with eight, 1.31 with one.
+constexpr int STATS_FEW = 16;
+template <int LANES>
 __global__ void __launch_bounds__(PREP_THREADS)
 rescale_stats_kernel(const TaskDev* __restrict__ tasks, const RescaleStat* __restrict__ stats,
                      const PwTree* __restrict__ trees, const int2* __restrict__ nodes,
                      const int32_t* __restrict__ levels, double* __restrict__ scratch,
                      double2* __restrict__ ms) {
+  __shared__ double rows[2 * ROW_STAGE];
   const RescaleStat rs = stats[blockIdx.x];
   const TaskDev t = tasks[rs.task];
   const double* x = t.x64 + (int64_t)rs.col * t.ld;
   const double n = (double)t.n;
   if (rs.group > 1) {  // axis-0 reduction of an (n, group) array: in row order
-    if (threadIdx.x == 0) {
-      double s = pw_value(x, rs.inv, 0, false, 0.0);
-      for (int i = 1; i < t.n; ++i) s = __dadd_rn(s, pw_value(x, rs.inv, i, false, 0.0));
-      const double m = __ddiv_rn(s, n);
-      double q = pw_value(x, rs.inv, 0, true, m);
-      for (int i = 1; i < t.n; ++i) q = __dadd_rn(q, pw_value(x, rs.inv, i, true, m));
-      ms[blockIdx.x] = make_double2(m, __dsqrt_rn(__ddiv_rn(q, n)));
-    }
+    const double mean = __ddiv_rn(row_sum(x, rs.inv, t.n, rows, false, 0.0), n);
+    const double q = row_sum(x, rs.inv, t.n, rows, true, mean);
+    if (threadIdx.x == 0) ms[blockIdx.x] = make_double2(mean, __dsqrt_rn(__ddiv_rn(q, n)));
     return;
   }
   const PwTree tr = trees[rs.tree];
   double* ns = scratch + rs.scratch;
-  const double mean = __ddiv_rn(pw_sum(x, rs.inv, tr, nodes, levels, ns, false, 0.0), n);
+  const double mean = __ddiv_rn(pw_sum<LANES>(x, rs.inv, tr, nodes, levels, ns, false, 0.0), n);
   __syncthreads();  // every thread has read the root before the slots are reused
-  const double sd = __dsqrt_rn(__ddiv_rn(pw_sum(x, rs.inv, tr, nodes, levels, ns, true, mean), n));
+  const double sd = __dsqrt_rn(__ddiv_rn(pw_sum<LANES>(x, rs.inv, tr, nodes, levels, ns, true, mean), n));
   if (threadIdx.x == 0) ms[blockIdx.x] = make_double2(mean, sd);
 }
 
@@ -448,84 +600,118 @@ __device__ __forceinline__ double psi_of(const double* __restrict__ tab, int64_t
   return tab[n];  // entry 0 is a placeholder; zero counts are flagged
 }
 
-__global__ void combine_kernel(const TaskDev* __restrict__ tasks,
-                               const CombineJob* __restrict__ jobs,
-                               const int32_t* __restrict__ chunk_job,
-                               const double* __restrict__ psi_tab, int64_t psi_len,
-                               double* __restrict__ partial, uint32_t* __restrict__ zero_flags,
-                               uint32_t* __restrict__ err) {
-  const int chunk = blockIdx.x;
+// The sample's term of a combine job, with its zero-count flags.
+__device__ __forceinline__ double combine_term(const TaskDev& t, int kind, int64_t i,
+                                               const double* __restrict__ psi_tab, int64_t psi_len,
+                                               uint32_t& zf, uint32_t& bad) {
+  double term;
+  switch (kind) {
+    case EGB_MI: {
+      const int32_t a = t.cnt[0][i], b = t.cnt[1][i];
+      zf |= (a == 0 ? 1u : 0u) | (b == 0 ? 2u : 0u);
+      term = psi_of(psi_tab, psi_len, a, bad) + psi_of(psi_tab, psi_len, b, bad);
+      break;
+    }
+    case EGB_CMI:
+    case EGB_CSEMI: {
+      const int32_t a = t.cnt[0][i], b = t.cnt[1][i], c = t.cnt[2][i];
+      zf |= (a == 0 ? 1u : 0u) | (b == 0 ? 2u : 0u) | (c == 0 ? 4u : 0u);
+      term = (psi_of(psi_tab, psi_len, a, bad) + psi_of(psi_tab, psi_len, b, bad)) -
+             psi_of(psi_tab, psi_len, c, bad);
+      break;
+    }
+    case EGB_SEMI: {
+      const int32_t a = t.cnt[0][i];
+      zf |= (a == 0 ? 1u : 0u);
+      term = psi_of(psi_tab, psi_len, a, bad);
+      break;
+    }
+    case EGB_DISCRETE_ENTROPY: {   // log(c / N)
+      term = log((double)t.cnt[0][i] / (double)t.n);
+      break;
+    }
+    case EGB_DISCRETE_MI: {        // log(N c_xy / (c_x c_y)), integer products exact
+      const int64_t num = (int64_t)t.n * t.cnt[0][i];
+      const int64_t den = (int64_t)t.cnt[1][i] * t.cnt[2][i];
+      term = log((double)num / (double)den);
+      break;
+    }
+    case EGB_DISCRETE_CMI: {       // log(c_z c_xyz / (c_xz c_yz))
+      const int64_t num = (int64_t)t.cnt[3][i] * t.cnt[0][i];
+      const int64_t den = (int64_t)t.cnt[1][i] * t.cnt[2][i];
+      term = log((double)num / (double)den);
+      break;
+    }
+    default: {  // EGB_ENTROPY: log(0) = -inf propagates exactly as in NumPy
+      const double e = t.eps[i];
+      zf |= (e == 0.0 ? 1u : 0u);
+      term = log(e);
+      break;
+    }
+  }
+  return term;
+}
+
+// Sum of a chunk's terms in a fixed order: term(j) = the chunk's j-th, thread
+// i the terms i, i + 256, ..., then warp shuffles, then warp 0 over the warps.
+constexpr int COMBINE_THREADS = 256;
+template <typename F>
+__device__ __forceinline__ void chunk_sum(int cnt, F term, double* out) {
+  __shared__ double wsum[COMBINE_THREADS / 32];
+  double acc = 0.0;
+  for (int j = threadIdx.x; j < cnt; j += COMBINE_THREADS) acc += term(j);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) wsum[warp] = acc;
+  __syncthreads();
+  if (warp == 0) {
+    double v = lane < COMBINE_THREADS / 32 ? wsum[lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) *out = v;
+  }
+}
+
+// CL blocks (a cluster) share a chunk of COMBINE_CHUNK samples: each evaluates
+// 1 / CL of its terms and leaves them in the first block's shared memory,
+// which adds them -- the same order, so the same bits, for every CL.  CL = 8
+// while chunks are fewer than the SMs (the loads, or an entropy's FP64
+// logarithms, are then the time): 3 chunks of an MI 11.6 -> 6 us, 49 of an
+// entropy 41 -> 10 us; CL = 1 where they fill the GPU.
+template <int CL>
+__global__ void __launch_bounds__(COMBINE_THREADS)
+combine_kernel(const TaskDev* __restrict__ tasks, const CombineJob* __restrict__ jobs,
+               const int32_t* __restrict__ chunk_job, const double* __restrict__ psi_tab,
+               int64_t psi_len, double* __restrict__ partial, uint32_t* __restrict__ zero_flags,
+               uint32_t* __restrict__ err) {
+  __shared__ double terms[CL > 1 ? COMBINE_CHUNK : 1];
+  const int chunk = blockIdx.x / CL;
   const CombineJob jb = jobs[chunk_job[chunk]];
   const TaskDev t = tasks[jb.task];
   const int64_t p0 = (int64_t)(chunk - jb.chunk0) * COMBINE_CHUNK;
-  const int64_t p1 = p0 + COMBINE_CHUNK < (int64_t)t.n ? p0 + COMBINE_CHUNK : (int64_t)t.n;
-  double acc = 0.0;
+  const int cnt = (int)min((int64_t)COMBINE_CHUNK, (int64_t)t.n - p0);
   uint32_t zf = 0, bad = 0;
-  for (int64_t i = p0 + threadIdx.x; i < p1; i += blockDim.x) {
-    double term;
-    switch (jb.kind) {
-      case EGB_MI: {
-        const int32_t a = t.cnt[0][i], b = t.cnt[1][i];
-        zf |= (a == 0 ? 1u : 0u) | (b == 0 ? 2u : 0u);
-        term = psi_of(psi_tab, psi_len, a, bad) + psi_of(psi_tab, psi_len, b, bad);
-        break;
-      }
-      case EGB_CMI:
-      case EGB_CSEMI: {
-        const int32_t a = t.cnt[0][i], b = t.cnt[1][i], c = t.cnt[2][i];
-        zf |= (a == 0 ? 1u : 0u) | (b == 0 ? 2u : 0u) | (c == 0 ? 4u : 0u);
-        term = (psi_of(psi_tab, psi_len, a, bad) + psi_of(psi_tab, psi_len, b, bad)) -
-               psi_of(psi_tab, psi_len, c, bad);
-        break;
-      }
-      case EGB_SEMI: {
-        const int32_t a = t.cnt[0][i];
-        zf |= (a == 0 ? 1u : 0u);
-        term = psi_of(psi_tab, psi_len, a, bad);
-        break;
-      }
-      case EGB_DISCRETE_ENTROPY: {   // log(c / N)
-        term = log((double)t.cnt[0][i] / (double)t.n);
-        break;
-      }
-      case EGB_DISCRETE_MI: {        // log(N c_xy / (c_x c_y)), integer products exact
-        const int64_t num = (int64_t)t.n * t.cnt[0][i];
-        const int64_t den = (int64_t)t.cnt[1][i] * t.cnt[2][i];
-        term = log((double)num / (double)den);
-        break;
-      }
-      case EGB_DISCRETE_CMI: {       // log(c_z c_xyz / (c_xz c_yz))
-        const int64_t num = (int64_t)t.cnt[3][i] * t.cnt[0][i];
-        const int64_t den = (int64_t)t.cnt[1][i] * t.cnt[2][i];
-        term = log((double)num / (double)den);
-        break;
-      }
-      default: {  // EGB_ENTROPY: log(0) = -inf propagates exactly as in NumPy
-        const double e = t.eps[i];
-        zf |= (e == 0.0 ? 1u : 0u);
-        term = log(e);
-        break;
-      }
-    }
-    acc += term;
-  }
-  // fixed-order block reduction: warp shuffles, then warp 0 over warp sums
-  __shared__ double wsum[32];
-#pragma unroll
-  for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  zf = __reduce_or_sync(0xffffffffu, zf);
-  bad = __reduce_or_sync(0xffffffffu, bad);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) wsum[warp] = acc;
-  if (lane == 0 && zf) atomicOr(&zero_flags[jb.task], zf);
-  if (lane == 0 && bad) atomicOr(err, (uint32_t)DERR_BAD_INDEX);
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-    double v = lane < nw ? wsum[lane] : 0.0;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) partial[chunk] = v;
+  auto flags = [&]() {
+    zf = __reduce_or_sync(0xffffffffu, zf);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0 && zf) atomicOr(&zero_flags[jb.task], zf);
+    if ((threadIdx.x & 31) == 0 && bad) atomicOr(err, (uint32_t)DERR_BAD_INDEX);
+  };
+  if constexpr (CL == 1) {
+    chunk_sum(cnt, [&](int j) { return combine_term(t, jb.kind, p0 + j, psi_tab, psi_len, zf, bad); },
+              partial + chunk);
+    flags();
+  } else {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    double* first = cl.map_shared_rank(terms, 0);
+    cl.sync();  // every block of the cluster has started
+    for (int j = (int)cl.block_rank() * COMBINE_THREADS + threadIdx.x; j < cnt; j += CL * COMBINE_THREADS)
+      first[j] = combine_term(t, jb.kind, p0 + j, psi_tab, psi_len, zf, bad);
+    flags();
+    cl.sync();
+    if (cl.block_rank() == 0) chunk_sum(cnt, [&](int j) { return terms[j]; }, partial + chunk);
   }
 }
 
@@ -544,10 +730,16 @@ void launch_rescale(const TaskDev* tasks_d, const RescaleStat* stats_d, int nsta
                     const int2* nodes_d, const int32_t* levels_d, double* scratch, double2* ms,
                     const double* noise, uint32_t* zero_flags, int64_t max_n, cudaStream_t st) {
   if (ncols <= 0 || nstats <= 0) return;
-  rescale_stats_kernel<<<nstats, PREP_THREADS, 0, st>>>(tasks_d, stats_d, trees_d, nodes_d, levels_d,
-                                                        scratch, ms);
+  auto stats_kernel = nstats <= STATS_FEW ? rescale_stats_kernel<8> : rescale_stats_kernel<1>;
+  stats_kernel<<<nstats, PREP_THREADS, 0, st>>>(tasks_d, stats_d, trees_d, nodes_d, levels_d, scratch,
+                                                ms);
   count_launch();
-  const dim3 agrid(grid_x_for((max_n + 3) / 4 / 8), grid_y_for(ncols));  // 32 samples a thread
+  // 32 samples a thread where the columns fill the GPU (one division per
+  // block), down to 4 where they do not: two columns of 10,000 samples took
+  // 16 us on two blocks each
+  const int gx = std::min(grid_x_for((max_n + 3) / 4),
+                          std::max(grid_x_for((max_n + 31) / 32), 2048 / std::min(ncols, 2048)));
+  const dim3 agrid(gx, grid_y_for(ncols));
   rescale_apply_kernel<<<agrid, PREP_THREADS, 0, st>>>(tasks_d, cols_d, ms, noise, zero_flags);
   count_launch();
 }
@@ -649,10 +841,26 @@ void launch_radius(const TaskDev* tasks_d, int ntasks, int64_t max_ld, cudaStrea
 
 void launch_combine(const TaskDev* tasks_d, const CombineJob* jobs_d, const int32_t* chunk_job_d,
                     int nchunks, const double* psi_tab, int64_t psi_len, double* partial,
-                    uint32_t* zero_flags, uint32_t* err, cudaStream_t st) {
+                    uint32_t* zero_flags, uint32_t* err, int num_sms, cudaStream_t st) {
   if (nchunks <= 0) return;
-  combine_kernel<<<nchunks, 256, 0, st>>>(tasks_d, jobs_d, chunk_job_d, psi_tab, psi_len,
-                                          partial, zero_flags, err);
+  if (nchunks >= num_sms) {
+    combine_kernel<1><<<nchunks, COMBINE_THREADS, 0, st>>>(tasks_d, jobs_d, chunk_job_d, psi_tab,
+                                                           psi_len, partial, zero_flags, err);
+  } else {
+    constexpr int CL = 8;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = CL;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(nchunks * CL));
+    cfg.blockDim = dim3(COMBINE_THREADS);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, combine_kernel<CL>, tasks_d, jobs_d, chunk_job_d, psi_tab, psi_len,
+                       partial, zero_flags, err);
+  }
   count_launch();
 }
 

@@ -69,6 +69,33 @@ def test_condition_columns_reduce_row_by_row(n, dz):
         assert np.array_equal(N.fetch(0, 18 + c, n).view(np.uint64), Zr[:, c].view(np.uint64)), c
 
 
+@pytest.mark.parametrize("n", [31, 33, 1023, 1025, 1056, 20011])
+@pytest.mark.parametrize("data", ["zero_mean", "ties", "scales", "cancel", "offset"])
+def test_row_sums_on_rounding_boundaries(n, data):
+    """Row-by-row sums that tie, change binade, cancel to zero or mix scales,
+    at lengths around the warp and the staged block: the bits of NumPy's
+    axis-0 reduction."""
+    rng = np.random.default_rng(n)
+    a = rng.normal(size=(n, 2))
+    if data == "ties":        # multiples of half an ulp of the running sum
+        a = rng.integers(-9, 9, (n, 2)) * 0.5 * 2.0 ** rng.integers(-54, 3, (n, 2))
+    elif data == "scales":
+        a *= 10.0 ** rng.integers(-20, 20, (n, 2))
+    elif data == "cancel":
+        a[1::2] = -a[0::2][:n // 2]
+    elif data == "offset":
+        a += 1e6
+    x, y = rng.normal(size=(2, n))
+    cols = [np.ascontiguousarray(c) for c in a.T]
+    res = []
+    N.run_tasks([N.Task(N.CMI, 3, [x], [y], cols, n=n)], flags=N.RESCALE | N.KEEP_INTERNALS,
+                results_out=res, noise=_noise)
+    assert res[0].status == 0
+    want = (a - a.mean(axis=0)) / a.std(axis=0) + _driver._noise.take(2 * n, (n, 2))
+    for c in range(2):
+        assert np.array_equal(N.fetch(0, 18 + c, n).view(np.uint64), want[:, c].view(np.uint64)), c
+
+
 def test_semidiscrete_columns_with_index():
     """Labels and an index together: the class order is applied on top of the
     index; the continuous column is rescaled from noise position 0."""
