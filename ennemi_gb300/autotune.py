@@ -80,8 +80,6 @@ def _tune_key(ctx, key: Key, size_classes: Sequence[int], repeats: int,
               prune: float, log) -> Dict[int, Tuple[int, Dict[int, float]]]:
     search, d, K = key
     alive = list(MODES)
-    if search == 0 and K > 8:
-        alive.remove(N.MODE_WARP_GRID)     # the warp grid runs kNN only for K <= 8
     if search == 0 or d != 2:
         alive.remove(N.MODE_RANK)          # rank-space counts: d = 2 ball counts only
     out = {}

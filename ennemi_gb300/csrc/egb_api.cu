@@ -654,7 +654,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     int sort_seg_c;
   };
   // layout of a multi-D job: EGB_FORCE_* flags, else the context's policy
-  // table, else the built-in rule; warp grid kNN needs K <= 8
+  // table, else the built-in rule; warp grid kNN needs K <= LIST_K_MAX (K <= 8
+  // in FP64)
   // mode 4: rank-space counts (d = 2 ball counts, FP32 path only)
   auto pick_mode = [&](bool is_knn, const Space& s) {
     const int64_t len = s.e - s.b;
@@ -669,8 +670,13 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       if (mode == EGB_MODE_AUTO) mode = len >= SLAB_MIN ? (rank_ok ? 4 : 3) : 0;
     }
     if (mode == 4 && !rank_ok) mode = 3;
-    if (mode == 3 && (cta_grid || (is_knn && s.K > 8))) mode = 2;
+    if (mode == 3 && (cta_grid || (is_knn && s.K > 8 && (plain || s.K > LIST_K_MAX)))) mode = 2;
     return mode;
+  };
+  // class of K that a kNN launch group is compiled for
+  auto kclass_of = [](const MJob& m) {
+    if (!m.is_knn || m.sel == 1) return 0;
+    return m.s.K <= 4 ? 4 : m.s.K <= 8 ? 8 : m.s.K <= 16 ? 16 : m.s.K <= 32 ? 32 : m.s.K <= 64 ? 64 : 128;
   };
   struct WmPlan { Space s; int seg_a, seg_b; };
   std::vector<WmPlan> wplans;
@@ -681,8 +687,17 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       sorted_knn.push_back({seg_for(s.task, s.sp.cols[0], s.b, s.e), s});
     } else {
       MJob m{s, true, 0, -1, 0, -1, 0, -1};
-      if (s.K > EGB_KREG_MAX) m.sel = 1;
-      else m.mode = pick_mode(true, s);
+      if (s.K <= EGB_KREG_MAX) {
+        m.mode = pick_mode(true, s);
+      } else if (plain || force_brute || force_slab || cta_grid || s.K > LIST_K_MAX) {
+        m.sel = 1;  // radix select on the FP64 distances to all points
+      } else {
+        m.mode = pick_mode(true, s);
+        if (m.mode != 3) {  // a warp's list over all points
+          m.mode = 0;
+          m.sel = 2;
+        }
+      }
       m.slab = m.mode >= 1 ? 1 : 0;
       if (m.slab) {
         m.sort_seg = seg_for(s.task, s.sp.cols[0], s.b, s.e);
@@ -866,8 +881,10 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
                        : tp.kind == KIND_COUNT_ONLY ? d + 1
                        : (tp.kind == EGB_SEMI || tp.kind == EGB_CSEMI) ? tp.ncol + 1
                        : std::max(tp.ncol, d + 1);
-        const double c = m.is_knn ? GRID_STRIPS_KNN_C : GRID_STRIPS_COUNT_C;
-        want = std::min<int64_t>(GRID_STRIPS_MAX, std::llround(c * std::pow((double)len, 1.0 / dj)));
+        const bool list = m.is_knn && m.s.K > 8;  // strips as high as its wider balls
+        const double c = list ? GRID_STRIPS_LIST_C : m.is_knn ? GRID_STRIPS_KNN_C : GRID_STRIPS_COUNT_C;
+        const double pts = list ? (double)len / m.s.K : (double)len;
+        want = std::min<int64_t>(GRID_STRIPS_MAX, std::llround(c * std::pow(pts, 1.0 / dj)));
       }
       J.nstrips = (int32_t)std::max<int64_t>(1, std::min<int64_t>(want, len / GRID_MIN_STRIP));
       if (m.sort_seg_c >= 0) {
@@ -1091,7 +1108,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     std::vector<WorkItem> items;  // tile groups: items built here
     std::vector<ItemRun> runs;    // grid groups: items built on the device
     std::vector<int32_t> cum;
-    int64_t nitems = 0, ncells = 0;
+    int64_t nitems = 0, ncells = 0, queries = 0;
     size_t tab_items = 0, tab_runs = 0, tab_cum = 0, off_items = 0;
     int64_t defer_cap = 0;   // slab groups: every query may be deferred once
     size_t off_defer = 0;
@@ -1106,8 +1123,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     const MJob& m = mjobs[j];
     const int d = m.s.sp.d;
     const int dclass = (d >= 2 && d <= 4) ? d : 0;
-    int kclass = 0;
-    if (m.is_knn && !m.sel) kclass = m.s.K <= 4 ? 4 : m.s.K <= 8 ? 8 : m.s.K <= 16 ? 16 : 32;
+    const int kclass = kclass_of(m);
     const auto key = std::make_tuple((int)m.is_knn, m.sel, kclass, dclass, m.slab, m.mode);
     auto it = gidx.find(key);
     int g;
@@ -1128,9 +1144,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     const MJob& m = mjobs[j];
     const int d = m.s.sp.d;
     const int dclass = (d >= 2 && d <= 4) ? d : 0;
-    int kclass = 0;
-    if (m.is_knn && !m.sel) kclass = m.s.K <= 4 ? 4 : m.s.K <= 8 ? 8 : m.s.K <= 16 ? 16 : 32;
+    const int kclass = kclass_of(m);
     Group& G = groups[(size_t)gidx[std::make_tuple((int)m.is_knn, m.sel, kclass, dclass, m.slab, m.mode)]];
+    G.queries += jobs[j].len;
     if (G.mode >= 2) {
       // items never straddle a strip (cell); the device writes them
       // (launch_emit_items) from these per-cell offsets
@@ -1160,7 +1176,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       continue;
     }
     int qb;
-    if (G.sel) qb = SELECT_WARPS;
+    if (G.sel) qb = G.sel == 1 ? SELECT_WARPS : LIST_QB;
     else if (G.is_knn) qb = knn_shape(G.kclass, G.dclass, plain, G.slab, G.dmax).queries();
     else qb = count_shape(G.dclass, plain, G.slab, G.dmax).queries();
     for (int64_t q0 = 0; q0 < jobs[j].len; q0 += qb) G.items.push_back({(int32_t)j, (int32_t)q0, 0, 0});
@@ -1177,8 +1193,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     const MJob& m = mjobs[j];
     const int d = m.s.sp.d;
     const int dclass = (d >= 2 && d <= 4) ? d : 0;
-    int kclass = 0;
-    if (m.is_knn && !m.sel) kclass = m.s.K <= 4 ? 4 : m.s.K <= 8 ? 8 : m.s.K <= 16 ? 16 : 32;
+    const int kclass = kclass_of(m);
     job_group[j] = gidx[std::make_tuple((int)m.is_knn, m.sel, kclass, dclass, m.slab, m.mode)];
   }
 
@@ -1648,6 +1663,17 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   // kNN groups after the first run on the side stream: each persistent
   // launch fills the GPU, so the next one starts in the previous one's tail
   // (a timed batch keeps them in line)
+  // A warp per query instead of a lane's walk (egb_wlist.cu): K beyond a
+  // lane's registers; four and more columns, where the 32 queries of a walk
+  // share few candidates (20,000 points, d = 4, K = 4: 115 us against 309;
+  // 200,000: 1.04 ms against 1.66); three columns while the launch has too
+  // few queries to fill the GPU with lanes (20,000, K = 4: 61 us against 115;
+  // the sides meet near 50,000 queries for K <= 4 and 100,000 for K <= 8).
+  auto list_form = [&](const Group& G) {
+    if (plain) return false;
+    if (G.kclass > 8 || (G.dclass != 2 && G.dclass != 3)) return true;
+    return G.dclass == 3 && G.queries <= (G.kclass <= 4 ? 49152 : 98304);
+  };
   int knn_groups = 0;
   for (const Group& G : groups) knn_groups += (G.is_knn && G.nitems > 0) ? 1 : 0;
   const bool fork_knn = !timing && knn_groups > 1;
@@ -1660,9 +1686,13 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     Group& G = groups[g];
     if (!G.is_knn || G.nitems == 0) continue;
     cudaStream_t gs = (fork_knn && knn_seen++ > 0) ? ctx->side_stream : st;
-    if (G.sel)
+    if (G.sel == 1)
       launch_knn_select((const JobDev*)dtab(tab_jobs), items_of(G),
                         (int)G.nitems, err_d, ctx->num_sms, gs);
+    else if (G.sel == 2 || (G.mode == 3 && list_form(G)))
+      launch_knn_list((const JobDev*)dtab(tab_jobs), items_of(G), (int)G.nitems,
+                      G.sel ? LIST_QB : WG_QB, G.kclass, G.dclass, G.mode == 3, counters + 2 * g,
+                      ctx->num_sms, gs);
     else if (G.mode == 3)
       launch_knn_wgrid((const JobDev*)dtab(tab_jobs), items_of(G),
                        (int)G.nitems, G.kclass, G.dclass, plain, G.dmax, counters + 2 * g,

@@ -311,7 +311,8 @@ __host__ __device__ __forceinline__ int32_t cell_start(int32_t s0, int32_t L, in
   return s0 + strip_start(c2, L, nsub);
 }
 constexpr int NEST_CELL_3D = 384;     // target points per nested-grid cell, kNN jobs of d = 3
-constexpr int NEST_CELL_4D = 256;     // the same for d >= 4 (measured best for each)
+constexpr int NEST_CELL_4D = 512;     // the same for d >= 4 (measured best for each:
+                                      // 200,000 4-D points 1.83 ms on 256, 1.04-1.46 on 512)
 constexpr int NEST_CELL_COUNT = 768;  // the same for count jobs, which also take at least
 constexpr double NEST_SIDE_C = 1.07;  // NEST_SIDE_C * len^(1/dj) cells per side (dj: see strips)
 constexpr int GRID_QB = 128;     // queries per grid work item
@@ -323,6 +324,10 @@ constexpr int GRID_MIN_STRIP = 64;
 // wide (balls shrink as len^(-1/dj)).  c measured on GB300: 500 kNN strips
 // and 128 count strips (3-D joint kNN) at 1e6 points.
 constexpr double GRID_STRIPS_KNN_C = 0.5;
+// K > 8 (egb_wlist.cu): c * (len / K)^(1/d) strips, as high as the wider balls
+// (20,000 to 1,000,000 2-D points, K = 13 to 100: 1.4 best or within 4 % of it
+// among 1 to 4).
+constexpr double GRID_STRIPS_LIST_C = 1.4;
 constexpr double GRID_STRIPS_COUNT_C = 1.28;
 constexpr int GRID_STRIPS_MAX = 1024;
 
@@ -571,7 +576,7 @@ void launch_count_grid(const JobDev* jobs_d, const WorkItem* items_d, int nitems
 constexpr int WG_QB = 32;
 void launch_knn_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int kclass,
                       int dclass, int plain, int dmax, int* counter, int num_sms, cudaStream_t st);
-// egb_wwalk.cu: FP32-path kNN of warp-grid jobs (K <= 8) by per-lane walks
+// egb_wwalk.cu: FP32-path kNN of warp-grid jobs (d = 2, 3; K <= 8) by per-lane walks
 void launch_knn_walk(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int kclass,
                      int dclass, int* counter, int num_sms, cudaStream_t st);
 // egb_wcount.cu: exact key-range ball counts of d = 2 / nested d = 3, 4
@@ -683,6 +688,12 @@ void launch_pairwise_matrix(const double* vals_d, const int32_t* pairs_d, int nt
 void launch_normalize(const double* in_d, int64_t n, double* out_d, cudaStream_t st);
 
 // egb_select.cu: any K (one warp per query, radix select on FP64 bits)
+// egb_wlist.cu: kNN of 9 <= K <= LIST_K_MAX over grid copies, and of
+// EGB_KREG_MAX < K over all points of a job without one
+constexpr int LIST_K_MAX = 128;
+constexpr int LIST_QB = 32;   // queries per item of a job without a grid copy
+void launch_knn_list(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int qb, int kclass,
+                     int dclass, bool grid, int* counter, int num_sms, cudaStream_t st);
 constexpr int SELECT_WARPS = 8;
 void launch_knn_select(const JobDev* jobs_d, const WorkItem* items_d, int nitems, uint32_t* err,
                        int num_sms, cudaStream_t st);

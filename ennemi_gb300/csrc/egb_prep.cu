@@ -41,6 +41,22 @@ int grid_x_for(int64_t n) {
 }
 int grid_y_for(int n) { return n > 65535 ? 65535 : (n < 1 ? 1 : n); }
 
+// n clusters of CL blocks each
+template <int CL, typename... P, typename... A>
+void launch_clusters(void (*kern)(P...), int n, int threads, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = CL;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(n * CL));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // Four loads in flight per thread before its stores: columns read in place
 // from host memory cross the CPU-GPU link, where throughput follows the
 // requests outstanding.
@@ -140,39 +156,50 @@ __device__ double pw_leaf8(const double* a, const int32_t* inv, int len, int r, 
   return s;
 }
 
-// The block's pairwise sum of x[0, n) (sq: of (x - m)^2): leaves in parallel,
-// then one height at a time; node sums in ns (global, read back through L2).
-// LANES: a leaf on one lane (fewest FP64 operations: the form for more
-// columns than the GPU holds blocks) or on eight (the shortest chain).
-template <int LANES>
+// The pairwise sum of x[0, n) (sq: of (x - m)^2) by a cluster of CL blocks:
+// leaves in parallel -- on one lane each (CL = 1: fewest FP64 operations) or
+// on eight (CL > 1: the shortest chain) -- then the first block one height at
+// a time, in shared memory where the tree fits.  Node sums pass through ns
+// (global, read back through L2); the first block returns the sum.
+constexpr int PW_SMEM_NODES = 4096;  // trees of n up to 180,000 and more
+template <int CL>
 __device__ double pw_sum(const double* x, const int32_t* inv, const PwTree& tr,
                          const int2* __restrict__ nodes, const int32_t* __restrict__ levels,
-                         double* ns, bool sq, double m) {
-  if (LANES == 1) {
+                         double* ns, double* sm, bool sq, double m) {
+  if constexpr (CL == 1) {
     for (int i = threadIdx.x; i < tr.nleaf; i += blockDim.x) {
       const int2 L = nodes[tr.node0 + i];
       ns[i] = inv ? pw_leaf(x, inv + L.x, L.y, sq, m) : pw_leaf(x + L.x, nullptr, L.y, sq, m);
     }
+    __syncthreads();
   } else {
-    const int r = threadIdx.x & 7, ngroup = blockDim.x >> 3;
-    for (int i0 = 0; i0 < tr.nleaf; i0 += ngroup) {
+    auto cl = cooperative_groups::this_cluster();
+    const int rank = (int)cl.block_rank(), r = threadIdx.x & 7, per = blockDim.x >> 3;
+    for (int i0 = rank * per; i0 < tr.nleaf; i0 += CL * per) {
       const int i = i0 + (threadIdx.x >> 3);
       const int2 L = i < tr.nleaf ? nodes[tr.node0 + i] : make_int2(0, 0);
       const double s = inv ? pw_leaf8(x, inv + L.x, L.y, r, sq, m)
                            : pw_leaf8(x + L.x, nullptr, L.y, r, sq, m);
       if (r == 0 && i < tr.nleaf) ns[i] = s;
     }
+    cl.sync();  // orders the leaf sums for the cluster
+    if (rank != 0) return 0.0;
   }
-  __syncthreads();
+  const bool fits = CL > 1 && tr.nnode <= PW_SMEM_NODES;
+  if (fits) {
+    for (int i = threadIdx.x; i < tr.nleaf; i += blockDim.x) sm[i] = __ldcg(ns + i);
+    __syncthreads();
+  }
   for (int h = 0; h < tr.nlvl; ++h) {
     const int a = levels[tr.lvl0 + h], b = levels[tr.lvl0 + h + 1];
     for (int i = a + threadIdx.x; i < b; i += blockDim.x) {
       const int2 c = nodes[tr.node0 + i];
-      ns[i] = __dadd_rn(__ldcg(ns + c.x), __ldcg(ns + c.y));
+      if (fits) sm[i] = __dadd_rn(sm[c.x], sm[c.y]);
+      else ns[i] = __dadd_rn(__ldcg(ns + c.x), __ldcg(ns + c.y));
     }
     __syncthreads();
   }
-  return __ldcg(ns + tr.nnode - 1);
+  return fits ? sm[tr.nnode - 1] : __ldcg(ns + tr.nnode - 1);
 }
 
 // s + x_0 + x_1 + ... in order, each addition rounded, for the 32 values of
@@ -286,34 +313,43 @@ __device__ double row_sum(const double* x, const int32_t* inv, int n, double* sm
   return s;
 }
 
-// LANES: pw_sum's form.  8 for a handful of columns (two of 10,000 samples:
-// 24 -> 10 us); 1 for more: 785 columns of 180,000 are FP64-bound (1.42 ms
-// against 1.65 on eight lanes), and a call of 44 columns of 1,000 measured
-// 1.40 ms with eight, 1.31 with one.
-constexpr int STATS_FEW = 16;
-template <int LANES>
+// One column per cluster of CL blocks.  A column's sums are FP64-bound on one
+// SM (two operations a clock), so a handful of columns takes CL = 8 and more
+// columns CL = 1 (785 columns of 180,000: 1.42 ms).
+constexpr int STATS_FEW = 16, STATS_CLUSTER = 8;
+template <int CL>
 __global__ void __launch_bounds__(PREP_THREADS)
 rescale_stats_kernel(const TaskDev* __restrict__ tasks, const RescaleStat* __restrict__ stats,
                      const PwTree* __restrict__ trees, const int2* __restrict__ nodes,
                      const int32_t* __restrict__ levels, double* __restrict__ scratch,
                      double2* __restrict__ ms) {
-  __shared__ double rows[2 * ROW_STAGE];
-  const RescaleStat rs = stats[blockIdx.x];
+  __shared__ double sm[CL > 1 ? PW_SMEM_NODES : 2 * ROW_STAGE];
+  __shared__ double mean_s;
+  const int stat = blockIdx.x / CL;
+  const RescaleStat rs = stats[stat];
   const TaskDev t = tasks[rs.task];
   const double* x = t.x64 + (int64_t)rs.col * t.ld;
   const double n = (double)t.n;
   if (rs.group > 1) {  // axis-0 reduction of an (n, group) array: in row order
-    const double mean = __ddiv_rn(row_sum(x, rs.inv, t.n, rows, false, 0.0), n);
-    const double q = row_sum(x, rs.inv, t.n, rows, true, mean);
-    if (threadIdx.x == 0) ms[blockIdx.x] = make_double2(mean, __dsqrt_rn(__ddiv_rn(q, n)));
+    if (blockIdx.x % CL) return;
+    const double mean = __ddiv_rn(row_sum(x, rs.inv, t.n, sm, false, 0.0), n);
+    const double q = row_sum(x, rs.inv, t.n, sm, true, mean);
+    if (threadIdx.x == 0) ms[stat] = make_double2(mean, __dsqrt_rn(__ddiv_rn(q, n)));
     return;
   }
   const PwTree tr = trees[rs.tree];
   double* ns = scratch + rs.scratch;
-  const double mean = __ddiv_rn(pw_sum<LANES>(x, rs.inv, tr, nodes, levels, ns, false, 0.0), n);
-  __syncthreads();  // every thread has read the root before the slots are reused
-  const double sd = __dsqrt_rn(__ddiv_rn(pw_sum<LANES>(x, rs.inv, tr, nodes, levels, ns, true, mean), n));
-  if (threadIdx.x == 0) ms[blockIdx.x] = make_double2(mean, sd);
+  double mean = __ddiv_rn(pw_sum<CL>(x, rs.inv, tr, nodes, levels, ns, sm, false, 0.0), n);
+  if constexpr (CL > 1) {  // the first block's mean for all
+    auto cl = cooperative_groups::this_cluster();
+    if (cl.block_rank() == 0 && threadIdx.x == 0) mean_s = mean;
+    cl.sync();
+    mean = *cl.map_shared_rank(&mean_s, 0);
+  } else {
+    __syncthreads();  // every thread has read the root before the slots are reused
+  }
+  const double q = pw_sum<CL>(x, rs.inv, tr, nodes, levels, ns, sm, true, mean);
+  if (threadIdx.x == 0 && blockIdx.x % CL == 0) ms[stat] = make_double2(mean, __dsqrt_rn(__ddiv_rn(q, n)));
 }
 
 // RN(a / b) without a division per element.  q = RN(a * rb) (rb = RN(1/b))
@@ -730,9 +766,12 @@ void launch_rescale(const TaskDev* tasks_d, const RescaleStat* stats_d, int nsta
                     const int2* nodes_d, const int32_t* levels_d, double* scratch, double2* ms,
                     const double* noise, uint32_t* zero_flags, int64_t max_n, cudaStream_t st) {
   if (ncols <= 0 || nstats <= 0) return;
-  auto stats_kernel = nstats <= STATS_FEW ? rescale_stats_kernel<8> : rescale_stats_kernel<1>;
-  stats_kernel<<<nstats, PREP_THREADS, 0, st>>>(tasks_d, stats_d, trees_d, nodes_d, levels_d, scratch,
-                                                ms);
+  if (nstats <= STATS_FEW)
+    launch_clusters<STATS_CLUSTER>(rescale_stats_kernel<STATS_CLUSTER>, nstats, PREP_THREADS, st, tasks_d,
+                                   stats_d, trees_d, nodes_d, levels_d, scratch, ms);
+  else
+    rescale_stats_kernel<1><<<nstats, PREP_THREADS, 0, st>>>(tasks_d, stats_d, trees_d, nodes_d, levels_d,
+                                                             scratch, ms);
   count_launch();
   // 32 samples a thread where the columns fill the GPU (one division per
   // block), down to 4 where they do not: two columns of 10,000 samples took
@@ -848,18 +887,8 @@ void launch_combine(const TaskDev* tasks_d, const CombineJob* jobs_d, const int3
                                                            psi_len, partial, zero_flags, err);
   } else {
     constexpr int CL = 8;
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = CL;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)(nchunks * CL));
-    cfg.blockDim = dim3(COMBINE_THREADS);
-    cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, combine_kernel<CL>, tasks_d, jobs_d, chunk_job_d, psi_tab, psi_len,
-                       partial, zero_flags, err);
+    launch_clusters<CL>(combine_kernel<CL>, nchunks, COMBINE_THREADS, st, tasks_d, jobs_d, chunk_job_d,
+                        psi_tab, psi_len, partial, zero_flags, err);
   }
   count_launch();
 }

@@ -1,4 +1,5 @@
-// egb_wwalk.cu -- kNN distances of warp-grid jobs by per-lane walks.
+// egb_wwalk.cu -- kNN distances of warp-grid jobs of two and three columns
+// and K <= 8 by per-lane walks (more columns, larger K: egb_wlist.cu).
 //
 // (k+1)-th smallest max-norm distance per point, self included, over the
 // job's grid copy (strips by column 1; nested cells by column 2 for d >= 3;
@@ -102,7 +103,6 @@ template <int D, int KMAX, bool NEST>
 __global__ void __launch_bounds__(WW_WARPS * 32, walk_min_blocks(D, KMAX))
 wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items, int nitems,
              int* __restrict__ counter) {
-  constexpr int DQ = D ? D : EGB_DMAX;
   constexpr float FINF = __builtin_huge_valf();
   const int lane = threadIdx.x & 31;
 
@@ -113,7 +113,6 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     if (it >= nitems) break;
     const WorkItem wi = items[it];
     const JobDev* __restrict__ J = jobs + wi.job;
-    const int d = D ? D : J->sp.d;
     const int64_t lds = J->lds;
     const double* __restrict__ c64 = J->c64g;
     const float* __restrict__ g = J->c32g;
@@ -138,11 +137,10 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     // which gives M = max_c |q_c - c| and the planning bounds of columns 1
     // and 2 without FP64 instructions (jobs with clamped values run the FP64
     // pass, whose bounds are infinite)
-    float qv[DQ];
+    float qv[D];
     float am = 0.0f;
 #pragma unroll
-    for (int c = 0; c < DQ; ++c) {
-      if (D == 0 && c >= d) break;
+    for (int c = 0; c < D; ++c) {
       qv[c] = exists ? g[(int64_t)c * lds + qp] : 0.0f;
       am = fmaxf(am, fabsf(qv[c]));
     }
@@ -177,8 +175,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     auto exact_dist = [&](int j) -> uint64_t {
       uint64_t mm = 0;
 #pragma unroll
-      for (int c = 0; c < DQ; ++c) {
-        if (D == 0 && c >= d) break;
+      for (int c = 0; c < D; ++c) {
         const int64_t off = (int64_t)c * lds;
         const uint64_t v = absdiff_bits(c64[off + j], c64[off + qp]);
         mm = v > mm ? v : mm;
@@ -236,8 +233,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
         const int j = go_l ? L : R;
         float dd = dx;
 #pragma unroll
-        for (int c = 1; c < DQ; ++c) {
-          if (D == 0 && c >= d) break;
+        for (int c = 1; c < D; ++c) {
           dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - qv[c]));
         }
         visit(j, dd);
@@ -346,10 +342,9 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
       while (hm) {
         const int ol = __ffs(hm) - 1;
         hm &= hm - 1u;
-        float oq[DQ];
+        float oq[D];
 #pragma unroll
-        for (int c = 0; c < DQ; ++c) {
-          if (D == 0 && c >= d) break;
+        for (int c = 0; c < D; ++c) {
           oq[c] = __shfl_sync(0xffffffffu, qv[c], ol);
         }
         const float omq = __shfl_sync(0xffffffffu, mq, ol);
@@ -377,8 +372,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
             if (j < wh) {
               float dd = 0.0f;
 #pragma unroll
-              for (int c = 0; c < DQ; ++c) {
-                if (D == 0 && c >= d) break;
+              for (int c = 0; c < D; ++c) {
                 dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - oq[c]));
               }
               ++cvis;
@@ -545,12 +539,8 @@ void launch_t(const JobDev* jobs, const WorkItem* items, int nitems, int* counte
 template <int KMAX>
 void launch_k(int dclass, const JobDev* jobs, const WorkItem* items, int nitems, int* counter,
               int num_sms, cudaStream_t st) {
-  switch (dclass) {
-    case 2: launch_t<2, KMAX, false>(jobs, items, nitems, counter, num_sms, st); break;
-    case 3: launch_t<3, KMAX, true>(jobs, items, nitems, counter, num_sms, st); break;
-    case 4: launch_t<4, KMAX, true>(jobs, items, nitems, counter, num_sms, st); break;
-    default: launch_t<0, KMAX, true>(jobs, items, nitems, counter, num_sms, st); break;
-  }
+  if (dclass == 2) launch_t<2, KMAX, false>(jobs, items, nitems, counter, num_sms, st);
+  else launch_t<3, KMAX, true>(jobs, items, nitems, counter, num_sms, st);
 }
 
 }  // namespace

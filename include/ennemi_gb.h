@@ -254,7 +254,8 @@ int egb_last_stats(const egb_ctx* ctx, int64_t* out, int32_t max);
  *   EGB_MODE_SLAB       points sorted by column 0, tiles from a window
  *   EGB_MODE_GRID       equal-count strips, 128-query CTA work items
  *   EGB_MODE_WARP_GRID  equal-count strips, 32-query warp work items
- *                       (kNN only for K = k + 1 <= 8; otherwise GRID)
+ *                       (kNN: K = k + 1 <= 128, the all-FP64
+ *                       comparator <= 8; otherwise GRID)
  *   EGB_MODE_RANK       ball counts of d = 2 only: rank-space rectangle
  *                       counts on a wavelet matrix (otherwise WARP_GRID;
  *                       the all-FP64 comparator keeps WARP_GRID too)

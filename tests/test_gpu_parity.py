@@ -195,6 +195,28 @@ def test_primitives_against_oracle(oracle):
         assert np.array_equal(cnt, oracle.ball_count(pts, r)), d
 
 
+@pytest.mark.parametrize("data", ["normal", "rounded", "huge"])
+@pytest.mark.parametrize("d", [2, 3, 4, 5])
+def test_warp_list_knn(oracle, d, data):
+    """K at the edges of the list sizes and of the compiled classes, at the
+    smallest grid size, one point below it and odd sizes above; near ties that
+    overflow the list, and values that rule out the FP32 screen."""
+    rng = np.random.default_rng(10 * d)
+    sizes = [4095, 4096, 9001] if data == "normal" else [4097]
+    for n in sizes:
+        pts = rng.normal(size=(n, d)) * np.linspace(1.0, 3.0, d)
+        if data == "rounded":
+            pts = np.round(pts, 0 if d > 3 else 1)
+        elif data == "huge":
+            pts[:, 0] *= 1e300
+        for k in [3, 7, 8, 15, 16, 31, 32, 63, 64, 127, 128]:
+            eps = N.knn_eps(pts, k)
+            assert np.array_equal(eps, oracle.knn_eps(pts, k)), (n, k)
+    few = rng.normal(size=(40, d))
+    for k in [32, 38, 39, 40, 127]:
+        assert np.array_equal(N.knn_eps(few, k), oracle.knn_eps(few, k)), k
+
+
 def test_device_input_matches_host_input():
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(7)

@@ -96,6 +96,20 @@ def test_row_sums_on_rounding_boundaries(n, data):
         assert np.array_equal(N.fetch(0, 18 + c, n).view(np.uint64), want[:, c].view(np.uint64)), c
 
 
+@pytest.mark.parametrize("n,tasks", [(700, 1), (4097, 8), (4097, 9), (300_001, 1)])
+def test_statistics_of_few_and_many_columns(n, tasks):
+    """One column per cluster of blocks up to 16 distinct columns, one per
+    block beyond; trees within and beyond shared memory."""
+    rng = np.random.default_rng(n)
+    cols = [rng.normal(size=n) * (i + 1) - i for i in range(2 * tasks)]
+    batch = [N.Task(N.MI, 3, [cols[2 * i]], [cols[2 * i + 1]], n=n) for i in range(tasks)]
+    N.run_tasks(batch, flags=N.RESCALE | N.KEEP_INTERNALS, noise=_noise)
+    for i in range(tasks):
+        for c in range(2):
+            want = _reference_rescale(cols[2 * i + c], c * n, n)
+            assert np.array_equal(N.fetch(i, 16 + c, n).view(np.uint64), want.view(np.uint64)), (i, c)
+
+
 def test_semidiscrete_columns_with_index():
     """Labels and an index together: the class order is applied on top of the
     index; the continuous column is rescaled from noise position 0."""
