@@ -888,12 +888,16 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       }
       J.nstrips = (int32_t)std::max<int64_t>(1, std::min<int64_t>(want, len / GRID_MIN_STRIP));
       if (m.sort_seg_c >= 0) {
-        // nested: about NEST_CELL_* points per cell, as many strips as cells
-        // per strip, every cell at least GRID_MIN_STRIP / 2 points
-        const int target = m.is_knn ? (d == 3 ? NEST_CELL_3D : NEST_CELL_4D) : NEST_CELL_COUNT;
-        int64_t side = (int64_t)std::lround(std::sqrt((double)len / target));
+        // nested: as many strips as cells per strip, every cell at least
+        // GRID_MIN_STRIP / 2 points.  Counts (egb_lcount.cu) read the items as
+        // leaves: as many cells per side as items per cell, so that a leaf is
+        // as deep in each of the first three columns.  kNN jobs and the FP64
+        // comparator read windows of larger cells: about NEST_CELL_* points.
         const TaskPlan& tq = P[(size_t)m.s.task];
-        if (!m.is_knn && tq.kind != EGB_SEMI && tq.kind != EGB_CSEMI) {
+        const int target = !m.is_knn ? NEST_CELL_COUNT : d == 3 ? NEST_CELL_3D
+                           : plain ? NEST_CELL_4D_FP64 : NEST_CELL_4D;
+        int64_t side = (int64_t)std::lround(std::sqrt((double)len / target));
+        if (plain && !m.is_knn && tq.kind != EGB_SEMI && tq.kind != EGB_CSEMI) {
           // count jobs of small spaces with wide balls take finer cells: at
           // least NEST_SIDE_C * len^(1/dj) per side, dj as for the strips
           // (the semidiscrete kinds, whose radii come from per-class kNN,
@@ -901,6 +905,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
           const int dj = tq.kind == KIND_COUNT_ONLY ? d + 1 : std::max(tq.ncol, d + 1);
           side = std::max<int64_t>(side, std::llround(NEST_SIDE_C * std::pow((double)len, 1.0 / dj)));
         }
+        if (!plain && !m.is_knn) side = std::llround(std::cbrt((double)len / WG_QB));
         side = std::max<int64_t>(1, std::min<int64_t>(256, side));
         while (side > 1 && len / (side * side) < GRID_MIN_STRIP / 2) --side;
         J.nstrips = (int32_t)side;
@@ -1112,6 +1117,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     size_t tab_items = 0, tab_runs = 0, tab_cum = 0, off_items = 0;
     int64_t defer_cap = 0;   // slab groups: every query may be deferred once
     size_t off_defer = 0;
+    bool boxed = false;      // nested grids whose items' boxes are read
+    size_t off_box = 0;
   };
   std::vector<Group> groups;
   std::map<std::tuple<int, int, int, int, int, int>, int> gidx;
@@ -1139,6 +1146,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     }
     groups[(size_t)g].dmax = std::max(groups[(size_t)g].dmax, d);
   }
+  std::vector<int32_t> job_cum0(mjobs.size(), 0);  // grid jobs: their first entry of G.cum
   for (size_t oi = 0; oi < order.size(); ++oi) {
     const size_t j = order[oi];
     const MJob& m = mjobs[j];
@@ -1158,6 +1166,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       r.job = (int32_t)j;
       r.ncell = S * std::max(S2, 1);
       r.cum0 = (int32_t)G.cum.size();
+      job_cum0[j] = r.cum0;
       r.qb = qb;
       r.cell0 = G.ncells;
       for (int sidx = 0; sidx < S; ++sidx) {
@@ -1183,6 +1192,12 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     G.nitems = (int64_t)G.items.size();
     if (G.slab) G.defer_cap += jobs[j].len;
   }
+  // ball counts of three and more columns read the boxes of their items
+  for (Group& G : groups)
+    if (!plain && G.mode == 3 && G.dclass != 2 && !G.is_knn) {
+      G.boxed = true;
+      G.off_box = dl.take(sizeof(float) * 2 * (size_t)G.dmax * (size_t)std::max<int64_t>(G.nitems, 1));
+    }
   for (Group& G : groups)
     if (!G.runs.empty()) G.off_items = dl.take(sizeof(WorkItem) * (size_t)std::max<int64_t>(G.nitems, 1));
   for (Group& G : groups)
@@ -1466,6 +1481,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
             cs0[s1 * J.nsub + c2] = cell_start(st0[s1], st0[s1 + 1] - st0[s1], c2, J.nsub);
         cs0[J.nstrips * J.nsub] = J.len;
         J.cstart = (const int32_t*)(A + off_tab + tab_cstart[j]);
+        const Group& GJ = groups[(size_t)job_group[j]];
+        J.leaf0 = (const int32_t*)(A + off_tab + GJ.tab_cum) + job_cum0[j];
       }
     }
     J.jflags = (uint32_t*)(A + off_zr + zr_jflags) + j;
@@ -1654,6 +1671,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
                             (int)grid_jobs.size(), vals, (const SortSeg*)dtab(tab_segs),
                             max_gkey > 256 ? gva : gvb, (const SortSeg*)dtab(tab_gsegs),
                             max_lds, st);
+    for (const Group& G : groups)
+      if (G.boxed)
+        launch_leaf_boxes(jobs_d, items_of(G), (int)G.nitems, (float*)(A + G.off_box), st);
   }
   if (timing) EGB_CUDA(cudaEventRecord(ctx->ev[3], st));
 
@@ -1750,10 +1770,12 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       if (!plain && count_keys_supported(G.dclass))
         launch_count_keys((const JobDev*)dtab(tab_jobs), items_of(G),
                           (int)G.nitems, G.dclass, counters + 2 * g, ctx->num_sms, st);
+      else if (G.boxed)
+        launch_count_leaf((const JobDev*)dtab(tab_jobs), items_of(G), (int)G.nitems,
+                          (const float*)(A + G.off_box), G.dclass, counters + 2 * g, ctx->num_sms, st);
       else
         launch_count_wgrid((const JobDev*)dtab(tab_jobs), items_of(G),
-                           (int)G.nitems, G.dclass, plain, G.dmax, counters + 2 * g,
-                           ctx->num_sms, st);
+                           (int)G.nitems, G.dclass, G.dmax, counters + 2 * g, ctx->num_sms, st);
       continue;
     }
     if (G.mode == 2) {

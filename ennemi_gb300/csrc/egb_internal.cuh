@@ -285,6 +285,7 @@ struct JobDev {
   int32_t nsub;
   int32_t sort_seg_c;     // nested: sort segment of column 2
   const int32_t* cstart;  // nstrips * nsub + 1 cell starts (cell_start table)
+  const int32_t* leaf0;   // the same for the first work item of each cell
   double* czlo;           // smallest column-2 value of each cell
   double* czhi;           // largest column-2 value of each cell
   // the strip and cell bounds centred and rounded outward to FP32
@@ -310,11 +311,13 @@ __host__ __device__ __forceinline__ int32_t cell_start(int32_t s0, int32_t L, in
                                                        int32_t nsub) {
   return s0 + strip_start(c2, L, nsub);
 }
-constexpr int NEST_CELL_3D = 384;     // target points per nested-grid cell, kNN jobs of d = 3
-constexpr int NEST_CELL_4D = 512;     // the same for d >= 4 (measured best for each:
-                                      // 200,000 4-D points 1.83 ms on 256, 1.04-1.46 on 512)
-constexpr int NEST_CELL_COUNT = 768;  // the same for count jobs, which also take at least
-constexpr double NEST_SIDE_C = 1.07;  // NEST_SIDE_C * len^(1/dj) cells per side (dj: see strips)
+constexpr int NEST_CELL_3D = 384;     // points per nested-grid cell, kNN jobs of d = 3
+constexpr int NEST_CELL_4D = 512;     // d >= 4 (200,000 4-D points, K = 4: 1.83 ms on 256, 1.46 on 512)
+// the FP64 comparator's kNN jobs of d >= 4, and its count jobs, which take at
+// least NEST_SIDE_C * len^(1/dj) cells per side (dj: see strips)
+constexpr int NEST_CELL_4D_FP64 = 256;
+constexpr int NEST_CELL_COUNT = 768;
+constexpr double NEST_SIDE_C = 1.07;
 constexpr int GRID_QB = 128;     // queries per grid work item
 constexpr int GRID_TILE = 128;   // candidates per grid tile
 constexpr int GRID_MIN_STRIP = 64;
@@ -579,13 +582,13 @@ void launch_knn_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems,
 // egb_wwalk.cu: FP32-path kNN of warp-grid jobs (d = 2, 3; K <= 8) by per-lane walks
 void launch_knn_walk(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int kclass,
                      int dclass, int* counter, int num_sms, cudaStream_t st);
-// egb_wcount.cu: exact key-range ball counts of d = 2 / nested d = 3, 4
-// warp-grid jobs (FP32 path; the FP64 comparator keeps launch_count_wgrid)
+// egb_wcount.cu: exact key-range ball counts of d = 2 warp-grid jobs (FP32
+// path; the FP64 comparator keeps launch_count_wgrid)
 bool count_keys_supported(int dclass);
 void launch_count_keys(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass,
                        int* counter, int num_sms, cudaStream_t st);
-void launch_count_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass,
-                        int plain, int dmax, int* counter, int num_sms, cudaStream_t st);
+void launch_count_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass, int dmax,
+                        int* counter, int num_sms, cudaStream_t st);
 
 // egb_wavelet.cu: exact 2-D ball counts in rank space.  A count space of
 // columns (a, b) over len points is the permutation S[i] = position in the
@@ -694,6 +697,12 @@ constexpr int LIST_K_MAX = 128;
 constexpr int LIST_QB = 32;   // queries per item of a job without a grid copy
 void launch_knn_list(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int qb, int kclass,
                      int dclass, bool grid, int* counter, int num_sms, cudaStream_t st);
+// egb_lcount.cu: boxes of the items of nested-grid jobs ([2 d][nitems] floats)
+// and FP32-path ball counts of d >= 3 on them
+void launch_leaf_boxes(const JobDev* jobs_d, const WorkItem* items_d, int nitems, float* boxes,
+                       cudaStream_t st);
+void launch_count_leaf(const JobDev* jobs_d, const WorkItem* items_d, int nitems, const float* boxes,
+                       int dclass, int* counter, int num_sms, cudaStream_t st);
 constexpr int SELECT_WARPS = 8;
 void launch_knn_select(const JobDev* jobs_d, const WorkItem* items_d, int nitems, uint32_t* err,
                        int num_sms, cudaStream_t st);

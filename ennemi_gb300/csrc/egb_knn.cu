@@ -47,9 +47,7 @@ void launch_count_grid_f32(int, const JobDev*, const WorkItem*, int, int*, uint3
 void launch_count_grid_f64(int, const JobDev*, const WorkItem*, int, int*, uint32_t*, int,
                            DeferEntry*, int*, int, cudaStream_t);
 
-void launch_knn_wgrid_f32(int, int, const JobDev*, const WorkItem*, int, int*, int, int, cudaStream_t);
 void launch_knn_wgrid_f64(int, int, const JobDev*, const WorkItem*, int, int*, int, int, cudaStream_t);
-void launch_count_wgrid_f32(int, const JobDev*, const WorkItem*, int, int*, int, int, cudaStream_t);
 void launch_count_wgrid_f64(int, const JobDev*, const WorkItem*, int, int*, int, int, cudaStream_t);
 
 void launch_knn_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int kclass,
@@ -61,11 +59,12 @@ void launch_knn_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems,
   else launch_knn_walk(jobs_d, items_d, nitems, kclass, dclass, counter, num_sms, st);
 }
 
-void launch_count_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass,
-                        int plain, int dmax, int* counter, int num_sms, cudaStream_t st) {
+// the FP64 comparator's counts; the FP32 path has launch_count_keys (d = 2) and
+// launch_count_leaf
+void launch_count_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass, int dmax,
+                        int* counter, int num_sms, cudaStream_t st) {
   if (nitems <= 0) return;
-  if (plain) launch_count_wgrid_f64(dclass, jobs_d, items_d, nitems, counter, dmax, num_sms, st);
-  else launch_count_wgrid_f32(dclass, jobs_d, items_d, nitems, counter, dmax, num_sms, st);
+  launch_count_wgrid_f64(dclass, jobs_d, items_d, nitems, counter, dmax, num_sms, st);
 }
 
 TileShape grid_shape(int dclass, int plain, int dmax) {

@@ -308,9 +308,9 @@ void launch_t(const JobDev* jobs, const WorkItem* items, int nitems, int* counte
 
 }  // namespace
 
-// d = 2: measured faster than the FP32 union-window counts on every workload
-// here; for d = 3 and 4 the radii of those workloads are large and few cells
-// lie wholly inside a ball, so the FP32 kernel (egb_wgrid.cuh) is kept there
+// d = 2: measured faster than FP32 windows on every workload here; for d = 3
+// and 4 few cells lie wholly inside a ball, and the leaves of egb_lcount.cu
+// are read instead
 bool count_keys_supported(int dclass) { return dclass == 2; }
 
 void launch_count_keys(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass,

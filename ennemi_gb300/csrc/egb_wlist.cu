@@ -32,18 +32,14 @@
 // CTA grid; d = 4, K = 4, 200,000 points: 1.04 ms against 1.66 of the walks.
 #include <algorithm>
 
-#include "egb_wgrid.cuh"
+#include "egb_leaf.cuh"
 
 namespace egb {
 namespace {
 
-using wgrid_detail::dn_band32;
-using wgrid_detail::plan_margin;
-using wgrid_detail::up_band32;
-using wgrid_detail::warp_window;
+using namespace leaf_detail;
 
 constexpr int WL_WARPS = 4;
-constexpr unsigned FULL = 0xffffffffu;
 
 // K-th smallest (1-based) of the warp's R x 32 float bit patterns (distances
 // >= 0; unused slots +inf), at least K of them finite or +inf alike.
@@ -128,12 +124,7 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     const double* __restrict__ c64 = GRID ? J->c64g : J->c64;
     const float* __restrict__ g = GRID ? J->c32g : J->c32;
     const int32_t* __restrict__ sst = J->sstart;
-    const float* __restrict__ ylo = J->sylo32;
-    const float* __restrict__ yhi = J->syhi32;
     const int32_t* __restrict__ cst = J->cstart;
-    const float* __restrict__ zlo = J->czlo32;
-    const float* __restrict__ zhi = J->czhi32;
-    const int S = GRID ? J->nstrips : 1;
     const int S2 = NEST ? J->nsub : 1;
     const int sq = NEST ? (wi.strip & 0xffff) : wi.strip;
     const int hc = NEST ? (wi.strip >> 16) : 0;
@@ -152,14 +143,10 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
         qv[c] = g[(int64_t)c * lds + qp];
         am = fmaxf(am, fabsf(qv[c]));
       }
-      // |q_c - c| and the planning bounds of columns 0..2, from the FP32 copy
-      // (see wwalk_kernel)
-      const float mq = __fmaf_ru(am, 1.0f + 0x1p-22f, 0x1p-148f);
-      auto below = [](float v) { return __fsub_rd(v, __fmaf_ru(fabsf(v), 0x1p-22f, 0x1p-148f)); };
-      auto above = [](float v) { return __fadd_ru(v, __fmaf_ru(fabsf(v), 0x1p-22f, 0x1p-148f)); };
-      const float qxl = below(qv[0]), qxh = above(qv[0]);
-      const float qyl = below(qv[1]), qyh = above(qv[1]);
-      const float qzl = NEST ? below(qv[NEST ? 2 : 0]) : 0.0f, qzh = NEST ? above(qv[NEST ? 2 : 0]) : 0.0f;
+      const float mq = __fmaf_ru(am, 1.0f + 0x1p-22f, 0x1p-148f);  // >= max |q_c - c|
+      const QueryBox qbox{coord_below(qv[0]), coord_above(qv[0]), coord_below(qv[1]), coord_above(qv[1]),
+                          NEST ? coord_below(qv[NEST ? 2 : 0]) : 0.0f,
+                          NEST ? coord_above(qv[NEST ? 2 : 0]) : 0.0f};
       float thr = FINF;  // screen bound S
       float tb = FINF;   // planning bound plan_margin(U)
       int cnt = 0;       // listed candidates
@@ -229,47 +216,8 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
       // Every range of positions within the planning bound, nearest strips
       // first; f may tighten the bound.
       auto enumerate = [&](auto&& f) {
-        if constexpr (!GRID) {
-          f(0, len);
-        } else {
-          auto crange = [&](int a, int b) {
-            const float xl = fminf(__fsub_rd(qxl, tb), 1e37f), xh = fmaxf(__fadd_ru(qxh, tb), -1e37f);
-            int wl, wh;
-            if (b - a <= 1024) {
-              // whole blocks of 32 positions, from the first value of each:
-              // one load and two ballots, and no candidate block is split
-              const int p = a + 32 * lane;
-              const float x = p < b ? g[p] : FINF;
-              const int nl = __popc(__ballot_sync(FULL, x < xl)), nh = __popc(__ballot_sync(FULL, x <= xh));
-              wl = a + 32 * max(nl - 1, 0);
-              wh = min(b, a + 32 * nh);
-            } else {
-              warp_window<float>(g, a, b, xl, xh, wl, wh);
-            }
-            if (wl < wh) f(wl, wh);
-          };
-          auto cstrip = [&](int s) {
-            if constexpr (NEST) {
-              const int cb = s * S2;
-              int c0 = 0, c1 = 0;
-              for (int b = 0; b < S2; b += 32) {
-                const int c = b + lane;
-                c0 += __popc(__ballot_sync(FULL, c < S2 && __fsub_rd(qzl, zhi[cb + c]) > tb));
-                c1 += __popc(__ballot_sync(FULL, c < S2 && !(__fsub_rd(zlo[cb + c], qzh) > tb)));
-              }
-              for (int c = c0; c < c1; ++c) crange(cst[cb + c], cst[cb + c + 1]);
-            } else {
-              crange(sst[s], sst[s + 1]);
-            }
-          };
-          cstrip(sq);
-          for (int up = sq + 1, dn = sq - 1;;) {
-            const bool ou = up < S && !(__fsub_rd(ylo[up], qyh) > tb);
-            const bool od = dn >= 0 && !(__fsub_rd(qyl, yhi[dn]) > tb);
-            if (!ou && !od) break;
-            cstrip(ou && (!od || (up - sq) <= (sq - dn)) ? up++ : dn--);
-          }
-        }
+        if constexpr (!GRID) f(0, len);
+        else query_ranges<NEST>(J, g, sq, qbox, tb, f);
       };
 
       uint64_t kth = INF_BITS;

@@ -217,6 +217,34 @@ def test_warp_list_knn(oracle, d, data):
         assert np.array_equal(N.knn_eps(few, k), oracle.knn_eps(few, k)), k
 
 
+@pytest.mark.parametrize("data", ["normal", "dyadic", "duplicates", "huge"])
+@pytest.mark.parametrize("d", [3, 4, 5])
+def test_leaf_counts(oracle, d, data):
+    """Ball counts over leaf boxes: the smallest grid, odd sizes, radii from
+    nothing to everything in one item (leaf lists that overflow), boundaries
+    on exact distances, and values that rule out the FP32 screen."""
+    rng = np.random.default_rng(100 + d)
+    for n in [4096, 4097, 9001]:
+        pts = rng.normal(size=(n, d)) * np.linspace(1.0, 2.0, d)
+        r = np.abs(rng.normal(0.3, 0.2, size=n))
+        if data == "dyadic":
+            pts = rng.integers(-300, 300, size=(n, d)) / 64.0
+            r = rng.integers(0, 120, size=n) / 64.0
+        elif data == "duplicates":
+            pts = rng.integers(0, 6, size=(n, d)).astype(np.float64)
+            r = rng.integers(0, 4, size=n) - 1e-12
+        elif data == "huge":
+            pts[:, 1] *= 1e300
+            r[::2] *= 1e300
+        r[::97] = -1e-13
+        r[1::97] = 0.0
+        r[2::97] = np.inf
+        r[3::97] = 1e3
+        r[4::97] = np.nan
+        r[5::97] = -0.0
+        assert np.array_equal(N.ball_count(pts, r), oracle.ball_count(pts, r)), n
+
+
 def test_device_input_matches_host_input():
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(7)
