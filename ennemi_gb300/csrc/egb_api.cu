@@ -63,6 +63,8 @@ constexpr int NKTIME = 7;   // kNN tile, kNN deferred, count tile, count deferre
 constexpr int NSTATS = 16;
 // finish_batch: the batch must run again with the full sort (not a public code)
 constexpr int RC_SORT_RETRY = 1;
+// run_direct: the batch must run on the general path
+constexpr int RC_DIRECT_REDO = 2;
 
 // Digamma of a positive integer with the reference's formula
 // (ennemi/_entropy_estimators.py:341-348): the SciPy constant for psi(1),
@@ -402,11 +404,259 @@ uint64_t replay_key(const egb_ctx* ctx, const egb_task* tasks, int ntasks, int f
   return h ? h : 1;
 }
 
+// ------------------------------------------------------ small batches --
+// Whether a batch takes the direct path (egb_direct.cu): every task small and
+// of a kind with a search kernel, columns the kernels can read where they are
+// (device memory, or host memory through the host's page tables), and no flag
+// or policy entry that asks for a layout, a graph or phase times.
+bool direct_batch(const egb_ctx* ctx, const egb_task* tasks, const std::vector<TaskPlan>& P, int flags) {
+  if (flags & ~(EGB_INPUT_DEVICE | EGB_KEEP_INTERNALS | EGB_RESCALE)) return false;
+  if (!(flags & EGB_INPUT_DEVICE) && !ctx->host_direct) return false;
+  double pairs = 0.0;
+  int64_t longest = 0;
+  for (size_t t = 0; t < P.size(); ++t) {
+    const TaskPlan& p = P[t];
+    if (p.n > DIRECT_MAX_N || !direct_supported(p.kind, p.dx, p.dy, p.dz, p.K)) return false;
+    pairs += (double)p.n * (double)p.n;
+    longest = std::max(longest, p.n);
+    const int d = p.ncol;
+    for (int e = 2; e <= d; ++e)  // the kNN space and the multi-column counts
+      if (ctx->policy[egb_policy_index(0, e, p.K, p.n)] != EGB_MODE_AUTO ||
+          ctx->policy[egb_policy_index(1, e, p.K, p.n)] != EGB_MODE_AUTO)
+        return false;
+  }
+  return longest <= DIRECT_ANY_N || pairs <= DIRECT_MAX_PAIRS;
+}
+
+int run_direct(egb_ctx* ctx, const egb_task* tasks, std::vector<TaskPlan>& P, int flags,
+               egb_result* results, int ncols, int64_t max_n,
+               std::chrono::steady_clock::time_point t_entry) {
+  using clk = std::chrono::steady_clock;
+  const int ntasks = (int)P.size();
+  const bool rescale = (flags & EGB_RESCALE) != 0;
+  const long long launches0 = g_launches.load();
+  cudaStream_t st = ctx->stream;
+
+  // tasks in launch groups: (estimator, columns, list size)
+  std::vector<int> order((size_t)ntasks);
+  for (int t = 0; t < ntasks; ++t) order[(size_t)t] = t;
+  auto group_of = [&](int t) {
+    const TaskPlan& p = P[(size_t)t];
+    return (p.kind * 8 + p.ncol) * 2 + (p.K > 16 ? 1 : 0);
+  };
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return group_of(a) < group_of(b); });
+  struct Run { int first, count, queries, kmax, per, part0, nparts; };
+  std::vector<Run> runs;
+  for (int i = 0; i < ntasks; ++i) {
+    const TaskPlan& p = P[(size_t)order[(size_t)i]];
+    if (i == 0 || group_of(order[(size_t)i]) != group_of(order[(size_t)i - 1]))
+      runs.push_back({i, 0, 0, 0, 1, 0, 0});
+    Run& r = runs.back();
+    ++r.count;
+    r.queries += (int)p.n;
+    r.kmax = std::max(r.kmax, p.K);
+  }
+
+  Layout dl, tl;
+  for (TaskPlan& p : P) {
+    p.off_x64 = dl.take(sizeof(double) * (size_t)(p.ncol * p.ld));
+    p.off_eps = dl.take(sizeof(double) * (size_t)p.ld);
+    p.off_rad = dl.take(sizeof(float) * (size_t)(p.ncol * p.ld));  // here: the FP32 copy
+    for (int s = 0; s < p.nslot; ++s) p.off_cnt[s] = dl.take(sizeof(int32_t) * (size_t)p.ld);
+  }
+  // tables: one blob, followed by the zeroed flags and the read-back, so that
+  // one copy goes each way
+  const size_t tab_tasks = tl.take(sizeof(DirectTask) * (size_t)ntasks);
+  const size_t tab_cols = tl.take(sizeof(DirectCol) * (size_t)ncols);
+  const size_t tab_tdev = tl.take(sizeof(TaskDev) * (size_t)ntasks);
+  const size_t tab_cjobs = tl.take(sizeof(CombineJob) * (size_t)ntasks);
+  const size_t tab_chunk = tl.take(sizeof(int32_t) * (size_t)ntasks);
+  std::vector<PwTree> trees;
+  std::vector<int2> nodes;
+  std::vector<int32_t> levels;
+  std::map<int64_t, int32_t> tree_of;
+  std::map<std::pair<const int32_t*, int64_t>, size_t> index_tab;
+  std::vector<size_t> inv_tab((size_t)ntasks, 0), cls_tab((size_t)ntasks, 0);
+  for (int t = 0; t < ntasks; ++t) {
+    TaskPlan& p = P[(size_t)t];
+    if (rescale && p.kind != EGB_ENTROPY && !tree_of.count(p.n))
+      tree_of[p.n] = pw_build(p.n, trees, nodes, levels);
+    if (!p.perm.empty()) {
+      p.tab_perm = tl.take(sizeof(int32_t) * p.perm.size());
+      if (rescale) inv_tab[(size_t)t] = tl.take(sizeof(int32_t) * p.perm.size());
+      cls_tab[(size_t)t] = tl.take(sizeof(int32_t) * p.cls_off.size());
+    }
+    if (p.index) {
+      auto it = index_tab.find({p.index, p.n});
+      if (it == index_tab.end())
+        it = index_tab.emplace(std::make_pair(p.index, p.n), tl.take(sizeof(int32_t) * (size_t)p.n)).first;
+      p.tab_index = it->second;
+    }
+  }
+  const size_t tab_trees = tl.take(sizeof(PwTree) * trees.size());
+  const size_t tab_nodes = tl.take(sizeof(int2) * nodes.size());
+  const size_t tab_levels = tl.take(sizeof(int32_t) * levels.size());
+  const size_t zr = tl.take(0);
+  const size_t zr_zero = 0, zr_err = align_up(sizeof(uint32_t) * (size_t)ntasks, 16);
+  const size_t zr_bytes = align_up(zr_err + 16, 256);
+  const size_t tab_bytes = zr + zr_bytes;
+  const size_t off_tab = dl.take(tab_bytes);
+  const size_t off_partial = dl.take(sizeof(double) * (size_t)ntasks);  // directly after the flags
+  const size_t back_bytes = off_partial + sizeof(double) * (size_t)ntasks - (off_tab + zr);
+  const size_t pin_back = align_up(tab_bytes, 256);
+
+  int rc = ensure_arena(ctx, align_up(dl.off, 256));
+  if (rc) return rc;
+  rc = ensure_pinned(ctx, pin_back + back_bytes);
+  if (rc) return rc;
+  rc = ensure_psi(ctx, max_n + 1);
+  if (rc) return rc;
+  char* A = (char*)ctx->arena;
+  char* H = (char*)ctx->pinned;
+  char* T = A + off_tab;
+
+  DirectTask* dt = (DirectTask*)(H + tab_tasks);
+  DirectCol* dc = (DirectCol*)(H + tab_cols);
+  TaskDev* tdev = (TaskDev*)(H + tab_tdev);
+  CombineJob* cj = (CombineJob*)(H + tab_cjobs);
+  int32_t* chunk = (int32_t*)(H + tab_chunk);
+  std::memset(H + zr, 0, zr_bytes);
+  for (const auto& e : index_tab)
+    std::memcpy(H + e.second, e.first.first, sizeof(int32_t) * (size_t)e.first.second);
+  if (!trees.empty()) {
+    std::memcpy(H + tab_trees, trees.data(), sizeof(PwTree) * trees.size());
+    std::memcpy(H + tab_nodes, nodes.data(), sizeof(int2) * nodes.size());
+    std::memcpy(H + tab_levels, levels.data(), sizeof(int32_t) * levels.size());
+  }
+  // queries per warp: one while they do not fill the GPU (32 warps per SM)
+  int parts = 0, nc = 0;
+  for (Run& r : runs) {
+    r.per = std::max(1, std::min(16, r.queries / (ctx->num_sms * 32)));
+    r.part0 = parts;
+    for (int i = r.first; i < r.first + r.count; ++i) {
+      const int t = order[(size_t)i];
+      TaskPlan& p = P[(size_t)t];
+      DirectTask& D = dt[i];
+      std::memset(&D, 0, sizeof(D));
+      D.x64 = (const double*)(A + p.off_x64);
+      D.x32 = (const float*)(A + p.off_rad);
+      D.eps = (double*)(A + p.off_eps);
+      for (int s = 0; s < p.nslot && s < 3; ++s) D.cnt[s] = (int32_t*)(A + p.off_cnt[s]);
+      D.ld = p.ld;
+      D.n = (int32_t)p.n;
+      D.K = p.K;
+      D.nclass = p.nclass;
+      D.part0 = parts;
+      D.id = t;
+      parts += (int)((p.n + r.per - 1) / r.per);
+      const int32_t* perm = nullptr;
+      if (!p.perm.empty()) {
+        const std::vector<int32_t>& gp = p.gperm.empty() ? p.perm : p.gperm;
+        std::memcpy(H + p.tab_perm, gp.data(), sizeof(int32_t) * gp.size());
+        perm = (const int32_t*)(T + p.tab_perm);
+        int32_t* cls = (int32_t*)(H + cls_tab[(size_t)t]);
+        for (size_t c = 0; c < p.cls_off.size(); ++c) cls[c] = (int32_t)p.cls_off[c];
+        D.cls = (const int32_t*)(T + cls_tab[(size_t)t]);
+        if (rescale) {
+          int32_t* inv = (int32_t*)(H + inv_tab[(size_t)t]);
+          for (size_t w = 0; w < p.perm.size(); ++w) inv[p.perm[w]] = (int32_t)w;
+        }
+      } else if (p.index) {
+        perm = (const int32_t*)(T + p.tab_index);
+      }
+      for (int c = 0; c < p.ncol; ++c) {
+        DirectCol& C = dc[nc++];
+        std::memset(&C, 0, sizeof(C));
+        C.src = tasks[t].cols[c].data;
+        C.stride = tasks[t].cols[c].stride;
+        C.perm = perm;
+        C.task = i;
+        C.col = c;
+        C.tree = -1;
+        C.group = 1;
+        if (rescale && p.kind != EGB_ENTROPY) {  // noise positions as in the general path
+          const int zc = c - p.dx - p.dy;
+          C.inv = p.perm.empty() ? nullptr : (const int32_t*)(T + inv_tab[(size_t)t]);
+          C.group = zc >= 0 && p.dz > 1 ? p.dz : 1;
+          C.noise_pos = zc >= 0 ? (int64_t)(p.dx + p.dy) * p.n + zc : (int64_t)c * p.n;
+          C.tree = tree_of[p.n];
+        }
+      }
+      TaskDev& V = tdev[t];
+      std::memset(&V, 0, sizeof(V));
+      V.x64 = D.x64;
+      V.eps = D.eps;
+      for (int s = 0; s < 3; ++s) V.cnt[s] = D.cnt[s];
+      V.ld = p.ld;
+      V.n = (int32_t)p.n;
+      V.ncol = p.ncol;
+      CombineJob J{};
+      J.task = t;
+      J.kind = p.kind;
+      J.chunk0 = t;
+      J.nchunk = 1;
+      cj[t] = J;
+      chunk[t] = t;
+    }
+    r.nparts = parts - r.part0;
+  }
+  static_assert(DIRECT_MAX_N <= COMBINE_CHUNK, "one combine chunk per task");
+  ReplayState R;
+  R.cjobs.assign(cj, cj + ntasks);
+
+  const int64_t plan_us =
+      std::chrono::duration_cast<std::chrono::microseconds>(clk::now() - t_entry).count();
+  const clk::time_point t_issue = clk::now();
+  uint32_t* flags_d = (uint32_t*)(T + zr + zr_zero);
+  uint32_t* err_d = (uint32_t*)(T + zr + zr_err);
+  EGB_CUDA(cudaMemcpyAsync(T, H, tab_bytes, cudaMemcpyHostToDevice, st));
+  launch_direct_prep((const DirectTask*)(T + tab_tasks), (const DirectCol*)(T + tab_cols), nc,
+                     (const PwTree*)(T + tab_trees), (const int2*)(T + tab_nodes),
+                     (const int32_t*)(T + tab_levels), ctx->noise_d, flags_d, st);
+  for (const Run& r : runs) {
+    const TaskPlan& p = P[(size_t)order[(size_t)r.first]];
+    launch_direct_search(p.kind, p.ncol, (const DirectTask*)(T + tab_tasks) + r.first, r.count, r.kmax,
+                         r.part0, r.nparts, r.per, st);
+  }
+  launch_combine((const TaskDev*)(T + tab_tdev), (const CombineJob*)(T + tab_cjobs),
+                 (const int32_t*)(T + tab_chunk), ntasks, ctx->psi_d, ctx->psi_len,
+                 (double*)(A + off_partial), flags_d, err_d, ctx->num_sms, st);
+  EGB_CUDA(cudaGetLastError());
+  EGB_CUDA(cudaMemcpyAsync(H + pin_back, T + zr, back_bytes, cudaMemcpyDeviceToHost, st));
+  const int64_t issue_us =
+      std::chrono::duration_cast<std::chrono::microseconds>(clk::now() - t_issue).count();
+  EGB_CUDA(cudaStreamSynchronize(st));
+  const uint32_t* fl = (const uint32_t*)(H + pin_back + zr_zero);
+  for (int t = 0; t < ntasks; ++t)
+    if (fl[t] & DIRECT_REDO) return RC_DIRECT_REDO;
+
+  ctx->h2d_bytes = (int64_t)tab_bytes;
+  ctx->d2h_bytes = (int64_t)back_bytes;
+  if (!(flags & EGB_INPUT_DEVICE))
+    for (int c = 0; c < nc; ++c) ctx->h2d_bytes += (int64_t)sizeof(double) * dt[dc[c].task].n;
+  R.P = std::move(P);
+  R.pin_zr = pin_back;
+  R.zr_zero = zr_zero;
+  R.zr_err = zr_err;
+  R.pin_rb = pin_back + (off_partial - (off_tab + zr));
+  const int rc_fin = finish_batch(ctx, R, H, (int64_t)(g_launches.load() - launches0), results);
+  ctx->stats[11] = 1;
+  ctx->stats[14] = plan_us;
+  ctx->stats[15] = issue_us;
+  if (rc_fin != EGB_OK) return rc_fin;
+  if (flags & EGB_KEEP_INTERNALS) {
+    ctx->keep = std::move(R.P);
+    ctx->kept = true;
+  }
+  return EGB_OK;
+}
+
 // extra: per-task extras for the internal kinds (radius for KIND_COUNT_ONLY)
 // One batch.  sort_first: the first 8-bit key digit the batch sort passes
 // over (2: the high 48 bits and a repair of tied runs; 0: all eight).
+// small_ok: a batch of small tasks may take the direct path (run_direct).
 int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
-                     egb_result* results, const double* count_radius, int sort_first) {
+                     egb_result* results, const double* count_radius, int sort_first, bool small_ok) {
   if (!ctx) return EGB_ERR_ARG;
   if (ntasks < 0 || (ntasks > 0 && !tasks)) return fail(ctx, EGB_ERR_ARG, "invalid task list");
   if (ntasks == 0) return EGB_OK;
@@ -539,6 +789,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       p.cls_off = {0, T.n};
     }
   }
+
+  if (small_ok && !inject && !count_radius && direct_batch(ctx, tasks, P, flags))
+    return run_direct(ctx, tasks, P, flags, results, ncols_total, max_n, t_entry);
 
   // ------------------------------------------------------------- spaces --
   std::vector<Space> knn, cnt;
@@ -1914,12 +2167,15 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
 
 // A batch whose sort met keys tied in their high 48 bits over a run too long
 // to repair (finish_batch: RC_SORT_RETRY) runs again with the full sort,
-// planned and issued directly.
+// planned and issued directly; a batch of small tasks with values that the
+// direct path does not take (RC_DIRECT_REDO) runs again on the general path.
 int run_batch(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags, egb_result* results,
               const double* count_radius) {
-  const int rc = run_batch_sorted(ctx, tasks, ntasks, flags, results, count_radius, 2);
+  int rc = run_batch_sorted(ctx, tasks, ntasks, flags, results, count_radius, 2, true);
+  if (rc == RC_DIRECT_REDO)
+    rc = run_batch_sorted(ctx, tasks, ntasks, flags, results, count_radius, 2, false);
   if (rc != RC_SORT_RETRY) return rc;
-  return run_batch_sorted(ctx, tasks, ntasks, flags & ~EGB_GRAPH, results, count_radius, 0);
+  return run_batch_sorted(ctx, tasks, ntasks, flags & ~EGB_GRAPH, results, count_radius, 0, false);
 }
 
 bool create_fork_events(egb_ctx* ctx) {

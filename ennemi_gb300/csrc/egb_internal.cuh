@@ -654,6 +654,45 @@ struct KeyIndexOut {
 void launch_samples(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
                     const uint64_t* keys, const KeyIndexOut& out, cudaStream_t st);
 
+// egb_direct.cu: batches of small tasks (run_direct in egb_api.cu)
+constexpr int DIRECT_MAX_N = 4095;       // most samples of a task (shared memory)
+// The search is brute force: batches of any length up to DIRECT_ANY_N samples a
+// task, beyond while the batch has at most DIRECT_MAX_PAIRS point pairs
+// (measured against the general path: 20 tasks of 4,000 samples 0.90 ms
+// against 1.07, 60 of them 2.43 against 1.61; 60 of 2,000 0.95 against 1.07,
+// 200 of them 2.76 against 2.47; 800 of 1,000 6.0 against 6.4).
+constexpr int DIRECT_ANY_N = 1024;
+constexpr double DIRECT_MAX_PAIRS = 4.5e8;
+constexpr uint32_t DIRECT_REDO = 1u << 30;  // flag word of a task: run the general path
+struct DirectTask {
+  const double* x64;      // working columns, column c at + c * ld
+  const float* x32;       // the same less their midranges, in FP32
+  double* eps;
+  int32_t* cnt[3];
+  const int32_t* cls;     // class starts (nclass + 1), SEMI / CSEMI
+  int64_t ld;
+  int32_t n, K, nclass;
+  int32_t part0;          // first search part
+  int32_t id;             // task of the batch
+  int32_t pad_;
+};
+struct DirectCol {        // one task column to prepare
+  const double* src;      // sample w at src[perm[w] * stride] (perm null: w)
+  int64_t stride;
+  const int32_t* perm;
+  const int32_t* inv;     // sample -> working position (class-ordered), or null
+  int64_t noise_pos;
+  int32_t task, col;      // task: index of its DirectTask
+  int32_t tree;           // summation tree of a rescaled column, or -1
+  int32_t group;          // > 1: one of `group` columns reduced row by row
+};
+bool direct_supported(int kind, int dx, int dy, int dz, int K);
+void launch_direct_prep(const DirectTask* tasks_d, const DirectCol* cols_d, int ncols, const PwTree* trees_d,
+                        const int2* nodes_d, const int32_t* levels_d, const double* noise, uint32_t* flags,
+                        cudaStream_t st);
+void launch_direct_search(int kind, int d, const DirectTask* tasks_d, int ntasks, int kmax, int part_base,
+                          int nparts, int per, cudaStream_t st);
+
 // egb_discrete.cu: exact group-by of the rows of one column subset of a
 // discrete task: the rows equal to each row, into count slot `slot`.
 struct GroupJob {

@@ -33,82 +33,28 @@
 #include <algorithm>
 
 #include "egb_leaf.cuh"
+#include "egb_list.cuh"
 
 namespace egb {
 namespace {
 
-using namespace leaf_detail;
+using leaf_detail::QueryBox;
+using leaf_detail::coord_above;
+using leaf_detail::coord_below;
+using leaf_detail::query_ranges;
+using list_detail::CandidateList;
+using list_detail::FULL;
+using list_detail::radix_kth;
 
 constexpr int WL_WARPS = 4;
-
-// K-th smallest (1-based) of the warp's R x 32 float bit patterns (distances
-// >= 0; unused slots +inf), at least K of them finite or +inf alike.
-template <int R>
-__device__ __forceinline__ uint32_t kth_bits(const uint32_t (&v)[R], int K) {
-  uint32_t lo = 0xffffffffu, hi = 0u;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    lo = min(lo, v[r]);
-    hi = max(hi, v[r]);
-  }
-  lo = __reduce_min_sync(FULL, lo);
-  if (K <= 8) {  // a few minima in turn are cheaper than a bisection
-    uint32_t w[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) w[r] = v[r];
-    for (int left = K;;) {
-      int c = 0;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        c += __popc(__ballot_sync(FULL, w[r] == lo));
-        w[r] = w[r] == lo ? 0xffffffffu : w[r];
-      }
-      left -= c;
-      if (left <= 0) return lo;
-      uint32_t m = w[0];
-#pragma unroll
-      for (int r = 1; r < R; ++r) m = min(m, w[r]);
-      lo = __reduce_min_sync(FULL, m);
-    }
-  }
-  hi = __reduce_max_sync(FULL, hi);
-  while (lo < hi) {
-    const uint32_t mid = lo + ((hi - lo) >> 1);
-    int c = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) c += __popc(__ballot_sync(FULL, v[r] <= mid));
-    if (c == K) {  // the largest of the K values up to mid
-      uint32_t m = 0;
-#pragma unroll
-      for (int r = 0; r < R; ++r) m = max(m, v[r] <= mid ? v[r] : 0u);
-      return __reduce_max_sync(FULL, m);
-    }
-    if (c > K) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
-__device__ __forceinline__ uint64_t warp_min64(uint64_t v) {
-  const uint32_t h = __reduce_min_sync(FULL, (uint32_t)(v >> 32));
-  const uint32_t l = __reduce_min_sync(FULL, (uint32_t)(v >> 32) == h ? (uint32_t)v : 0xffffffffu);
-  return ((uint64_t)h << 32) | l;
-}
 
 template <int D, int R, bool GRID, bool NEST>
 __global__ void __launch_bounds__(WL_WARPS * 32)
 wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items, int nitems, int qb,
              int per, int* __restrict__ counter) {
   constexpr int DQ = D ? D : EGB_DMAX;
-  constexpr int CAP = 32 * R;
-  constexpr float FINF = __builtin_huge_valf();
-  struct Entry { float d; int j; };
-  constexpr int WORDS = 2 * CAP > 256 ? 2 * CAP : 256;  // the list, or 256 radix counters
-  __shared__ __align__(8) uint32_t store[WL_WARPS][WORDS];
+  __shared__ __align__(8) uint32_t store[WL_WARPS][CandidateList<R>::WORDS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  Entry* list = reinterpret_cast<Entry*>(store[warp]);
-  uint32_t* hist = store[warp];
   const int split = (qb + per - 1) / per;  // parts of `per` queries of an item
 
   for (;;) {
@@ -147,11 +93,7 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
       const QueryBox qbox{coord_below(qv[0]), coord_above(qv[0]), coord_below(qv[1]), coord_above(qv[1]),
                           NEST ? coord_below(qv[NEST ? 2 : 0]) : 0.0f,
                           NEST ? coord_above(qv[NEST ? 2 : 0]) : 0.0f};
-      float thr = FINF;  // screen bound S
-      float tb = FINF;   // planning bound plan_margin(U)
-      int cnt = 0;       // listed candidates
-      bool over = unsafe;
-
+      CandidateList<R> list(store[warp], K, mq);
       auto exact_dist = [&](int j) -> uint64_t {
         uint64_t mm = 0;
 #pragma unroll
@@ -163,39 +105,11 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
         }
         return mm;
       };
-      // New bounds from the list's K-th smallest; entries beyond them leave.
-      auto tighten = [&]() {
-        __syncwarp();
-        uint32_t v[R];
-        int ix[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const bool in = r * 32 + lane < cnt;
-          const Entry e = in ? list[r * 32 + lane] : Entry{FINF, 0};
-          v[r] = __float_as_uint(e.d);
-          ix[r] = e.j;
-        }
-        const float u = up_band32(__uint_as_float(kth_bits<R>(v, K)), mq);
-        thr = up_band32(u, mq);
-        tb = plan_margin(u);
-        __syncwarp();
-        int kept = 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const bool keep = r * 32 + lane < cnt && __uint_as_float(v[r]) <= thr;
-          const uint32_t m = __ballot_sync(FULL, keep);
-          if (keep) list[kept + __popc(m & lt)] = Entry{__uint_as_float(v[r]), ix[r]};
-          kept += __popc(m);
-        }
-        cnt = kept;
-        over = over || cnt > CAP - 32;  // more near ties than the list holds
-        __syncwarp();
-      };
       auto screen = [&](int a, int b, int ea, int eb) {  // [a, b) without [ea, eb)
         pairs += (unsigned)(b - a);
-        for (int j0 = a; j0 < b && !over; j0 += 32) {
+        for (int j0 = a; j0 < b && !list.over; j0 += 32) {
           const int j = j0 + lane;
-          float dd = FINF;
+          float dd = __builtin_huge_valf();
           if (j < b && !(j >= ea && j < eb)) {
             dd = fabsf(g[j] - qv[0]);
 #pragma unroll
@@ -204,24 +118,18 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
               dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - qv[c]));
             }
           }
-          const bool hit = dd <= thr && dd < FINF;
-          const uint32_t m = __ballot_sync(FULL, hit);
-          if (m) {
-            if (hit) list[cnt + __popc(m & lt)] = Entry{dd, j};
-            cnt += __popc(m);
-            if (cnt > CAP - 32) tighten();
-          }
+          list.push(dd, j);
         }
       };
-      // Every range of positions within the planning bound, nearest strips
-      // first; f may tighten the bound.
+      // every range of positions within the planning bound, nearest strips
+      // first; f may tighten the bound
       auto enumerate = [&](auto&& f) {
         if constexpr (!GRID) f(0, len);
-        else query_ranges<NEST>(J, g, sq, qbox, tb, f);
+        else query_ranges<NEST>(J, g, sq, qbox, list.tb, f);
       };
 
       uint64_t kth = INF_BITS;
-      if (!over) {
+      if (!unsafe) {
         int e0 = 0, e1 = 0;
         if (GRID) {
           // first bound: the query's neighbours in its own strip or cell
@@ -231,114 +139,24 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
           e0 = max(ha, qp - w);
           e1 = min(hb, e0 + 2 * w);
           screen(e0, e1, 0, 0);
-          if (cnt >= K) tighten();
+          if (list.cnt >= K) list.tighten();
         }
         enumerate([&](int a, int b) {
-          if (over) return;
-          const int had = cnt;
+          if (list.over) return;
+          const int had = list.cnt;
           screen(a, b, e0, e1);
-          if (cnt >= K && (cnt - had >= 8 || !(thr < FINF))) tighten();
+          if (list.cnt >= K && (list.cnt - had >= 8 || !(list.thr < __builtin_huge_valf()))) list.tighten();
         });
       }
-      if (!over) {
-        __syncwarp();
-        float v[R];
-        int ix[R];
-        uint32_t vb[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const bool in = r * 32 + lane < cnt;
-          const Entry e = in ? list[r * 32 + lane] : Entry{FINF, 0};
-          v[r] = e.d;
-          vb[r] = __float_as_uint(e.d);
-          ix[r] = e.j;
-        }
-        if (cnt >= K) {
-          const float t32 = __uint_as_float(kth_bits<R>(vb, K));
-          const float lo = dn_band32(t32, mq), hi = up_band32(t32, mq);
-          int rank = K;
-          uint64_t e[R];
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            rank -= __popc(__ballot_sync(FULL, up_band32(v[r], mq) < lo));  // false for +inf
-            e[r] = ~0ull;
-          }
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-            if (v[r] < FINF && !(up_band32(v[r], mq) < lo) && !(dn_band32(v[r], mq) > hi))
-              e[r] = exact_dist(ix[r]);
-          for (;;) {  // the rank-th smallest of e (ties leave together)
-            uint64_t m = ~0ull;
-#pragma unroll
-            for (int r = 0; r < R; ++r) m = e[r] < m ? e[r] : m;
-            m = warp_min64(m);
-            int c = 0;
-#pragma unroll
-            for (int r = 0; r < R; ++r) c += __popc(__ballot_sync(FULL, e[r] == m));
-            if (c >= rank || m == ~0ull) {
-              kth = m;
-              break;
-            }
-            rank -= c;
-#pragma unroll
-            for (int r = 0; r < R; ++r) e[r] = e[r] == m ? ~0ull : e[r];
-          }
-        }
-        __syncwarp();
+      if (!unsafe && !list.over) {
+        kth = list.kth(exact_dist);
       } else if (len >= K) {
-        // radix select on the exact distances, 8 bits a pass, over the
-        // candidates within the bound (U was set from K listed candidates)
+        // the exact distances of the candidates within the bound (U was set
+        // from K listed candidates; none in a job with clamped values)
         ++redone;
-        uint64_t prefix = 0, mask = 0;
-        uint32_t rank = (uint32_t)K;
-        for (int shift = 56; shift >= 0; shift -= 8) {
-          __syncwarp();
-          for (int b = lane; b < 256; b += 32) hist[b] = 0u;
-          __syncwarp();
-          enumerate([&](int a, int b) {
-            pairs += (unsigned)(b - a);
-            for (int j = a + lane; j < b; j += 32) {
-              const uint64_t m = exact_dist(j);
-              if ((m & mask) == prefix) atomicAdd(&hist[(m >> shift) & 255u], 1u);
-            }
-            __syncwarp();
-          });
-          __syncwarp();
-          uint32_t s = 0, loc[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            loc[i] = hist[8 * lane + i];
-            s += loc[i];
-          }
-          uint32_t incl = s;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += y;
-          }
-          const uint32_t excl = incl - s;
-          const unsigned hit = __ballot_sync(FULL, excl < rank && rank <= incl);
-          const int src = hit ? __ffs(hit) - 1 : 0;
-          uint32_t run = excl, digit = 255, before = excl;
-#pragma unroll
-          for (int i = 7; i >= 0; --i) {  // the first bucket that reaches the rank
-            run = excl;
-#pragma unroll
-            for (int k = 0; k < i; ++k) run += loc[k];
-            if (run < rank && rank <= run + loc[i]) {
-              digit = (uint32_t)(8 * lane + i);
-              before = run;
-            }
-          }
-          digit = __shfl_sync(FULL, digit, src);
-          before = __shfl_sync(FULL, before, src);
-          prefix |= (uint64_t)digit << shift;
-          mask |= 255ull << shift;
-          rank -= before;
-        }
+        kth = radix_kth(store[warp], K, enumerate, exact_dist);
         // distances of non-finite data, as the lists and the select rank them
-        kth = K <= EGB_KREG_MAX && prefix > INF_BITS ? INF_BITS : prefix;
-        __syncwarp();
+        if (K <= EGB_KREG_MAX && kth > INF_BITS) kth = INF_BITS;
       }
       if (lane == 0) J->eps[GRID ? J->idxg[qp] : J->idx[qp]] = bits_to_double(kth);
     }

@@ -245,6 +245,85 @@ def test_leaf_counts(oracle, d, data):
         assert np.array_equal(N.ball_count(pts, r), oracle.ball_count(pts, r)), n
 
 
+def _small_tasks(rng, n, k, data):
+    """Every estimator that the direct path serves, over n samples."""
+    lab = rng.integers(0, 3, size=n).astype(np.int32)
+    c = rng.normal(size=(n, 5))
+    c[:, 1] += 0.6 * c[:, 0]
+    if data == "rounded":
+        c = np.round(c, 1)
+    elif data == "duplicates":
+        c = rng.integers(0, 3, size=(n, 5)).astype(np.float64)
+    elif data == "huge":
+        c[:, 0] *= 1e300
+    elif data == "infinite":
+        c[n // 2, 1] = np.inf
+    col = [np.ascontiguousarray(v) for v in c.T]
+    seen = np.unique(lab)
+    lab = np.searchsorted(seen, lab).astype(np.int32)
+    T, m = N.Task, len(seen)
+    return [T(N.MI, k, col[:1], col[1:2], n=n), T(N.CMI, k, col[:1], col[1:2], col[2:3], n=n),
+            T(N.CMI, k, col[:1], col[1:2], col[2:4], n=n), T(N.CMI, k, col[:1], col[1:2], col[2:], n=n),
+            T(N.SEMI, k, col[:1], labels=lab, nclass=m, n=n), T(N.SEMI, k, col[:3], labels=lab, nclass=m, n=n),
+            T(N.CSEMI, k, col[:1], (), col[1:2], labels=lab, nclass=m, n=n),
+            T(N.CSEMI, k, col[:1], (), col[1:3], labels=lab, nclass=m, n=n),
+            T(N.ENTROPY, k, col[:1], n=n), T(N.ENTROPY, k, col[:2], n=n), T(N.ENTROPY, k, col[:4], n=n)]
+
+
+@pytest.mark.parametrize("data", ["normal", "rounded", "duplicates", "huge", "infinite"])
+@pytest.mark.parametrize("n,k", [(1, 1), (2, 1), (5, 4), (31, 3), (32, 3), (33, 31), (64, 15), (65, 16),
+                                 (257, 63), (300, 64), (1000, 3), (1024, 5), (1025, 3), (4095, 3), (4096, 3)])
+def test_small_batches_equal_the_general_path(n, k, data):
+    """The direct path's results -- values, distances and counts -- are those of
+    the general path bit for bit: below, at and beyond its limits, with lists
+    that near ties overflow and values that send the batch back."""
+    tasks = _small_tasks(np.random.default_rng(n + k), n, k, data)
+    slots = {N.MI: 2, N.CMI: 3, N.SEMI: 1, N.CSEMI: 3, N.ENTROPY: 0}
+
+    def results(flags, batch):
+        v = N.run_tasks(batch, flags=flags | N.KEEP_INTERNALS)
+        return v, [[N.fetch(i, w, n) for w in range(1 + slots[t.kind])] for i, t in enumerate(batch)]
+
+    want, inner = results(N.FORCE_BRUTE, tasks)
+    got, kept = results(0, tasks)
+    assert np.array_equal(got, want, equal_nan=True)
+    for a, b in zip(kept, inner):
+        for u, w in zip(a, b):
+            assert np.array_equal(u.view(np.int64), w.view(np.int64))
+    for i in (0, 2, 7):   # a task alone, and as device columns
+        alone, k1 = results(0, tasks[i:i + 1])
+        assert np.array_equal(alone, want[i:i + 1], equal_nan=True)
+        for u, w in zip(k1[0], inner[i]):
+            assert np.array_equal(u.view(np.int64), w.view(np.int64))
+
+
+@pytest.mark.parametrize("n", [9, 129, 1000, 4095])
+def test_small_batches_rescale_and_index(n):
+    """Strided views, a shared sample index, class orders and conditions of one
+    and two columns: the rescaled columns are the general path's bits."""
+    from ennemi_gb300 import _driver
+    rng = np.random.default_rng(n)
+    raw = rng.normal(size=(n + 40, 4)) * [1.0, 3.0, 0.1, 2.0] + [0.0, 5.0, -1.0, 0.0]
+    idx = np.sort(rng.choice(n + 30, size=n, replace=False)).astype(np.int32)
+    lab = (np.arange(n) % 3).astype(np.int32)
+    v = [raw[5:, c] for c in range(4)]
+    k = min(3, n - 2)
+    tasks = [N.Task(N.MI, k, [v[0]], [v[1]], n=n, index=idx), N.Task(N.MI, k, [v[1]], [v[2]], n=n),
+             N.Task(N.CMI, k, [v[0]], [v[1]], [v[2]], n=n, index=idx),
+             N.Task(N.CMI, k, [v[0]], [v[1]], [v[2], v[3]], n=n, index=idx),
+             N.Task(N.SEMI, k, [v[0]], labels=lab, nclass=3, n=n, index=idx),
+             N.Task(N.CSEMI, k, [v[0]], (), [v[1]], labels=lab, nclass=3, n=n)]
+    noise = lambda m: _driver._noise.take(0, (m,))
+    out = []
+    for flags in (N.FORCE_BRUTE, 0):
+        r = N.run_tasks(tasks, flags=flags | N.RESCALE | N.KEEP_INTERNALS, noise=noise)
+        out.append((r, [N.fetch(t, 16 + c, n) for t, task in enumerate(tasks)
+                        for c in range(len(task.x) + len(task.y) + len(task.z))]))
+    assert np.array_equal(out[0][0], out[1][0])
+    for a, b in zip(out[0][1], out[1][1]):
+        assert np.array_equal(a.view(np.uint64), b.view(np.uint64))
+
+
 def test_device_input_matches_host_input():
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(7)
