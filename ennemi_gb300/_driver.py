@@ -341,45 +341,56 @@ def _estimate_mi(y: FloatArray, x: FloatArray, lag: FloatArray, k: int,
         raise ValueError("lag is too large, no observations left")
 
     nvar = 1 if x.ndim == 1 else x.shape[1]
-    indices = [(li, vi) for li in range(len(lag)) for vi in range(nvar)]
+    nlag = len(lag)
     prep = _Prep(mask, min_lag, max_lag)
-    jobs = []
-    for li, vi in indices:
+
+    def job(t):   # the host preparation of task t
+        li, vi = divmod(t, nvar)
         xv = x if x.ndim == 1 else x[:, vi]
-        jobs.append(_task_job(prep, ("x", vi), xv, ("y",), y, lag[li], max_lag, min_lag, k, mask,
-                              cond, cond_lag[li], discrete_x, discrete_y, preprocess, drop_nan,
-                              share_x=False))
+        return _task_job(prep, ("x", vi), xv, ("y",), y, lag[li], max_lag, min_lag, k, mask,
+                         cond, cond_lag[li], discrete_x, discrete_y, preprocess, drop_nan,
+                         share_x=False)
+
     if _device_prep_ok((x, y) + (() if cond is None else (cond,)), cond, preprocess, drop_nan,
                        discrete_x or discrete_y, nan_rows_ok=True):
         lo, hi = min(min_lag, 0), max(max_lag, 0)
-        n = len(y) - hi + lo if prep.idx is None else len(prep.idx)
-        specs = []
-        ycol = _native.Col(y[hi:])
-        zcols = {}   # condition columns by lag: shared by the tasks of a lag row
-        for li, vi in indices:
-            xv = x if x.ndim == 1 else x[:, vi]
-            zv = None
-            if cond is not None:
-                zkey = tuple(int(c) for c in cond_lag[li])
-                zv = zcols.get(zkey)
-                if zv is None:
-                    zv = zcols[zkey] = [_native.Col(cond[hi - cond_lag[li][c]:, c])
-                                        for c in range(cond.shape[1])]
-            specs.append((_native.Col(xv[hi - lag[li]:]), ycol, zv))
-        rows = None
-        if drop_nan:
-            rows = _kept_rows(x, y, cond, lag, cond_lag, indices, hi, len(y) - hi + lo, prep.idx,
-                              max_threads)
-        values = _run_device_prep(specs, n, k, prep.idx, jobs, max_threads, rows)
+        n0 = len(y) - hi + lo
+        xc, yc = _native.Columns(x), _native.Columns(y)
+        zc = None if cond is None else _native.Columns(cond)
+        dz = 0 if cond is None else cond.shape[1]
+
+        def addresses():
+            # the lagged views: task (li, vi) starts at row hi - lag of x, hi of
+            # y and hi - cond_lag of each condition column
+            ptr = np.empty((nlag, nvar, 2 + dz), dtype=np.uint64)
+            stride = np.empty((nlag, nvar, 2 + dz), dtype=np.int64)
+            ptr[:, :, 0] = xc.address((hi - np.asarray(lag)).astype(np.int64)[:, None], np.arange(nvar)[None, :])
+            ptr[:, :, 1] = yc.address(hi)
+            stride[:, :, 0], stride[:, :, 1] = xc.row // 8, yc.row // 8
+            if dz:
+                ptr[:, :, 2:] = zc.address((hi - np.asarray(cond_lag)).astype(np.int64),
+                                           np.arange(dz)[None, :])[:, None, :]
+                stride[:, :, 2:] = zc.row // 8
+            return ptr.reshape(nlag * nvar, -1), stride.reshape(nlag * nvar, -1)
+
+        def spec(t):
+            li, vi = divmod(t, nvar)
+            xv = xc.array if x.ndim == 1 else xc.array[:, vi]
+            return (_native.Col(xv[hi - lag[li]:]), _native.Col(yc.array[hi:]),
+                    [_native.Col(zc.array[hi - cond_lag[li][c]:, c]) for c in range(dz)] if dz else None)
+
+        values = _run_device_prep(nlag * nvar, 2 + dz, addresses, spec, n0, k, prep.idx, job, max_threads,
+                                  drop_nan, (xc, yc, zc))
     else:
         batch = _Batch()
+        jobs = [job(t) for t in range(nlag * nvar)]
         slots = [_add_prepared(batch, p) for p in _prepare_all(jobs, max_threads)]
         values = batch.run()[slots]
-    result = np.empty((len(lag), nvar))
-    for (li, vi), v in zip(indices, values):
-        result[li, vi] = v
-        if callback is not None:
-            callback(vi, lag[li])
+    result = np.array(values, dtype=np.float64).reshape(nlag, nvar)
+    if callback is not None:
+        for li in range(nlag):
+            for vi in range(nvar):
+                callback(vi, lag[li])
     return result
 
 
@@ -488,29 +499,46 @@ def _pairwise_mi(data: FloatArray, k: int, cond: Optional[FloatArray], preproces
     cond_lag = np.full(cond.shape[1], 0) if cond is not None else np.asarray(0)
 
     prep = _Prep(mask, 0, 0)
-    pairs = []
-    jobs = []
-    for i in range(nvar):
-        for j in range(i + 1, nvar):
-            pairs.append((i, j))
-            jobs.append(_task_job(prep, ("d", i), data[:, i], ("d", j), data[:, j], 0, 0, 0, k, mask,
-                                  cond, cond_lag, discrete[i], discrete[j], preprocess, drop_nan,
-                                  share_x=True))
-    if pairs and _device_prep_ok((data,) + (() if cond is None else (cond,)), cond, preprocess,
-                                 drop_nan, bool(np.any(discrete))):
-        n = len(data) if prep.idx is None else len(prep.idx)
-        cols = [_native.Col(data[:, i]) for i in range(nvar)]
-        zv = None if cond is None else [_native.Col(cond[:, c]) for c in range(cond.shape[1])]
-        specs = [(cols[i], cols[j], zv) for i, j in pairs]
-        values = _run_device_prep(specs, n, k, prep.idx, jobs, max_threads)
+    first, second = np.triu_indices(nvar, 1)   # (i, j), i < j, row by row
+
+    def job(t):   # the host preparation of pair t
+        i, j = int(first[t]), int(second[t])
+        return _task_job(prep, ("d", i), data[:, i], ("d", j), data[:, j], 0, 0, 0, k, mask,
+                         cond, cond_lag, discrete[i], discrete[j], preprocess, drop_nan,
+                         share_x=True)
+
+    if len(first) and _device_prep_ok((data,) + (() if cond is None else (cond,)), cond, preprocess,
+                                      drop_nan, bool(np.any(discrete))):
+        dc = _native.Columns(data)
+        zc = None if cond is None else _native.Columns(cond)
+        dz = 0 if cond is None else cond.shape[1]
+
+        def addresses():
+            ptr = np.empty((len(first), 2 + dz), dtype=np.uint64)
+            stride = np.empty((len(first), 2 + dz), dtype=np.int64)
+            ptr[:, 0], ptr[:, 1] = dc.address(0, first), dc.address(0, second)
+            stride[:, :2] = dc.row // 8
+            if dz:
+                ptr[:, 2:] = zc.address(0, np.arange(dz))
+                stride[:, 2:] = zc.row // 8
+            return ptr, stride
+
+        def spec(t):
+            return (_native.Col(dc.array[:, first[t]]), _native.Col(dc.array[:, second[t]]),
+                    [_native.Col(zc.array[:, c]) for c in range(dz)] if dz else None)
+
+        values = _run_device_prep(len(first), 2 + dz, addresses, spec, len(data), k, prep.idx, job,
+                                  max_threads, False, (dc, zc))
     else:
         batch = _Batch()
+        jobs = [job(t) for t in range(len(first))]
         slots = [_add_prepared(batch, p) for p in _prepare_all(jobs, max_threads)]
         values = batch.run()[slots] if slots else np.empty(0)
     # the symmetric matrix with a NaN diagonal, assembled on the device
-    result = _native.pairwise_matrix(values, pairs, nvar) if pairs else np.full((nvar, nvar), np.nan)
+    pairs = np.stack((first, second), axis=1)
+    result = _native.pairwise_matrix(values, pairs, nvar) if len(pairs) else np.full((nvar, nvar), np.nan)
     if callback is not None:
-        for i, j in pairs:
+        for i, j in pairs.tolist():
             callback(i, j)
     return result
 
@@ -609,56 +637,54 @@ def _device_prep_ok(arrays, cond, preprocess: bool, drop_nan: bool, any_discrete
     return _numpy_sums_pairwise()
 
 
-def _kept_rows(x, y, cond, lag, cond_lag, indices, hi: int, n0: int, idx, max_threads):
-    """Per task of a lagged estimate_mi with drop_nan: the sample index of
-    the rows it keeps -- the masked rows (idx; None: all n0) whose x, y and
-    condition values in the task's lagged views are all numbers, the rows
-    _apply_masks keeps (_driver.py:834-854) -- or None where that is every
-    masked row (such tasks share the call's index)."""
-    base = None if idx is None else np.asarray(idx, dtype=np.int32)
-    cols = lambda a: [a] if a.ndim == 1 else [a[:, c] for c in range(a.shape[1])]
-    fin_x = [~np.isnan(c) for c in cols(x)]
-    fin_y = ~np.isnan(y[hi: hi + n0])
-    fin_z = [] if cond is None else [~np.isnan(c) for c in cols(cond)]
-
-    def one(li, vi):
-        keep = fin_x[vi][hi - lag[li]: hi - lag[li] + n0] & fin_y
-        for c, fz in enumerate(fin_z):
-            keep &= fz[hi - cond_lag[li][c]: hi - cond_lag[li][c] + n0]
-        if base is not None:
-            keep = keep[base]
-        if keep.all():
-            return None
-        return base[keep] if base is not None else np.flatnonzero(keep).astype(np.int32)
-
-    jobs = [lambda li=li, vi=vi: one(li, vi) for li, vi in indices]
-    return _prepare_all(jobs, max_threads)
-
-
-def _run_device_prep(specs, n: int, k: int, idx, jobs, max_threads, rows=None) -> np.ndarray:
-    """Estimates of the tasks (x, y, condition columns or None): the columns
-    are lagged views of the caller's arrays, sample w at view[idx[w]] (idx
-    None: the first n), rescaled on the device.  rows: per task, its own
-    sample index (drop_nan) or None for idx.  Tasks with a constant column
-    are prepared on the host (`jobs`, same order) and run in a second batch."""
+def _run_device_prep(nt: int, nc: int, addresses, spec, n0: int, k: int, idx, job, max_threads,
+                     drop_nan: bool, keep) -> np.ndarray:
+    """Estimates of nt tasks of nc columns (x, y, then the condition): lagged
+    views of the caller's arrays, sample w at view[idx[w]] (idx None: the first
+    n0), rescaled on the device.  spec(t): the views of task t; addresses():
+    the first addresses and strides of all, (nt, nc) each, of the arrays that
+    `keep` holds.  With drop_nan every task keeps the masked rows whose
+    values are all numbers, the rows _apply_masks keeps (_driver.py:834-854).
+    Tasks with a constant column are prepared on the host (job(t)) and run in a
+    second batch."""
     index = None if idx is None else np.ascontiguousarray(idx, dtype=np.int32)
-    tasks = []
-    for t, (xv, yv, zv) in enumerate(specs):
+    most = n0 if index is None else len(index)
+    if nt and most <= k:
+        raise ValueError(K_TOO_LARGE_MSG)
+    few = nt < 4 and not drop_nan   # filling a table costs as much as four task objects
+    ptr, stride = (None, None) if few else addresses()
+    n = np.full(nt, most, dtype=np.int64)
+    rows = None      # per task: its own sample index, or None for the shared one
+    table_index = index
+    if drop_nan:
+        threads = max_threads if max_threads is not None else min(16, os.cpu_count() or 1)
+        kept, n = _native.kept_rows(ptr, stride, n0, index, threads)
+        if (n < most).any():
+            rows = [None if n[t] == most else kept[t, :n[t]] for t in range(nt)]
+            shared = 0 if index is None else index.ctypes.data
+            table_index = kept.ctypes.data + np.arange(nt, dtype=np.uint64) * np.uint64(kept.strides[0])
+            table_index[n == most] = shared
+            keep = keep + (kept,)
+    if (n <= k).any():
+        raise ValueError(K_TOO_LARGE_MSG)
+
+    kind = _native.MI if nc == 2 else _native.CMI
+
+    def make(t):
+        xv, yv, zv = spec(t)
         own = None if rows is None else rows[t]
-        tn, tix = (n, index) if own is None else (len(own), own)
-        if tn <= k:  # the first task in order that keeps too few rows raises
-            raise ValueError(K_TOO_LARGE_MSG)
-        if zv is None:
-            tasks.append(_native.Task(_native.MI, k, [xv], [yv], n=tn, index=tix))
-        else:
-            tasks.append(_native.Task(_native.CMI, k, [xv], [yv], list(zv), n=tn, index=tix))
+        return _native.Task(kind, k, [xv], [yv], [] if zv is None else list(zv), n=int(n[t]),
+                            index=index if own is None else own)
+
+    tasks = [make(t) for t in range(nt)] if few else \
+        _native.TaskTable(kind, k, nc - 2, ptr, stride, n, table_index, make, keep + (index,))
     res = []
     values = _native.run_tasks(tasks, flags=run_flags | _native.RESCALE, results_out=res,
                                noise=lambda m: _noise.take(0, (m,)))
     redo = [i for i, r in enumerate(res) if r.status == _native.TASK_CONSTANT]
     if redo:
         batch = _Batch()
-        slots = [_add_prepared(batch, p) for p in _prepare_all([jobs[i] for i in redo], max_threads)]
+        slots = [_add_prepared(batch, p) for p in _prepare_all([job(i) for i in redo], max_threads)]
         again = batch.run()
         for i, s in zip(redo, slots):
             values[i] = again[s]

@@ -15,6 +15,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+from collections.abc import Sequence as _SequenceABC
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
@@ -69,6 +70,15 @@ class EgbTask(ctypes.Structure):
                 ("nclass", ctypes.c_int32), ("cols", ctypes.POINTER(EgbColumn)),
                 ("labels", ctypes.POINTER(ctypes.c_int32)),
                 ("index", ctypes.POINTER(ctypes.c_int32))]
+
+
+# The same layouts as NumPy records, filled column-wise for long batches.
+_COL_DTYPE = np.dtype([("data", np.uint64), ("stride", np.int64)])
+_TASK_DTYPE = np.dtype([("kind", np.int32), ("k", np.int32), ("n", np.int64), ("dx", np.int32),
+                        ("dy", np.int32), ("dz", np.int32), ("nclass", np.int32),
+                        ("cols", np.uint64), ("labels", np.uint64), ("index", np.uint64)])
+_RESULT_DTYPE = np.dtype([("value", np.float64), ("term_sum", np.float64),
+                          ("zero_mask", np.uint32), ("status", np.int32)])
 
 
 class EgbResult(ctypes.Structure):
@@ -132,6 +142,8 @@ def load():
         lib.egb_pairwise_matrix.restype = ctypes.c_int
         lib.egb_normalize.argtypes = [vp, vp, i64, i32, vp]
         lib.egb_normalize.restype = ctypes.c_int
+        lib.egb_kept_rows.argtypes = [i32, i32, vp, vp, i64, vp, i64, i32, vp, vp]
+        lib.egb_kept_rows.restype = ctypes.c_int
         lib.egb_debug_inject_device_error.argtypes = [vp, ctypes.c_uint32]
         lib.egb_debug_inject_device_error.restype = ctypes.c_int
         lib.egb_debug_divide.argtypes = [vp, vp, vp, ctypes.c_int64, vp]
@@ -299,14 +311,107 @@ class Col:
         self.length = int(ref.shape[0])
 
 
+class Columns:
+    """The columns of a float64 array resolved once: address of element (0, c)
+    and strides in bytes.  Arrays whose rows the library cannot step through
+    (stride not a positive multiple of 8, unaligned) are copied."""
+
+    __slots__ = ("array", "ptr", "row", "col")
+
+    def __init__(self, a: np.ndarray):
+        if a.strides[0] <= 0 or a.strides[0] % 8 or not a.flags.aligned:
+            a = np.ascontiguousarray(a)
+        self.array, self.ptr, self.row = a, a.ctypes.data, a.strides[0]
+        self.col = a.strides[1] if a.ndim > 1 else 0
+
+    def address(self, row, col=0):
+        """Address of element (row, col); arrays of either give arrays."""
+        return self.ptr + row * self.row + col * self.col
+
+
+class TaskTable(_SequenceABC):
+    """Tasks of one estimator whose columns are views of a few host arrays, as
+    arrays of addresses: what a lagged estimate_mi or a pairwise_mi call has
+    hundreds of.  ptr, stride (elements): (tasks, columns), x first, then y,
+    then z; n: samples per task; index: int32 sample positions shared by all
+    tasks, an array of addresses per task (0: none), or None.  Indexing gives
+    the equivalent :class:`Task` (make(i))."""
+
+    def __init__(self, kind: int, k: int, dz: int, ptr, stride, n, index, make, keep):
+        self.kind, self.k, self.dz = kind, k, dz
+        self.ptr, self.stride, self.n, self.index = ptr, stride, n, index
+        self.make, self.keep = make, keep
+
+    def __len__(self) -> int:
+        return len(self.n)
+
+    def __getitem__(self, i):
+        if isinstance(i, slice):
+            return [self.make(j) for j in range(*i.indices(len(self)))]
+        if not -len(self) <= i < len(self):
+            raise IndexError(i)
+        return self.make(i % len(self))
+
+
+def kept_rows(ptr, stride, n0: int, base, threads: int):
+    """Per task (a row of ptr / stride): the rows of 0..n0-1, or of the int32
+    array `base`, whose values are numbers in every column.  Returns (rows
+    (tasks, most), counts)."""
+    nt, nc = ptr.shape
+    most = n0 if base is None else len(base)
+    rows = np.empty((nt, most), dtype=np.int32)
+    counts = np.empty(nt, dtype=np.int64)
+    ptr = np.ascontiguousarray(ptr, dtype=np.uint64)
+    stride = np.ascontiguousarray(stride, dtype=np.int64)
+    rc = load().egb_kept_rows(nt, nc, ptr.ctypes.data, stride.ctypes.data, n0,
+                              None if base is None else base.ctypes.data, most, int(threads),
+                              rows.ctypes.data, counts.ctypes.data)
+    if rc != 0:
+        raise RuntimeError(f"egb_kept_rows failed ({rc})")
+    return rows, counts
+
+
 def _length(col) -> int:
     return col.length if type(col) is Col else len(col)
+
+
+def _ensure_noise(ctx: Context, need: int, noise) -> None:
+    if ctx.noise_len < need:
+        if noise is None:
+            raise ValueError("RESCALE needs the noise stream")
+        ctx.set_noise(noise(max(need, 2 * ctx.noise_len)))
+
+
+def _run_table(ctx: Context, table: TaskTable, flags: int, results_out, noise) -> np.ndarray:
+    """run_tasks of a TaskTable.  results_out receives the results only when
+    some status is not 0 (in order, one per task)."""
+    nt, nc = table.ptr.shape
+    if flags & RESCALE:
+        _ensure_noise(ctx, int(table.n.max()) * nc, noise)
+    cols = np.empty((nt, nc), dtype=_COL_DTYPE)
+    cols["data"], cols["stride"] = table.ptr, table.stride
+    tasks = np.zeros(nt, dtype=_TASK_DTYPE)
+    tasks["kind"], tasks["k"], tasks["n"] = table.kind, table.k, table.n
+    tasks["dx"] = tasks["dy"] = 1
+    tasks["dz"] = table.dz
+    tasks["cols"] = cols.ctypes.data + np.arange(nt, dtype=np.uint64) * np.uint64(cols.strides[0])
+    if table.index is not None:
+        tasks["index"] = table.index.ctypes.data if table.index.dtype == np.int32 else table.index
+    res = np.empty(nt, dtype=_RESULT_DTYPE)
+    with ctx.lock:
+        rc = ctx.lib.egb_run_batch(ctx.h, ctypes.cast(tasks.ctypes.data, ctypes.POINTER(EgbTask)), nt,
+                                   flags, ctypes.cast(res.ctypes.data, ctypes.POINTER(EgbResult)))
+        ctx.check(rc, "egb_run_batch")
+    if results_out is not None and res["status"].any():
+        results_out.extend((EgbResult * nt).from_buffer(res))
+    return res["value"].copy()
 
 
 def run_tasks(tasks: List[Task], flags: int = 0, device: int = 0,
               results_out: Optional[list] = None, noise=None,
               groups_out: Optional[dict] = None) -> np.ndarray:
-    """Evaluate the tasks in one batched call; returns the estimates.
+    """Evaluate the tasks (a list, or a TaskTable) in one batched call; returns
+    the estimates.
 
     groups_out (a dict) receives, for each task of a discrete kind, the six
     distinct-value figures of egb_last_groups under the task's index.
@@ -317,12 +422,11 @@ def run_tasks(tasks: List[Task], flags: int = 0, device: int = 0,
     if not tasks:
         return np.empty(0)
     ctx = context(device)
+    if isinstance(tasks, TaskTable):
+        return _run_table(ctx, tasks, flags, results_out, noise)
     if flags & RESCALE:
         need = max((t.n or _length(t.x[0])) * (len(t.x) + len(t.y) + len(t.z)) for t in tasks)
-        if ctx.noise_len < need:
-            if noise is None:
-                raise ValueError("RESCALE needs the noise stream")
-            ctx.set_noise(noise(max(need, 2 * ctx.noise_len)))
+        _ensure_noise(ctx, need, noise)
     is_dev = bool(flags & INPUT_DEVICE)
     ctasks = (EgbTask * len(tasks))()
     keep = []

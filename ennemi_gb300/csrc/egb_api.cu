@@ -36,7 +36,10 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <tuple>
+#include <unordered_map>
 #include <vector>
 
 #include "egb_internal.cuh"
@@ -103,6 +106,29 @@ struct TaskPlan {
   size_t tab_perm = 0;            // offset of perm inside the table blob
   size_t tab_rad = 0;             // KIND_COUNT_ONLY: caller radii (host input)
   int center0 = 0;                // first column of the task in the centre array
+};
+
+// What makes two working columns the same bits: the caller's column, the
+// sample index, the length and how it is rescaled.
+struct ColKey {
+  uintptr_t data;
+  int64_t stride;
+  uintptr_t index;
+  int64_t n, noise_pos;
+  int32_t group;
+  bool operator==(const ColKey& o) const {
+    return data == o.data && stride == o.stride && index == o.index && n == o.n &&
+           noise_pos == o.noise_pos && group == o.group;
+  }
+};
+struct ColKeyHash {
+  size_t operator()(const ColKey& k) const {
+    uint64_t h = 0;
+    for (uint64_t v : {(uint64_t)k.data, (uint64_t)k.stride, (uint64_t)k.index, (uint64_t)k.n,
+                       (uint64_t)k.noise_pos, (uint64_t)k.group})
+      h = (h ^ v) * 0x9e3779b97f4a7c15ull, h ^= h >> 29;
+    return (size_t)h;
+  }
 };
 
 // A sort segment: a range of one working column, named by the column's
@@ -707,7 +733,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   for (int t = 0; t < ntasks; ++t) {
     const egb_task& T = tasks[t];
     TaskPlan& p = P[(size_t)t];
-    const std::string who = "task " + std::to_string(t) + ": ";
+    auto who = [&] { return "task " + std::to_string(t) + ": "; };
     p.kind = T.kind;
     p.k = T.k;
     p.n = T.n;
@@ -717,42 +743,43 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     p.ncol = T.dx + T.dy + T.dz;
     const bool internal = T.kind == KIND_KNN_ONLY || T.kind == KIND_COUNT_ONLY;
     if (!(T.kind >= EGB_MI && T.kind <= EGB_DISCRETE_CMI) && !internal)
-      return fail(ctx, EGB_ERR_ARG, who + "unknown estimator kind");
-    if (T.n < 1 || T.n > (int64_t)0x3fffffff) return fail(ctx, EGB_ERR_ARG, who + "n out of range");
-    if (T.k < 1 && T.kind != KIND_COUNT_ONLY) return fail(ctx, EGB_ERR_ARG, who + "k must be greater than zero");
+      return fail(ctx, EGB_ERR_ARG, who() + "unknown estimator kind");
+    if (T.n < 1 || T.n > (int64_t)0x3fffffff) return fail(ctx, EGB_ERR_ARG, who() + "n out of range");
+    if (T.k < 1 && T.kind != KIND_COUNT_ONLY) return fail(ctx, EGB_ERR_ARG, who() + "k must be greater than zero");
     if (T.dx < 1 || T.dy < 0 || T.dz < 0 || p.ncol > EGB_DMAX)
-      return fail(ctx, EGB_ERR_ARG, who + "column counts out of range (at most 32 columns)");
+      return fail(ctx, EGB_ERR_ARG, who() + "column counts out of range (at most 32 columns)");
     const bool needs_y = T.kind == EGB_MI || T.kind == EGB_CMI || T.kind == EGB_DISCRETE_MI ||
                          T.kind == EGB_DISCRETE_CMI;
     const bool needs_z = T.kind == EGB_CMI || T.kind == EGB_CSEMI || T.kind == EGB_DISCRETE_CMI;
     if ((needs_y != (T.dy > 0)) || (needs_z != (T.dz > 0)))
-      return fail(ctx, EGB_ERR_ARG, who + "column counts do not match the estimator kind");
-    if (!T.cols) return fail(ctx, EGB_ERR_ARG, who + "null column list");
+      return fail(ctx, EGB_ERR_ARG, who() + "column counts do not match the estimator kind");
+    if (!T.cols) return fail(ctx, EGB_ERR_ARG, who() + "null column list");
     for (int c = 0; c < p.ncol; ++c)
       if (!T.cols[c].data || T.cols[c].stride < 1)
-        return fail(ctx, EGB_ERR_ARG, who + "invalid column " + std::to_string(c));
+        return fail(ctx, EGB_ERR_ARG, who() + "invalid column " + std::to_string(c));
     p.src_len = T.n;
     if (T.index) {
-      if (internal) return fail(ctx, EGB_ERR_ARG, who + "index not supported for this kind");
+      if (internal) return fail(ctx, EGB_ERR_ARG, who() + "index not supported for this kind");
       auto it = index_max.find({T.index, T.n});
       if (it == index_max.end()) {
-        int64_t mx = -1;
+        int32_t mx = -1, mn = 0;
         for (int64_t i = 0; i < T.n; ++i) {
-          if (T.index[i] < 0) return fail(ctx, EGB_ERR_ARG, who + "negative sample index");
-          mx = std::max<int64_t>(mx, T.index[i]);
+          mx = std::max(mx, T.index[i]);
+          mn = std::min(mn, T.index[i]);
         }
-        it = index_max.emplace(std::make_pair(T.index, T.n), mx).first;
+        if (mn < 0) return fail(ctx, EGB_ERR_ARG, who() + "negative sample index");
+        it = index_max.emplace(std::make_pair(T.index, T.n), (int64_t)mx).first;
       }
       p.src_len = it->second + 1;
       p.index = T.index;
     }
     if (rescale && T.kind >= EGB_MI && T.kind <= EGB_CSEMI) {
-      if (internal) return fail(ctx, EGB_ERR_ARG, who + "EGB_RESCALE applies to estimator tasks only");
+      if (internal) return fail(ctx, EGB_ERR_ARG, who() + "EGB_RESCALE applies to estimator tasks only");
       if (T.dx != 1 || T.dy > 1)
-        return fail(ctx, EGB_ERR_ARG, who + "EGB_RESCALE needs one x column and at most one y column");
+        return fail(ctx, EGB_ERR_ARG, who() + "EGB_RESCALE needs one x column and at most one y column");
       const int64_t draws = T.n * (int64_t)(T.dx + T.dy + T.dz);
       if (!ctx->noise_d || draws > ctx->noise_len)
-        return fail(ctx, EGB_ERR_ARG, who + "EGB_RESCALE needs " + std::to_string(draws) +
+        return fail(ctx, EGB_ERR_ARG, who() + "EGB_RESCALE needs " + std::to_string(draws) +
                                           " noise values (egb_set_noise)");
     }
     p.K = T.k + 1;
@@ -766,12 +793,12 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
               : T.kind == EGB_MI ? 2 : (T.kind == EGB_CMI || T.kind == EGB_CSEMI) ? 3
               : (T.kind == EGB_SEMI || T.kind == KIND_COUNT_ONLY) ? 1 : 0;
     if (T.kind == EGB_SEMI || T.kind == EGB_CSEMI) {
-      if (!T.labels || T.nclass < 1) return fail(ctx, EGB_ERR_ARG, who + "labels required");
+      if (!T.labels || T.nclass < 1) return fail(ctx, EGB_ERR_ARG, who() + "labels required");
       p.nclass = T.nclass;
       std::vector<int64_t> cnt((size_t)T.nclass + 1, 0);
       for (int64_t i = 0; i < T.n; ++i) {
         const int32_t c = T.labels[i];
-        if (c < 0 || c >= T.nclass) return fail(ctx, EGB_ERR_ARG, who + "label out of range");
+        if (c < 0 || c >= T.nclass) return fail(ctx, EGB_ERR_ARG, who() + "label out of range");
         ++cnt[(size_t)c + 1];
       }
       p.cls_off.assign((size_t)T.nclass + 1, 0);
@@ -858,7 +885,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   // lagged estimate_mi, every column of a pairwise_mi, a shared condition.
   std::vector<std::vector<int>> colid((size_t)ntasks);
   {
-    std::map<std::tuple<uintptr_t, int64_t, uintptr_t, int64_t, int64_t, int>, int> ids;
+    std::unordered_map<ColKey, int, ColKeyHash> ids;
     int next_id = 0;
     for (int t = 0; t < ntasks; ++t) {
       const TaskPlan& p = P[(size_t)t];
@@ -872,8 +899,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
         const int zc = c - p.dx - p.dy;
         const int64_t noise_pos = !resc ? -1 : zc >= 0 ? (int64_t)(p.dx + p.dy) * p.n + zc : (int64_t)c * p.n;
         const int group = !resc ? 0 : (zc >= 0 && p.dz > 1 ? p.dz : 1);
-        const auto key = std::make_tuple((uintptr_t)tasks[t].cols[c].data, tasks[t].cols[c].stride,
-                                         (uintptr_t)p.index, p.n, noise_pos, group);
+        const ColKey key{(uintptr_t)tasks[t].cols[c].data, tasks[t].cols[c].stride, (uintptr_t)p.index,
+                         p.n, noise_pos, group};
         auto it = ids.find(key);
         if (it == ids.end()) it = ids.emplace(key, next_id++).first;
         colid[(size_t)t][(size_t)c] = it->second;
@@ -1496,7 +1523,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     std::map<int64_t, int32_t> tree_of;
     // a column read through the same pointer, stride and sample index (and
     // summed the same way) has the same statistics in every task
-    std::map<std::tuple<uintptr_t, int64_t, uintptr_t, int64_t, int>, int32_t> stat_of;
+    std::unordered_map<ColKey, int32_t, ColKeyHash> stat_of;
     size_t scratch_elems = 0;
     for (int t = 0; t < ntasks; ++t) {
       const TaskPlan& p = P[(size_t)t];
@@ -1519,8 +1546,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
         const int zc = c - p.dx - p.dy;  // condition column, or negative
         rc.group = zc >= 0 && p.dz > 1 ? p.dz : 1;
         rc.noise_pos = zc >= 0 ? (int64_t)(p.dx + p.dy) * p.n + zc : (int64_t)c * p.n;
-        const auto key = std::make_tuple((uintptr_t)tasks[t].cols[c].data, tasks[t].cols[c].stride,
-                                         (uintptr_t)p.index, p.n, rc.group);
+        const ColKey key{(uintptr_t)tasks[t].cols[c].data, tasks[t].cols[c].stride, (uintptr_t)p.index,
+                         p.n, 0, rc.group};
         const bool ordered = !p.perm.empty();  // its own class order: not shared
         auto f = ordered ? stat_of.end() : stat_of.find(key);
         if (f == stat_of.end()) {
@@ -1566,10 +1593,17 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   const size_t tab_rcols = tl.take(sizeof(RescaleCol) * std::max<size_t>(rcols.size(), 1));
   const size_t tab_rstats = tl.take(sizeof(RescaleStat) * std::max<size_t>(rstats.size(), 1));
   const size_t tab_rinv = tl.take(sizeof(int32_t) * std::max<size_t>(rinv.size(), 1));
-  // shared sample indices: one copy per (array, n)
+  // shared sample indices: one copy per (array, n); an index that few columns
+  // read is read where it is
   std::map<std::pair<const int32_t*, int64_t>, size_t> index_tab;
+  std::unordered_map<const int32_t*, int> index_cols;
+  for (const TaskPlan& p : P)
+    if (p.index) index_cols[p.index] += p.ncol;
+  auto index_in_place = [&](const TaskPlan& p) {
+    return ctx->host_direct && !(flags & (EGB_STAGE_HOST | EGB_GRAPH)) && index_cols[p.index] <= 4;
+  };
   for (TaskPlan& p : P) {
-    if (!p.index) continue;
+    if (!p.index || index_in_place(p)) continue;
     auto it = index_tab.find({p.index, p.n});
     if (it == index_tab.end())
       it = index_tab.emplace(std::make_pair(p.index, p.n), tl.take(sizeof(int32_t) * (size_t)p.n)).first;
@@ -1639,7 +1673,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     D.ncol = p.ncol;
     D.rad_given = p.kind == KIND_COUNT_ONLY ? 1 : 0;
     const std::vector<int32_t>& gp = p.gperm.empty() ? p.perm : p.gperm;
-    const int32_t* perm_dev = p.index ? (const int32_t*)(A + off_tab + p.tab_index)
+    const int32_t* perm_dev = p.index ? (index_in_place(p) ? p.index
+                                                           : (const int32_t*)(A + off_tab + p.tab_index))
                               : gp.empty() ? nullptr : (const int32_t*)(A + off_tab + p.tab_perm);
     if (!gp.empty()) std::memcpy(H + p.tab_perm, gp.data(), sizeof(int32_t) * gp.size());
     if (p.kind == KIND_COUNT_ONLY && !dev_in)
@@ -2492,6 +2527,43 @@ int egb_last_groups(const egb_ctx* ctx, int32_t task, int64_t* out, int32_t max)
   const int n = std::min(max, 6);
   for (int i = 0; i < n; ++i) out[i] = ctx->groups[(size_t)task][(size_t)i];
   return n;
+}
+
+int egb_kept_rows(int32_t ntasks, int32_t ncol, const double* const* data, const int64_t* stride,
+                  int64_t n0, const int32_t* base, int64_t nrows, int32_t threads, int32_t* rows,
+                  int64_t* counts) {
+  if (ntasks < 0 || ncol < 1 || n0 < 0 || nrows < 0 || (!base && nrows != n0) ||
+      (ntasks > 0 && (!data || !stride || !rows || !counts)))
+    return EGB_ERR_ARG;
+  auto one = [&](int32_t t) {
+    const double* const* d = data + (size_t)t * ncol;
+    const int64_t* st = stride + (size_t)t * ncol;
+    int32_t* out = rows + (size_t)t * nrows;
+    int64_t m = 0;
+    for (int64_t i = 0; i < nrows; ++i) {
+      const int64_t r = base ? base[i] : i;
+      bool ok = true;
+      for (int32_t c = 0; c < ncol; ++c) ok &= !std::isnan(d[c][r * st[c]]);
+      out[m] = (int32_t)r;  // overwritten by the next row unless kept
+      m += ok;
+    }
+    counts[t] = m;
+  };
+  // about a quarter of a million values a thread
+  const int64_t want = std::min<int64_t>({(int64_t)threads, (int64_t)ntasks,
+                                          (int64_t)ntasks * nrows * ncol / 250000 + 1});
+  std::atomic<int32_t> next{0};
+  auto work = [&]() {
+    for (int32_t t; (t = next.fetch_add(1)) < ntasks;) one(t);
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (int64_t w = 1; w < want; ++w) pool.emplace_back(work);
+  } catch (const std::system_error&) {  // fewer threads then
+  }
+  work();
+  for (std::thread& th : pool) th.join();
+  return EGB_OK;
 }
 
 int egb_debug_inject_device_error(egb_ctx* ctx, uint32_t word) {

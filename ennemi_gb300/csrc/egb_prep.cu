@@ -527,9 +527,9 @@ __device__ __forceinline__ void chunk_sum(int cnt, F term, double* out) {
 // CL blocks (a cluster) share a chunk of COMBINE_CHUNK samples: each evaluates
 // 1 / CL of its terms and leaves them in the first block's shared memory,
 // which adds them -- the same order, so the same bits, for every CL.  CL = 8
-// while chunks are fewer than the SMs (the loads, or an entropy's FP64
-// logarithms, are then the time): 3 chunks of an MI 11.6 -> 6 us, 49 of an
-// entropy 41 -> 10 us; CL = 1 where they fill the GPU.
+// while chunks are fewer than a third of the SMs (the loads, or an entropy's
+// FP64 logarithms, are then the time): 3 chunks of an MI 11.6 -> 6 us, 49 of an
+// entropy 41 -> 21 us; CL = 1 beyond (125 chunks: 25 us against 31).
 template <int CL>
 __global__ void __launch_bounds__(COMBINE_THREADS)
 combine_kernel(const TaskDev* __restrict__ tasks, const CombineJob* __restrict__ jobs,
@@ -697,7 +697,7 @@ void launch_combine(const TaskDev* tasks_d, const CombineJob* jobs_d, const int3
                     int nchunks, const double* psi_tab, int64_t psi_len, double* partial,
                     uint32_t* zero_flags, uint32_t* err, int num_sms, cudaStream_t st) {
   if (nchunks <= 0) return;
-  if (nchunks >= num_sms) {
+  if (3 * nchunks >= num_sms) {
     combine_kernel<1><<<nchunks, COMBINE_THREADS, 0, st>>>(tasks_d, jobs_d, chunk_job_d, psi_tab,
                                                            psi_len, partial, zero_flags, err);
   } else {

@@ -373,6 +373,19 @@ int egb_normalize(egb_ctx* ctx, const double* mi, int64_t n, int32_t flags, doub
 int egb_last_groups(const egb_ctx* ctx, int32_t task, int64_t* out, int32_t max);
 
 /*
+ * Host only (no context, no device): the rows that each task of a lagged call
+ * keeps when rows with NaNs are dropped, as _apply_masks of the reference
+ * (_driver.py:834-854).  Column c of task t is data[t * ncol + c] with element
+ * stride stride[t * ncol + c]; row r is kept when every column's value there
+ * is a number.  Candidate rows are base[0 .. nrows) (each in [0, n0)), or 0 ..
+ * n0 - 1 with base null and nrows = n0.  Task t's rows go to rows[t * nrows],
+ * their number to counts[t].  At most `threads` host threads.
+ */
+int egb_kept_rows(int32_t ntasks, int32_t ncol, const double* const* data, const int64_t* stride,
+                  int64_t n0, const int32_t* base, int64_t nrows, int32_t threads, int32_t* rows,
+                  int64_t* counts);
+
+/*
  * Test hook for the device-error path: the next egb_run_batch on this context
  * starts with `word` already in its device error word, as though one of its
  * kernels had reported it (bit 0: a bounded wait gave up; bit 1: an index

@@ -357,3 +357,23 @@ def test_device_preprocessing_columns_are_the_reference_slices(monkeypatch, case
         assert kind == (_native.CMI if dz else _native.MI)
         for got, r in zip(cols, ref):
             assert np.array_equal(got.view(np.uint64), np.ascontiguousarray(r).view(np.uint64))
+
+
+@pytest.mark.parametrize("n,share,threads", [(1, 0.0, 1), (7, 1.0, 2), (4099, 0.1, 1), (60_001, 0.02, 4)])
+def test_kept_rows_are_the_rows_without_nans(n, share, threads):
+    """egb_kept_rows against NumPy: strided views, a base of rows, tasks that
+    keep everything or nothing, and more than one host thread."""
+    rng = np.random.default_rng(n)
+    a = rng.normal(size=(n + 3, 3))
+    a[rng.random(a.shape) < share] = np.nan
+    y = rng.normal(size=n + 3)
+    ac, yc = _native.Columns(a), _native.Columns(y)
+    views = [(a[lag:, c], y[1:], lag, c) for lag in (0, 3) for c in range(3)]
+    ptr = np.array([[ac.address(lag, c), yc.address(1)] for _, _, lag, c in views], dtype=np.uint64)
+    stride = np.tile(np.array([3, 1], dtype=np.int64), (len(views), 1))
+    for base in (None, np.flatnonzero(rng.random(n) < 0.7).astype(np.int32)):
+        rows, counts = _native.kept_rows(ptr, stride, n, base, threads)
+        for t, (u, v, _, _) in enumerate(views):
+            r = np.arange(n) if base is None else base
+            want = r[~(np.isnan(u[r]) | np.isnan(v[r]))]
+            assert counts[t] == len(want) and np.array_equal(rows[t, :counts[t]], want)
