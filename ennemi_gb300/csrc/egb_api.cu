@@ -105,7 +105,9 @@ struct TaskPlan {
   size_t off_x64 = 0, off_eps = 0, off_rad = 0, off_cnt[4] = {0, 0, 0, 0};
   size_t tab_perm = 0;            // offset of perm inside the table blob
   size_t tab_rad = 0;             // KIND_COUNT_ONLY: caller radii (host input)
-  int center0 = 0;                // first column of the task in the centre array
+  int center0 = 0;                // first column of the task in the per-column tables
+  std::vector<int> slot;          // general path: the batch column of each column,
+  std::vector<size_t> off_col;    // and its arena offset
 };
 
 // What makes two working columns the same bits: the caller's column, the
@@ -161,6 +163,7 @@ struct ReplayState {
   std::vector<CombineJob> cjobs;
   std::vector<GroupStat> groups;
   size_t pin_rb = 0, pin_zr = 0, zr_stats = 0, zr_err = 0, zr_zero = 0, zr_groups = 0, zr_warn = 0;
+  size_t zr_const = 0;   // per batch column: constant under EGB_RESCALE
   std::vector<std::pair<int, int>> group_of;  // per group job: (task, slot)
   std::vector<int> warn_of;                   // per level check: its task
   size_t tab_bytes = 0, zr_bytes = 0;
@@ -334,6 +337,7 @@ int finish_batch(egb_ctx* ctx, const ReplayState& R, const char* H, int64_t laun
   }
   const double* partial = (const double*)(H + R.pin_rb);
   const uint32_t* zf = (const uint32_t*)(H + R.pin_zr + R.zr_zero);
+  const uint32_t* cf = (const uint32_t*)(H + R.pin_zr + R.zr_const);
   const double INF = HUGE_VAL;
   int ci = 0;
   for (size_t t = 0; t < R.P.size(); ++t) {
@@ -348,7 +352,9 @@ int finish_batch(egb_ctx* ctx, const ReplayState& R, const char* H, int64_t laun
     double S = 0.0;
     for (int i = 0; i < c.nchunk; ++i) S += partial[c.chunk0 + i];
     const uint32_t z = zf[t] & ~RESCALE_CONSTANT;
-    if (zf[t] & RESCALE_CONSTANT) {  // the caller preprocesses this task itself
+    bool constant = (zf[t] & RESCALE_CONSTANT) != 0;
+    for (int sl : p.slot) constant |= cf[sl] != 0;
+    if (constant) {  // the caller preprocesses this task itself
       r.value = NAN;
       r.status = EGB_TASK_CONSTANT;
       if (results) results[t] = r;
@@ -610,7 +616,6 @@ int run_direct(egb_ctx* ctx, const egb_task* tasks, std::vector<TaskPlan>& P, in
       }
       TaskDev& V = tdev[t];
       std::memset(&V, 0, sizeof(V));
-      V.x64 = D.x64;
       V.eps = D.eps;
       for (int s = 0; s < 3; ++s) V.cnt[s] = D.cnt[s];
       V.ld = p.ld;
@@ -881,19 +886,21 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   // the same caller column (pointer, stride), the same sample index and
   // length, in sample order (no class order), with the same preprocessing
   // (EGB_RESCALE: the same noise positions; statistics depend on the rest):
-  // such columns share one sort segment -- the y column of every task of a
-  // lagged estimate_mi, every column of a pairwise_mi, a shared condition.
-  std::vector<std::vector<int>> colid((size_t)ntasks);
+  // the y column of every task of a lagged estimate_mi, every column of a
+  // pairwise_mi, a shared condition.
+  // Each is one batch column: gathered, rescaled, ranged and sorted once.
+  struct SlotPlan { int task, col; size_t off; };
+  std::vector<SlotPlan> slots;
   {
     std::unordered_map<ColKey, int, ColKeyHash> ids;
-    int next_id = 0;
     for (int t = 0; t < ntasks; ++t) {
-      const TaskPlan& p = P[(size_t)t];
-      colid[(size_t)t].resize((size_t)p.ncol);
+      TaskPlan& p = P[(size_t)t];
+      p.slot.resize((size_t)p.ncol);
       const bool resc = rescale && p.kind >= EGB_MI && p.kind <= EGB_CSEMI;
       for (int c = 0; c < p.ncol; ++c) {
         if (!p.perm.empty()) {  // class-ordered working columns are the task's own
-          colid[(size_t)t][(size_t)c] = next_id++;
+          p.slot[(size_t)c] = (int)slots.size();
+          slots.push_back({t, c, 0});
           continue;
         }
         const int zc = c - p.dx - p.dy;
@@ -902,20 +909,23 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
         const ColKey key{(uintptr_t)tasks[t].cols[c].data, tasks[t].cols[c].stride, (uintptr_t)p.index,
                          p.n, noise_pos, group};
         auto it = ids.find(key);
-        if (it == ids.end()) it = ids.emplace(key, next_id++).first;
-        colid[(size_t)t][(size_t)c] = it->second;
+        if (it == ids.end()) {
+          it = ids.emplace(key, (int)slots.size()).first;
+          slots.push_back({t, c, 0});
+        }
+        p.slot[(size_t)c] = it->second;
       }
     }
   }
   std::map<SegKey, int> seg_index;
   std::vector<SortSeg> segs;
   auto seg_for = [&](int task, int col, int64_t b, int64_t e) {
-    const SegKey key{colid[(size_t)task][(size_t)col], b, e};
+    const int slot = P[(size_t)task].slot[(size_t)col];
+    const SegKey key{slot, b, e};
     auto it = seg_index.find(key);
     if (it != seg_index.end()) return it->second;
     SortSeg s{};
-    s.task = task;
-    s.col = col;
+    s.slot = slot;
     s.src_begin = (int32_t)b;
     s.len = (int32_t)(e - b);
     const int id = (int)segs.size();
@@ -1082,16 +1092,19 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
 
   for (int t = 0; t < ntasks; ++t) {
     TaskPlan& p = P[(size_t)t];
-    p.off_x64 = dl.take(sizeof(double) * (size_t)(p.ncol * p.ld));
     p.off_eps = dl.take(sizeof(double) * (size_t)p.ld);
-    p.off_rad = dl.take(sizeof(double) * (size_t)p.ld);
+    if (p.kind == KIND_COUNT_ONLY) p.off_rad = dl.take(sizeof(double) * (size_t)p.ld);
     for (int s = 0; s < p.nslot; ++s) p.off_cnt[s] = dl.take(sizeof(int32_t) * (size_t)p.ld);
     const std::vector<int32_t>& gp = p.gperm.empty() ? p.perm : p.gperm;
     if (!gp.empty()) p.tab_perm = tl.take(sizeof(int32_t) * gp.size());
     if (p.kind == KIND_COUNT_ONLY && !dev_in) p.tab_rad = tl.take(sizeof(double) * (size_t)p.n);
   }
-  const size_t off_centers = dl.take(sizeof(double) * (size_t)ncols_total);
-  const size_t off_minmax = dl.take(sizeof(unsigned long long) * 2 * (size_t)ncols_total);
+  const int nslots = (int)slots.size();
+  for (SlotPlan& sl : slots) sl.off = dl.take(sizeof(double) * (size_t)P[(size_t)sl.task].ld);
+  for (TaskPlan& p : P)
+    for (int sl : p.slot) p.off_col.push_back(slots[(size_t)sl].off);
+  const size_t off_centers = dl.take(sizeof(double) * (size_t)nslots);
+  const size_t off_minmax = dl.take(sizeof(unsigned long long) * 2 * (size_t)nslots);
   const size_t off_keys_a = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(sort_total, 1));
   const size_t off_keys_b = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(sort_total, 1));
   const size_t off_vals_a = dl.take(sizeof(int32_t) * (size_t)std::max<int64_t>(sort_total, 1));
@@ -1102,7 +1115,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   const size_t off_fs1 = dl.take(sizeof(float) * (size_t)std::max<int64_t>(s1_total, 1));
   const size_t off_fs2 = dl.take(sizeof(float) * (size_t)std::max<int64_t>(s2_total, 1));
   const size_t sweep_bytes = sort_sweep_bytes(nblk_os, (int)segs.size());
-  const size_t off_sweep = dl.take(sweep_bytes);
 
   // multi-D job blocks
   std::vector<JobDev> jobs(mjobs.size());
@@ -1208,7 +1220,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       g.len = (int32_t)len;
       g.blk0 = nblk_grid;
       g.nblk = (int32_t)((len + SORT_TILE - 1) / SORT_TILE);
-      g.task = m.s.task;
       gsegs.push_back(g);
       grid_jobs.push_back((int32_t)j);
       gsort_total += len;
@@ -1324,7 +1335,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     wbuild.push_back(J);
     wjobs.push_back(J);
   }
-  const size_t off_wmz = dl.take(std::max<size_t>(wmz_bytes, 16));
 
   // discrete tasks: one exact group-by per column subset (egb_discrete.cu);
   // hash tables of twice the rows, zeroed by one memset with the rest
@@ -1385,7 +1395,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     lchecks.push_back(L);
     lcheck_jobs.push_back({(int)g - 2, (int)g - 1, (int)g, G.task});
   }
-  const size_t off_gbz = dl.take(std::max<size_t>(gbz_bytes, 16));
 
   // tile launch groups
   struct Group {
@@ -1539,9 +1548,10 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
         for (size_t w = 0; w < p.perm.size(); ++w) inv[p.perm[w]] = (int32_t)w;
       }
       for (int c = 0; c < p.ncol; ++c) {
+        const int sl = p.slot[(size_t)c];
+        if (slots[(size_t)sl].task != t || slots[(size_t)sl].col != c) continue;  // another's column
         RescaleCol rc{};
-        rc.task = t;
-        rc.col = c;
+        rc.slot = sl;
         // x from noise position 0, then y, then z (n x dz, row-major)
         const int zc = c - p.dx - p.dy;  // condition column, or negative
         rc.group = zc >= 0 && p.dz > 1 ? p.dz : 1;
@@ -1552,8 +1562,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
         auto f = ordered ? stat_of.end() : stat_of.find(key);
         if (f == stat_of.end()) {
           RescaleStat rs{};
-          rs.task = t;
-          rs.col = c;
+          rs.slot = sl;
           rs.tree = it->second;
           rs.group = rc.group;
           rs.scratch = (int64_t)scratch_elems;
@@ -1572,12 +1581,10 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   }
 
   // tables (pinned blob -> device)
-  std::vector<GatherCol> gcols;
-  std::vector<int32_t> col_task, col_idx;
   const size_t tab_tasks = tl.take(sizeof(TaskDev) * (size_t)ntasks);
-  const size_t tab_gcols = tl.take(sizeof(GatherCol) * (size_t)ncols_total);
-  const size_t tab_coltask = tl.take(sizeof(int32_t) * (size_t)ncols_total);
-  const size_t tab_colidx = tl.take(sizeof(int32_t) * (size_t)ncols_total);
+  const size_t tab_slots = tl.take(sizeof(BatchCol) * (size_t)nslots);
+  const size_t tab_colptr = tl.take(sizeof(double*) * (size_t)ncols_total);
+  const size_t tab_colslot = tl.take(sizeof(int32_t) * (size_t)ncols_total);
   const size_t tab_segs = tl.take(sizeof(SortSeg) * std::max<size_t>(segs.size(), 1));
   const size_t tab_blkseg = tl.take(sizeof(int32_t) * (size_t)std::max(nblk_sort, 1));
   const size_t tab_osblkseg = tl.take(sizeof(int32_t) * (size_t)std::max(nblk_os, 1));
@@ -1638,8 +1645,14 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   const size_t zr_err = align_up(zr_zero + sizeof(uint32_t) * (size_t)ntasks, 16);
   const size_t zr_groups = align_up(zr_err + 16, 16);  // distinct rows per group job
   const size_t zr_warn = zr_groups + sizeof(unsigned long long) * gbjobs.size();  // 2 per check
-  const size_t zr_bytes = align_up(zr_warn + 2 * sizeof(unsigned long long) * lchecks.size(), 256);
+  const size_t zr_const = align_up(zr_warn + 2 * sizeof(unsigned long long) * lchecks.size(), 16);
+  const size_t zr_bytes = align_up(zr_const + sizeof(uint32_t) * (size_t)nslots, 256);
+  // everything that starts zeroed, in one run
   const size_t off_zr = dl.take(zr_bytes);
+  const size_t off_sweep = dl.take(sweep_bytes);
+  const size_t off_wmz = dl.take(wmz_bytes);
+  const size_t off_gbz = dl.take(gbz_bytes);
+  const size_t zero_bytes = dl.off - off_zr;
   // readback region: partial sums, then a copy of zero flags + error word
   const size_t off_partial = dl.take(sizeof(double) * (size_t)std::max(nchunks, 1));
   const size_t arena_bytes = align_up(dl.off, 256);
@@ -1663,36 +1676,39 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     TaskPlan& p = P[(size_t)t];
     TaskDev& D = tdev[(size_t)t];
     std::memset(&D, 0, sizeof(D));
-    D.x64 = (const double*)devp(p.off_x64);
-    D.center = (const double*)(A + off_centers) + p.center0;
+    D.col = (double* const*)(A + off_tab + tab_colptr) + p.center0;
+    D.slot = (const int32_t*)(A + off_tab + tab_colslot) + p.center0;
+    D.centers = (const double*)(A + off_centers);
     D.eps = (double*)devp(p.off_eps);
-    D.rad = (double*)devp(p.off_rad);
+    D.rad = p.kind == KIND_COUNT_ONLY ? (double*)devp(p.off_rad) : D.eps;
     for (int s = 0; s < p.nslot; ++s) D.cnt[s] = (int32_t*)devp(p.off_cnt[s]);
     D.ld = p.ld;
     D.n = (int32_t)p.n;
     D.ncol = p.ncol;
     D.rad_given = p.kind == KIND_COUNT_ONLY ? 1 : 0;
     const std::vector<int32_t>& gp = p.gperm.empty() ? p.perm : p.gperm;
-    const int32_t* perm_dev = p.index ? (index_in_place(p) ? p.index
-                                                           : (const int32_t*)(A + off_tab + p.tab_index))
-                              : gp.empty() ? nullptr : (const int32_t*)(A + off_tab + p.tab_perm);
     if (!gp.empty()) std::memcpy(H + p.tab_perm, gp.data(), sizeof(int32_t) * gp.size());
     if (p.kind == KIND_COUNT_ONLY && !dev_in)
       std::memcpy(H + p.tab_rad, count_radius, sizeof(double) * (size_t)p.n);
     for (int c = 0; c < p.ncol; ++c) {
-      GatherCol g{};
-      g.src = dev_col(t, c);
-      g.stride = tasks[t].cols[c].stride;
-      g.perm = perm_dev;
-      g.task = t;
-      g.col = c;
-      gcols.push_back(g);
-      col_task.push_back(t);
-      col_idx.push_back(c);
+      ((double**)(H + tab_colptr))[p.center0 + c] = (double*)devp(p.off_col[(size_t)c]);
+      ((int32_t*)(H + tab_colslot))[p.center0 + c] = p.slot[(size_t)c];
     }
   }
+  for (int i = 0; i < nslots; ++i) {
+    const SlotPlan& sl = slots[(size_t)i];
+    const TaskPlan& p = P[(size_t)sl.task];
+    BatchCol b{};
+    b.x = (double*)devp(sl.off);
+    b.src = dev_col(sl.task, sl.col);
+    b.stride = tasks[sl.task].cols[sl.col].stride;
+    b.perm = p.index ? (index_in_place(p) ? p.index : (const int32_t*)(A + off_tab + p.tab_index))
+             : p.perm.empty() ? nullptr : (const int32_t*)(A + off_tab + p.tab_perm);
+    b.ld = p.ld;
+    b.n = (int32_t)p.n;
+    std::memcpy(H + tab_slots + sizeof(BatchCol) * (size_t)i, &b, sizeof(BatchCol));
+  }
   std::memcpy(H + tab_tasks, tdev.data(), sizeof(TaskDev) * tdev.size());
-  std::memcpy(H + tab_gcols, gcols.data(), sizeof(GatherCol) * gcols.size());
   for (const auto& e : index_tab)
     std::memcpy(H + e.second, e.first.first, sizeof(int32_t) * (size_t)e.first.second);
   if (!rcols.empty()) {
@@ -1703,14 +1719,12 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       const size_t o = rinv_task[(size_t)task];
       return o == SIZE_MAX ? nullptr : (const int32_t*)(A + off_tab + tab_rinv) + o;
     };
-    for (RescaleCol& rc : rcols) rc.inv = inv_of(rc.task);
-    for (RescaleStat& rs : rstats) rs.inv = inv_of(rs.task);
+    for (RescaleCol& rc : rcols) rc.inv = inv_of(slots[(size_t)rc.slot].task);
+    for (RescaleStat& rs : rstats) rs.inv = inv_of(slots[(size_t)rs.slot].task);
     std::memcpy(H + tab_rcols, rcols.data(), sizeof(RescaleCol) * rcols.size());
     std::memcpy(H + tab_rstats, rstats.data(), sizeof(RescaleStat) * rstats.size());
     if (!rinv.empty()) std::memcpy(H + tab_rinv, rinv.data(), sizeof(int32_t) * rinv.size());
   }
-  std::memcpy(H + tab_coltask, col_task.data(), sizeof(int32_t) * col_task.size());
-  std::memcpy(H + tab_colidx, col_idx.data(), sizeof(int32_t) * col_idx.size());
   if (!segs.empty()) std::memcpy(H + tab_segs, segs.data(), sizeof(SortSeg) * segs.size());
   {
     int32_t* bs = (int32_t*)(H + tab_blkseg);
@@ -1777,6 +1791,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     J.stats = (unsigned long long*)(A + off_zr + zr_stats) + 4 * job_group[j];
     J.eps = D.eps;
     J.rad = D.rad;
+    J.rad_given = D.rad_given;
     J.cnt = mjobs[j].is_knn ? nullptr : D.cnt[mjobs[j].s.slot];
     std::memcpy(H + tab_jobs + sizeof(JobDev) * j, &J, sizeof(JobDev));
   }
@@ -1867,10 +1882,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   // or captured once into a CUDA graph and replayed for identical batches.
   auto enqueue = [&]() -> int {
   EGB_CUDA(cudaMemcpyAsync(A + off_tab, H, tab_bytes, cudaMemcpyHostToDevice, st));
-  EGB_CUDA(cudaMemsetAsync(A + off_zr, 0, zr_bytes, st));
-  if (wmz_bytes) EGB_CUDA(cudaMemsetAsync(A + off_wmz, 0, wmz_bytes, st));
-  if (gbz_bytes) EGB_CUDA(cudaMemsetAsync(A + off_gbz, 0, gbz_bytes, st));
-  if (nblk_sort) EGB_CUDA(cudaMemsetAsync(A + off_sweep, 0, sweep_bytes, st));
+  EGB_CUDA(cudaMemsetAsync(A + off_zr, 0, zero_bytes, st));
   if (inject)  // the device error word as if a kernel had set these bits
     for (int i = 0; i < 4; ++i)
       EGB_CUDA(cudaMemsetAsync((char*)err_d + i, (int)((inject >> (8 * i)) & 0xffu), 1, st));
@@ -1891,22 +1903,22 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       launch_emit_items((const JobDev*)dtab(tab_jobs), (const ItemRun*)dtab(G.tab_runs),
                         (int)G.runs.size(), (const int32_t*)dtab(G.tab_cum), G.nitems,
                         (WorkItem*)(A + G.off_items), st);
-  launch_gather(tasks_d, (const GatherCol*)dtab(tab_gcols), ncols_total, max_ld, st);
+  const BatchCol* slots_d = (const BatchCol*)dtab(tab_slots);
+  launch_gather(slots_d, nslots, max_ld, (unsigned long long*)(A + off_minmax), st);
   if (!rcols.empty())
-    launch_rescale(tasks_d, (const RescaleStat*)dtab(tab_rstats), (int)rstats.size(),
+    launch_rescale(slots_d, (const RescaleStat*)dtab(tab_rstats), (int)rstats.size(),
                    (const RescaleCol*)dtab(tab_rcols), (int)rcols.size(),
                    (const PwTree*)dtab(tab_pwtrees), (const int2*)dtab(tab_pwnodes),
                    (const int32_t*)dtab(tab_pwlevels), (double*)(A + off_pw_scratch),
-                   (double2*)(A + off_pw_ms), ctx->noise_d, zero_d, max_n, st);
-  launch_prepare(tasks_d, (const int32_t*)dtab(tab_coltask), (const int32_t*)dtab(tab_colidx),
-                 ncols_total, max_n, (unsigned long long*)(A + off_minmax), (double*)(A + off_centers),
-                 st);
+                   (double2*)(A + off_pw_ms), ctx->noise_d, (uint32_t*)(A + off_zr + zr_const), max_n, st);
+  launch_prepare(slots_d, nslots, max_n, tasks_d, (const JobDev*)dtab(tab_jobs), (int)jobs.size(),
+                 (unsigned long long*)(A + off_minmax), (double*)(A + off_centers), st);
   if (timing) EGB_CUDA(cudaEventRecord(ctx->ev[2], st));
 
   uint64_t* keys = (uint64_t*)(A + off_keys_a);
   int32_t* vals = (int32_t*)(A + off_vals_a);
   if (timing) EGB_CUDA(cudaEventRecord(ctx->kev[8], st));
-  launch_sort(tasks_d, (const SortSeg*)dtab(tab_segs), (const int32_t*)dtab(tab_blkseg), nblk_sort,
+  launch_sort(slots_d, (const SortSeg*)dtab(tab_segs), (const int32_t*)dtab(tab_blkseg), nblk_sort,
               (const int32_t*)dtab(tab_osblkseg), nblk_os, (int)segs.size(), keys,
               (uint64_t*)(A + off_keys_b), vals, (int32_t*)(A + off_vals_b), A + off_sweep,
               sort_first, err_d, st, timing ? ctx->kev + 12 : nullptr);
@@ -1926,8 +1938,11 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     EGB_CUDA(cudaEventRecord(ctx->join_ev[0], ctx->side_stream));
   }
   if (timing) EGB_CUDA(cudaEventRecord(ctx->kev[9], st));
-  launch_materialize(tasks_d, (const JobDev*)dtab(tab_jobs), (int)jobs.size(), vals,
-                     (const SortSeg*)dtab(tab_segs), max_lds, st);
+  bool any_plain_copy = false;  // jobs with working-order or sorted copies
+  for (const JobDev& J : jobs) any_plain_copy |= J.c64 != nullptr;
+  if (any_plain_copy)
+    launch_materialize(tasks_d, (const JobDev*)dtab(tab_jobs), (int)jobs.size(), vals,
+                       (const SortSeg*)dtab(tab_segs), max_lds, st);
   if (!grid_jobs.empty()) {
     const JobDev* jobs_d = (const JobDev*)dtab(tab_jobs);
     const int32_t* gj_d = (const int32_t*)dtab(tab_gridjobs);
@@ -2031,7 +2046,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   if (timing) EGB_CUDA(cudaEventRecord(ctx->kev[3], st));
   if (timing) EGB_CUDA(cudaEventRecord(ctx->ev[4], st));
 
-  launch_radius(tasks_d, ntasks, max_ld, st);
   if (timing) EGB_CUDA(cudaEventRecord(ctx->kev[10], st));
   // the 1-D counts overlap the rank-space and multi-D counts on the side
   // stream (a timed batch keeps them in line, for their own event times)
@@ -2175,6 +2189,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   R.zr_warn = zr_warn;
   for (const auto& j : lcheck_jobs) R.warn_of.push_back(j[3]);
   R.zr_zero = zr_zero;
+  R.zr_const = zr_const;
   R.nchunks = nchunks;
   R.tab_bytes = tab_bytes;
   R.zr_bytes = zr_bytes;
@@ -2311,7 +2326,8 @@ int egb_fetch(egb_ctx* ctx, int32_t task, int32_t which, void* host_out) {
   const size_t n = (size_t)p.n;
   std::vector<char> buf(n * 8);
   const char* src = (const char*)ctx->arena +
-                    (column ? p.off_x64 + sizeof(double) * (size_t)((which - 16) * p.ld)
+                    (column ? (p.off_col.empty() ? p.off_x64 + sizeof(double) * (size_t)((which - 16) * p.ld)
+                                                 : p.off_col[(size_t)which - 16])
                             : which == 0 ? p.off_eps : p.off_cnt[which - 1]);
   const size_t esz = (which == 0 || column) ? 8 : 4;
   EGB_CUDA(cudaMemcpyAsync(buf.data(), src, n * esz, cudaMemcpyDeviceToHost, ctx->stream));

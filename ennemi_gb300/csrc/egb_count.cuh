@@ -80,7 +80,7 @@ count_tile_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ 
     for (int q = 0; q < QPT; ++q) {
       qp[q] = q0 + tid + q * THREADS;
       const bool exists = qp[q] < len;
-      const double r = exists ? sj.rad[sj.idx[qp[q]]] : -1.0;
+      const double r = exists ? radius_of(sj.rad, sj.rad_given, sj.idx[qp[q]]) : -1.0;
       qok[q] = exists && (r >= 0.0);
       qr[q] = r;
       rbits[q] = qok[q] ? (uint64_t)__double_as_longlong(r) : 0ull;

@@ -48,7 +48,7 @@ group_insert_kernel(const TaskDev* __restrict__ tasks, const GroupJob* __restric
   const int d = J.sp.d;
   uint64_t h = 0x243f6a8885a308d3ull;
   for (int c = 0; c < d; ++c) {
-    uint64_t u = (uint64_t)__double_as_longlong(t.x64[(int64_t)J.sp.cols[c] * t.ld + row]);
+    uint64_t u = (uint64_t)__double_as_longlong(t.col[J.sp.cols[c]][row]);
     u = u == 0x8000000000000000ull ? 0ull : u;  // -0 hashes as +0
     h = mix64(h ^ u);
   }
@@ -67,7 +67,7 @@ group_insert_kernel(const TaskDev* __restrict__ tasks, const GroupJob* __restric
     bool same = true;
     const int j = owner - 1;
     for (int c = 0; c < d && same; ++c) {
-      const double* col = t.x64 + (int64_t)J.sp.cols[c] * t.ld;
+      const double* col = t.col[J.sp.cols[c]];
       same = col[j] == col[row];
     }
     if (same) break;

@@ -204,7 +204,7 @@ grid_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items,
     int cntq = 0;
     bool qok = exists;
     if constexpr (COUNT) {
-      qr = exists ? sj.rad[sj.idxg[qp]] : -1.0;
+      qr = exists ? radius_of(sj.rad, sj.rad_given, sj.idxg[qp]) : -1.0;
       qok = exists && (qr >= 0.0);
       rbits = qok ? (uint64_t)__double_as_longlong(qr) : 0ull;
       if (!PLAIN && qok) {

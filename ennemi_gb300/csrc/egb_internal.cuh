@@ -216,17 +216,27 @@ __device__ __forceinline__ double band(double m, double t) {
 
 constexpr uint64_t INF_BITS = 0x7ff0000000000000ull;
 
+#ifdef __CUDACC__
+// The count radius of working index w: the caller's, or fl64(eps - 1e-12), the
+// reference's (ennemi/_entropy_estimators.py:109-110, :152-154, :196, :243-245).
+__device__ __forceinline__ double radius_of(const double* rad, int given, int64_t w) {
+  const double v = rad[w];
+  return given ? v : v - 1e-12;
+}
+#endif
+
 // ------------------------------------------------------------ job structs --
 struct TaskDev {          // per-task device view
-  const double* x64;      // working FP64 columns, column c at x64 + c*ld
-  const double* center;   // [ncol] column midranges (FP32 copies are x - center)
+  double* const* col;     // [ncol] working FP64 columns (shared between tasks)
+  const int32_t* slot;    // [ncol] the batch column behind each
+  const double* centers;  // per batch column: its midrange (FP32 copies are x - it)
   double* eps;            // [ld]
-  double* rad;            // [ld] count radius per sample
+  double* rad;            // [ld] caller radii (rad_given), else eps
   int32_t* cnt[4];        // count slots (working order)
   int64_t ld;
   int32_t n;
   int32_t ncol;
-  int32_t rad_given;      // 1: rad holds caller radii (egb_ball_count)
+  int32_t rad_given;      // 1: rad holds caller radii (egb_ball_count), else eps
   int32_t pad_;
 };
 
@@ -249,7 +259,7 @@ struct JobDev {
   double* center;         // [d]
   uint32_t* jflags;       // TF_* bits of this job (set by materialise)
   double* eps;            // task eps  (kNN: written; counts: unused)
-  const double* rad;      // task radius (counts)
+  const double* rad;      // task radii (counts), see radius_of
   int32_t* cnt;           // task count slot (counts)
   int64_t lds;
   int32_t task;
@@ -259,6 +269,7 @@ struct JobDev {
   int32_t slab;           // 1: sorted by the first column
   int32_t sort_seg;       // slab: index of the sort segment of column 0
   int32_t sort_seg_b;     // slab: sort segment of column 1 (second order)
+  int32_t rad_given;
   int32_t kform;          // grid copy holds order-preserving keys, not values:
                           // column c's high words at (uint32*)c64g + 2c*lds,
                           // low words at + (2c+1)*lds (key-range count jobs)
@@ -389,19 +400,23 @@ struct SortSeg {          // one segment of the batched radix sort
   int32_t len;
   int32_t blk0;           // first tile (block) of the segment
   int32_t nblk;
-  int32_t task;
-  int32_t col;            // source column of the task
+  int32_t slot;           // batch column
   int32_t src_begin;      // first working index of the segment
   int32_t os_blk0;        // its first tile of the single-sweep passes (OS_TILE keys)
   int32_t os_nblk;
 };
 
-struct GatherCol {        // working column <- caller column (strided, permuted)
-  const double* src;
+// A working column of the batch.  Task columns with the same bits (the y of
+// every lag, a column of many pairs) are one: gathered, rescaled, ranged and
+// sorted once.
+struct BatchCol {
+  double* x;              // [ld], zero padded
+  const double* src;      // sample w at src[perm[w] * stride] (perm null: w)
   int64_t stride;
-  const int32_t* perm;    // working -> caller index, or null (identity)
-  int32_t task;
-  int32_t col;
+  const int32_t* perm;
+  int64_t ld;
+  int32_t n;
+  int32_t pad_;
 };
 
 // Device rescale (EGB_RESCALE).  A column's sum in NumPy's pairwise order
@@ -414,15 +429,15 @@ struct PwTree {
   int32_t node0, nleaf, nnode, lvl0, nlvl;
 };
 struct RescaleStat {      // one distinct column of the batch: its mean and std
-  int32_t task, col;      // a task column holding it (working order)
+  int32_t slot;           // a batch column holding it (working order, not rescaled yet)
   int32_t tree;           // its summation tree (group == 1)
   int32_t group;          // > 1: one of `group` condition columns, which NumPy
                           // reduces along axis 0 -- row by row, in order
   int64_t scratch;        // first node-sum slot (tree.nnode doubles)
   const int32_t* inv;     // sample -> working position (class-ordered tasks), or null
 };
-struct RescaleCol {       // one task column to rescale in place
-  int32_t task, col;
+struct RescaleCol {       // one batch column to rescale in place
+  int32_t slot;
   int32_t stat;           // its RescaleStat
   int32_t group;          // noise stride: condition columns of an n x group array
   int64_t noise_pos;      // noise value of the column's first sample
@@ -433,10 +448,10 @@ struct RescaleCol {       // one task column to rescale in place
 constexpr uint32_t RESCALE_CONSTANT = 1u << 31;
 // stats: one block per distinct column -> ms[u] = (mean, std); then one block
 // per task column: x = (x - mean) / std + noise
-void launch_rescale(const TaskDev* tasks_d, const RescaleStat* stats_d, int nstats,
+void launch_rescale(const BatchCol* slots_d, const RescaleStat* stats_d, int nstats,
                     const RescaleCol* cols_d, int ncols, const PwTree* trees_d,
                     const int2* nodes_d, const int32_t* levels_d, double* scratch, double2* ms,
-                    const double* noise, uint32_t* zero_flags, int64_t max_n, cudaStream_t st);
+                    const double* noise, uint32_t* const_flags, int64_t max_n, cudaStream_t st);
 // egb_debug_divide: the rescale's division (div_rn) over n pairs
 void launch_divide(const double* a_d, const double* b_d, int64_t n, double* out_d, cudaStream_t st);
 
@@ -457,11 +472,11 @@ void count_launch();
 // launches on `st` and never synchronises.
 
 // egb_prep.cu
-void launch_gather(const TaskDev* tasks_d, const GatherCol* cols_d, int ncols,
-                   int64_t max_ld, cudaStream_t st);
-void launch_prepare(const TaskDev* tasks_d, const int32_t* col_task_d, const int32_t* col_idx_d,
-                    int ncols_total, int64_t max_n, unsigned long long* minmax_d,
-                    double* centers_d, cudaStream_t st);
+void launch_gather(const BatchCol* slots_d, int nslots, int64_t max_ld, unsigned long long* minmax_d,
+                   cudaStream_t st);
+void launch_prepare(const BatchCol* slots_d, int nslots, int64_t max_n, const TaskDev* tasks_d,
+                    const JobDev* jobs_d, int njobs, unsigned long long* minmax_d, double* centers_d,
+                    cudaStream_t st);
 void launch_materialize(const TaskDev* tasks_d, const JobDev* jobs_d, int njobs,
                         const int32_t* sorted_vals, const SortSeg* segs_d, int64_t max_lds,
                         cudaStream_t st);
@@ -469,7 +484,6 @@ void launch_materialize_grid(const TaskDev* tasks_d, const JobDev* jobs_d,
                              const int32_t* grid_jobs_d, int ngrid, const int32_t* sorted_vals,
                              const SortSeg* segs_d, const int32_t* gvals_sorted,
                              const SortSeg* gsegs_d, int64_t max_lds, cudaStream_t st);
-void launch_radius(const TaskDev* tasks_d, int ntasks, int64_t max_ld, cudaStream_t st);
 void launch_emit_items(const JobDev* jobs_d, const ItemRun* runs_d, int nruns, const int32_t* cum_d,
                        int64_t nitems, WorkItem* items_d, cudaStream_t st);
 void launch_combine(const TaskDev* tasks_d, const CombineJob* jobs_d, const int32_t* chunk_job_d,
@@ -532,7 +546,7 @@ size_t sort_sweep_bytes(int os_nblk, int nseg);
 // Once per context, on its device: lets the passes use their shared memory
 // (above the 48 KB default); returns the cudaError_t.
 int init_sort_kernels();
-void launch_sort(const TaskDev* tasks_d, const SortSeg* segs_d, const int32_t* blk_seg_d,
+void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d,
                  int nblk, const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys_a,
                  uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b, void* sweep, int first,
                  uint32_t* err, cudaStream_t st,

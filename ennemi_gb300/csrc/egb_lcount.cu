@@ -101,7 +101,7 @@ lcount_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ item
     }
     const float mq = __fmaf_ru(am, 1.0f + 0x1p-22f, 0x1p-148f);
     const int32_t w = exists ? J->idxg[qp] : 0;
-    const double qr = exists ? J->rad[w] : -1.0;
+    const double qr = exists ? radius_of(J->rad, J->rad_given, w) : -1.0;
     const int rc = exists ? radius_class(qr) : 0;  // 0 none, 1 finite, 2 every point
     const uint64_t rbits = rc == 1 ? (uint64_t)__double_as_longlong(fabs(qr)) : 0ull;
     float lo = -1.0f, hi = -1.0f;  // inside up to lo, outside beyond hi

@@ -1,7 +1,7 @@
 // egb_prep.cu -- data movement around the search kernels.
 //
 // gather       caller columns (strided, optionally class-permuted) -> the
-//              task's working FP64 columns, zero padded up to ld;
+//              batch's working FP64 columns, zero padded up to ld;
 // prepare      per working column the midrange centre (min/max over the
 //              order-preserving integer keys, so -0.0/+0.0 and any finite
 //              values compare exactly);
@@ -9,9 +9,6 @@
 //              working or sorted order, with the FP32 centred copy and the
 //              job's "FP32 unsafe" flag (a centred value >= 1e37 or not
 //              finite: every candidate of that job is then decided in FP64);
-// radius       rad = fl64(eps - 1e-12): the reference's count radius
-//              (ennemi/_entropy_estimators.py:109-110, :152-154, :196,
-//              :243-245);
 // combine      per-sample estimator term summed in fixed 4096-sample chunks
 //              (deterministic order), plus per-slot "a count was zero" flags.
 //              Terms, from ennemi/_entropy_estimators.py:
@@ -62,29 +59,31 @@ void launch_clusters(void (*kern)(P...), int n, int threads, cudaStream_t st, A.
 // from host memory cross the CPU-GPU link, where throughput follows the
 // requests outstanding.
 constexpr int GATHER_UNROLL = 4;
-__global__ void gather_kernel(const TaskDev* __restrict__ tasks,
-                              const GatherCol* __restrict__ cols, int ncols) {
-  for (int g = blockIdx.y; g < ncols; g += gridDim.y) {
-    const GatherCol gc = cols[g];
-    const TaskDev t = tasks[gc.task];
-    double* dst = const_cast<double*>(t.x64) + (int64_t)gc.col * t.ld;
+__global__ void gather_kernel(const BatchCol* __restrict__ slots, int nslots,
+                              unsigned long long* __restrict__ minmax) {
+  for (int g = blockIdx.y; g < nslots; g += gridDim.y) {
+    const BatchCol bc = slots[g];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // for minmax_kernel
+      minmax[2 * g] = ~0ull;
+      minmax[2 * g + 1] = 0ull;
+    }
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t w0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w0 < t.ld;
+    for (int64_t w0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w0 < bc.ld;
          w0 += GATHER_UNROLL * step) {
       double v[GATHER_UNROLL];
 #pragma unroll
       for (int u = 0; u < GATHER_UNROLL; ++u) {
         const int64_t w = w0 + u * step;
         v[u] = 0.0;
-        if (w < t.n) {
-          const int64_t s = gc.perm ? (int64_t)gc.perm[w] : w;
-          v[u] = gc.src[s * gc.stride];
+        if (w < bc.n) {
+          const int64_t s = bc.perm ? (int64_t)bc.perm[w] : w;
+          v[u] = bc.src[s * bc.stride];
         }
       }
 #pragma unroll
       for (int u = 0; u < GATHER_UNROLL; ++u) {
         const int64_t w = w0 + u * step;
-        if (w < t.ld) dst[w] = v[u];
+        if (w < bc.ld) bc.x[w] = v[u];
       }
     }
   }
@@ -177,7 +176,7 @@ constexpr int STATS_FEW = 16, STATS_CLUSTER = 8;
 constexpr int ROW_STAGE = 1024;  // rows staged at a time
 template <int CL>
 __global__ void __launch_bounds__(PREP_THREADS)
-rescale_stats_kernel(const TaskDev* __restrict__ tasks, const RescaleStat* __restrict__ stats,
+rescale_stats_kernel(const BatchCol* __restrict__ slots, const RescaleStat* __restrict__ stats,
                      const PwTree* __restrict__ trees, const int2* __restrict__ nodes,
                      const int32_t* __restrict__ levels, double* __restrict__ scratch,
                      double2* __restrict__ ms) {
@@ -185,13 +184,13 @@ rescale_stats_kernel(const TaskDev* __restrict__ tasks, const RescaleStat* __res
   __shared__ double mean_s;
   const int stat = blockIdx.x / CL;
   const RescaleStat rs = stats[stat];
-  const TaskDev t = tasks[rs.task];
-  const double* x = t.x64 + (int64_t)rs.col * t.ld;
-  const double n = (double)t.n;
+  const int len = slots[rs.slot].n;
+  const double* x = slots[rs.slot].x;
+  const double n = (double)len;
   if (rs.group > 1) {  // axis-0 reduction of an (n, group) array: in row order
     if (blockIdx.x % CL) return;
-    const double mean = __ddiv_rn(row_sum<ROW_STAGE>(x, rs.inv, t.n, sm, false, 0.0), n);
-    const double q = row_sum<ROW_STAGE>(x, rs.inv, t.n, sm, true, mean);
+    const double mean = __ddiv_rn(row_sum<ROW_STAGE>(x, rs.inv, len, sm, false, 0.0), n);
+    const double q = row_sum<ROW_STAGE>(x, rs.inv, len, sm, true, mean);
     if (threadIdx.x == 0) ms[stat] = make_double2(mean, __dsqrt_rn(__ddiv_rn(q, n)));
     return;
   }
@@ -213,16 +212,16 @@ rescale_stats_kernel(const TaskDev* __restrict__ tasks, const RescaleStat* __res
 // x = RN(RN(RN(x - mean) / sd) + noise) per sample of a task column (one
 // y-row of blocks per column, four samples in flight per thread)
 __global__ void __launch_bounds__(PREP_THREADS)
-rescale_apply_kernel(const TaskDev* __restrict__ tasks, const RescaleCol* __restrict__ cols,
+rescale_apply_kernel(const BatchCol* __restrict__ slots, const RescaleCol* __restrict__ cols,
                      const double2* __restrict__ ms, const double* __restrict__ noise,
-                     uint32_t* __restrict__ zero_flags) {
+                     uint32_t* __restrict__ const_flags) {
   const RescaleCol rc = cols[blockIdx.y];
-  const TaskDev t = tasks[rc.task];
-  double* x = const_cast<double*>(t.x64) + (int64_t)rc.col * t.ld;
+  const int n = slots[rc.slot].n;
+  double* x = slots[rc.slot].x;
   const double2 m = ms[rc.stat];
   const double mean = m.x, sd = m.y;
   if (fabs(sd) < 1e-20) {  // np.abs(std) < 1e-20: the reference warns and keeps x
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(zero_flags + rc.task, RESCALE_CONSTANT);
+    if (blockIdx.x == 0 && threadIdx.x == 0) const_flags[rc.slot] = 1u;
     return;
   }
   __shared__ double rsd_s;  // RN(1 / sd), once per block
@@ -231,14 +230,14 @@ rescale_apply_kernel(const TaskDev* __restrict__ tasks, const RescaleCol* __rest
   const double rsd = rsd_s;
   const double* nz = noise + rc.noise_pos;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < t.n; i0 += 4 * step) {
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
     int w[4];
     double v[4], z[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {  // sample i0 + u * step
       const int64_t i = i0 + u * step;
       w[u] = -1;
-      if (i < t.n) {
+      if (i < n) {
         w[u] = rc.inv ? rc.inv[i] : (int)i;
         v[u] = x[w[u]];
         z[u] = nz[i * rc.group];
@@ -258,23 +257,21 @@ __global__ void divide_kernel(const double* __restrict__ a, const double* __rest
     out[i] = div_rn(a[i], b[i], __ddiv_rn(1.0, b[i]));
 }
 
-__global__ void minmax_kernel(const TaskDev* __restrict__ tasks,
-                              const int32_t* __restrict__ col_task,
-                              const int32_t* __restrict__ col_idx, int ncols,
+__global__ void minmax_kernel(const BatchCol* __restrict__ slots, int nslots,
                               unsigned long long* __restrict__ minmax) {
-  for (int g = blockIdx.y; g < ncols; g += gridDim.y) {
-    const TaskDev t = tasks[col_task[g]];
-    const double* x = t.x64 + (int64_t)col_idx[g] * t.ld;
+  for (int g = blockIdx.y; g < nslots; g += gridDim.y) {
+    const int n = slots[g].n;
+    const double* x = slots[g].x;
     unsigned long long lo = ~0ull, hi = 0ull;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (; i + 3 * stride < t.n; i += 4 * stride) {  // four loads in flight
+    for (; i + 3 * stride < n; i += 4 * stride) {  // four loads in flight
       const double v0 = x[i], v1 = x[i + stride], v2 = x[i + 2 * stride], v3 = x[i + 3 * stride];
       const unsigned long long k0 = key_of(v0), k1 = key_of(v1), k2 = key_of(v2), k3 = key_of(v3);
       lo = min(min(lo, k0), min(k1, min(k2, k3)));
       hi = max(max(hi, k0), max(k1, max(k2, k3)));
     }
-    for (; i < t.n; i += stride) {
+    for (; i < n; i += stride) {
       const unsigned long long k = key_of(x[i]);
       lo = k < lo ? k : lo;
       hi = k > hi ? k : hi;
@@ -307,13 +304,18 @@ __global__ void minmax_kernel(const TaskDev* __restrict__ tasks,
   }
 }
 
-__global__ void center_kernel(const unsigned long long* __restrict__ minmax, int ncols,
-                              double* __restrict__ centers) {
+// Midranges per batch column, and per column of every job.
+__global__ void center_kernel(const unsigned long long* __restrict__ minmax, int nslots,
+                              double* __restrict__ centers, const TaskDev* __restrict__ tasks,
+                              const JobDev* __restrict__ jobs, int njobs) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= ncols) return;
-  const double lo = value_of(minmax[2 * g]);
-  const double hi = value_of(minmax[2 * g + 1]);
-  centers[g] = 0.5 * lo + 0.5 * hi;
+  auto mid = [&](int slot) { return 0.5 * value_of(minmax[2 * slot]) + 0.5 * value_of(minmax[2 * slot + 1]); };
+  if (g < nslots) centers[g] = mid(g);
+  if (g < njobs) {
+    const JobDev& J = jobs[g];
+    const int32_t* slot = tasks[J.task].slot;
+    for (int c = 0; c < J.sp.d; ++c) J.center[c] = mid(slot[J.sp.cols[c]]);
+  }
 }
 
 __device__ __forceinline__ bool materialize_copy(const TaskDev& t, const JobDev& J, int d,
@@ -327,8 +329,8 @@ __device__ __forceinline__ bool materialize_copy(const TaskDev& t, const JobDev&
       idx[p] = w;
       for (int c = 0; c < d; ++c) {
         const int tc = J.sp.cols[c];
-        const double v = t.x64[(int64_t)tc * t.ld + w];
-        const double cv = v - t.center[tc];
+        const double v = t.col[tc][w];
+        const double cv = v - J.center[c];
         bad |= !(fabs(cv) < 1e37);
         c64[(int64_t)c * J.lds + p] = v;
         // clamped so that FP32 distances stay finite; a job with a clamped
@@ -354,7 +356,6 @@ __global__ void materialize_kernel(const TaskDev* __restrict__ tasks,
     const JobDev J = jobs[jb];
     const TaskDev t = tasks[J.task];
     const int d = J.sp.d;
-    if (blockIdx.x == 0 && threadIdx.x < d) J.center[threadIdx.x] = t.center[J.sp.cols[threadIdx.x]];
     if (J.c64 == nullptr) continue;  // grid copy only (materialize_grid_kernel)
     const int32_t* sv = J.slab ? sorted_vals + segs[J.sort_seg].out_base : nullptr;
     bool bad = materialize_copy(t, J, d, J.c64, J.c32, J.idx, sv);
@@ -381,7 +382,7 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
     const int32_t* gv = gvals_sorted + gsegs[J.gseg].out_base;
     // column-1 bounds of each strip, from the column-1 sort
     const int32_t* vb = sorted_vals + segs[J.sort_seg_b].out_base;
-    const double* x1 = t.x64 + (int64_t)J.sp.cols[1] * t.ld;
+    const double* x1 = t.col[J.sp.cols[1]];
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < J.nstrips; s += gridDim.x * blockDim.x) {
       const double lo = x1[vb[J.sstart[s]]];
       const double hi = x1[vb[J.sstart[s + 1] - 1]];
@@ -400,14 +401,14 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
         J.idxg[p] = w;
         for (int c = 0; c < d; ++c) {
           const int tc = J.sp.cols[c];
-          const double v = t.x64[(int64_t)tc * t.ld + w];
+          const double v = t.col[tc][w];
           if (J.kform) {
             const uint64_t k = raw_key((uint64_t)__double_as_longlong(v));
             uint32_t* kw = reinterpret_cast<uint32_t*>(J.c64g);
             kw[(int64_t)(2 * c) * J.lds + p] = (uint32_t)(k >> 32);
             kw[(int64_t)(2 * c + 1) * J.lds + p] = (uint32_t)k;
           } else {
-            const double cv = v - t.center[tc];
+            const double cv = v - J.center[c];
             bad |= !(fabs(cv) < 1e37);
             J.c64g[(int64_t)c * J.lds + p] = v;
             J.c32g[(int64_t)c * J.lds + p] = __double2float_rn(fmin(fmax(cv, -1e37), 1e37));
@@ -429,16 +430,6 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
       }
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(J.jflags, (uint32_t)TF_UNSAFE32);
-  }
-}
-
-__global__ void radius_kernel(const TaskDev* __restrict__ tasks, int ntasks) {
-  for (int ti = blockIdx.y; ti < ntasks; ti += gridDim.y) {
-    const TaskDev t = tasks[ti];
-    if (t.rad_given) continue;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.n;
-         i += (int64_t)gridDim.x * blockDim.x)
-      t.rad[i] = t.eps[i] - 1e-12;
   }
 }
 
@@ -568,24 +559,24 @@ combine_kernel(const TaskDev* __restrict__ tasks, const CombineJob* __restrict__
 
 }  // namespace
 
-void launch_gather(const TaskDev* tasks_d, const GatherCol* cols_d, int ncols, int64_t max_ld,
+void launch_gather(const BatchCol* slots_d, int nslots, int64_t max_ld, unsigned long long* minmax_d,
                    cudaStream_t st) {
-  if (ncols <= 0) return;
-  dim3 grid(grid_x_for((max_ld + GATHER_UNROLL - 1) / GATHER_UNROLL), grid_y_for(ncols));
-  gather_kernel<<<grid, PREP_THREADS, 0, st>>>(tasks_d, cols_d, ncols);
+  if (nslots <= 0) return;
+  dim3 grid(grid_x_for((max_ld + GATHER_UNROLL - 1) / GATHER_UNROLL), grid_y_for(nslots));
+  gather_kernel<<<grid, PREP_THREADS, 0, st>>>(slots_d, nslots, minmax_d);
   count_launch();
 }
 
-void launch_rescale(const TaskDev* tasks_d, const RescaleStat* stats_d, int nstats,
+void launch_rescale(const BatchCol* slots_d, const RescaleStat* stats_d, int nstats,
                     const RescaleCol* cols_d, int ncols, const PwTree* trees_d,
                     const int2* nodes_d, const int32_t* levels_d, double* scratch, double2* ms,
-                    const double* noise, uint32_t* zero_flags, int64_t max_n, cudaStream_t st) {
+                    const double* noise, uint32_t* const_flags, int64_t max_n, cudaStream_t st) {
   if (ncols <= 0 || nstats <= 0) return;
   if (nstats <= STATS_FEW)
-    launch_clusters<STATS_CLUSTER>(rescale_stats_kernel<STATS_CLUSTER>, nstats, PREP_THREADS, st, tasks_d,
+    launch_clusters<STATS_CLUSTER>(rescale_stats_kernel<STATS_CLUSTER>, nstats, PREP_THREADS, st, slots_d,
                                    stats_d, trees_d, nodes_d, levels_d, scratch, ms);
   else
-    rescale_stats_kernel<1><<<nstats, PREP_THREADS, 0, st>>>(tasks_d, stats_d, trees_d, nodes_d, levels_d,
+    rescale_stats_kernel<1><<<nstats, PREP_THREADS, 0, st>>>(slots_d, stats_d, trees_d, nodes_d, levels_d,
                                                              scratch, ms);
   count_launch();
   // 32 samples a thread where the columns fill the GPU (one division per
@@ -594,7 +585,7 @@ void launch_rescale(const TaskDev* tasks_d, const RescaleStat* stats_d, int nsta
   const int gx = std::min(grid_x_for((max_n + 3) / 4),
                           std::max(grid_x_for((max_n + 31) / 32), 2048 / std::min(ncols, 2048)));
   const dim3 agrid(gx, grid_y_for(ncols));
-  rescale_apply_kernel<<<agrid, PREP_THREADS, 0, st>>>(tasks_d, cols_d, ms, noise, zero_flags);
+  rescale_apply_kernel<<<agrid, PREP_THREADS, 0, st>>>(slots_d, cols_d, ms, noise, const_flags);
   count_launch();
 }
 
@@ -604,20 +595,16 @@ void launch_divide(const double* a_d, const double* b_d, int64_t n, double* out_
   count_launch();
 }
 
-void launch_prepare(const TaskDev* tasks_d, const int32_t* col_task_d, const int32_t* col_idx_d,
-                    int ncols_total, int64_t max_n, unsigned long long* minmax_d,
-                    double* centers_d, cudaStream_t st) {
-  if (ncols_total <= 0) return;
-  // slot 2g holds the min key (starts all-ones), slot 2g+1 the max key
-  // (starts at zero)
-  cudaMemsetAsync(minmax_d, 0, sizeof(unsigned long long) * 2 * ncols_total, st);
-  cudaMemset2DAsync(minmax_d, 2 * sizeof(unsigned long long), 0xff, sizeof(unsigned long long),
-                    ncols_total, st);
-  dim3 grid(grid_x_for((max_n + 7) / 8), grid_y_for(ncols_total));  // eight values a thread
-  minmax_kernel<<<grid, PREP_THREADS, 0, st>>>(tasks_d, col_task_d, col_idx_d, ncols_total,
-                                                minmax_d);
+void launch_prepare(const BatchCol* slots_d, int nslots, int64_t max_n, const TaskDev* tasks_d,
+                    const JobDev* jobs_d, int njobs, unsigned long long* minmax_d, double* centers_d,
+                    cudaStream_t st) {
+  if (nslots <= 0) return;
+  // launch_gather set the slots: 2g holds the min key, 2g+1 the max key
+  dim3 grid(grid_x_for((max_n + 7) / 8), grid_y_for(nslots));  // eight values a thread
+  minmax_kernel<<<grid, PREP_THREADS, 0, st>>>(slots_d, nslots, minmax_d);
   count_launch();
-  center_kernel<<<(ncols_total + 255) / 256, 256, 0, st>>>(minmax_d, ncols_total, centers_d);
+  center_kernel<<<(std::max(nslots, njobs) + 255) / 256, 256, 0, st>>>(minmax_d, nslots, centers_d, tasks_d,
+                                                                       jobs_d, njobs);
   count_launch();
 }
 
@@ -683,13 +670,6 @@ void launch_materialize_grid(const TaskDev* tasks_d, const JobDev* jobs_d,
   dim3 grid(grid_x_for(max_lds), grid_y_for(ngrid));
   materialize_grid_kernel<<<grid, PREP_THREADS, 0, st>>>(tasks_d, jobs_d, grid_jobs_d, ngrid,
                                                          sorted_vals, segs_d, gvals_sorted, gsegs_d);
-  count_launch();
-}
-
-void launch_radius(const TaskDev* tasks_d, int ntasks, int64_t max_ld, cudaStream_t st) {
-  if (ntasks <= 0) return;
-  dim3 grid(grid_x_for(max_ld), grid_y_for(ntasks));
-  radius_kernel<<<grid, PREP_THREADS, 0, st>>>(tasks_d, ntasks);
   count_launch();
 }
 

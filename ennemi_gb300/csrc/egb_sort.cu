@@ -192,7 +192,7 @@ __device__ __forceinline__ uint64_t key_of_bits(uint64_t u) {
 }
 
 __global__ void __launch_bounds__(SORT_THREADS)
-onesweep_load_kernel(const TaskDev* __restrict__ tasks, const SortSeg* __restrict__ segs,
+onesweep_load_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict__ segs,
                      const int32_t* __restrict__ blk_seg, uint64_t* __restrict__ keys,
                      int32_t* __restrict__ vals, uint32_t* __restrict__ seg_hist, int first) {
   __shared__ uint32_t h[OS_PASSES * 256];
@@ -201,9 +201,7 @@ onesweep_load_kernel(const TaskDev* __restrict__ tasks, const SortSeg* __restric
   const SortSeg s = segs[si];
   for (int i = threadIdx.x; i < OS_PASSES * 256; i += SORT_THREADS) h[i] = 0;
   __syncthreads();
-  const TaskDev& t = tasks[s.task];
-  const uint64_t* __restrict__ x =
-      reinterpret_cast<const uint64_t*>(t.x64 + (int64_t)s.col * t.ld + s.src_begin);
+  const uint64_t* __restrict__ x = reinterpret_cast<const uint64_t*>(slots[s.slot].x + s.src_begin);
   const int i0 = (b - s.blk0) * SORT_TILE;
   const int i1 = min(i0 + SORT_TILE, s.len);
   for (int i = i0 + threadIdx.x; i < i1; i += SORT_THREADS) {
@@ -522,7 +520,7 @@ __global__ void sorted_jobs_kernel(const TaskDev* __restrict__ tasks,
     return;
   }
 
-  const double r = t.rad[i];
+  const double r = radius_of(t.rad, t.rad_given, i);
   const int rc = radius_class(r);
   int32_t count;
   if (rc == 0) {
@@ -624,7 +622,7 @@ __global__ void nest_sub_kernel(const TaskDev* __restrict__ tasks,
     const TaskDev& t = tasks[J.task];
     const int64_t out = gsegs[J.gseg].out_base;
     const int nsub = J.nsub;
-    const double* z = t.x64 + (int64_t)J.sp.cols[2] * t.ld + J.seg_begin;
+    const double* z = t.col[J.sp.cols[2]] + J.seg_begin;
     for (int64_t p2 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p2 < J.len;
          p2 += (int64_t)gridDim.x * blockDim.x) {
       const int s1 = (int)keys_sorted[out + p2];
@@ -720,7 +718,7 @@ size_t sort_sweep_bytes(int os_nblk, int nseg) {
          sizeof(uint32_t) * OS_PASSES * 256 * (size_t)std::max(nseg, 1) + 64;
 }
 
-void launch_sort(const TaskDev* tasks_d, const SortSeg* segs_d, const int32_t* blk_seg_d,
+void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d,
                  int nblk, const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys_a,
                  uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b, void* sweep, int first,
                  uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
@@ -729,7 +727,7 @@ void launch_sort(const TaskDev* tasks_d, const SortSeg* segs_d, const int32_t* b
   unsigned long long* flags = (unsigned long long*)sweep;
   uint32_t* seg_hist = (uint32_t*)(flags + 256 * (size_t)os_nblk);
   int* counters = (int*)(seg_hist + OS_PASSES * 256 * (size_t)std::max(nseg, 1));
-  onesweep_load_kernel<<<nblk, SORT_THREADS, 0, st>>>(tasks_d, segs_d, blk_seg_d, keys_a, vals_a,
+  onesweep_load_kernel<<<nblk, SORT_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, keys_a, vals_a,
                                                      seg_hist, first);
   count_launch();
   uint64_t* kin = keys_a;

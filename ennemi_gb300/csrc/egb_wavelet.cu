@@ -365,7 +365,7 @@ wm_count_kernel(const TaskDev* __restrict__ tasks, const WmJob* __restrict__ job
   if (i >= len) return;
   const TaskDev& t = tasks[J.task];
   const int32_t w = vals_all[J.base_a + i];          // working index of the query
-  const double r = t.rad[w];
+  const double r = radius_of(t.rad, t.rad_given, w);
   const int rc = radius_class(r);
   int32_t count;
   if (rc == 0) {

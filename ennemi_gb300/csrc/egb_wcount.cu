@@ -194,7 +194,7 @@ wcount_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ item
 
     const int qp = wi.q0 + lane;
     const bool exists = qp < wi.q1;
-    const double qr = exists ? J->rad[J->idxg[qp]] : -1.0;
+    const double qr = exists ? radius_of(J->rad, J->rad_given, J->idxg[qp]) : -1.0;
     const bool qok = exists && qr >= 0.0;
     const bool every = qok && isinf(qr);  // an infinite radius holds every point
     uint64_t kxl = 1, kxr = 0, kyl = 1, kyr = 0, kzl = 1, kzr = 0, kwl = 1, kwr = 0;  // empty

@@ -309,7 +309,7 @@ wgrid_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     bool qok = exists;
     int pass = TWO_PASS ? 0 : 1;
     if constexpr (COUNT) {
-      qr = exists ? J->rad[J->idxg[qp]] : -1.0;
+      qr = exists ? radius_of(J->rad, J->rad_given, J->idxg[qp]) : -1.0;
       qok = exists && (qr >= 0.0);
       rbits = qok ? (uint64_t)__double_as_longlong(qr) : 0ull;
       if (!PLAIN && qok) tcnt = plan_margin(__double2float_ru(qr));
