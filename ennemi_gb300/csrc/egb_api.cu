@@ -1120,6 +1120,12 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   std::vector<JobDev> jobs(mjobs.size());
   std::vector<SortSeg> gsegs;        // strip-key sort, one segment per grid job
   std::vector<int32_t> grid_jobs;    // job index of each grid job
+  std::vector<int32_t> strip_table_jobs;  // grid jobs and strip jobs: those with a strip table
+  std::vector<StripJob> strip_jobs;  // two-column jobs built by strip
+  std::vector<InvSeg> inv_segs;      // their column-0 segments, inverted once each
+  std::unordered_map<int, size_t> inv_of_seg;
+  int nstrips_built = 0, strip_largest = 0;
+  int64_t max_inv_len = 1;
   int64_t gsort_total = 0, max_glen = 1;
   bool any_nested = false;
   int64_t max_gkey = 1;  // largest strip / cell key of the grid jobs
@@ -1161,7 +1167,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       J.c64g = (double*)(uintptr_t)dl.take(sizeof(double) * (size_t)(d * J.lds));
       J.c32g = (float*)(uintptr_t)dl.take(sizeof(float) * (size_t)(d * J.lds));
       J.idxg = (int32_t*)(uintptr_t)dl.take(sizeof(int32_t) * (size_t)J.lds);
-      J.posg = (int32_t*)(uintptr_t)dl.take(sizeof(int32_t) * (size_t)J.lds);
+      // (read by the deferred queries of the CTA grid only)
+      if (m.mode == 2) J.posg = (int32_t*)(uintptr_t)dl.take(sizeof(int32_t) * (size_t)J.lds);
       // strips of at least GRID_MIN_STRIP points: about c * len^(1/dj) of them
       // for warp-grid jobs (GRID_STRIPS_*_C), 256 for the CTA grid
       int64_t want = 256;
@@ -1209,11 +1216,39 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
         J.czlo32 = (float*)(uintptr_t)dl.take(sizeof(float) * (size_t)(side * side));
         J.czhi32 = (float*)(uintptr_t)dl.take(sizeof(float) * (size_t)(side * side));
       }
-      max_gkey = std::max<int64_t>(max_gkey, (int64_t)J.nstrips * std::max<int32_t>(1, J.nsub));
       J.sylo = (double*)(uintptr_t)dl.take(sizeof(double) * (size_t)J.nstrips);
       J.syhi = (double*)(uintptr_t)dl.take(sizeof(double) * (size_t)J.nstrips);
       J.sylo32 = (float*)(uintptr_t)dl.take(sizeof(float) * (size_t)J.nstrips);
       J.syhi32 = (float*)(uintptr_t)dl.take(sizeof(float) * (size_t)J.nstrips);
+      const int64_t strip_len = (len + J.nstrips - 1) / J.nstrips;
+      if (m.mode == 3 && J.nsub == 0 && !J.kform && strip_len <= STRIP_CAP) {
+        // two columns in strips that a block orders (egb_strips.cu)
+        const SortSeg& sa = segs[(size_t)m.sort_seg];
+        auto iv = inv_of_seg.find(m.sort_seg);
+        if (iv == inv_of_seg.end()) {
+          iv = inv_of_seg.emplace(m.sort_seg, inv_segs.size()).first;
+          InvSeg v{};
+          v.base = sa.out_base;
+          v.inv = (int32_t*)(uintptr_t)dl.take(sizeof(int32_t) * (size_t)len);
+          v.len = (int32_t)len;
+          v.src_begin = sa.src_begin;
+          inv_segs.push_back(v);
+          max_inv_len = std::max(max_inv_len, len);
+        }
+        StripJob sj{};
+        sj.base_a = sa.out_base;
+        sj.base_b = segs[(size_t)m.sort_seg_b].out_base;
+        sj.inv = inv_segs[iv->second].inv;  // an arena offset for now
+        sj.job = (int32_t)j;
+        sj.blk0 = nstrips_built;
+        strip_jobs.push_back(sj);
+        nstrips_built += J.nstrips;
+        strip_largest = std::max(strip_largest, (int)strip_len);
+        strip_table_jobs.push_back((int32_t)j);
+        continue;
+      }
+      strip_table_jobs.push_back((int32_t)j);
+      max_gkey = std::max<int64_t>(max_gkey, (int64_t)J.nstrips * std::max<int32_t>(1, J.nsub));
       J.gseg = (int32_t)gsegs.size();
       SortSeg g{};
       g.out_base = gsort_total;
@@ -1618,7 +1653,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   }
   std::vector<size_t> tab_sstart(jobs.size(), 0);
   std::vector<size_t> tab_cstart(jobs.size(), 0);
-  for (int32_t gj : grid_jobs) {
+  for (int32_t gj : strip_table_jobs) {
     const JobDev& J = jobs[(size_t)gj];
     tab_sstart[(size_t)gj] = tl.take(sizeof(int32_t) * (size_t)(J.nstrips + 1));
     if (J.nsub > 0) tab_cstart[(size_t)gj] = tl.take(sizeof(int32_t) * (size_t)(J.nstrips * J.nsub + 1));
@@ -1628,6 +1663,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     G.tab_runs = tl.take(sizeof(ItemRun) * G.runs.size());
     G.tab_cum = tl.take(sizeof(int32_t) * G.cum.size());
   }
+  const size_t tab_sjobs = tl.take(sizeof(StripJob) * strip_jobs.size());
+  const size_t tab_invsegs = tl.take(sizeof(InvSeg) * inv_segs.size());
   const size_t tab_wjobs = tl.take(sizeof(WmJob) * std::max<size_t>(wjobs.size(), 1));
   const size_t tab_wbuild = tl.take(sizeof(WmJob) * std::max<size_t>(wbuild.size(), 1));
   const size_t tab_gbjobs = tl.take(sizeof(GroupJob) * std::max<size_t>(gbjobs.size(), 1));
@@ -1764,7 +1801,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       J.c64g = (double*)(A + (uintptr_t)J.c64g);
       J.c32g = (float*)(A + (uintptr_t)J.c32g);
       J.idxg = (int32_t*)(A + (uintptr_t)J.idxg);
-      J.posg = (int32_t*)(A + (uintptr_t)J.posg);
+      if (J.posg) J.posg = (int32_t*)(A + (uintptr_t)J.posg);
       J.sylo = (double*)(A + (uintptr_t)J.sylo);
       J.syhi = (double*)(A + (uintptr_t)J.syhi);
       J.sylo32 = (float*)(A + (uintptr_t)J.sylo32);
@@ -1794,6 +1831,16 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     J.rad_given = D.rad_given;
     J.cnt = mjobs[j].is_knn ? nullptr : D.cnt[mjobs[j].s.slot];
     std::memcpy(H + tab_jobs + sizeof(JobDev) * j, &J, sizeof(JobDev));
+  }
+  for (size_t i = 0; i < strip_jobs.size(); ++i) {
+    StripJob sj = strip_jobs[i];
+    sj.inv = (const int32_t*)(A + (uintptr_t)sj.inv);
+    std::memcpy(H + tab_sjobs + sizeof(StripJob) * i, &sj, sizeof(sj));
+  }
+  for (size_t i = 0; i < inv_segs.size(); ++i) {
+    InvSeg v = inv_segs[i];
+    v.inv = (int32_t*)(A + (uintptr_t)v.inv);
+    std::memcpy(H + tab_invsegs + sizeof(InvSeg) * i, &v, sizeof(v));
   }
   for (Group& G : groups) {
     if (!G.items.empty()) std::memcpy(H + G.tab_items, G.items.data(), sizeof(WorkItem) * G.items.size());
@@ -1943,6 +1990,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   if (any_plain_copy)
     launch_materialize(tasks_d, (const JobDev*)dtab(tab_jobs), (int)jobs.size(), vals,
                        (const SortSeg*)dtab(tab_segs), max_lds, st);
+  launch_seg_inv((const InvSeg*)dtab(tab_invsegs), (int)inv_segs.size(), max_inv_len, vals, st);
+  launch_strip_build((const JobDev*)dtab(tab_jobs), (const StripJob*)dtab(tab_sjobs), (int)strip_jobs.size(),
+                     nstrips_built, strip_largest, keys, vals, st);
   if (!grid_jobs.empty()) {
     const JobDev* jobs_d = (const JobDev*)dtab(tab_jobs);
     const int32_t* gj_d = (const int32_t*)dtab(tab_gridjobs);
@@ -2254,6 +2304,7 @@ int egb_create(int device, egb_ctx** out) {
   egb_ctx* ctx = new egb_ctx();
   ctx->device = device;
   if (cudaSetDevice(device) != cudaSuccess || init_sort_kernels() != (int)cudaSuccess ||
+      init_strip_kernels() != (int)cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
       !create_fork_events(ctx)) {

@@ -104,6 +104,22 @@ __device__ __forceinline__ double bits_to_double(uint64_t u) {
   return __longlong_as_double((long long)u);
 }
 
+// fl32(d), rounded to nearest even, by integer operations in the normal float
+// range: the conversion instruction runs on the FP64 pipe (two lanes a clock).
+__device__ __forceinline__ float f32_nearest(double d) {
+  const uint64_t u = (uint64_t)__double_as_longlong(d);
+  const uint64_t a = u & 0x7fffffffffffffffull;
+  const uint32_t e = (uint32_t)(a >> 52);
+  if (e - (1023u - 126u) >= 253u) return __double2float_rn(d);  // below 2^-126, or 2^127 and beyond
+  const uint64_t r = a - ((uint64_t)(1023 - 127) << 52);
+  const uint32_t f = (uint32_t)((r + 0x0fffffffull + ((r >> 29) & 1ull)) >> 29);
+  return __uint_as_float(f | (uint32_t)(u >> 63) << 31);
+}
+// |d| < 1e37 (false for NaN), by the bits
+__device__ __forceinline__ bool fits32(double d) {
+  return ((uint64_t)__double_as_longlong(d) & 0x7fffffffffffffffull) < (uint64_t)__double_as_longlong(1e37);
+}
+
 // Order-preserving integer image of a double's bit pattern (raw: -0 sorts
 // just below +0) and its inverse.
 __device__ __forceinline__ uint64_t raw_key(uint64_t u) {
@@ -667,6 +683,25 @@ struct KeyIndexOut {
 };
 void launch_samples(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
                     const uint64_t* keys, const KeyIndexOut& out, cudaStream_t st);
+
+// egb_strips.cu: grid copies of two-column jobs by strip
+constexpr int STRIP_CAP = 4096;   // most points of a strip
+struct InvSeg {           // a sorted segment whose order is inverted
+  int64_t base;
+  int32_t* inv;
+  int32_t len, src_begin;
+};
+struct StripJob {
+  int64_t base_a, base_b; // its sorted segments of columns 0 and 1
+  const int32_t* inv;     // inverse of the column-0 order
+  int32_t job;
+  int32_t blk0;           // block of its first strip
+};
+int init_strip_kernels();
+void launch_seg_inv(const InvSeg* segs_d, int nsegs, int64_t max_len, const int32_t* sorted_vals,
+                    cudaStream_t st);
+void launch_strip_build(const JobDev* jobs_d, const StripJob* sjobs_d, int nsjobs, int nstrips, int largest,
+                        const uint64_t* keys, const int32_t* vals, cudaStream_t st);
 
 // egb_direct.cu: batches of small tasks (run_direct in egb_api.cu)
 constexpr int DIRECT_MAX_N = 4095;       // most samples of a task (shared memory)

@@ -330,12 +330,15 @@ __device__ __forceinline__ bool materialize_copy(const TaskDev& t, const JobDev&
       for (int c = 0; c < d; ++c) {
         const int tc = J.sp.cols[c];
         const double v = t.col[tc][w];
-        const double cv = v - J.center[c];
-        bad |= !(fabs(cv) < 1e37);
+        double cv = v - J.center[c];
+        if (!fits32(cv)) {
+          bad = true;
+          cv = fmin(fmax(cv, -1e37), 1e37);
+        }
         c64[(int64_t)c * J.lds + p] = v;
         // clamped so that FP32 distances stay finite; a job with a clamped
         // value never trusts its FP32 copy (TF_UNSAFE32)
-        c32[(int64_t)c * J.lds + p] = __double2float_rn(fmin(fmax(cv, -1e37), 1e37));
+        c32[(int64_t)c * J.lds + p] = f32_nearest(cv);
       }
     } else {
       idx[p] = J.seg_begin;
@@ -397,7 +400,7 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
       if (p < J.len) {
         const int32_t pa = gv[p];
         const int32_t w = va[pa];
-        J.posg[p] = pa;
+        if (J.posg) J.posg[p] = pa;
         J.idxg[p] = w;
         for (int c = 0; c < d; ++c) {
           const int tc = J.sp.cols[c];
@@ -408,14 +411,17 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
             kw[(int64_t)(2 * c) * J.lds + p] = (uint32_t)(k >> 32);
             kw[(int64_t)(2 * c + 1) * J.lds + p] = (uint32_t)k;
           } else {
-            const double cv = v - J.center[c];
-            bad |= !(fabs(cv) < 1e37);
+            double cv = v - J.center[c];
+            if (!fits32(cv)) {
+              bad = true;
+              cv = fmin(fmax(cv, -1e37), 1e37);
+            }
             J.c64g[(int64_t)c * J.lds + p] = v;
-            J.c32g[(int64_t)c * J.lds + p] = __double2float_rn(fmin(fmax(cv, -1e37), 1e37));
+            J.c32g[(int64_t)c * J.lds + p] = f32_nearest(cv);
           }
         }
       } else {
-        J.posg[p] = 0;
+        if (J.posg) J.posg[p] = 0;
         J.idxg[p] = J.seg_begin;
         for (int c = 0; c < d; ++c) {
           if (J.kform) {

@@ -245,6 +245,22 @@ def test_leaf_counts(oracle, d, data):
         assert np.array_equal(N.ball_count(pts, r), oracle.ball_count(pts, r)), n
 
 
+@pytest.mark.parametrize("data", ["independent", "cubic", "square", "steps", "constant", "huge"])
+@pytest.mark.parametrize("n", [4096, 4099, 20_001])
+def test_strip_layouts(oracle, n, data):
+    """Two-column grids built strip by strip: column-0 ranks spread over a
+    strip's buckets, crowded into few of them (columns that are functions of
+    each other), ties, and values that rule out the FP32 copy."""
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=n)
+    y = {"independent": rng.normal(size=n), "cubic": x ** 3, "square": x ** 2, "steps": np.round(x),
+         "constant": np.full(n, 2.5), "huge": x * 1e300}[data]
+    pts = np.column_stack((x, y))
+    for k in (3, 20):
+        assert np.array_equal(N.knn_eps(pts, k), oracle.knn_eps(pts, k)), k
+    assert np.array_equal(N.knn_eps(pts[:, ::-1], 3), oracle.knn_eps(pts, 3))
+
+
 def _small_tasks(rng, n, k, data):
     """Every estimator that the direct path serves, over n samples."""
     lab = rng.integers(0, 3, size=n).astype(np.int32)
