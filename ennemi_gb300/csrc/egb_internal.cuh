@@ -298,9 +298,11 @@ struct JobDev {
   // equal-count strips by their rank in column 1, each strip sorted by
   // column 0 -- with, per position, its position in the column-0 order
   double* c64g;
-  float* c32g;
+  float* c32g;            // [d][lds], or by point for the kNN kernels of d = 2, 3
+                          // (aos): grid_aos(d) floats each
   int32_t* idxg;
   int32_t* posg;
+  int32_t aos;
   int32_t nstrips;
   int32_t gseg;           // grid: its segment in the strip-key sort
   const int32_t* sstart;  // grid: nstrips + 1 strip starts (strip_start table)
@@ -345,6 +347,8 @@ constexpr int NEST_CELL_4D = 512;     // d >= 4 (200,000 4-D points, K = 4: 1.83
 constexpr int NEST_CELL_4D_FP64 = 256;
 constexpr int NEST_CELL_COUNT = 768;
 constexpr double NEST_SIDE_C = 1.07;
+// Floats per point of a by-point FP32 copy: a walk's next candidate is one load.
+__host__ __device__ constexpr int grid_aos(int d) { return d == 2 ? 2 : 4; }
 constexpr int GRID_QB = 128;     // queries per grid work item
 constexpr int GRID_TILE = 128;   // candidates per grid tile
 constexpr int GRID_MIN_STRIP = 64;

@@ -219,7 +219,7 @@ lcount_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ item
         // jobs with clamped values search everything
         const float tb = unsafe ? FINF : plan_margin(f32_up_of_bits(ob));
         int c0 = 0;
-        query_ranges<true>(J, g, sq, qb, tb, [&](int a, int b) {
+        query_ranges<true, 1>(J, g, sq, qb, tb, [&](int a, int b) {
           pairs += (unsigned)(b - a);
           for (int p0 = a; p0 < b; p0 += 32) {
             const bool in = p0 + lane < b;

@@ -41,7 +41,8 @@ __device__ __forceinline__ float coord_above(float v) {
 
 // Every range of positions within the planning bound tb of one query (warp
 // uniform), its strip sq first and then outward; f(a, b) may tighten tb.
-template <bool NEST, typename F>
+// STRIDE: floats from one position's column 0 to the next.
+template <bool NEST, int STRIDE, typename F>
 __device__ __forceinline__ void query_ranges(const JobDev* __restrict__ J, const float* __restrict__ g,
                                              int sq, const QueryBox& q, const float& tb, F&& f) {
   const int lane = threadIdx.x & 31;
@@ -57,12 +58,12 @@ __device__ __forceinline__ void query_ranges(const JobDev* __restrict__ J, const
       // whole blocks of 32 positions, from the first value of each: one load
       // and two ballots, and no candidate block is split
       const int p = a + 32 * lane;
-      const float x = p < b ? g[p] : __builtin_huge_valf();
+      const float x = p < b ? g[(int64_t)p * STRIDE] : __builtin_huge_valf();
       const int nl = __popc(__ballot_sync(FULL, x < xl)), nh = __popc(__ballot_sync(FULL, x <= xh));
       wl = a + 32 * max(nl - 1, 0);
       wh = min(b, a + 32 * nh);
     } else {
-      warp_window<float>(g, a, b, xl, xh, wl, wh);
+      warp_window<float, STRIDE>(g, a, b, xl, xh, wl, wh);
     }
     if (wl < wh) f(wl, wh);
   };

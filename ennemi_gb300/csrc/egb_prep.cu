@@ -417,7 +417,7 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
               cv = fmin(fmax(cv, -1e37), 1e37);
             }
             J.c64g[(int64_t)c * J.lds + p] = v;
-            J.c32g[(int64_t)c * J.lds + p] = f32_nearest(cv);
+            J.c32g[J.aos ? p * grid_aos(d) + c : (int64_t)c * J.lds + p] = f32_nearest(cv);
           }
         }
       } else {
@@ -430,7 +430,7 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
             kw[(int64_t)(2 * c + 1) * J.lds + p] = 0u;
           } else {
             J.c64g[(int64_t)c * J.lds + p] = 0.0;
-            J.c32g[(int64_t)c * J.lds + p] = 0.0f;
+            J.c32g[J.aos ? p * grid_aos(d) + c : (int64_t)c * J.lds + p] = 0.0f;
           }
         }
       }

@@ -175,15 +175,20 @@ strip_build_kernel(const JobDev* __restrict__ jobs, const StripJob* __restrict__
     J.idxg[p] = vb[i];
     J.c64g[p] = x0;
     J.c64g[J.lds + p] = x1;
-    J.c32g[p] = f32_nearest(d0);
-    J.c32g[J.lds + p] = f32_nearest(d1);
+    const float f0 = f32_nearest(d0), f1 = f32_nearest(d1);
+    if (J.aos) {
+      reinterpret_cast<float2*>(J.c32g)[p] = make_float2(f0, f1);
+    } else {
+      J.c32g[p] = f0;
+      J.c32g[J.lds + p] = f1;
+    }
   }
   if (s == J.nstrips - 1)  // the padding behind the last point
     for (int64_t p = J.len + tid; p < J.lds; p += THREADS) {
       J.idxg[p] = sb;
       for (int c = 0; c < 2; ++c) {
         J.c64g[c * J.lds + p] = 0.0;
-        J.c32g[c * J.lds + p] = 0.0f;
+        J.c32g[J.aos ? 2 * p + c : c * J.lds + p] = 0.0f;
       }
     }
   if (tid == 0) {

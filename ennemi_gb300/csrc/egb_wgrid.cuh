@@ -84,7 +84,8 @@ __device__ __forceinline__ float plan_margin(float t) { return __fmul_ru(t, 1.0f
 // Exact window of strip [s0, s1) for column-0 values [xlo, xhi]: the lower
 // half-warp finds the first position with x >= xlo, the upper half the first
 // with x > xhi.
-template <typename V>
+// STRIDE: elements from one position's column 0 to the next.
+template <typename V, int STRIDE = 1>
 __device__ __forceinline__ void warp_window(const V* x, int s0, int s1, V xlo, V xhi, int& wlo,
                                             int& whi) {
   const int lane = threadIdx.x & 31;
@@ -99,7 +100,7 @@ __device__ __forceinline__ void warp_window(const V* x, int s0, int s1, V xlo, V
     int p = small ? lo + l16 : lo + (int)((int64_t)(l16 + 1) * n / 17);
     const bool inr = p < hi;
     p = inr ? p : s0;
-    const V v = x[p];
+    const V v = x[(int64_t)p * STRIDE];
     const bool t = inr && (upper ? (v <= xhi) : (v < xlo));
     const unsigned b = __ballot_sync(0xffffffffu, t) & m;
     const int c = __popc(b);

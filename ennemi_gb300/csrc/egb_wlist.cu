@@ -53,6 +53,8 @@ __global__ void __launch_bounds__(WL_WARPS * 32)
 wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items, int nitems, int qb,
              int per, int* __restrict__ counter) {
   constexpr int DQ = D ? D : EGB_DMAX;
+  // two and three columns: grid copies by point (JobDev::aos)
+  constexpr int AOS = GRID && (D == 2 || D == 3) ? grid_aos(D) : 0;
   __shared__ __align__(8) uint32_t store[WL_WARPS][CandidateList<R>::WORDS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int split = (qb + per - 1) / per;  // parts of `per` queries of an item
@@ -86,7 +88,7 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
 #pragma unroll
       for (int c = 0; c < DQ; ++c) {
         if (D == 0 && c >= d) break;
-        qv[c] = g[(int64_t)c * lds + qp];
+        qv[c] = AOS ? g[(int64_t)qp * AOS + c] : g[(int64_t)c * lds + qp];
         am = fmaxf(am, fabsf(qv[c]));
       }
       const float mq = __fmaf_ru(am, 1.0f + 0x1p-22f, 0x1p-148f);  // >= max |q_c - c|
@@ -111,11 +113,19 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
           const int j = j0 + lane;
           float dd = __builtin_huge_valf();
           if (j < b && !(j >= ea && j < eb)) {
-            dd = fabsf(g[j] - qv[0]);
+            if constexpr (AOS == 2) {
+              const float2 p = reinterpret_cast<const float2*>(g)[j];
+              dd = fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1]));
+            } else if constexpr (AOS == 4) {
+              const float4 p = reinterpret_cast<const float4*>(g)[j];
+              dd = fmaxf(fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1])), fabsf(p.z - qv[D == 3 ? 2 : 0]));
+            } else {
+              dd = fabsf(g[j] - qv[0]);
 #pragma unroll
-            for (int c = 1; c < DQ; ++c) {
-              if (D == 0 && c >= d) break;
-              dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - qv[c]));
+              for (int c = 1; c < DQ; ++c) {
+                if (D == 0 && c >= d) break;
+                dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - qv[c]));
+              }
             }
           }
           list.push(dd, j);
@@ -125,7 +135,7 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
       // first; f may tighten the bound
       auto enumerate = [&](auto&& f) {
         if constexpr (!GRID) f(0, len);
-        else query_ranges<NEST>(J, g, sq, qbox, list.tb, f);
+        else query_ranges<NEST, AOS ? AOS : 1>(J, g, sq, qbox, list.tb, f);
       };
 
       uint64_t kth = INF_BITS;

@@ -33,6 +33,8 @@
 // Lanes without that margin (near ties, fewer than K candidates, jobs whose
 // centred values reach 1e37) walk again with U fixed, deciding in FP64 every
 // candidate with FP32 distance <= S.
+#include <type_traits>
+
 #include "egb_wgrid.cuh"
 
 namespace egb {
@@ -47,14 +49,15 @@ using wgrid_detail::dn_band32;
 constexpr int WW_WARPS = 4;
 // A lane whose walks screen more candidates than this in pass 0 leaves its
 // query to the cooperative phase (far-out queries of sparse regions).
-constexpr int WALK_BUDGET = 192;
+constexpr unsigned WALK_BUDGET = 192;
 
 // First position of [a, b) with x[p] >= v (x ascending).
+template <int P>  // floats per point
 __device__ __forceinline__ int lower_bound_f(const float* __restrict__ x, int a, int b, float v) {
   int n = b - a;
   while (n > 0) {
     const int h = n >> 1;
-    if (x[a + h] < v) {
+    if (x[(int64_t)(a + h) * P] < v) {
       a += h + 1;
       n -= h + 1;
     } else {
@@ -66,18 +69,19 @@ __device__ __forceinline__ int lower_bound_f(const float* __restrict__ x, int a,
 
 // The same from a guessed position g in [a, b): gallop towards the answer,
 // then bisect (exact for any g; a few steps when g is close).
+template <int P>
 __device__ __forceinline__ int lower_bound_from(const float* __restrict__ x, int a, int b, float v,
                                                 int g) {
   if (b <= a) return a;
   g = g < a ? a : (g >= b ? b - 1 : g);
   int lo, hi;  // x[lo - 1] < v <= x[hi] (lo = a, hi = b when absent)
-  if (x[g] < v) {
+  if (x[(int64_t)g * P] < v) {
     lo = g + 1;
     int step = 1;
     for (;;) {
       const int t = g + step;
       if (t >= b) { hi = b; break; }
-      if (!(x[t] < v)) { hi = t; break; }
+      if (!(x[(int64_t)t * P] < v)) { hi = t; break; }
       lo = t + 1;
       step <<= 1;
     }
@@ -87,23 +91,29 @@ __device__ __forceinline__ int lower_bound_from(const float* __restrict__ x, int
     for (;;) {
       const int t = g - step;
       if (t < a) { lo = a; break; }
-      if (x[t] < v) { lo = t + 1; break; }
+      if (x[(int64_t)t * P] < v) { lo = t + 1; break; }
       hi = t;
       step <<= 1;
     }
   }
-  return lower_bound_f(x, lo, hi, v);
+  return lower_bound_f<P>(x, lo, hi, v);
 }
 
-// Resident blocks per SM the register budget is cut for (measured: 2-D at
-// six, 3-D with K <= 4 at five; the others keep what they need)
-constexpr int walk_min_blocks(int D, int KMAX) { return D == 2 ? 6 : (D == 3 && KMAX == 4 ? 5 : 1); }
+// Resident blocks per SM the register budget is cut for: the walks are
+// latency-bound, so warps count for more than the registers spilled outside
+// them.  Measured (784 jobs of 180,000 2-D points, K = 4): 16.9, 14.1, 14.0, 16.5
+// ms at 6, 8, 10, 12 blocks; 1,000,000 3-D points, K = 4: 636, 604, 622 us at 5, 6,
+// 8; K = 7: 1131, 969, 971 at 3, 4, 6; 2-D at K = 8 (325 us) gains nothing from 8.
+constexpr int walk_min_blocks(int D, int KMAX) {
+  return D == 2 ? (KMAX == 4 ? 8 : 6) : (KMAX == 4 ? 6 : 4);
+}
 
 template <int D, int KMAX, bool NEST>
 __global__ void __launch_bounds__(WW_WARPS * 32, walk_min_blocks(D, KMAX))
 wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items, int nitems,
              int* __restrict__ counter) {
   constexpr float FINF = __builtin_huge_valf();
+  constexpr int P = grid_aos(D);  // floats per point of the FP32 copy
   const int lane = threadIdx.x & 31;
 
   for (;;) {
@@ -141,7 +151,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     float am = 0.0f;
 #pragma unroll
     for (int c = 0; c < D; ++c) {
-      qv[c] = exists ? g[(int64_t)c * lds + qp] : 0.0f;
+      qv[c] = exists ? g[(int64_t)qp * P + c] : 0.0f;
       am = fmaxf(am, fabsf(qv[c]));
     }
     const float mq = __fmaf_ru(am, 1.0f + 0x1p-22f, 0x1p-148f);
@@ -170,7 +180,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     float ufix = FINF, sfix = FINF;
     bool act = exists;     // this lane searches in the current pass
     bool heavy = false;    // pass 0 gave up: the warp finishes the query together
-    unsigned long long visited = 0;
+    unsigned visited = 0;
 
     auto exact_dist = [&](int j) -> uint64_t {
       uint64_t mm = 0;
@@ -182,22 +192,19 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
       }
       return mm;
     };
-    // screen bound S and planning bound plan_margin(U), kept current as the
-    // list changes (refresh); the planning bound is -1 when inactive
-    float sb_c = FINF, pb_c = FINF;
+    // up_band32(t, mq) with its constant part once (t = +inf stays +inf)
+    const float mqb = __fmaf_ru(mq, 0x1p-21f, 0x1p-100f);
+    auto up_band = [&](float t) { return __fmaf_ru(t, 1.0f + 0x1p-21f, mqb); };
+    // screen bound S, kept current as the list changes, at most FLT_MAX (gaps
+    // of real points are finite, those of an exhausted side +inf); U, the
+    // bound of the K-th distance; the planning bound is -1 when inactive
+    float sb_c = 0.0f, ub_c = 0.0f;
     auto refresh = [&]() {
-      if (pass1) {
-        sb_c = sfix;
-        pb_c = plan_margin(ufix);
-      } else {
-        const float u = up_band32(l32[KMAX - 1], mq);
-        sb_c = up_band32(u, mq);
-        pb_c = plan_margin(u);
-      }
+      ub_c = pass1 ? ufix : up_band(l32[KMAX - 1]);
+      sb_c = fminf(pass1 ? sfix : up_band(ub_c), __int_as_float(0x7f7fffff));
     };
     refresh();
-    auto sbound = [&]() -> float { return sb_c; };
-    auto pbound = [&]() -> float { return act ? pb_c : -1.0f; };
+    auto pbound = [&]() -> float { return act ? plan_margin(ub_c) : -1.0f; };
     auto visit = [&](int j, float dd) {
       ++visited;
       if (!pass1) {
@@ -214,45 +221,68 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     };
     // This lane's walk of [a, b) outward from p0 (the first position whose
     // column 0 is >= the query's): nearer side first, until both sides pass
-    // S or end.
-    auto walk = [&](int a, int b, int p0) {
+    // S or end.  more(a, b, p0): the lane's next range, if any; a warp's lanes
+    // need not finish their ranges together.
+    auto walk = [&](int a, int b, int p0, auto&& more) {
+      // the next candidates on both sides, loaded ahead of their visit
+      using Point = typename std::conditional<D == 2, float2, float4>::type;
+      const Point* __restrict__ pt = reinterpret_cast<const Point*>(g);
       int L = p0 - 1, R = p0;
-      float dl = L >= a ? qv[0] - g[L] : FINF;
-      float dr = R < b ? g[R] - qv[0] : FINF;
+      Point cl{}, cr{};
+      float dl = FINF, dr = FINF;
+      auto next_l = [&]() {
+        dl = FINF;
+        if (L >= a) {
+          cl = pt[L];
+          dl = qv[0] - cl.x;
+        }
+      };
+      auto next_r = [&]() {
+        dr = FINF;
+        if (R < b) {
+          cr = pt[R];
+          dr = cr.x - qv[0];
+        }
+      };
+      next_l();
+      next_r();
       for (;;) {
         const bool go_l = dl <= dr;
         const float dx = go_l ? dl : dr;
-        // both sides exhausted (real gaps are finite: values are clamped to
-        // +-1e37), or the nearer side is beyond the screen bound
-        if (!(dx < FINF) || !(dx <= sbound())) break;
-        if (!pass1 && visited >= (unsigned long long)WALK_BUDGET) {
+        if (!(dx <= sb_c)) {  // both sides exhausted or beyond the screen bound
+          if (!more(a, b, p0)) break;
+          L = p0 - 1;
+          R = p0;
+          next_l();
+          next_r();
+          continue;
+        }
+        if (!pass1 && visited >= WALK_BUDGET) {
           heavy = true;  // leave it to the cooperative phase
           act = false;
           break;
         }
         const int j = go_l ? L : R;
-        float dd = dx;
-#pragma unroll
-        for (int c = 1; c < D; ++c) {
-          dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - qv[c]));
-        }
-        visit(j, dd);
+        float dd = fmaxf(dx, fabsf((go_l ? cl.y : cr.y) - qv[1]));
+        if constexpr (D == 3) dd = fmaxf(dd, fabsf((go_l ? cl.z : cr.z) - qv[2]));
         if (go_l) {
           --L;
-          dl = L >= a ? qv[0] - g[L] : FINF;
+          next_l();
         } else {
           ++R;
-          dr = R < b ? g[R] - qv[0] : FINF;
+          next_r();
         }
+        visit(j, dd);
       }
     };
+    auto none = [](int&, int&, int&) { return false; };
     // the query's relative position in its own strip (cell): where to guess
     // its column 0 in another
     const int ha = NEST ? cst[sq * S2 + hc2] : sst[sq];
     const int hb = NEST ? cst[sq * S2 + hc2 + 1] : sst[sq + 1];
     const float frel = hb > ha ? (float)(qp - ha) / (float)(hb - ha) : 0.0f;
     auto walk_range = [&](int a, int b) {
-      walk(a, b, lower_bound_from(g, a, b, qv[0], a + (int)(frel * (float)(b - a))));
+      walk(a, b, lower_bound_from<P>(g, a, b, qv[0], a + (int)(frel * (float)(b - a))), none);
     };
     // The warp visits strips and cells together; a lane walks the ones its
     // planning bound reaches.
@@ -299,10 +329,10 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     auto search = [&]() {
       if (NEST) {
         const int cb = sq * S2;
-        if (act) walk(cst[cb + hc2], cst[cb + hc2 + 1], qp);
+        if (act) walk(cst[cb + hc2], cst[cb + hc2 + 1], qp, none);
         cells(sq, hc2, hc2);
       } else {
-        if (act) walk(sst[sq], sst[sq + 1], qp);
+        if (act) walk(sst[sq], sst[sq + 1], qp, none);
       }
       int up = sq + 1, dn = sq - 1;
       bool tu = true;
@@ -313,6 +343,35 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
         const bool any_u = __any_sync(0xffffffffu, ou);
         const bool any_d = __any_sync(0xffffffffu, od);
         if (!any_u && !any_d) break;
+        if constexpr (!NEST) {
+          // the next strips above and below in one loop of walks
+          const bool nu = any_u && strip_reach(up, t), nd = any_d && strip_reach(dn, t);
+          const int s1 = up, s2 = dn;
+          up += any_u;
+          dn -= any_d;
+          int a1 = 0, b1 = 0, p1 = 0, a2 = 0, b2 = 0, p2 = 0;
+          if (nu) {
+            a1 = sst[s1];
+            b1 = sst[s1 + 1];
+            p1 = lower_bound_from<P>(g, a1, b1, qv[0], a1 + (int)(frel * (float)(b1 - a1)));
+          }
+          if (nd) {
+            a2 = sst[s2];
+            b2 = sst[s2 + 1];
+            p2 = lower_bound_from<P>(g, a2, b2, qv[0], a2 + (int)(frel * (float)(b2 - a2)));
+          }
+          bool pending = nu && nd;
+          auto second = [&](int& a, int& b, int& p0) {
+            if (!pending || !strip_reach(s2, pbound())) return false;
+            pending = false;
+            a = a2;
+            b = b2;
+            p0 = p2;
+            return true;
+          };
+          if (nu || nd) walk(nu ? a1 : a2, nu ? b1 : b2, nu ? p1 : p2, second);
+          continue;
+        }
         int s;
         if ((tu && any_u) || !any_d) {
           s = up++;
@@ -321,11 +380,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
           s = dn--;
           tu = true;
         }
-        if (NEST) {
-          cells(s, start_cell(s), -1);
-        } else if (strip_reach(s, t)) {
-          walk_range(sst[s], sst[s + 1]);
-        }
+        cells(s, start_cell(s), -1);
       }
     };
 
@@ -362,10 +417,10 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
           ix2[s2] = 0;
         }
         float rej2 = FINF;
-        unsigned long long cvis = 0;
+        unsigned cvis = 0;
         auto crange = [&](int a, int b) {
           int wl, wh;
-          wgrid_detail::warp_window<float>(g, a, b, fminf(__fsub_rd(oxl, tb), 1e37f),
+          wgrid_detail::warp_window<float, P>(g, a, b, fminf(__fsub_rd(oxl, tb), 1e37f),
                                            fmaxf(__fadd_ru(oxh, tb), -1e37f), wl, wh);
           for (int j0 = wl; j0 < wh; j0 += 32) {
             const int j = j0 + lane;
@@ -373,7 +428,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
               float dd = 0.0f;
 #pragma unroll
               for (int c = 0; c < D; ++c) {
-                dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - oq[c]));
+                dd = fmaxf(dd, fabsf(g[(int64_t)j * P + c] - oq[c]));
               }
               ++cvis;
               // <= : the owner's own K-th candidate lies exactly at the cap
@@ -461,7 +516,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
           float lo2 = fminf(rej2, v);
 #pragma unroll
           for (int o = 16; o; o >>= 1) lo2 = fminf(lo2, __shfl_xor_sync(0xffffffffu, lo2, o));
-          const unsigned long long cv = __reduce_add_sync(0xffffffffu, (unsigned)cvis);
+          const unsigned cv = __reduce_add_sync(0xffffffffu, cvis);
           if (lane == ol) {
 #pragma unroll
             for (int s2 = 0; s2 < KMAX; ++s2) {
@@ -512,7 +567,7 @@ wwalk_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
     }
     if (exists) J->eps[J->idxg[qp]] = bits_to_double(kth);
 
-    const unsigned long long tot = __reduce_add_sync(0xffffffffu, (unsigned)visited);
+    const unsigned long long tot = __reduce_add_sync(0xffffffffu, visited);
     const unsigned agm = __ballot_sync(0xffffffffu, again);
     if (lane == 0) {
       atomicAdd(J->stats + 0, tot);
