@@ -14,7 +14,7 @@
 //   kNN         1-D: merge on sorted keys; multi-D: tile kernels (brute force
 //               or slab), any-K select for k + 1 > 32
 //   radius      rad = eps - 1e-12
-//   counts      1-D: gallop + bisect on sorted keys; multi-D: tile kernels
+//   counts      1-D: windows of the sorted values; multi-D: tile kernels
 //   combine     per-task term sums (psi table / log) + zero flags
 //   download    partial sums, flags, device error word
 //
@@ -1281,19 +1281,22 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   for (auto& pr : sorted_knn) {
     const SortSeg& sg = segs[(size_t)pr.first];
     SortedJob j{};
-    j.task = pr.second.task; j.kind = 0; j.slot = 0; j.K = pr.second.K;
+    j.task = pr.second.task; j.slot = 0; j.K = pr.second.K;
     j.base = sg.out_base; j.s1_base = sg.s1_base; j.s2_base = sg.s2_base;
     j.len = sg.len; j.blk0 = blk_knn;
     blk_knn += (sg.len + SORTED_BLOCK - 1) / SORTED_BLOCK;
     sj_knn.push_back(j);
   }
+  int64_t cnt_total = 0;
+  for (auto& pr : sorted_cnt) cnt_total += segs[(size_t)pr.first].len;
+  const int ball_span = cnt_total < (int64_t)BALL_SPAN * 2 * ctx->num_sms ? BALL_SPAN_FEW : BALL_SPAN;
   for (auto& pr : sorted_cnt) {
     const SortSeg& sg = segs[(size_t)pr.first];
     SortedJob j{};
-    j.task = pr.second.task; j.kind = 1; j.slot = pr.second.slot; j.K = 0;
+    j.task = pr.second.task; j.slot = pr.second.slot; j.K = 0;
     j.base = sg.out_base; j.s1_base = sg.s1_base; j.s2_base = sg.s2_base;
     j.len = sg.len; j.blk0 = blk_cnt;
-    blk_cnt += (sg.len + SORTED_BLOCK - 1) / SORTED_BLOCK;
+    blk_cnt += (sg.len + ball_span - 1) / ball_span;
     sj_cnt.push_back(j);
   }
 
@@ -2108,8 +2111,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     EGB_CUDA(cudaEventRecord(ctx->fork_ev[2], st));
     EGB_CUDA(cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev[2], 0));
   }
-  launch_sorted_jobs(tasks_d, (const SortedJob*)dtab(tab_sjc), (int)sj_cnt.size(), blk_cnt, kx, vals,
-                     fork_1d ? ctx->side_stream : st);
+  launch_ball_jobs(tasks_d, (const SortedJob*)dtab(tab_sjc), (int)sj_cnt.size(), blk_cnt, ball_span, kx,
+                   vals, fork_1d ? ctx->side_stream : st);
   if (fork_1d) EGB_CUDA(cudaEventRecord(ctx->join_ev[2], ctx->side_stream));
   if (timing) EGB_CUDA(cudaEventRecord(ctx->kev[11], st));
   if (timing) EGB_CUDA(cudaEventRecord(ctx->kev[4], st));

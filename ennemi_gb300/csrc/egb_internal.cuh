@@ -397,10 +397,11 @@ constexpr int DEFER_FRAC = 8;    // an item stops when <= 1/8 of its threads
                                  // still have unfinished queries
 constexpr int SIDE_CAP = 128;    // ... or after this many tiles beyond home
 
-// 1-D jobs on sorted arrays: one thread per sorted position.
+// 1-D jobs on sorted arrays, by sorted position: kNN (writes eps, one thread
+// per position) or counts (writes cnt[slot], see ball_jobs_kernel).
 struct SortedJob {
   int32_t task;
-  int32_t kind;           // 0 = kNN (writes eps), 1 = count (writes cnt[slot])
+  int32_t pad_;
   int32_t slot;
   int32_t K;              // k + 1 for kNN
   int64_t base;           // offset of the sorted segment in the key buffer
@@ -574,6 +575,14 @@ void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* 
 constexpr int SORTED_BLOCK = 128;
 void launch_sorted_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njobs,
                         int total_blocks, const KeyIndex& kx, const int32_t* perm, cudaStream_t st);
+// 1-D counts: sorted positions per block, and the same while a launch has
+// fewer than two blocks per SM (two jobs of 10,000 points: 5.2 us, against 8.0
+// with one thread per position and no window); the window's fill is then paid
+// for by 256 queries instead of 1024.
+constexpr int BALL_SPAN = 1024;
+constexpr int BALL_SPAN_FEW = 256;
+void launch_ball_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njobs, int total_blocks,
+                      int span, const KeyIndex& kx, const int32_t* perm, cudaStream_t st);
 
 // egb_knn.cu / egb_count.cu: tile kernels over materialised jobs.
 // dclass in {2, 3, 4} or 0 (generic d <= EGB_DMAX); kclass in {4, 8, 16, 32}.

@@ -152,52 +152,125 @@ __device__ __forceinline__ float f32_above(double v) {
 // bracket that is not finite or holds more than BALL_SCAN values (values far
 // outside the FP32 range, or all crowded into a few FP32 ulps) takes the
 // exact FP64 search of ball_keys on the 8-byte keys instead.
-//
-// g: the query's own position in the segment, the start of galloping
-// searches (measured faster for the 1-D counts, whose warps hold
-// consecutive positions), or -1: searches from the top of the samples.
 constexpr int BALL_SCAN = 16;
-__device__ __forceinline__ void ball_positions(const SegView& v, double q, double r, int g, int& lo,
-                                               int& hi) {
-  const int len = v.len;
+struct BallEnds {  // the brackets of one ball; ok: they decide (all finite)
+  float a1, b1, a0, b0;
+  bool ok;
+};
+__device__ __forceinline__ BallEnds ball_ends(double q, double r) {
   const uint64_t rb = (uint64_t)__double_as_longlong(r) & 0x7fffffffffffffffull;  // -0 as +0
   const float qd = f32_below(q), qu = f32_above(q);
   const float rd = f32_down_of_bits(rb), ru = f32_up_of_bits(rb);  // ru >= 2^-126
   const float rn = __int_as_float(__float_as_int(ru) + 1);         // next float above ru
+  BallEnds e;
+  e.a1 = __fadd_rd(qd, rd), e.b1 = __fadd_ru(qu, rn);
+  e.a0 = __fsub_rd(qd, rn), e.b0 = __fsub_ru(qu, rd);
+  const uint64_t qb = (uint64_t)__double_as_longlong(q);
+  e.ok = isfinite(e.a1) && isfinite(e.b1) && isfinite(e.a0) && isfinite(e.b0) &&
+         ((qb >> 52) & 0x7ffu) != 0x7ffu;  // q finite, by its exponent bits
+  return e;
+}
+// The ends from the first positions whose FP32 value is >= a1 / >= a0: past
+// the values of the bracket that the FP64 predicate lets through.  False: the
+// bracket holds more than BALL_SCAN of them.
+__device__ __forceinline__ bool ball_right(const SegView& v, const BallEnds& e, double q, double r,
+                                           int p, int& hi) {  // the first value failing P
+  int n = 0;
+  for (; p < v.len; ++p, ++n) {
+    if (__ldg(v.fk + p) > e.b1 || n == BALL_SCAN) break;  // value > b1: fails P
+    if (!(value_of(__ldg(v.keys + p)) - q <= r)) break;
+  }
+  hi = p;
+  return n < BALL_SCAN;
+}
+__device__ __forceinline__ bool ball_left(const SegView& v, const BallEnds& e, double q, double r,
+                                          int p, int& lo) {  // the first value satisfying Q
+  int n = 0;
+  for (; p < v.len; ++p, ++n) {
+    if (__ldg(v.fk + p) > e.b0 || n == BALL_SCAN) break;  // value > b0: satisfies Q
+    if (q - value_of(__ldg(v.keys + p)) <= r) break;
+  }
+  lo = p;
+  return n < BALL_SCAN;
+}
+// The exact key range, then its positions.
+__device__ __forceinline__ void ball_exact(const SegView& v, double q, double r, int& lo, int& hi) {
+  uint64_t kl, kr;
+  ball_keys(q, r, kl, kr);
+  kl = kl == 0x7fffffffffffffffull ? 0x8000000000000000ull : kl;  // raw -0 -> +0
+  lo = sampled_bound<uint64_t, false>(v.keys, v.s1, v.s2, v.len, kl);
+  hi = sampled_bound<uint64_t, true>(v.keys, v.s1, v.s2, v.len, kr);
+}
+// Searches from the top of the samples (queries in no order of this segment).
+__device__ __forceinline__ void ball_positions(const SegView& v, double q, double r, int& lo,
+                                               int& hi) {
+  const BallEnds e = ball_ends(q, r);
+  if (e.ok && ball_right(v, e, q, r, sampled_bound<float, false>(v.fk, v.fs1, v.fs2, v.len, e.a1), hi) &&
+      ball_left(v, e, q, r, sampled_bound<float, false>(v.fk, v.fs1, v.fs2, v.len, e.a0), lo))
+    return;
+  ball_exact(v, q, r, lo, hi);
+}
+// The ball of the value at position p of the segment itself, through a window
+// of the FP32 keys in shared memory: win[i] is the value at position
+// p - at + i (-inf before position 0, +inf from position len on), for i in
+// [at - HALF, at + HALF + 1).  p
+// is inside its ball, so the right end is searched in (p, p + HALF] and the
+// left end in [p - HALF, p), both in one branch-free loop; an end beyond the
+// window is found by galloping over the samples from the window's edge.
+//
+// win[at], the largest float <= q, stands for q itself: q lies in it and the
+// next float, r in rd and below the next one, rn.  The 8-byte key of p is
+// read, and FP64 arithmetic done, only for ends with values inside a bracket;
+// one loop serves both ends, so a warp pays for the longer of its lanes'
+// checks rather than for each end in turn.
+template <int HALF>
+__device__ __forceinline__ void ball_positions_at(const SegView& v, const float* win, int at, int p,
+                                                  double r, int& lo, int& hi) {
+  const int64_t rb = __double_as_longlong(r) & 0x7fffffffffffffffll;  // -0 as +0
+  const float qd = win[at], rd = f32_down_of_bits((uint64_t)rb);
+  const int qi = __float_as_int(qd);
+  const float qu = __int_as_float(qd < 0.0f ? qi - 1 : (qi & 0x7fffffff) + 1);
+  const float rn = __int_as_float(max(__float_as_int(rd) + 1, 0x00800000));
   const float a1 = __fadd_rd(qd, rd), b1 = __fadd_ru(qu, rn);
   const float a0 = __fsub_rd(qd, rn), b0 = __fsub_ru(qu, rd);
-  const uint64_t qb = (uint64_t)__double_as_longlong(q);
-  bool exact = isfinite(a1) && isfinite(b1) && isfinite(a0) && isfinite(b0) &&
-               ((qb >> 52) & 0x7ffu) != 0x7ffu;  // q finite, by its exponent bits
-  auto fbound = [&](float a) {  // first position whose value is >= a
-    return g >= 0 ? sampled_bound_from<float, false>(v.fk, v.fs1, len, a, g)
-                  : sampled_bound<float, false>(v.fk, v.fs1, v.fs2, len, a);
-  };
-  if (exact) {  // right end: the first value failing P
-    int p = fbound(a1), n = 0;
-    for (; p < len; ++p, ++n) {
-      if (__ldg(v.fk + p) > b1 || n == BALL_SCAN) break;  // value > b1: fails P
-      if (!(value_of(__ldg(v.keys + p)) - q <= r)) break;
+  bool ok = isfinite(b1) && isfinite(a0);  // a1 and b0 lie between
+  if (ok) {
+    int a = at + 1, b = at - HALF;
+#pragma unroll
+    for (int h = HALF / 2; h; h >>= 1) {
+      if (win[a + h - 1] < a1) a += h;
+      if (win[b + h - 1] < a0) b += h;
     }
-    hi = p;
-    exact = n < BALL_SCAN;
-  }
-  if (exact) {  // left end: the first value satisfying Q
-    int p = fbound(a0), n = 0;
-    for (; p < len; ++p, ++n) {
-      if (__ldg(v.fk + p) > b0 || n == BALL_SCAN) break;  // value > b0: satisfies Q
-      if (q - value_of(__ldg(v.keys + p)) <= r) break;
+    if (win[a] < a1) ++a;
+    if (win[b] < a0) ++b;
+    hi = p + (a - at);
+    lo = p + (b - at);
+    const bool out1 = a > at + HALF && hi < v.len, out0 = b == at - HALF && lo > 0;
+    bool more1 = out1 || !(win[a] > b1), more0 = out0 || !(win[b] > b0);
+    if (more1 || more0) {
+      if (out1) hi = sampled_bound_from<float, false>(v.fk, v.fs1, v.len, a1, hi);
+      if (out0) lo = sampled_bound_from<float, false>(v.fk, v.fs1, v.len, a0, lo);
+      const double q = value_of(__ldg(v.keys + p));
+      int n = 0;
+      do {  // one value of one end: hi to the first past P, lo to the first in Q
+        const int c = more1 ? hi : lo;
+        if (c >= v.len || __ldg(v.fk + c) > (more1 ? b1 : b0)) {
+          if (more1) more1 = false; else more0 = false;
+        } else {
+          const double x = value_of(__ldg(v.keys + c));
+          const bool in = (__double_as_longlong(x - q) & 0x7fffffffffffffffll) <= rb;  // |x - q| <= r
+          if (more1) {
+            if (in) ++hi; else more1 = false;
+          } else {
+            if (in) more0 = false; else ++lo;
+          }
+          ok = ++n < 2 * BALL_SCAN;
+        }
+      } while (ok && (more1 || more0));
     }
-    lo = p;
-    exact = n < BALL_SCAN;
+    if (ok) return;
   }
-  if (!exact) {  // the exact key range, then its positions
-    uint64_t kl, kr;
-    ball_keys(q, r, kl, kr);
-    kl = kl == 0x7fffffffffffffffull ? 0x8000000000000000ull : kl;  // raw -0 -> +0
-    lo = sampled_bound<uint64_t, false>(v.keys, v.s1, v.s2, len, kl);
-    hi = sampled_bound<uint64_t, true>(v.keys, v.s1, v.s2, len, kr);
-  }
+  ball_exact(v, value_of(__ldg(v.keys + p)), r, lo, hi);
 }
 #endif
 

@@ -487,55 +487,117 @@ __global__ void scan_down_kernel(uint32_t* __restrict__ data, int64_t n,
 }
 
 // --------------------------------------------------------- sorted jobs ----
-__global__ void sorted_jobs_kernel(const TaskDev* __restrict__ tasks,
-                                   const SortedJob* __restrict__ jobs, int njobs,
-                                   const KeyIndex kx, const int32_t* __restrict__ perm_all) {
-  // the job of this block: last j with jobs[j].blk0 <= blockIdx.x
+// the job of this block: last j with jobs[j].blk0 <= blockIdx.x
+__device__ __forceinline__ int sorted_job_of(const SortedJob* __restrict__ jobs, int njobs) {
   int lo = 0, hi = njobs;
   while (hi - lo > 1) {
     const int m = (lo + hi) >> 1;
     if (jobs[m].blk0 <= (int)blockIdx.x) lo = m; else hi = m;
   }
-  const SortedJob jb = jobs[lo];
+  return lo;
+}
+
+// 1-D kNN distances: one thread per sorted position.
+__global__ void sorted_jobs_kernel(const TaskDev* __restrict__ tasks,
+                                   const SortedJob* __restrict__ jobs, int njobs,
+                                   const KeyIndex kx, const int32_t* __restrict__ perm_all) {
+  const SortedJob jb = jobs[sorted_job_of(jobs, njobs)];
   const int64_t p = (int64_t)((int)blockIdx.x - jb.blk0) * SORTED_THREADS + threadIdx.x;
   const int64_t len = jb.len;
   if (p >= len) return;
   const uint64_t* __restrict__ keys = kx.keys + jb.base;
-  const int32_t i = perm_all[jb.base + p];
-  const TaskDev t = tasks[jb.task];
   const double q = value_of(keys[p]);
   const double INF = __longlong_as_double((long long)INF_BITS);
-
-  if (jb.kind == 0) {  // (k+1)-NN distance, self included; +inf if too few
-    int64_t L = p - 1, R = p + 1;
-    double d = (jb.K <= len) ? 0.0 : INF;
-    if (jb.K <= len) {
-      for (int s = 1; s < jb.K; ++s) {
-        const double dl = L >= 0 ? q - value_of(keys[L]) : INF;
-        const double dr = R < len ? value_of(keys[R]) - q : INF;
-        if (dl <= dr) { d = dl; --L; } else { d = dr; ++R; }
-      }
+  // (k+1)-NN distance, self included; +inf if too few
+  int64_t L = p - 1, R = p + 1;
+  double d = (jb.K <= len) ? 0.0 : INF;
+  if (jb.K <= len) {
+    for (int s = 1; s < jb.K; ++s) {
+      const double dl = L >= 0 ? q - value_of(keys[L]) : INF;
+      const double dr = R < len ? value_of(keys[R]) - q : INF;
+      if (dl <= dr) { d = dl; --L; } else { d = dr; ++R; }
     }
-    t.eps[i] = d;
-    return;
   }
+  tasks[jb.task].eps[perm_all[jb.base + p]] = d;
+}
 
-  const double r = radius_of(t.rad, t.rad_given, i);
-  const int rc = radius_class(r);
-  int32_t count;
-  if (rc == 0) {
-    count = 0;
-  } else if (rc == 2) {
-    count = (int32_t)len;
-  } else {
-    // The ball is one run of sorted positions; its ends come from FP32
-    // brackets and the segment's samples (ball_positions, egb_search.cuh).
-    int lo, hi;
-    ball_positions(seg_view(kx, jb.base, jb.s1_base, jb.s2_base, (int)len), q, r, (int)p, lo, hi);
-    count = (int32_t)(hi - lo);
-    if (jb.ranges) jb.ranges[i] = make_int2(lo, hi);
+// 1-D ball counts.  A block takes BALL_SPAN consecutive sorted
+// positions and searches the ends of their balls in the FP32 values of those
+// positions and BALL_HALF to either side, held in shared memory (21 KB).
+//
+// Bound by the latency of the search (12 dependent shared loads, both ends at
+// once) and of the two gathers by working index (radius in, count out), with
+// the L1 pipe about half busy, so what counts is warps in flight: 32
+// registers, 8 blocks an SM.  784 jobs of 180,000 points: 11.5 ms with
+// galloping searches over global samples, one position per thread; 8.1 ms
+// from the window at 5 or 6 blocks an SM; 6.5 ms at 8.  2016 pairs of 50,000:
+// 7.8 -> 4.3 ms.  BALL_HALF: with 4096 five or six blocks fit (8.1 / 5.4 ms);
+// with 1024 too many ends fall outside (10.5 / 6.3 ms at 5 blocks against 8.7
+// / 5.6).  Blocks of 512 threads: 7.6 / 5.2 ms.
+constexpr int BALL_THREADS = 256;
+constexpr int BALL_HALF = 2048;
+template <int PER>
+__global__ void __launch_bounds__(BALL_THREADS, 8)
+ball_jobs_kernel(const TaskDev* __restrict__ tasks, const SortedJob* __restrict__ jobs, int njobs,
+                 const KeyIndex kx, const int32_t* __restrict__ perm_all) {
+  constexpr int SPAN = BALL_THREADS * PER;
+  constexpr int WIN = SPAN + 2 * BALL_HALF + 4;
+  __shared__ __align__(16) float win[WIN];
+  const SortedJob& jb = jobs[sorted_job_of(jobs, njobs)];
+  const int64_t base = jb.base;
+  const int len = jb.len;
+  const int p0 = ((int)blockIdx.x - jb.blk0) * SPAN;
+  const TaskDev& t = tasks[jb.task];
+
+  int32_t idx[PER];
+  double rad[PER];
+#pragma unroll
+  for (int s = 0; s < PER; ++s) {
+    const int p = p0 + s * BALL_THREADS + (int)threadIdx.x;
+    idx[s] = p < len ? __ldg(perm_all + base + p) : -1;
   }
-  t.cnt[jb.slot][i] = count;
+  // the window of FP32 keys, from a position whose address is 16-byte aligned
+  const int off = (int)(base & 3);
+  const int w0 = p0 - BALL_HALF - off;
+  const float* fk = kx.fkeys + base;
+  for (int j = (int)threadIdx.x; j < WIN / 4; j += BALL_THREADS) {
+    const int g = w0 + 4 * j;
+    float4 v;
+    if (g >= 0 && g + 4 <= len) {
+      v = __ldg((const float4*)(fk + g));
+    } else {
+      const float INF = __int_as_float(0x7f800000);
+      auto at = [&](int p) { return p < 0 ? -INF : p < len ? __ldg(fk + p) : INF; };
+      v = make_float4(at(g), at(g + 1), at(g + 2), at(g + 3));
+    }
+    *(float4*)(win + 4 * j) = v;
+  }
+#pragma unroll
+  for (int s = 0; s < PER; ++s) rad[s] = idx[s] >= 0 ? radius_of(t.rad, t.rad_given, idx[s]) : 0.0;
+  __syncthreads();
+
+  const SegView v = seg_view(kx, base, jb.s1_base, jb.s2_base, len);
+  int32_t* __restrict__ cnt = t.cnt[jb.slot];
+  int2* __restrict__ ranges = jb.ranges;
+#pragma unroll
+  for (int s = 0; s < PER; ++s) {
+    if (idx[s] < 0) break;
+    const int at = off + BALL_HALF + s * BALL_THREADS + (int)threadIdx.x;
+    const int p = w0 + at;
+    const int rc = radius_class(rad[s]);
+    int32_t count;
+    if (rc == 0) {
+      count = 0;
+    } else if (rc == 2) {
+      count = len;
+    } else {
+      int lo, hi;
+      ball_positions_at<BALL_HALF>(v, win, at, p, rad[s], lo, hi);
+      count = hi - lo;
+      if (ranges) ranges[idx[s]] = make_int2(lo, hi);
+    }
+    cnt[idx[s]] = count;
+  }
 }
 
 // ----------------------------------------------------------- grid keys ----
@@ -768,6 +830,17 @@ void launch_sorted_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njo
   if (njobs <= 0 || total_blocks <= 0) return;
   sorted_jobs_kernel<<<(unsigned)total_blocks, SORTED_THREADS, 0, st>>>(tasks_d, jobs_d, njobs, kx,
                                                                         perm);
+  count_launch();
+}
+
+void launch_ball_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njobs, int total_blocks,
+                      int span, const KeyIndex& kx, const int32_t* perm, cudaStream_t st) {
+  if (njobs <= 0 || total_blocks <= 0) return;
+  const unsigned nb = (unsigned)total_blocks;
+  if (span == BALL_THREADS)
+    ball_jobs_kernel<1><<<nb, BALL_THREADS, 0, st>>>(tasks_d, jobs_d, njobs, kx, perm);
+  else
+    ball_jobs_kernel<4><<<nb, BALL_THREADS, 0, st>>>(tasks_d, jobs_d, njobs, kx, perm);
   count_launch();
 }
 

@@ -375,7 +375,7 @@ wm_count_kernel(const TaskDev* __restrict__ tasks, const WmJob* __restrict__ job
   } else {
     const SegView va = seg_view(kx, J.base_a, J.s1_a, J.s2_a, len);
     int alo, ahi, blo, bhi;
-    ball_positions(va, value_of(va.keys[i]), r, -1, alo, ahi);
+    ball_positions(va, value_of(va.keys[i]), r, alo, ahi);
     if (J.brange) {  // the b ball, as the 1-D count of column b found it
       const int2 br = __ldg(J.brange + w);
       blo = br.x;
@@ -383,7 +383,7 @@ wm_count_kernel(const TaskDev* __restrict__ tasks, const WmJob* __restrict__ job
     } else {
       const SegView vb = seg_view(kx, J.base_b, J.s1_b, J.s2_b, len);
       const int jb = min(max(J.inv_b[w - J.seg_begin], 0), len - 1);
-      ball_positions(vb, value_of(__ldg(vb.keys + jb)), r, -1, blo, bhi);
+      ball_positions(vb, value_of(__ldg(vb.keys + jb)), r, blo, bhi);
     }
     count = wm_rect(J, alo, ahi, blo, bhi);
   }

@@ -245,6 +245,44 @@ def test_leaf_counts(oracle, d, data):
         assert np.array_equal(N.ball_count(pts, r), oracle.ball_count(pts, r)), n
 
 
+@pytest.mark.parametrize("data", ["normal", "dyadic", "duplicates", "fine", "tiny", "huge"])
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 2049, 9001, 311_295, 311_297, 400_003])
+def test_window_counts(n, data):
+    """1-D ball counts through windows of the sorted values: a few points and
+    the first sizes of each block span, balls from nothing to everything (ends
+    inside the window, past its edge and past the segment), boundaries on exact
+    distances, and values that an FP32 bracket cannot tell apart or hold."""
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=n)
+    r = np.abs(rng.normal(0.0, 3.0 / np.sqrt(n), size=n))
+    if data == "dyadic":
+        x = rng.integers(-3000, 3000, size=n) / 64.0
+        r = rng.integers(0, 120, size=n) / 64.0
+    elif data == "duplicates":
+        x = rng.integers(0, 6, size=n).astype(np.float64)
+        r = rng.integers(0, 4, size=n) - 1e-12
+    elif data == "fine":
+        x = 1.0 + x * 1e-9
+        r *= 1e-9
+    elif data == "tiny":
+        x *= 1e-42
+        r *= 1e-42
+    elif data == "huge":
+        x[::2] *= 1e300
+        r[::3] *= 1e300
+    r[::97] = -1e-13
+    r[1::97] = 0.0
+    r[2::97] = np.inf
+    r[3::97] = 1e3
+    r[4::97] = np.nan
+    r[5::97] = -0.0
+    r[6::97] = 0.5
+    got = N.ball_count(x[:, None], r)
+    rows = np.unique(np.concatenate([np.arange(min(n, 40)), np.argsort(x)[[0, -1]], rng.integers(0, n, 160)]))
+    for i in rows:
+        assert got[i] == np.count_nonzero(np.abs(x - x[i]) <= r[i]), i
+
+
 @pytest.mark.parametrize("data", ["independent", "cubic", "square", "steps", "constant", "huge"])
 @pytest.mark.parametrize("n", [4096, 4099, 20_001])
 def test_strip_layouts(oracle, n, data):
