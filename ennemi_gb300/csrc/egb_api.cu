@@ -1115,6 +1115,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   const size_t off_fs1 = dl.take(sizeof(float) * (size_t)std::max<int64_t>(s1_total, 1));
   const size_t off_fs2 = dl.take(sizeof(float) * (size_t)std::max<int64_t>(s2_total, 1));
   const size_t sweep_bytes = sort_sweep_bytes(nblk_os, (int)segs.size());
+  const bool sort_codes = sort_first > 0 && sort_total >= SORT_CODES_MIN;
 
   // multi-D job blocks
   std::vector<JobDev> jobs(mjobs.size());
@@ -1970,15 +1971,14 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   uint64_t* keys = (uint64_t*)(A + off_keys_a);
   int32_t* vals = (int32_t*)(A + off_vals_a);
   if (timing) EGB_CUDA(cudaEventRecord(ctx->kev[8], st));
-  launch_sort(slots_d, (const SortSeg*)dtab(tab_segs), (const int32_t*)dtab(tab_blkseg), nblk_sort,
-              (const int32_t*)dtab(tab_osblkseg), nblk_os, (int)segs.size(), keys,
-              (uint64_t*)(A + off_keys_b), vals, (int32_t*)(A + off_vals_b), A + off_sweep,
-              sort_first, err_d, st, timing ? ctx->kev + 12 : nullptr);
   const KeyIndexOut ko{(float*)(A + off_fk), (uint64_t*)(A + off_s1), (uint64_t*)(A + off_s2),
                        (float*)(A + off_fs1), (float*)(A + off_fs2)};
   const KeyIndex kx{keys, ko.fkeys, ko.s1, ko.s2, ko.fs1, ko.fs2};
-  launch_samples((const SortSeg*)dtab(tab_segs), (const int32_t*)dtab(tab_blkseg), nblk_sort, keys,
-                 ko, st);
+  launch_sort(slots_d, (const double*)(A + off_centers), (const SortSeg*)dtab(tab_segs),
+              (const int32_t*)dtab(tab_blkseg), nblk_sort, (const int32_t*)dtab(tab_osblkseg), nblk_os,
+              (int)segs.size(), keys, (uint64_t*)(A + off_keys_b), vals, (int32_t*)(A + off_vals_b), ko,
+              A + off_sweep, sort_first, sort_codes, ctx->num_sms, err_d, st,
+              timing ? ctx->kev + 12 : nullptr);
   // the rank-space matrices need only the sorted values: they build on the
   // side stream, joined back before their counts
   const bool fork_wm = !wbuild.empty();
@@ -2250,7 +2250,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   R.zr_bytes = zr_bytes;
   R.sort_keys = sort_total;
   R.sort_segs = (int64_t)segs.size();
-  R.sort_passes = 8 - sort_first;
+  R.sort_passes = sort_codes ? 4 : 8 - sort_first;
   const int64_t launches =
       use_graph ? (int64_t)ctx->graph_launches : (int64_t)(g_launches.load() - launches0);
   const int rc_fin = finish_batch(ctx, R, H, launches, results);

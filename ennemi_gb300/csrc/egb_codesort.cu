@@ -1,0 +1,275 @@
+// egb_codesort.cu -- the batch sort of large batches: four passes over 32-bit
+// codes instead of six over 64-bit keys.
+//
+// A value's code is the order-preserving image of its FP32 distance from the
+// column's midrange, rounded to nearest.  Subtraction and rounding are
+// monotone, so codes never order two values wrongly; values that FP32 cannot
+// tell apart share one.  A pass moves one 8-byte word per point (code, working
+// index), 16 bytes of traffic against the 24 of key and index apart, and four
+// digits stand for six.  The last kernel reads each point's value through its
+// index (the column lies in L2), orders the runs of equal codes by the full
+// key, and writes keys, indices and the samples of the searches
+// (egb_search.cuh): the stable order of the full keys, exactly.
+//
+// A run of more than TIE_RUN equal codes that is out of order, and any pair
+// that is (NaNs), marks its segment in Sweep::redo, and the passes over the
+// keys' own digits (egb_sort.cu) run for the marked segments.  They are
+// launched always and return at once when nothing is marked, so nothing waits
+// for the host.  Exact duplicates are in order as they come and mark nothing.
+//
+// 785 segments of 180,000 keys: load, passes, repair and samples 0.54 + 7.60 +
+// 0.35 + 0.28 ms with the keys' digits; here load, passes and unpack 0.57 + 3.23
+// + 1.19.  Eleven columns of a million: 0.81 -> 0.50 ms; 126 of 50,000: 0.45 ->
+// 0.28.  A pass moves 16 bytes a point at 2.8 TB/s and is bound by the chain
+// from digit counts to slots: barriers and shared-memory latency.  Blocks of
+// 256 threads, one per digit and sixteen words each, five to an SM (with a few
+// spills): 3.23 ms; four 3.27; 512 threads, three to an SM: 3.65; two: 4.48.
+// The unpack is bound by its gathers from L2: 512 threads 1.19 ms, 256 1.30.
+#include "egb_internal.cuh"
+#include "egb_search.cuh"
+#include "egb_sweep.cuh"
+
+namespace egb {
+
+namespace {
+
+constexpr int LOAD_THREADS = 256;
+constexpr int UNPACK_THREADS = 512;
+constexpr int PASS_THREADS = 256;          // one per digit
+constexpr int PASS_NW = PASS_THREADS / 32;
+constexpr int PASS_CH = OS_TILE / PASS_NW;   // words per warp
+constexpr int PASS_R = PASS_CH / 32;         // rounds per warp
+constexpr int TIE_RUN = 32;
+
+__device__ __forceinline__ uint32_t code_of(double x, double c) {
+  uint32_t b = __float_as_uint(f32_nearest(x - c));
+  if (b == 0x80000000u) b = 0u;  // -0 and +0 are one value
+  return (b >> 31) ? ~b : (b | 0x80000000u);
+}
+
+__global__ void __launch_bounds__(LOAD_THREADS)
+code_load_kernel(const BatchCol* __restrict__ slots, const double* __restrict__ centers,
+                 const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg,
+                 uint64_t* __restrict__ words, uint32_t* __restrict__ seg_hist) {
+  __shared__ uint32_t h[CODE_PASSES * 256];
+  const int si = blk_seg[blockIdx.x];
+  const SortSeg& s = segs[si];
+  for (int i = threadIdx.x; i < CODE_PASSES * 256; i += LOAD_THREADS) h[i] = 0;
+  __syncthreads();
+  const double mid = centers[s.slot], c = isfinite(mid) ? mid : 0.0;
+  const double* __restrict__ x = slots[s.slot].x + s.src_begin;
+  uint64_t* __restrict__ out = words + s.out_base;
+  const int i0 = ((int)blockIdx.x - s.blk0) * SORT_TILE;
+  const int i1 = min(i0 + SORT_TILE, s.len);
+  const int w0 = s.src_begin;
+  for (int i = i0 + (int)threadIdx.x; i < i1; i += LOAD_THREADS) {
+    const uint32_t code = code_of(__ldg(x + i), c);
+    out[i] = (uint64_t)code << 32 | (uint32_t)(w0 + i);
+#pragma unroll
+    for (int p = 0; p < CODE_PASSES; ++p) atomicAdd(&h[p * 256 + ((code >> (8 * p)) & 255u)], 1u);
+  }
+  __syncthreads();
+  uint32_t* g = seg_hist + ((size_t)si * ALL_PASSES + OS_PASSES) * 256;
+  for (int i = threadIdx.x; i < CODE_PASSES * 256; i += LOAD_THREADS)
+    if (h[i]) atomicAdd(g + i, h[i]);
+}
+
+// One digit of the codes: the single-sweep pass of egb_sort.cu on words.  A
+// tile's missing words read as the largest digit, behind all others.
+struct PassSmem {
+  uint32_t wcnt[PASS_NW][256];  // per-warp digit counts, then offsets
+  uint32_t dstart[256];         // first tile slot of each digit
+  uint32_t gbase[256];          // first output position of each digit, less dstart
+  uint2 warp_sum[PASS_NW];      // of the two digit scans
+  int tile;
+  uint64_t sk[OS_TILE];
+};
+
+__global__ void __launch_bounds__(PASS_THREADS, 5)
+code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ os_blk_seg,
+                 const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int digit,
+                 const uint32_t* __restrict__ seg_hist, unsigned long long* flags, int* tile_counter,
+                 uint32_t* err) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  PassSmem& S = *reinterpret_cast<PassSmem*>(raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) S.tile = atomicAdd(tile_counter, 1);
+  for (int i = tid; i < PASS_NW * 256; i += PASS_THREADS) (&S.wcnt[0][0])[i] = 0u;
+  __syncthreads();
+  const int b = S.tile;
+  const int si = os_blk_seg[b];
+  const int64_t base = segs[si].out_base;
+  const int len = segs[si].len, first = segs[si].os_blk0;
+  const int i0 = (b - first) * OS_TILE;
+  const int n = min(OS_TILE, len - i0);
+  const int shift = 8 * digit;
+  const uint32_t lt = (1u << lane) - 1u;
+  uint64_t key[PASS_R];
+  const uint64_t* __restrict__ src = in + base + i0 + warp * PASS_CH + lane;
+#pragma unroll
+  for (int r = 0; r < PASS_R; ++r)
+    key[r] = warp * PASS_CH + r * 32 + lane < n ? __ldg(src + r * 32) : ~0ull;
+  uint32_t rk[PASS_R];
+#pragma unroll
+  for (int r = 0; r < PASS_R; ++r) {
+    const uint32_t d = ((uint32_t)(key[r] >> 32) >> shift) & 255u;
+    uint32_t peers = 0xffffffffu;  // lanes with the same digit
+#pragma unroll
+    for (int bit = 0; bit < 8; ++bit) {
+      const uint32_t bb = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
+      peers &= ((d >> bit) & 1u) ? bb : ~bb;
+    }
+    const uint32_t before = S.wcnt[warp][d];
+    __syncwarp();
+    if ((peers & lt) == 0) S.wcnt[warp][d] = before + __popc(peers);
+    __syncwarp();
+    rk[r] = before + __popc(peers & lt);
+  }
+  __syncthreads();
+  uint32_t cnt = 0;  // digit tid: offsets of the warps, then its count in the tile
+#pragma unroll
+  for (int w = 0; w < PASS_NW; ++w) {
+    const uint32_t c = S.wcnt[w][tid];
+    S.wcnt[w][tid] = cnt;
+    cnt += c;
+  }
+  if (tid == 255) cnt -= (uint32_t)(OS_TILE - n);
+  const int pass = OS_PASSES + digit;
+  // exclusive scans over the digits of the tile's counts and of the segment's
+  const uint32_t tot = seg_hist[((size_t)si * ALL_PASSES + pass) * 256 + tid];
+  uint2 sum = make_uint2(cnt, tot);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t a = __shfl_up_sync(0xffffffffu, sum.x, o), c = __shfl_up_sync(0xffffffffu, sum.y, o);
+    if (lane >= o) sum.x += a, sum.y += c;
+  }
+  if (lane == 31) S.warp_sum[warp] = sum;
+  const uint32_t excl = sweep_look_back(flags, b, first, tid, pass, cnt, err);
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) sum.x += S.warp_sum[w].x, sum.y += S.warp_sum[w].y;
+  S.gbase[tid] = (sum.y - tot) + excl - (sum.x - cnt);
+  S.dstart[tid] = sum.x - cnt;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < PASS_R; ++r) {
+    const uint32_t d = ((uint32_t)(key[r] >> 32) >> shift) & 255u;
+    S.sk[S.dstart[d] + S.wcnt[warp][d] + rk[r]] = key[r];
+  }
+  __syncthreads();
+  for (int t = tid; t < n; t += PASS_THREADS) {
+    const uint64_t k = S.sk[t];
+    const uint32_t d = ((uint32_t)(k >> 32) >> shift) & 255u;
+    const uint32_t pos = S.gbase[d] + (uint32_t)t;
+    if (pos < (uint32_t)len)
+      out[base + pos] = k;
+    else
+      atomicOr(err, DERR_BAD_INDEX);
+  }
+}
+
+// Sorted words -> keys, indices and samples.  A block takes SORT_TILE
+// positions and 32 to either side: enough to see all of a run of TIE_RUN.
+// Warps with no inversion in sight write their positions as they are.
+__global__ void __launch_bounds__(UNPACK_THREADS)
+code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict__ segs,
+                   const int32_t* __restrict__ blk_seg, const uint64_t* __restrict__ words,
+                   uint64_t* __restrict__ keys, int32_t* __restrict__ vals, KeyIndexOut ko,
+                   uint32_t* redo, int nseg) {
+  constexpr int SPAN = SORT_TILE + 64;
+  __shared__ uint64_t sk[SPAN];
+  __shared__ uint32_t sc[SPAN];
+  __shared__ uint32_t inv[SPAN / 32];  // bit: below its predecessor
+  const int si = blk_seg[blockIdx.x];
+  const SortSeg& s = segs[si];
+  const int len = s.len;
+  const int i0 = ((int)blockIdx.x - s.blk0) * SORT_TILE;
+  const int64_t base = s.out_base;
+  const double* __restrict__ x = slots[s.slot].x;
+  const int lane = threadIdx.x & 31;
+  const int w0 = s.src_begin;
+  constexpr int R = SORT_TILE / UNPACK_THREADS;
+  uint32_t idx[R];
+#pragma unroll
+  for (int r = 0; r <= R; ++r) {  // the last round: the positions to either side
+    const int u = r < R ? 32 + r * UNPACK_THREADS + (int)threadIdx.x
+                        : (int)threadIdx.x < 32 ? (int)threadIdx.x : SORT_TILE + (int)threadIdx.x;
+    if (r == R && threadIdx.x >= 64) break;
+    const int p = i0 - 32 + u;
+    if (p >= 0 && p < len) {
+      const uint64_t w = __ldg(words + base + p);
+      const uint32_t i = min(max((int)(uint32_t)w, w0), w0 + len - 1);
+      if (r < R) idx[r] = i;
+      sk[u] = key_of_bits((uint64_t)__double_as_longlong(__ldg(x + i)));
+      sc[u] = (uint32_t)(w >> 32);
+    }
+  }
+  __syncthreads();
+  bool bad = false;
+  for (int u = threadIdx.x; u < SPAN; u += UNPACK_THREADS) {
+    const int p = i0 - 32 + u;
+    const bool below = u > 0 && p > 0 && p < len && sk[u] < sk[u - 1];
+    bad |= below && sc[u] != sc[u - 1];
+    const uint32_t m = __ballot_sync(__activemask(), below);
+    if (lane == 0) inv[u / 32] = m;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int u = 32 + r * UNPACK_THREADS + (int)threadIdx.x;
+    const int p = i0 - 32 + u;
+    if (p >= len) break;
+    const uint64_t k = sk[u];
+    int pos = p;
+    if (inv[u / 32 - 1] | inv[u / 32] | inv[u / 32 + 1]) {
+      const uint32_t c = sc[u];
+      const int ml = min(TIE_RUN, p), mr = min(TIE_RUN, len - 1 - p);
+      int l = 0, g = 0;
+      while (l < ml && sc[u - 1 - l] == c) ++l;
+      while (g < mr && sc[u + 1 + g] == c) ++g;
+      if (l + g + 1 <= TIE_RUN) {  // the rank among the run
+        int below = 0;
+        for (int j = u - l; j < u; ++j) below += sk[j] <= k;
+        for (int j = u + 1; j <= u + g; ++j) below += sk[j] < k;
+        pos = p - l + below;
+      } else {
+        bad |= l > 0 && k < sk[u - 1];
+      }
+    }
+    keys[base + pos] = k;
+    vals[base + pos] = (int32_t)idx[r];
+    put_samples(ko, s, pos, k);
+  }
+  if (bad) redo[si] = redo[nseg] = 1u;
+}
+static_assert(PASS_THREADS == 256, "one thread per digit");
+static_assert((SORT_TILE + 64) % 32 == 0 && TIE_RUN <= 32, "inversion words");
+
+}  // namespace
+
+int init_code_sort() {
+  return (int)cudaFuncSetAttribute(code_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(PassSmem));
+}
+
+void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
+                      const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
+                      int nseg, uint64_t* keys, uint64_t* words, int32_t* vals, const KeyIndexOut& ko,
+                      const Sweep& w, uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
+  code_load_kernel<<<nblk, LOAD_THREADS, 0, st>>>(slots_d, centers_d, segs_d, blk_seg_d, words, w.seg_hist);
+  count_launch();
+  if (pass_events) cudaEventRecord(pass_events[0], st);
+  uint64_t* in = words;  // an even number of passes: back in words
+  uint64_t* out = keys;
+  for (int d = 0; d < CODE_PASSES; ++d) {
+    code_pass_kernel<<<os_nblk, PASS_THREADS, sizeof(PassSmem), st>>>(
+        segs_d, os_blk_seg_d, in, out, d, w.seg_hist, w.flags, w.counters + OS_PASSES + d, err);
+    count_launch();
+    uint64_t* t = in; in = out; out = t;
+  }
+  if (pass_events) cudaEventRecord(pass_events[1], st);
+  code_unpack_kernel<<<nblk, UNPACK_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, words, keys, vals, ko, w.redo,
+                                                   nseg);
+  count_launch();
+}
+
+}  // namespace egb

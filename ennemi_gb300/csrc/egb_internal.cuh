@@ -115,6 +115,16 @@ __device__ __forceinline__ float f32_nearest(double d) {
   const uint32_t f = (uint32_t)((r + 0x0fffffffull + ((r >> 29) & 1ull)) >> 29);
   return __uint_as_float(f | (uint32_t)(u >> 63) << 31);
 }
+// The largest float <= d, with integer operations where d is in the normal
+// FP32 range.
+__device__ __forceinline__ float f32_floor(double d) {
+  const uint64_t u = (uint64_t)__double_as_longlong(d);
+  const uint64_t a = u & 0x7fffffffffffffffull;
+  if ((uint32_t)(a >> 52) - (1023u - 126u) >= 253u) return __double2float_rd(d);
+  const uint64_t r = a - ((uint64_t)(1023 - 127) << 52);
+  const uint32_t neg = (uint32_t)(u >> 63);
+  return __uint_as_float((uint32_t)((r + (neg ? 0x1fffffffull : 0ull)) >> 29) | neg << 31);
+}
 // |d| < 1e37 (false for NaN), by the bits
 __device__ __forceinline__ bool fits32(double d) {
   return ((uint64_t)__double_as_longlong(d) & 0x7fffffffffffffffull) < (uint64_t)__double_as_longlong(1e37);
@@ -526,6 +536,17 @@ struct KeyIndex {
   const float* fs1;       // fkeys[32 j]
   const float* fs2;       // fkeys[1024 j]
 };
+// The same arrays as the sort writes them.
+struct KeyIndexOut {
+  float* fkeys;
+  uint64_t* s1;
+  uint64_t* s2;
+  float* fs1;
+  float* fs2;
+};
+void launch_samples(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk, int grid,
+                    const uint64_t* keys, const KeyIndexOut& out, const uint32_t* redo, int nseg,
+                    cudaStream_t st);
 // Strip keys of the grid jobs.  launch_grid_inv: inv[p_B] = column-1 rank
 // of each point (by working offset).  launch_grid_key: keys[p] = cell key of
 // the point at column-0 position p -- its strip (column-1 rank * nstrips /
@@ -567,11 +588,26 @@ size_t sort_sweep_bytes(int os_nblk, int nseg);
 // Once per context, on its device: lets the passes use their shared memory
 // (above the 48 KB default); returns the cudaError_t.
 int init_sort_kernels();
-void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d,
-                 int nblk, const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys_a,
-                 uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b, void* sweep, int first,
+// codes: the code sort (egb_codesort.cu) does the work, and the passes run for
+// the segments it leaves over.  Writes the samples (ko) too.  Taken for large
+// batches, where it is faster in spite of the nine launches that then usually
+// find nothing to do.  Whole calls, digits and codes: 600,000 keys 383 and 388
+// us (segments of 20,000), 329 and 336 (100,000); a million 504 and 497, 405
+// and 403, 425 and 416 (500,000); 2.2 million 841 and 801, 648 and 604; five
+// million 1639 and 1522, 1190 and 1076, 1201 and 1081.
+constexpr int64_t SORT_CODES_MIN = 1 << 20;
+void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
+                 const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
+                 int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
+                 const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
                  uint32_t* err, cudaStream_t st,
                  cudaEvent_t* pass_events = nullptr);  // recorded around the passes alone
+struct Sweep;
+int init_code_sort();
+void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
+                      const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
+                      int nseg, uint64_t* keys, uint64_t* words, int32_t* vals, const KeyIndexOut& ko,
+                      const Sweep& w, uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events);
 constexpr int SORTED_BLOCK = 128;
 void launch_sorted_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njobs,
                         int total_blocks, const KeyIndex& kx, const int32_t* perm, cudaStream_t st);
@@ -685,17 +721,6 @@ void launch_wm_build(const WmJob* jobs_d, int njobs, int total_tiles, int max_le
 // Counts: one thread per query, in the a order; writes cnt[slot] of the task.
 void launch_wm_count(const TaskDev* tasks_d, const WmJob* jobs_d, int njobs, int total_blocks,
                      const KeyIndex& kx, const int32_t* sorted_vals, cudaStream_t st);
-// The arrays launch_samples writes: the FP32 copy and the samples of every
-// sorted segment (read back through a KeyIndex), after the sort.
-struct KeyIndexOut {
-  float* fkeys;
-  uint64_t* s1;
-  uint64_t* s2;
-  float* fs1;
-  float* fs2;
-};
-void launch_samples(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
-                    const uint64_t* keys, const KeyIndexOut& out, cudaStream_t st);
 
 // egb_strips.cu: grid copies of two-column jobs by strip
 constexpr int STRIP_CAP = 4096;   // most points of a strip

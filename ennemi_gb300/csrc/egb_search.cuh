@@ -42,6 +42,20 @@ __device__ __forceinline__ SegView seg_view(const KeyIndex& I, int64_t base, int
   return SegView{I.keys + base, I.fkeys + base, I.s1 + s1b, I.s2 + s2b, I.fs1 + s1b, I.fs2 + s2b, len};
 }
 
+// The entries of position p of a sorted segment, its key k given.
+__device__ __forceinline__ void put_samples(const KeyIndexOut& out, const SortSeg& sg, int p, uint64_t k) {
+  const float f = f32_floor(value_of(k));
+  out.fkeys[sg.out_base + p] = f;
+  if (p % SAMPLE1 == 0) {
+    out.s1[sg.s1_base + p / SAMPLE1] = k;
+    out.fs1[sg.s1_base + p / SAMPLE1] = f;
+    if (p % SAMPLE2 == 0) {
+      out.s2[sg.s2_base + p / SAMPLE2] = k;
+      out.fs2[sg.s2_base + p / SAMPLE2] = f;
+    }
+  }
+}
+
 // First index i in [lo, hi) with a[i] > x (UPPER) or a[i] >= x (lower);
 // hi if none.
 template <typename T, bool UPPER>

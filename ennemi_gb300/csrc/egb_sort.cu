@@ -5,7 +5,8 @@
 // concatenated key array.  Keys are the order-preserving uint64 image of the
 // FP64 value (key_of), the payload is the working index of the point.  The
 // batch sort takes stable 8-bit single-sweep LSD passes over the high 48 key
-// bits and repairs the rare runs tied there (below); the three-kernel pass
+// bits and repairs the rare runs tied there (below), for large batches only
+// over what the sort of 32-bit codes leaves (egb_codesort.cu); the three-kernel pass
 // -- histogram, exclusive scan, stable scatter -- serves the strip-key
 // passes of the grid layouts: its per-block histograms are laid out
 // segment-major, digit-next, block-minor, so ONE global exclusive scan
@@ -24,6 +25,7 @@
 
 #include "egb_internal.cuh"
 #include "egb_search.cuh"
+#include "egb_sweep.cuh"
 
 namespace egb {
 
@@ -183,39 +185,40 @@ sort_scatter_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict_
 // whole, so no other data needs ordering.  Every wait is bounded: past
 // OS_SPIN_LIMIT polls the tile records DERR_WAIT_TIMEOUT (the batch then
 // reports EGB_ERR_DEVICE) and goes on.
-constexpr int OS_PASSES = 8;
-constexpr int OS_SPIN_LIMIT = 1 << 22;
-
-__device__ __forceinline__ uint64_t key_of_bits(uint64_t u) {
-  u = u == 0x8000000000000000ull ? 0ull : u;  // -0 -> +0
-  return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
-}
-
+//
+// redo (else null): the kernels run after the code sort (egb_codesort.cu), for
+// the segments marked there alone -- usually none, so a launch has few blocks
+// and each takes many tiles.
 __global__ void __launch_bounds__(SORT_THREADS)
 onesweep_load_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict__ segs,
-                     const int32_t* __restrict__ blk_seg, uint64_t* __restrict__ keys,
-                     int32_t* __restrict__ vals, uint32_t* __restrict__ seg_hist, int first) {
+                     const int32_t* __restrict__ blk_seg, int nblk, uint64_t* __restrict__ keys,
+                     int32_t* __restrict__ vals, uint32_t* __restrict__ seg_hist, int first,
+                     const uint32_t* __restrict__ redo, int nseg) {
   __shared__ uint32_t h[OS_PASSES * 256];
-  const int b = blockIdx.x;
-  const int si = blk_seg[b];
-  const SortSeg s = segs[si];
-  for (int i = threadIdx.x; i < OS_PASSES * 256; i += SORT_THREADS) h[i] = 0;
-  __syncthreads();
-  const uint64_t* __restrict__ x = reinterpret_cast<const uint64_t*>(slots[s.slot].x + s.src_begin);
-  const int i0 = (b - s.blk0) * SORT_TILE;
-  const int i1 = min(i0 + SORT_TILE, s.len);
-  for (int i = i0 + threadIdx.x; i < i1; i += SORT_THREADS) {
-    const uint64_t k = key_of_bits(x[i]);
-    keys[s.out_base + i] = k;
-    vals[s.out_base + i] = s.src_begin + i;
+  if (redo && !redo[nseg]) return;
+  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    const int si = blk_seg[b];
+    if (redo && !redo[si]) continue;
+    const SortSeg s = segs[si];
+    for (int i = threadIdx.x; i < OS_PASSES * 256; i += SORT_THREADS) h[i] = 0;
+    __syncthreads();
+    const uint64_t* __restrict__ x = reinterpret_cast<const uint64_t*>(slots[s.slot].x + s.src_begin);
+    const int i0 = (b - s.blk0) * SORT_TILE;
+    const int i1 = min(i0 + SORT_TILE, s.len);
+    for (int i = i0 + threadIdx.x; i < i1; i += SORT_THREADS) {
+      const uint64_t k = key_of_bits(x[i]);
+      keys[s.out_base + i] = k;
+      vals[s.out_base + i] = s.src_begin + i;
 #pragma unroll
-    for (int p = 0; p < OS_PASSES; ++p)
-      if (p >= first) atomicAdd(&h[p * 256 + (uint32_t)((k >> (8 * p)) & 255u)], 1u);
+      for (int p = 0; p < OS_PASSES; ++p)
+        if (p >= first) atomicAdd(&h[p * 256 + (uint32_t)((k >> (8 * p)) & 255u)], 1u);
+    }
+    __syncthreads();
+    uint32_t* g = seg_hist + (size_t)si * ALL_PASSES * 256;
+    for (int i = threadIdx.x; i < OS_PASSES * 256; i += SORT_THREADS)
+      if (h[i]) atomicAdd(g + i, h[i]);
+    __syncthreads();
   }
-  __syncthreads();
-  uint32_t* g = seg_hist + (size_t)si * OS_PASSES * 256;
-  for (int i = threadIdx.x; i < OS_PASSES * 256; i += SORT_THREADS)
-    if (h[i]) atomicAdd(g + i, h[i]);
 }
 
 // A pass tile is OS_TILE keys on OS_THREADS threads (eight keys a thread);
@@ -233,151 +236,101 @@ struct OsSmem {
 };
 static_assert(OS_TILE % OS_NW == 0 && (OS_TILE / OS_NW) % 32 == 0, "whole warp rounds");
 
-// Exclusive scan over the 256 digits, one value per digit thread (tid <
-// 256: warps 0-7); every thread of the block calls it.
-__device__ __forceinline__ uint32_t digit_excl_scan(uint32_t v, uint32_t* ws) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t x = v;
-  if (tid < 256) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) ws[warp] = x;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = lane < 8 ? ws[lane] : 0u;
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    if (lane < 8) ws[lane] = w;
-  }
-  __syncthreads();
-  const uint32_t r = tid < 256 ? (warp ? ws[warp - 1] : 0u) + x - v : 0u;
-  __syncthreads();
-  return r;
-}
-
 __global__ void __launch_bounds__(OS_THREADS)
-onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ os_blk_seg,
+onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ os_blk_seg, int nblk,
                      const uint64_t* __restrict__ kin, const int32_t* __restrict__ vin,
                      uint64_t* __restrict__ kout, int32_t* __restrict__ vout, int pass,
                      const uint32_t* __restrict__ seg_hist, unsigned long long* flags,
-                     int* tile_counter, uint32_t* err) {
+                     int* tile_counter, uint32_t* err, const uint32_t* __restrict__ redo, int nseg) {
   constexpr int CH = OS_TILE / OS_NW;  // keys per warp
   constexpr int R = CH / 32;           // rounds per warp
   extern __shared__ __align__(16) unsigned char os_raw[];
   OsSmem& S = *reinterpret_cast<OsSmem*>(os_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) S.tile = atomicAdd(tile_counter, 1);
-  for (int i = tid; i < OS_NW * 256; i += OS_THREADS) (&S.wcnt[0][0])[i] = 0u;
-  __syncthreads();
-  const int b = S.tile;
-  const int si = os_blk_seg[b];
-  const SortSeg s = segs[si];
-  const int lb = b - s.os_blk0;
-  const int shift = 8 * pass;
-  const int i0 = lb * OS_TILE;
-  const int n = min(OS_TILE, s.len - i0);
-  const uint32_t lt = (1u << lane) - 1u;
-  uint64_t key[R];
-  int32_t val[R];
-  uint32_t dg[R], rk[R];
+  if (redo && !redo[nseg]) return;
+  for (bool more = true; more; more = redo != nullptr) {
+    if (tid == 0) S.tile = atomicAdd(tile_counter, 1);
+    for (int i = tid; i < OS_NW * 256; i += OS_THREADS) (&S.wcnt[0][0])[i] = 0u;
+    __syncthreads();
+    const int b = S.tile;
+    if (b >= nblk) break;
+    const int si = os_blk_seg[b];
+    __syncthreads();  // S.tile is read before the next tile's id lands
+    if (redo && !redo[si]) continue;
+    const SortSeg s = segs[si];
+    const int lb = b - s.os_blk0;
+    const int shift = 8 * pass;
+    const int i0 = lb * OS_TILE;
+    const int n = min(OS_TILE, s.len - i0);
+    const uint32_t lt = (1u << lane) - 1u;
+    uint64_t key[R];
+    int32_t val[R];
+    uint32_t dg[R], rk[R];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int t = warp * CH + r * 32 + lane;
-    const bool valid = t < n;
-    key[r] = valid ? kin[s.out_base + i0 + t] : 0ull;
-    val[r] = valid ? vin[s.out_base + i0 + t] : 0;
-    const uint32_t d = valid ? (uint32_t)(key[r] >> shift) & 255u : 256u + lane;
-    dg[r] = d;
-    uint32_t peers = 0xffffffffu;  // lanes with the same 9-bit digit
+    for (int r = 0; r < R; ++r) {
+      const int t = warp * CH + r * 32 + lane;
+      const bool valid = t < n;
+      key[r] = valid ? kin[s.out_base + i0 + t] : 0ull;
+      val[r] = valid ? vin[s.out_base + i0 + t] : 0;
+      const uint32_t d = valid ? (uint32_t)(key[r] >> shift) & 255u : 256u + lane;
+      dg[r] = d;
+      uint32_t peers = 0xffffffffu;  // lanes with the same 9-bit digit
 #pragma unroll
-    for (int bit = 0; bit < 9; ++bit) {
-      const uint32_t bb = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
-      peers &= ((d >> bit) & 1u) ? bb : ~bb;
-    }
-    const uint32_t before = valid ? S.wcnt[warp][d] : 0u;
-    __syncwarp();
-    if (valid && (peers & lt) == 0) S.wcnt[warp][d] = before + __popc(peers);
-    __syncwarp();
-    rk[r] = before + __popc(peers & lt);
-  }
-  __syncthreads();
-  uint32_t cnt = 0;  // digit tid: offsets of the warps, then its count in the tile
-  if (tid < 256) {
-#pragma unroll
-    for (int w = 0; w < OS_NW; ++w) {
-      const uint32_t c = S.wcnt[w][tid];
-      S.wcnt[w][tid] = cnt;
-      cnt += c;
-    }
-  }
-  // publish this tile's count of digit tid, then look back for the count of
-  // digit tid in the segment's earlier tiles
-  uint32_t excl = 0;
-  if (tid < 256) {
-    const unsigned long long tag = (unsigned long long)(pass + 1) << 56;
-    const unsigned long long INCL = 1ull << 55;
-    unsigned long long* mine = flags + (size_t)b * 256 + tid;
-    if (lb == 0) {
-      atomicExch(mine, tag | INCL | cnt);
-    } else {
-      atomicExch(mine, tag | cnt);
-      int pb = b - 1;
-      for (;;) {
-        const volatile unsigned long long* f = flags + (size_t)pb * 256 + tid;
-        unsigned long long w = *f;
-        int spins = 0;
-        while ((w >> 56) != (unsigned long long)(pass + 1)) {
-          if (++spins > OS_SPIN_LIMIT) {
-            atomicOr(err, DERR_WAIT_TIMEOUT);
-            w = tag | INCL;
-            break;
-          }
-          w = *f;
-        }
-        excl += (uint32_t)w;
-        if ((w & INCL) || pb <= s.os_blk0) break;
-        --pb;
+      for (int bit = 0; bit < 9; ++bit) {
+        const uint32_t bb = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
+        peers &= ((d >> bit) & 1u) ? bb : ~bb;
       }
-      atomicExch(mine, tag | INCL | (excl + cnt));
+      const uint32_t before = valid ? S.wcnt[warp][d] : 0u;
+      __syncwarp();
+      if (valid && (peers & lt) == 0) S.wcnt[warp][d] = before + __popc(peers);
+      __syncwarp();
+      rk[r] = before + __popc(peers & lt);
     }
-  }
-  // digit tid of the whole segment starts after the smaller digits
-  const uint32_t seg_tot = tid < 256 ? seg_hist[((size_t)si * OS_PASSES + pass) * 256 + tid] : 0u;
-  const uint32_t seg_off = digit_excl_scan(seg_tot, S.ws);
-  const uint32_t ds = digit_excl_scan(cnt, S.ws);
-  if (tid < 256) {
-    S.gbase[tid] = seg_off + excl;
-    S.dstart[tid] = ds;
-  }
-  __syncthreads();
+    __syncthreads();
+    uint32_t cnt = 0;  // digit tid: offsets of the warps, then its count in the tile
+    if (tid < 256) {
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int t = warp * CH + r * 32 + lane;
-    if (t < n) {
-      const uint32_t d = dg[r];
-      const uint32_t slot = S.dstart[d] + S.wcnt[warp][d] + rk[r];
-      S.sk[slot] = key[r];
-      S.sv[slot] = val[r];
+      for (int w = 0; w < OS_NW; ++w) {
+        const uint32_t c = S.wcnt[w][tid];
+        S.wcnt[w][tid] = cnt;
+        cnt += c;
+      }
     }
-  }
-  __syncthreads();
-  for (int t = tid; t < n; t += OS_THREADS) {
-    const uint64_t k = S.sk[t];
-    const uint32_t d = (uint32_t)(k >> shift) & 255u;
-    const uint32_t pos = S.gbase[d] + ((uint32_t)t - S.dstart[d]);
-    if (pos < (uint32_t)s.len) {
-      kout[s.out_base + pos] = k;
-      vout[s.out_base + pos] = S.sv[t];
-    } else {
-      atomicOr(err, DERR_BAD_INDEX);
+    // publish this tile's count of digit tid, then look back for the count of
+    // digit tid in the segment's earlier tiles
+    const uint32_t excl = tid < 256 ? sweep_look_back(flags, b, s.os_blk0, tid, pass, cnt, err) : 0u;
+    // digit tid of the whole segment starts after the smaller digits
+    const uint32_t seg_tot = tid < 256 ? seg_hist[((size_t)si * ALL_PASSES + pass) * 256 + tid] : 0u;
+    const uint32_t seg_off = digit_excl_scan(seg_tot, S.ws);
+    const uint32_t ds = digit_excl_scan(cnt, S.ws);
+    if (tid < 256) {
+      S.gbase[tid] = seg_off + excl;
+      S.dstart[tid] = ds;
     }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int t = warp * CH + r * 32 + lane;
+      if (t < n) {
+        const uint32_t d = dg[r];
+        const uint32_t slot = S.dstart[d] + S.wcnt[warp][d] + rk[r];
+        S.sk[slot] = key[r];
+        S.sv[slot] = val[r];
+      }
+    }
+    __syncthreads();
+    for (int t = tid; t < n; t += OS_THREADS) {
+      const uint64_t k = S.sk[t];
+      const uint32_t d = (uint32_t)(k >> shift) & 255u;
+      const uint32_t pos = S.gbase[d] + ((uint32_t)t - S.dstart[d]);
+      if (pos < (uint32_t)s.len) {
+        kout[s.out_base + pos] = k;
+        vout[s.out_base + pos] = S.sv[t];
+      } else {
+        atomicOr(err, DERR_BAD_INDEX);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -396,45 +349,51 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
 constexpr int TIE_RUN = 32;
 
 __global__ void __launch_bounds__(SORT_THREADS)
-tie_fix_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg,
-               uint64_t* keys_all, int32_t* vals_all, uint32_t* __restrict__ err) {
-  const SortSeg sg = segs[blk_seg[blockIdx.x]];
-  const int len = sg.len;
-  const int i0 = ((int)blockIdx.x - sg.blk0) * SORT_TILE;
-  const int i1 = min(i0 + SORT_TILE, len);
-  uint64_t* keys = keys_all + sg.out_base;  // written by run owners: no __restrict__
-  int32_t* vals = vals_all + sg.out_base;
-  for (int q = i0 + (int)threadIdx.x; q < i1; q += SORT_THREADS) {
-    const uint64_t k = keys[q];
-    const uint64_t hi = k >> 16;
-    const bool starts = q == 0 || (keys[q - 1] >> 16) != hi;
-    if (!starts) {
-      // inside a run: out of order against the previous key and the run
-      // too long to be repaired -> the batch needs the full sort
-      if (k < keys[q - 1]) {
-        int s = q - 1, e = q + 1;
-        while (s > 0 && (keys[s - 1] >> 16) == hi && q - s <= TIE_RUN) --s;
-        while (e < len && (keys[e] >> 16) == hi && e - s <= TIE_RUN) ++e;
-        if (e - s > TIE_RUN) atomicOr(err, (uint32_t)DERR_SORT_TIES);
+tie_fix_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg, int nblk,
+               uint64_t* keys_all, int32_t* vals_all, uint32_t* __restrict__ err,
+               const uint32_t* __restrict__ redo, int nseg) {
+  if (redo && !redo[nseg]) return;
+  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    const int si = blk_seg[b];
+    if (redo && !redo[si]) continue;
+    const SortSeg sg = segs[si];
+    const int len = sg.len;
+    const int i0 = (b - sg.blk0) * SORT_TILE;
+    const int i1 = min(i0 + SORT_TILE, len);
+    uint64_t* keys = keys_all + sg.out_base;  // written by run owners: no __restrict__
+    int32_t* vals = vals_all + sg.out_base;
+    for (int q = i0 + (int)threadIdx.x; q < i1; q += SORT_THREADS) {
+      const uint64_t k = keys[q];
+      const uint64_t hi = k >> 16;
+      const bool starts = q == 0 || (keys[q - 1] >> 16) != hi;
+      if (!starts) {
+        // inside a run: out of order against the previous key and the run
+        // too long to be repaired -> the batch needs the full sort
+        if (k < keys[q - 1]) {
+          int s = q - 1, e = q + 1;
+          while (s > 0 && (keys[s - 1] >> 16) == hi && q - s <= TIE_RUN) --s;
+          while (e < len && (keys[e] >> 16) == hi && e - s <= TIE_RUN) ++e;
+          if (e - s > TIE_RUN) atomicOr(err, (uint32_t)DERR_SORT_TIES);
+        }
+        continue;
       }
-      continue;
-    }
-    if (q + 1 >= len || (keys[q + 1] >> 16) != hi) continue;  // a run of one
-    int e = q + 1;
-    while (e < len && (keys[e] >> 16) == hi && e - q <= TIE_RUN) ++e;
-    if (e - q > TIE_RUN) continue;
-    for (int i = q + 1; i < e; ++i) {  // stable insertion sort of [q, e)
-      const uint64_t ki = keys[i];
-      if (ki >= keys[i - 1]) continue;
-      const int32_t vi = vals[i];
-      int j = i;
-      while (j > q && keys[j - 1] > ki) {
-        keys[j] = keys[j - 1];
-        vals[j] = vals[j - 1];
-        --j;
+      if (q + 1 >= len || (keys[q + 1] >> 16) != hi) continue;  // a run of one
+      int e = q + 1;
+      while (e < len && (keys[e] >> 16) == hi && e - q <= TIE_RUN) ++e;
+      if (e - q > TIE_RUN) continue;
+      for (int i = q + 1; i < e; ++i) {  // stable insertion sort of [q, e)
+        const uint64_t ki = keys[i];
+        if (ki >= keys[i - 1]) continue;
+        const int32_t vi = vals[i];
+        int j = i;
+        while (j > q && keys[j - 1] > ki) {
+          keys[j] = keys[j - 1];
+          vals[j] = vals[j - 1];
+          --j;
+        }
+        keys[j] = ki;
+        vals[j] = vi;
       }
-      keys[j] = ki;
-      vals[j] = vi;
     }
   }
 }
@@ -771,46 +730,52 @@ static void excl_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t st)
 }
 
 int init_sort_kernels() {
+  const int rc = init_code_sort();
+  if (rc) return rc;
   return (int)cudaFuncSetAttribute(onesweep_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sizeof(OsSmem));
 }
 
-size_t sort_sweep_bytes(int os_nblk, int nseg) {
-  return sizeof(unsigned long long) * 256 * (size_t)std::max(os_nblk, 1) +
-         sizeof(uint32_t) * OS_PASSES * 256 * (size_t)std::max(nseg, 1) + 64;
-}
+size_t sort_sweep_bytes(int os_nblk, int nseg) { return sweep_layout(nullptr, os_nblk, nseg, nullptr) + 64; }
 
-void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d,
-                 int nblk, const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys_a,
-                 uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b, void* sweep, int first,
+void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
+                 const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
+                 int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
+                 const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
                  uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
   if (nblk <= 0 || os_nblk <= 0) return;
-  // sweep (zeroed by the caller): flag words, segment digit totals, tile counters
-  unsigned long long* flags = (unsigned long long*)sweep;
-  uint32_t* seg_hist = (uint32_t*)(flags + 256 * (size_t)os_nblk);
-  int* counters = (int*)(seg_hist + OS_PASSES * 256 * (size_t)std::max(nseg, 1));
-  onesweep_load_kernel<<<nblk, SORT_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, keys_a, vals_a,
-                                                     seg_hist, first);
+  Sweep w;
+  sweep_layout(sweep, os_nblk, nseg, &w);
+  if (codes)
+    launch_code_sort(slots_d, centers_d, segs_d, blk_seg_d, nblk, os_blk_seg_d, os_nblk, nseg, keys_a,
+                     keys_b, vals_a, ko, w, err, st, pass_events);
+  const uint32_t* redo = codes ? w.redo : nullptr;
+  const int gl = codes ? std::min(nblk, 4 * num_sms) : nblk;
+  const int gp = codes ? std::min(os_nblk, 2 * num_sms) : os_nblk;
+  onesweep_load_kernel<<<gl, SORT_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, nblk, keys_a, vals_a,
+                                                   w.seg_hist, first, redo, nseg);
   count_launch();
   uint64_t* kin = keys_a;
   uint64_t* kout = keys_b;
   int32_t* vin = vals_a;
   int32_t* vout = vals_b;
-  if (pass_events) cudaEventRecord(pass_events[0], st);
+  if (pass_events && !codes) cudaEventRecord(pass_events[0], st);
   for (int pass = first; pass < OS_PASSES; ++pass) {
-    onesweep_pass_kernel<<<os_nblk, OS_THREADS, sizeof(OsSmem), st>>>(
-        segs_d, os_blk_seg_d, kin, vin, kout, vout, pass, seg_hist, flags, counters + pass, err);
+    onesweep_pass_kernel<<<gp, OS_THREADS, sizeof(OsSmem), st>>>(segs_d, os_blk_seg_d, os_nblk, kin, vin,
+                                                                 kout, vout, pass, w.seg_hist, w.flags,
+                                                                 w.counters + pass, err, redo, nseg);
     count_launch();
     uint64_t* tk = kin; kin = kout; kout = tk;
     int32_t* tv = vin; vin = vout; vout = tv;
   }
-  if (pass_events) cudaEventRecord(pass_events[1], st);
+  if (pass_events && !codes) cudaEventRecord(pass_events[1], st);
   // an even number of passes: the sorted keys and values are back in
   // keys_a / vals_a
   if (first > 0) {
-    tie_fix_kernel<<<nblk, SORT_THREADS, 0, st>>>(segs_d, blk_seg_d, keys_a, vals_a, err);
+    tie_fix_kernel<<<gl, SORT_THREADS, 0, st>>>(segs_d, blk_seg_d, nblk, keys_a, vals_a, err, redo, nseg);
     count_launch();
   }
+  launch_samples(segs_d, blk_seg_d, nblk, gl, keys_a, ko, redo, nseg, st);
 }
 
 void launch_radix_pass(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,

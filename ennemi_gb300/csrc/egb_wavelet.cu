@@ -392,26 +392,22 @@ wm_count_kernel(const TaskDev* __restrict__ tasks, const WmJob* __restrict__ job
 
 // fkeys[p] = the largest float <= the value of keys[p]; s1[j] = keys[32 j],
 // s2[j] = keys[1024 j] and the same of fkeys, for every sorted segment.
-// One block of SAMPLE_THREADS per 2048-key tile of the sort.
+// One block of SAMPLE_THREADS per 2048-key tile of the sort (after the code
+// sort, which writes them itself: for the segments it left over).
 constexpr int SAMPLE_THREADS = 256;
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-samples_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg,
-               const uint64_t* __restrict__ keys, KeyIndexOut out) {
-  const SortSeg sg = segs[blk_seg[blockIdx.x]];
-  const int i0 = ((int)blockIdx.x - sg.blk0) * SORT_TILE;
-  const int i1 = min(i0 + SORT_TILE, sg.len);
-  for (int p = i0 + (int)threadIdx.x; p < i1; p += SAMPLE_THREADS) {
-    const uint64_t k = __ldg(keys + sg.out_base + p);
-    const float f = __double2float_rd(value_of(k));
-    out.fkeys[sg.out_base + p] = f;
-    if (p % SAMPLE1 == 0) {
-      out.s1[sg.s1_base + p / SAMPLE1] = k;
-      out.fs1[sg.s1_base + p / SAMPLE1] = f;
-      if (p % SAMPLE2 == 0) {
-        out.s2[sg.s2_base + p / SAMPLE2] = k;
-        out.fs2[sg.s2_base + p / SAMPLE2] = f;
-      }
-    }
+samples_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg, int nblk,
+               const uint64_t* __restrict__ keys, KeyIndexOut out, const uint32_t* __restrict__ redo,
+               int nseg) {
+  if (redo && !redo[nseg]) return;
+  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    const int si = blk_seg[b];
+    if (redo && !redo[si]) continue;
+    const SortSeg sg = segs[si];
+    const int i0 = (b - sg.blk0) * SORT_TILE;
+    const int i1 = min(i0 + SORT_TILE, sg.len);
+    for (int p = i0 + (int)threadIdx.x; p < i1; p += SAMPLE_THREADS)
+      put_samples(out, sg, p, __ldg(keys + sg.out_base + p));
   }
 }
 static_assert(SORT_TILE % SAMPLE1 == 0, "sample grid");
@@ -438,10 +434,11 @@ void launch_wm_count(const TaskDev* tasks_d, const WmJob* jobs_d, int njobs, int
   count_launch();
 }
 
-void launch_samples(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
-                    const uint64_t* keys, const KeyIndexOut& out, cudaStream_t st) {
+void launch_samples(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk, int grid,
+                    const uint64_t* keys, const KeyIndexOut& out, const uint32_t* redo, int nseg,
+                    cudaStream_t st) {
   if (nblk <= 0) return;
-  samples_kernel<<<nblk, SAMPLE_THREADS, 0, st>>>(segs_d, blk_seg_d, keys, out);
+  samples_kernel<<<grid, SAMPLE_THREADS, 0, st>>>(segs_d, blk_seg_d, nblk, keys, out, redo, nseg);
   count_launch();
 }
 

@@ -283,6 +283,54 @@ def test_window_counts(n, data):
         assert got[i] == np.count_nonzero(np.abs(x - x[i]) <= r[i]), i
 
 
+def _code_columns(data, n, rng):
+    x = rng.normal(size=n)
+    if data == "offset":
+        x += 1e6
+    elif data == "near":      # short runs of equal codes, out of order
+        x = rng.permutation(np.concatenate([x[: n // 4] + j * 2.0 ** -40 for j in range(4)] + [x[: n % 4]]))
+    elif data == "levels":    # long runs of equal values
+        x = np.round(x * 2.0)
+    elif data == "zeros":     # both zeros
+        x = np.where(rng.random(n) < 0.5, np.copysign(0.0, x), x)
+    elif data == "cluster":   # a long run of equal codes, out of order
+        x[: n // 50] = 3.0 + rng.permutation(n // 50) * 2.0 ** -40
+    elif data == "twins":     # runs around the longest that is repaired
+        x = rng.permutation(np.concatenate([v + rng.permutation(m) * 2.0 ** -45 for m in (31, 32, 33, 34)
+                                            for v in rng.normal(size=n // 8 // m)] + [x])[:n])
+    elif data == "huge":
+        x[::3] *= 1e300
+    elif data == "tiny":
+        x *= 1e-300
+    elif data == "one_huge":  # everything else shares a code
+        x[0] = 1e308
+    return x
+
+
+@pytest.mark.parametrize("data", ["normal", "offset", "near", "levels", "zeros", "cluster", "twins", "huge",
+                                  "tiny", "one_huge"])
+def test_code_sort_equals_the_digit_sort(data):
+    """A batch large enough for the code sort returns, for segments of one
+    point up to several tiles, exactly what each of its tasks returns alone."""
+    rng = np.random.default_rng(17)
+    sizes = [5, 40, 2047, 2049, 4096, 4097, 60_001, 500_000, 500_003]
+    tasks = []
+    for n in sizes:
+        x = _code_columns(data, n, rng)
+        tasks.append(N.Task(N.MI, 3, [x], [0.5 * x + rng.normal(size=n)]))
+    ctx = N.context(0)
+    both = N.run_tasks(tasks, flags=N.KEEP_INTERNALS)
+    # "twins": runs too long to repair both in their codes and in 48 key bits
+    assert ctx.stats()["sort_passes"] == (8 if data == "twins" else 4)
+    kept = [[N.fetch(t, w, n) for w in (0, 1, 2)] for t, n in enumerate(sizes)]
+    for t, n in enumerate(sizes):
+        alone = N.run_tasks([tasks[t]], flags=N.KEEP_INTERNALS)
+        assert ctx.stats()["sort_passes"] != 4
+        assert np.array_equal(alone[0], both[t], equal_nan=True), n
+        for w in (0, 1, 2):
+            assert np.array_equal(N.fetch(0, w, n), kept[t][w], equal_nan=True), (n, w)
+
+
 @pytest.mark.parametrize("data", ["independent", "cubic", "square", "steps", "constant", "huge"])
 @pytest.mark.parametrize("n", [4096, 4099, 20_001])
 def test_strip_layouts(oracle, n, data):
