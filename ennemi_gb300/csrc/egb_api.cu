@@ -59,7 +59,20 @@ namespace {
 
 constexpr int KIND_KNN_ONLY = 100;    // egb_knn_eps
 constexpr int KIND_COUNT_ONLY = 101;  // egb_ball_count
-constexpr int SLAB_MIN = 4096;        // shorter multi-D segments use brute force
+// Multi-D segments below SLAB_MIN points have no grid copy, but for kNN jobs
+// of at least KNN_GRID_MIN where the batch holds enough of their dimension to
+// pay for the launches that build it (pairs of points in such jobs above
+// SMALL_GRID_*).  The others take a warp per query over all points
+// (egb_wlist.cu), and the tiles of SMALL_TILE queries, which serve a query in
+// fewer instructions, when two columns fill two of them per SM.  Whole calls,
+// tile / list / grid (us): one set of 2000 points, d = 2: 691 / 210 / 228; d = 4:
+// 1130 / 352 / 499; 40 sets of 2000, d = 2: 904 / 697 / 435; d = 3: 1327 / 993 / 879;
+// d = 4: 1621 / 1175 / 1156; 496 of 1100, d = 2: 3480 / 3784 / 2330; d = 3: 5312 /
+// 4930 / 3954; 1225 sets of 700, d = 2: 6272 / 6675 / -; 40 of 700: 595 / 447 / -.
+constexpr int64_t KNN_GRID_MIN = 1024;
+constexpr int64_t SMALL_GRID_2D = 10'000'000, SMALL_GRID_ND = 100'000'000;
+constexpr int SMALL_TILE = 1024;
+constexpr int SLAB_MIN = 4096;
 constexpr int NPHASE = 7;
 constexpr int NKTIME = 7;   // kNN tile, kNN deferred, count tile, count deferred,
                             // radix sort, 1-D counts, the sort's digit passes
@@ -943,6 +956,21 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     Space s; bool is_knn; int slab; int sort_seg; int sel; int sort_seg_b; int mode;
     int sort_seg_c;
   };
+  // kNN jobs of fewer than SLAB_MIN points, by d: pairs of those that could
+  // take a grid, CTAs of all of them as tiles
+  int64_t small_pairs[EGB_DMAX + 1] = {}, small_tiles[EGB_DMAX + 1] = {};
+  for (const Space& s : knn) {
+    const int64_t len = s.e - s.b;
+    if (s.sp.d < 2 || len >= SLAB_MIN) continue;
+    if (len >= KNN_GRID_MIN) small_pairs[s.sp.d] += len * len;
+    small_tiles[s.sp.d] += (len + SMALL_TILE - 1) / SMALL_TILE;
+  }
+  auto small_grid = [&](int d, int64_t len) {
+    return !plain && len >= KNN_GRID_MIN && small_pairs[d] > (d == 2 ? SMALL_GRID_2D : SMALL_GRID_ND);
+  };
+  auto small_list = [&](int d, int64_t len) {
+    return !plain && !force_brute && len < SLAB_MIN && (d > 2 || small_tiles[d] < 2 * ctx->num_sms);
+  };
   // layout of a multi-D job: EGB_FORCE_* flags, else the context's policy
   // table, else the built-in rule; warp grid kNN needs K <= LIST_K_MAX (K <= 8
   // in FP64)
@@ -957,7 +985,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     else if (force_grid || cta_grid) mode = 3;
     else {
       mode = ctx->policy[egb_policy_index(is_knn ? 0 : 1, s.sp.d, s.K, len)];
-      if (mode == EGB_MODE_AUTO) mode = len >= SLAB_MIN ? (rank_ok ? 4 : 3) : 0;
+      if (mode == EGB_MODE_AUTO) mode = (is_knn && len < SLAB_MIN ? small_grid(s.sp.d, len) : len >= SLAB_MIN) ? (rank_ok ? 4 : 3) : 0;
     }
     if (mode == 4 && !rank_ok) mode = 3;
     if (mode == 3 && (cta_grid || (is_knn && s.K > 8 && (plain || s.K > LIST_K_MAX)))) mode = 2;
@@ -979,6 +1007,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       MJob m{s, true, 0, -1, 0, -1, 0, -1};
       if (s.K <= EGB_KREG_MAX) {
         m.mode = pick_mode(true, s);
+        if (m.mode == 0 && small_list(s.sp.d, s.e - s.b)) m.sel = 2;
       } else if (plain || force_brute || force_slab || cta_grid || s.K > LIST_K_MAX) {
         m.sel = 1;  // radix select on the FP64 distances to all points
       } else {

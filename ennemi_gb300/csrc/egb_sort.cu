@@ -743,7 +743,10 @@ void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg
                  int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
                  const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
                  uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
-  if (nblk <= 0 || os_nblk <= 0) return;
+  if (nblk <= 0 || os_nblk <= 0) {
+    if (pass_events) cudaEventRecord(pass_events[0], st), cudaEventRecord(pass_events[1], st);
+    return;
+  }
   Sweep w;
   sweep_layout(sweep, os_nblk, nseg, &w);
   if (codes)

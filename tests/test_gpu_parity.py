@@ -331,6 +331,50 @@ def test_code_sort_equals_the_digit_sort(data):
             assert np.array_equal(N.fetch(0, w, n), kept[t][w], equal_nan=True), (n, w)
 
 
+def _small_points(data, n, d, rng):
+    x = rng.normal(size=(n, d))
+    if data == "duplicates":
+        x = rng.integers(0, 4, size=(n, d)).astype(np.float64)
+    elif data == "huge":
+        x[:, 0] *= 1e300
+    elif data == "offset":
+        x += 1e9
+    return x
+
+
+@pytest.mark.parametrize("data", ["normal", "duplicates", "huge", "offset"])
+@pytest.mark.parametrize("d", [2, 3, 4, 5])
+def test_small_knn(oracle, d, data):
+    """kNN of sets too small for a layout of their own: fewer points than
+    neighbours, the warp's widths, both sides of the smallest grid."""
+    rng = np.random.default_rng(40 + d)
+    for n in [1, 2, 9, 31, 33, 65, 700, 1023, 1025, 4095]:
+        pts = _small_points(data, n, d, rng)
+        for k in [1, 3, 7, 8, 31] if n < 1000 else [3, 8]:
+            assert np.array_equal(N.knn_eps(pts, k), oracle.knn_eps(pts, k)), (n, k)
+
+
+@pytest.mark.parametrize("data", ["normal", "duplicates", "huge", "offset"])
+@pytest.mark.parametrize("count, n", [(3, 2000), (26, 2000), (11, 4095), (100, 1024), (320, 40), (320, 900)])
+def test_small_batches_take_the_form_that_fits(count, n, data):
+    """Batches of small sets, from a few to those that get grids or fill the
+    tile kernel, against brute force."""
+    rng = np.random.default_rng(count)
+    tasks = []
+    for i in range(count):
+        x = _small_points(data, n, 4, rng)
+        y = 0.5 * x[:, 0] + rng.normal(size=n)
+        tasks.append(N.Task(N.MI, 3, [x[:, 0].copy()], [y]) if i % 2 else
+                     N.Task(N.CMI, 3, [x[:, 0].copy()], [y], [x[:, 1].copy(), x[:, 2].copy()][: 1 + i % 4 // 2]))
+    flags = N.KEEP_INTERNALS | N.TIMING
+    got = N.run_tasks(tasks, flags=flags)
+    kept = [N.fetch(t, 0, n) for t in range(0, count, 7)]
+    want = N.run_tasks(tasks, flags=flags | N.FORCE_BRUTE)
+    assert np.array_equal(got, want, equal_nan=True)
+    for t, e in zip(range(0, count, 7), kept):
+        assert np.array_equal(N.fetch(t, 0, n), e, equal_nan=True), t
+
+
 @pytest.mark.parametrize("data", ["independent", "cubic", "square", "steps", "constant", "huge"])
 @pytest.mark.parametrize("n", [4096, 4099, 20_001])
 def test_strip_layouts(oracle, n, data):
