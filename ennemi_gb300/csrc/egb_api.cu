@@ -44,6 +44,7 @@
 
 #include "egb_internal.cuh"
 #include "egb_search.cuh"
+#include "egb_sweep.cuh"
 #include "egb_pwtree.h"
 #include "ennemi_gb.h"
 
@@ -1285,25 +1286,21 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       SortSeg g{};
       g.out_base = gsort_total;
       g.len = (int32_t)len;
-      g.blk0 = nblk_grid;
-      g.nblk = (int32_t)((len + SORT_TILE - 1) / SORT_TILE);
+      g.os_blk0 = nblk_grid;
+      g.os_nblk = (int32_t)((len + OS_TILE - 1) / OS_TILE);
       gsegs.push_back(g);
       grid_jobs.push_back((int32_t)j);
       gsort_total += len;
-      nblk_grid += g.nblk;
+      nblk_grid += g.os_nblk;
       max_glen = std::max(max_glen, len);
     }
   }
 
-  // strip-key sort of the grid jobs (one extra 8-bit radix pass)
+  // strip-key sort of the grid jobs: words, ping-pong
   const size_t off_gkeys_a = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(gsort_total, 1));
   const size_t off_gkeys_b = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(gsort_total, 1));
-  const size_t off_gvals_a = dl.take(sizeof(int32_t) * (size_t)std::max<int64_t>(gsort_total, 1));
-  const size_t off_gvals_b = dl.take(sizeof(int32_t) * (size_t)std::max<int64_t>(gsort_total, 1));
   const size_t off_ginv = dl.take(sizeof(int32_t) * (size_t)std::max<int64_t>(gsort_total, 1));
   const size_t off_gsub = any_nested ? dl.take(sizeof(int32_t) * (size_t)std::max<int64_t>(gsort_total, 1)) : 0;
-  const size_t off_ghist = dl.take(sizeof(uint32_t) * 256 * (size_t)std::max(nblk_grid, 1));
-  const size_t off_gscan = dl.take(sizeof(uint32_t) * sort_scan_tmp_elems(std::max(nblk_grid, 1)));
 
   // sorted jobs
   std::vector<SortedJob> sj_knn, sj_cnt;
@@ -1722,6 +1719,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   // everything that starts zeroed, in one run
   const size_t off_zr = dl.take(zr_bytes);
   const size_t off_sweep = dl.take(sweep_bytes);
+  const size_t off_gsweep = nblk_grid ? dl.take(sort_sweep_bytes(nblk_grid, (int)gsegs.size())) : 0;
   const size_t off_wmz = dl.take(wmz_bytes);
   const size_t off_gbz = dl.take(gbz_bytes);
   const size_t zero_bytes = dl.off - off_zr;
@@ -1810,7 +1808,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   {
     int32_t* bs = (int32_t*)(H + tab_blkgseg);
     for (size_t g = 0; g < gsegs.size(); ++g)
-      for (int b = 0; b < gsegs[g].nblk; ++b) bs[gsegs[g].blk0 + b] = (int32_t)g;
+      for (int b = 0; b < gsegs[g].os_nblk; ++b) bs[gsegs[g].os_blk0 + b] = (int32_t)g;
   }
   if (!grid_jobs.empty())
     std::memcpy(H + tab_gridjobs, grid_jobs.data(), sizeof(int32_t) * grid_jobs.size());
@@ -2035,29 +2033,28 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     const int32_t* blkg_d = (const int32_t*)dtab(tab_blkgseg);
     uint64_t* gka = (uint64_t*)(A + off_gkeys_a);
     uint64_t* gkb = (uint64_t*)(A + off_gkeys_b);
-    int32_t* gva = (int32_t*)(A + off_gvals_a);
-    int32_t* gvb = (int32_t*)(A + off_gvals_b);
-    uint32_t* ghist = (uint32_t*)(A + off_ghist);
-    uint32_t* gscan = (uint32_t*)(A + off_gscan);
+    Sweep gw;
+    sweep_layout(A + off_gsweep, nblk_grid, (int)gsegs.size(), &gw);
+    auto pass = [&](const uint64_t* in, uint64_t* out, int digit, int id) {
+      launch_word_pass(gsegs_d, blkg_d, nblk_grid, in, out, digit, id, gw, err_d, st);
+    };
     int32_t* ginv = (int32_t*)(A + off_ginv);
     int32_t* gsub = any_nested ? (int32_t*)(A + off_gsub) : nullptr;
     launch_grid_inv(jobs_d, gj_d, ngrid, gsegs_d, vals, (const SortSeg*)dtab(tab_segs), ginv, max_glen, st);
     if (any_nested) {
       // strips of the column-2 order -> cell of every point within its strip
-      launch_nest_key(jobs_d, gj_d, ngrid, gsegs_d, vals, (const SortSeg*)dtab(tab_segs), ginv, gka,
-                      gva, max_glen, st);
-      launch_radix_pass(gsegs_d, blkg_d, nblk_grid, gka, gva, gkb, gvb, 0, ghist, gscan, st);
-      launch_nest_sub(tasks_d, jobs_d, gj_d, ngrid, gsegs_d, gkb, gvb, gsub, max_glen, st);
+      launch_nest_key(jobs_d, gj_d, ngrid, gsegs_d, vals, (const SortSeg*)dtab(tab_segs), ginv, gka, gw,
+                      max_glen, st);
+      pass(gka, gkb, 0, NEST_PASS);
+      launch_nest_sub(tasks_d, jobs_d, gj_d, ngrid, gsegs_d, gkb, gsub, max_glen, st);
     }
-    launch_grid_key(jobs_d, gj_d, ngrid, gsegs_d, vals, (const SortSeg*)dtab(tab_segs), ginv, gsub, gka,
-                    gva, max_glen, st);
-    launch_radix_pass(gsegs_d, blkg_d, nblk_grid, gka, gva, gkb, gvb, 0, ghist, gscan, st);
-    if (max_gkey > 256)  // strip / cell keys above 8 bits: second digit
-      launch_radix_pass(gsegs_d, blkg_d, nblk_grid, gkb, gvb, gka, gva, 8, ghist, gscan, st);
+    launch_grid_key(jobs_d, gj_d, ngrid, gsegs_d, vals, (const SortSeg*)dtab(tab_segs), ginv, gsub, gka, gw,
+                    max_glen, st);
+    pass(gka, gkb, 0, GRID_PASS);
+    if (max_gkey > 256) pass(gkb, gka, 1, GRID_PASS + 1);  // strip / cell keys above 8 bits
     launch_materialize_grid(tasks_d, (const JobDev*)dtab(tab_jobs), (const int32_t*)dtab(tab_gridjobs),
                             (int)grid_jobs.size(), vals, (const SortSeg*)dtab(tab_segs),
-                            max_gkey > 256 ? gva : gvb, (const SortSeg*)dtab(tab_gsegs),
-                            max_lds, st);
+                            max_gkey > 256 ? gka : gkb, (const SortSeg*)dtab(tab_gsegs), max_lds, st);
     for (const Group& G : groups)
       if (G.boxed)
         launch_leaf_boxes(jobs_d, items_of(G), (int)G.nitems, (float*)(A + G.off_box), st);

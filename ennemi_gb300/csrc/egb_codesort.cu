@@ -87,7 +87,7 @@ struct PassSmem {
 
 __global__ void __launch_bounds__(PASS_THREADS, 5)
 code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ os_blk_seg,
-                 const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int digit,
+                 const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int digit, int pass,
                  const uint32_t* __restrict__ seg_hist, unsigned long long* flags, int* tile_counter,
                  uint32_t* err) {
   extern __shared__ __align__(16) unsigned char raw[];
@@ -134,7 +134,6 @@ code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ o
     cnt += c;
   }
   if (tid == 255) cnt -= (uint32_t)(OS_TILE - n);
-  const int pass = OS_PASSES + digit;
   // exclusive scans over the digits of the tile's counts and of the segment's
   const uint32_t tot = seg_hist[((size_t)si * ALL_PASSES + pass) * 256 + tid];
   uint2 sum = make_uint2(cnt, tot);
@@ -251,6 +250,14 @@ int init_code_sort() {
                                    (int)sizeof(PassSmem));
 }
 
+void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, const uint64_t* in,
+                      uint64_t* out, int digit, int pass, const Sweep& w, uint32_t* err, cudaStream_t st) {
+  if (os_nblk <= 0) return;
+  code_pass_kernel<<<os_nblk, PASS_THREADS, sizeof(PassSmem), st>>>(segs_d, os_blk_seg_d, in, out, digit, pass,
+                                                                    w.seg_hist, w.flags, w.counters + pass, err);
+  count_launch();
+}
+
 void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
                       const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
                       int nseg, uint64_t* keys, uint64_t* words, int32_t* vals, const KeyIndexOut& ko,
@@ -261,9 +268,7 @@ void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const So
   uint64_t* in = words;  // an even number of passes: back in words
   uint64_t* out = keys;
   for (int d = 0; d < CODE_PASSES; ++d) {
-    code_pass_kernel<<<os_nblk, PASS_THREADS, sizeof(PassSmem), st>>>(
-        segs_d, os_blk_seg_d, in, out, d, w.seg_hist, w.flags, w.counters + OS_PASSES + d, err);
-    count_launch();
+    launch_word_pass(segs_d, os_blk_seg_d, os_nblk, in, out, d, OS_PASSES + d, w, err, st);
     uint64_t* t = in; in = out; out = t;
   }
   if (pass_events) cudaEventRecord(pass_events[1], st);

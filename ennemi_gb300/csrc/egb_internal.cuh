@@ -513,7 +513,7 @@ void launch_materialize(const TaskDev* tasks_d, const JobDev* jobs_d, int njobs,
                         cudaStream_t st);
 void launch_materialize_grid(const TaskDev* tasks_d, const JobDev* jobs_d,
                              const int32_t* grid_jobs_d, int ngrid, const int32_t* sorted_vals,
-                             const SortSeg* segs_d, const int32_t* gvals_sorted,
+                             const SortSeg* segs_d, const uint64_t* words,
                              const SortSeg* gsegs_d, int64_t max_lds, cudaStream_t st);
 void launch_emit_items(const JobDev* jobs_d, const ItemRun* runs_d, int nruns, const int32_t* cum_d,
                        int64_t nitems, WorkItem* items_d, cudaStream_t st);
@@ -548,34 +548,38 @@ void launch_samples(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk, i
                     const uint64_t* keys, const KeyIndexOut& out, const uint32_t* redo, int nseg,
                     cudaStream_t st);
 // Strip keys of the grid jobs.  launch_grid_inv: inv[p_B] = column-1 rank
-// of each point (by working offset).  launch_grid_key: keys[p] = cell key of
-// the point at column-0 position p -- its strip (column-1 rank * nstrips /
-// len), times nsub plus its cell (nested grids, from sub[]) -- and vals[p] =
-// p; stable 8-bit radix passes then order each segment by (key, column 0).
+// of each point (by working offset).  launch_grid_key: the word (upper half,
+// lower half) of column-0 position p is the cell of its point -- its strip
+// (column-1 rank * nstrips / len), times nsub plus its cell (nested grids, from
+// sub[]) -- and p; stable 8-bit passes (launch_word_pass) then order each
+// segment by (cell, column 0).  The digit totals that a pass needs are sums of
+// the cells' sizes, which the key kernels write beside the words: a pass is one
+// launch, against five with a histogram and a scan of its own.
+struct Sweep;
 void launch_grid_inv(const JobDev* jobs_d, const int32_t* grid_jobs_d, int ngrid,
                      const SortSeg* gsegs_d, const int32_t* sorted_vals, const SortSeg* segs_d,
                      int32_t* inv_scratch, int64_t max_len, cudaStream_t st);
 void launch_grid_key(const JobDev* jobs_d, const int32_t* grid_jobs_d, int ngrid,
                      const SortSeg* gsegs_d, const int32_t* sorted_vals, const SortSeg* segs_d,
-                     const int32_t* inv_scratch, const int32_t* sub, uint64_t* gkeys,
-                     int32_t* gvals, int64_t max_len, cudaStream_t st);
+                     const int32_t* inv_scratch, const int32_t* sub, uint64_t* words, const Sweep& w,
+                     int64_t max_len, cudaStream_t st);
 // Nested grids.  launch_nest_key: over the column-2 order of each nested job,
-// keys[r] = strip of the point at column-2 position r, vals[r] = its working
-// offset (non-nested jobs: zeros).  After one stable radix pass (strips in
+// the word of position r is the strip of its point and the point's working
+// offset (non-nested jobs: strip 0).  After one stable pass (strips in
 // column-2 order), launch_nest_sub: sub[w] = cell of point w within its strip
 // (its within-strip column-2 rank * nsub / strip length), and the column-2
 // bounds czlo / czhi of every cell.
 void launch_nest_key(const JobDev* jobs_d, const int32_t* grid_jobs_d, int ngrid,
                      const SortSeg* gsegs_d, const int32_t* sorted_vals, const SortSeg* segs_d,
-                     const int32_t* inv_scratch, uint64_t* keys, int32_t* vals, int64_t max_len,
+                     const int32_t* inv_scratch, uint64_t* words, const Sweep& w, int64_t max_len,
                      cudaStream_t st);
 void launch_nest_sub(const TaskDev* tasks_d, const JobDev* jobs_d, const int32_t* grid_jobs_d,
-                     int ngrid, const SortSeg* gsegs_d, const uint64_t* keys_sorted,
-                     const int32_t* vals_sorted, int32_t* sub, int64_t max_len, cudaStream_t st);
-void launch_radix_pass(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
-                       const uint64_t* kin, const int32_t* vin, uint64_t* kout, int32_t* vout,
-                       int shift, uint32_t* hist, uint32_t* scan_tmp, cudaStream_t st);
-size_t sort_scan_tmp_elems(int nblk);
+                     int ngrid, const SortSeg* gsegs_d, const uint64_t* words, int32_t* sub,
+                     int64_t max_len, cudaStream_t st);
+// One stable pass (egb_codesort.cu) over the digit (bits 8 digit ..) of the
+// words' upper halves, the segments' OS_TILE tiles given.
+void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, const uint64_t* in,
+                      uint64_t* out, int digit, int pass, const Sweep& w, uint32_t* err, cudaStream_t st);
 // The batch sort: single-sweep LSD passes over the 8-bit digits first..7 of
 // the keys (first = 0: all; first = 2: the high 48 bits, then a repair of
 // the rare runs tied there, which sets DERR_SORT_TIES when one is too long);
@@ -602,7 +606,6 @@ void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg
                  const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
                  uint32_t* err, cudaStream_t st,
                  cudaEvent_t* pass_events = nullptr);  // recorded around the passes alone
-struct Sweep;
 int init_code_sort();
 void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
                       const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,

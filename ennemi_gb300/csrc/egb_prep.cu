@@ -369,20 +369,20 @@ __global__ void materialize_kernel(const TaskDev* __restrict__ tasks,
 }
 
 // Grid copy: position p_G of the strip order takes the point at column-0
-// position p_A = gvals_sorted[p_G].
+// position p_A, the lower half of the sorted word at p_G.
 __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
                                         const JobDev* __restrict__ jobs,
                                         const int32_t* __restrict__ grid_jobs, int ngrid,
                                         const int32_t* __restrict__ sorted_vals,
                                         const SortSeg* __restrict__ segs,
-                                        const int32_t* __restrict__ gvals_sorted,
+                                        const uint64_t* __restrict__ words,
                                         const SortSeg* __restrict__ gsegs) {
   for (int g = blockIdx.y; g < ngrid; g += gridDim.y) {
     const JobDev J = jobs[grid_jobs[g]];
     const TaskDev t = tasks[J.task];
     const int d = J.sp.d;
     const int32_t* va = sorted_vals + segs[J.sort_seg].out_base;
-    const int32_t* gv = gvals_sorted + gsegs[J.gseg].out_base;
+    const uint64_t* gv = words + gsegs[J.gseg].out_base;
     // column-1 bounds of each strip, from the column-1 sort
     const int32_t* vb = sorted_vals + segs[J.sort_seg_b].out_base;
     const double* x1 = t.col[J.sp.cols[1]];
@@ -398,7 +398,7 @@ __global__ void materialize_grid_kernel(const TaskDev* __restrict__ tasks,
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < J.lds;
          p += (int64_t)gridDim.x * blockDim.x) {
       if (p < J.len) {
-        const int32_t pa = gv[p];
+        const int32_t pa = (int32_t)(uint32_t)gv[p];
         const int32_t w = va[pa];
         if (J.posg) J.posg[p] = pa;
         J.idxg[p] = w;
@@ -670,12 +670,12 @@ void launch_emit_items(const JobDev* jobs_d, const ItemRun* runs_d, int nruns, c
 
 void launch_materialize_grid(const TaskDev* tasks_d, const JobDev* jobs_d,
                              const int32_t* grid_jobs_d, int ngrid, const int32_t* sorted_vals,
-                             const SortSeg* segs_d, const int32_t* gvals_sorted,
+                             const SortSeg* segs_d, const uint64_t* words,
                              const SortSeg* gsegs_d, int64_t max_lds, cudaStream_t st) {
   if (ngrid <= 0) return;
   dim3 grid(grid_x_for(max_lds), grid_y_for(ngrid));
   materialize_grid_kernel<<<grid, PREP_THREADS, 0, st>>>(tasks_d, jobs_d, grid_jobs_d, ngrid,
-                                                         sorted_vals, segs_d, gvals_sorted, gsegs_d);
+                                                         sorted_vals, segs_d, words, gsegs_d);
   count_launch();
 }
 

@@ -6,11 +6,8 @@
 // FP64 value (key_of), the payload is the working index of the point.  The
 // batch sort takes stable 8-bit single-sweep LSD passes over the high 48 key
 // bits and repairs the rare runs tied there (below), for large batches only
-// over what the sort of 32-bit codes leaves (egb_codesort.cu); the three-kernel pass
-// -- histogram, exclusive scan, stable scatter -- serves the strip-key
-// passes of the grid layouts: its per-block histograms are laid out
-// segment-major, digit-next, block-minor, so ONE global exclusive scan
-// yields absolute output positions that never leave a segment.
+// over what the sort of 32-bit codes leaves (egb_codesort.cu), whose passes
+// also order the strip keys of the grid layouts.
 //
 // 1-D kNN (entropy of one column, Ross MI with 1-D x): for the point at
 // sorted position p the (k+1)-th smallest |x_j - x_p| (self included) is
@@ -32,143 +29,7 @@ namespace egb {
 namespace {
 
 constexpr int SORT_THREADS = 256;
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 16;
-constexpr int SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
 constexpr int SORTED_THREADS = SORTED_BLOCK;
-
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total) {
-  __shared__ uint32_t ws[SCAN_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) ws[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = lane < SCAN_THREADS / 32 ? ws[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    if (lane < SCAN_THREADS / 32) ws[lane] = w;
-  }
-  __syncthreads();
-  const uint32_t wprefix = warp ? ws[warp - 1] : 0;
-  if (total) *total = ws[SCAN_THREADS / 32 - 1];
-  const uint32_t r = wprefix + x - v;
-  __syncthreads();
-  return r;
-}
-
-__global__ void sort_hist_kernel(const SortSeg* __restrict__ segs,
-                                 const int32_t* __restrict__ blk_seg,
-                                 const uint64_t* __restrict__ keys, int shift,
-                                 uint32_t* __restrict__ hist) {
-  __shared__ uint32_t h[256];
-  const int b = blockIdx.x;
-  const SortSeg s = segs[blk_seg[b]];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  const int i0 = (b - s.blk0) * SORT_TILE;
-  const int i1 = min(i0 + SORT_TILE, s.len);
-  for (int i = i0 + threadIdx.x; i < i1; i += SORT_THREADS)
-    atomicAdd(&h[(uint32_t)(keys[s.out_base + i] >> shift) & 255u], 1u);
-  __syncthreads();
-  const int lb = b - s.blk0;
-  hist[(int64_t)256 * s.blk0 + (int64_t)threadIdx.x * s.nblk + lb] = h[threadIdx.x];
-}
-
-// Stable scatter of one tile.  Warp w ranks the keys [w * CH, (w + 1) * CH)
-// of the tile in rounds of 32: per-bit ballots give a key's rank among the
-// equal digits of its round, per-warp counters carry the rank across rounds.  One
-// block scan then turns the per-warp digit counts into the tile's layout in
-// digit order, staged in shared memory and written out so that consecutive
-// threads store to consecutive addresses of each digit's output run.
-// offs[] holds absolute positions in the concatenated buffer.
-__global__ void __launch_bounds__(SORT_THREADS)
-sort_scatter_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg,
-                    const uint64_t* __restrict__ kin, const int32_t* __restrict__ vin, int shift,
-                    const uint32_t* __restrict__ offs, uint64_t* __restrict__ kout,
-                    int32_t* __restrict__ vout) {
-  constexpr int NW = SORT_THREADS / 32;
-  constexpr int CH = SORT_TILE / NW;  // keys per warp
-  constexpr int R = CH / 32;          // rounds per warp
-  static_assert(SORT_THREADS == 256 && SCAN_THREADS == 256, "one thread per digit");
-  __shared__ uint32_t wcnt[NW][256];  // per-warp digit counts, then offsets
-  __shared__ uint32_t dstart[256];    // first tile slot of each digit
-  __shared__ uint32_t gbase[256];     // first output position of each digit
-  __shared__ uint64_t sk[SORT_TILE];
-  __shared__ int32_t sv[SORT_TILE];
-  const int b = blockIdx.x;
-  const SortSeg s = segs[blk_seg[b]];
-  const int lb = b - s.blk0;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  gbase[tid] = offs[(int64_t)256 * s.blk0 + (int64_t)tid * s.nblk + lb];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) wcnt[w][tid] = 0;
-  __syncthreads();
-  const int i0 = lb * SORT_TILE;
-  const int n = min(SORT_TILE, s.len - i0);
-  const uint32_t lt = (1u << lane) - 1u;
-  uint64_t key[R];
-  int32_t val[R];
-  uint32_t dg[R], rk[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int t = warp * CH + r * 32 + lane;
-    const bool valid = t < n;
-    key[r] = valid ? kin[s.out_base + i0 + t] : 0ull;
-    val[r] = valid ? vin[s.out_base + i0 + t] : 0;
-    const uint32_t d = valid ? (uint32_t)(key[r] >> shift) & 255u : 256u + lane;
-    dg[r] = d;
-    // lanes with the same digit (9 bits: invalid lanes carry 256 + lane),
-    // from one ballot per bit (measured faster than match_any here)
-    uint32_t peers = 0xffffffffu;
-#pragma unroll
-    for (int bit = 0; bit < 9; ++bit) {
-      const uint32_t bb = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
-      peers &= ((d >> bit) & 1u) ? bb : ~bb;
-    }
-    const uint32_t before = valid ? wcnt[warp][d] : 0u;
-    __syncwarp();
-    if (valid && (peers & lt) == 0) wcnt[warp][d] = before + __popc(peers);
-    __syncwarp();
-    rk[r] = before + __popc(peers & lt);
-  }
-  __syncthreads();
-  uint32_t run = 0;  // digit tid: offsets of the warps, then of the digit
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    const uint32_t c = wcnt[w][tid];
-    wcnt[w][tid] = run;
-    run += c;
-  }
-  dstart[tid] = block_excl_scan(run, nullptr);
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int t = warp * CH + r * 32 + lane;
-    if (t < n) {
-      const uint32_t d = dg[r];
-      const uint32_t slot = dstart[d] + wcnt[warp][d] + rk[r];
-      sk[slot] = key[r];
-      sv[slot] = val[r];
-    }
-  }
-  __syncthreads();
-  for (int t = tid; t < n; t += SORT_THREADS) {
-    const uint64_t k = sk[t];
-    const uint32_t d = (uint32_t)(k >> shift) & 255u;
-    const uint32_t pos = gbase[d] + ((uint32_t)t - dstart[d]);
-    kout[pos] = k;
-    vout[pos] = sv[t];
-  }
-}
 
 // ------------------------------------------------------- single sweep --
 // The batch sort proper: stable 8-bit LSD passes, one launch each,
@@ -398,53 +259,6 @@ tie_fix_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk
   }
 }
 
-// ------------------------------------------------------------------ scan --
-__global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
-                                   uint32_t* __restrict__ sums) {
-  const int64_t c0 = (int64_t)blockIdx.x * SCAN_CHUNK;
-  uint32_t s = 0;
-  for (int j = 0; j < SCAN_ITEMS; ++j) {
-    const int64_t i = c0 + (int64_t)j * SCAN_THREADS + threadIdx.x;
-    if (i < n) s += in[i];
-  }
-  uint32_t tot;
-  block_excl_scan(s, &tot);
-  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
-}
-
-__global__ void scan_top_kernel(uint32_t* __restrict__ sums, int nchunks) {
-  uint32_t carry = 0;
-  for (int c0 = 0; c0 < nchunks; c0 += SCAN_THREADS) {
-    const int i = c0 + threadIdx.x;
-    const uint32_t v = i < nchunks ? sums[i] : 0;
-    uint32_t tot;
-    const uint32_t ex = block_excl_scan(v, &tot);
-    if (i < nchunks) sums[i] = carry + ex;
-    carry += tot;
-  }
-}
-
-__global__ void scan_down_kernel(uint32_t* __restrict__ data, int64_t n,
-                                 const uint32_t* __restrict__ sums) {
-  const int64_t c0 = (int64_t)blockIdx.x * SCAN_CHUNK;
-  // blocked arrangement: thread t owns items [t*ITEMS, (t+1)*ITEMS)
-  uint32_t v[SCAN_ITEMS];
-  uint32_t s = 0;
-#pragma unroll
-  for (int j = 0; j < SCAN_ITEMS; ++j) {
-    const int64_t i = c0 + (int64_t)threadIdx.x * SCAN_ITEMS + j;
-    v[j] = i < n ? data[i] : 0;
-    s += v[j];
-  }
-  uint32_t run = block_excl_scan(s, nullptr) + sums[blockIdx.x];
-#pragma unroll
-  for (int j = 0; j < SCAN_ITEMS; ++j) {
-    const int64_t i = c0 + (int64_t)threadIdx.x * SCAN_ITEMS + j;
-    if (i < n) data[i] = run;
-    run += v[j];
-  }
-}
-
 // --------------------------------------------------------- sorted jobs ----
 // the job of this block: last j with jobs[j].blk0 <= blockIdx.x
 __device__ __forceinline__ int sorted_job_of(const SortedJob* __restrict__ jobs, int njobs) {
@@ -576,54 +390,68 @@ __global__ void grid_inv_kernel(const JobDev* __restrict__ jobs,
   }
 }
 
-// keys[out + p_A] = cell key of the point at column-0 position p_A; vals = p_A.
-__global__ void grid_key_kernel(const JobDev* __restrict__ jobs,
-                                const int32_t* __restrict__ grid_jobs, int ngrid,
-                                const SortSeg* __restrict__ gsegs,
-                                const int32_t* __restrict__ sorted_vals,
-                                const SortSeg* __restrict__ segs,
-                                const int32_t* __restrict__ inv, const int32_t* __restrict__ sub,
-                                uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
+// Points per value of the digit threadIdx.x (256 threads), for keys that are
+// positions in a table of count + 1 starts.
+__device__ __forceinline__ uint32_t low_digit_total(const int32_t* __restrict__ starts, int count) {
+  uint32_t n = 0;
+  for (int k = (int)threadIdx.x; k < count; k += 256) n += (uint32_t)(starts[k + 1] - starts[k]);
+  return n;
+}
+__device__ __forceinline__ uint32_t high_digit_total(const int32_t* __restrict__ starts, int count) {
+  const int k = 256 * (int)threadIdx.x;
+  return (uint32_t)(starts[min(k + 256, count)] - starts[min(k, count)]);
+}
+
+// words[out + p_A] = cell key of the point at column-0 position p_A, and p_A.
+// The first block of a job writes its digit totals: the sizes of the cells.
+__global__ void __launch_bounds__(256)
+grid_key_kernel(const JobDev* __restrict__ jobs, const int32_t* __restrict__ grid_jobs, int ngrid,
+                const SortSeg* __restrict__ gsegs, const int32_t* __restrict__ sorted_vals,
+                const SortSeg* __restrict__ segs, const int32_t* __restrict__ inv,
+                const int32_t* __restrict__ sub, uint64_t* __restrict__ words,
+                uint32_t* __restrict__ seg_hist) {
   for (int g = blockIdx.y; g < ngrid; g += gridDim.y) {
     const JobDev& J = jobs[grid_jobs[g]];
     const int64_t out = gsegs[J.gseg].out_base;
     const int32_t* va = sorted_vals + segs[J.sort_seg].out_base;
     const int64_t len = J.len;
     const int nsub = J.nsub;
+    if (blockIdx.x == 0) {
+      const int32_t* starts = nsub > 0 ? J.cstart : J.sstart;
+      const int count = nsub > 0 ? J.nstrips * nsub : J.nstrips;
+      uint32_t* h = seg_hist + ((size_t)J.gseg * ALL_PASSES + GRID_PASS) * 256 + threadIdx.x;
+      h[0] = low_digit_total(starts, count);
+      h[256] = high_digit_total(starts, count);
+    }
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < len;
          p += (int64_t)gridDim.x * blockDim.x) {
       const int64_t w = va[p] - J.seg_begin;
       const int64_t strip = (int64_t)inv[out + w] * J.nstrips / len;
-      keys[out + p] = (uint64_t)(nsub > 0 ? strip * nsub + sub[out + w] : strip);
-      vals[out + p] = (int32_t)p;
+      words[out + p] = (uint64_t)(nsub > 0 ? strip * nsub + sub[out + w] : strip) << 32 | (uint32_t)p;
     }
   }
 }
 
-// keys[out + r] = strip of the point at column-2 position r; vals = its offset.
-__global__ void nest_key_kernel(const JobDev* __restrict__ jobs,
-                                const int32_t* __restrict__ grid_jobs, int ngrid,
-                                const SortSeg* __restrict__ gsegs,
-                                const int32_t* __restrict__ sorted_vals,
-                                const SortSeg* __restrict__ segs,
-                                const int32_t* __restrict__ inv, uint64_t* __restrict__ keys,
-                                int32_t* __restrict__ vals) {
+// words[out + r] = strip of the point at column-2 position r, and its offset.
+__global__ void __launch_bounds__(256)
+nest_key_kernel(const JobDev* __restrict__ jobs, const int32_t* __restrict__ grid_jobs, int ngrid,
+                const SortSeg* __restrict__ gsegs, const int32_t* __restrict__ sorted_vals,
+                const SortSeg* __restrict__ segs, const int32_t* __restrict__ inv,
+                uint64_t* __restrict__ words, uint32_t* __restrict__ seg_hist) {
   for (int g = blockIdx.y; g < ngrid; g += gridDim.y) {
     const JobDev& J = jobs[grid_jobs[g]];
     const int64_t out = gsegs[J.gseg].out_base;
     const int64_t len = J.len;
     const bool nested = J.nsub > 0;
     const int32_t* vc = nested ? sorted_vals + segs[J.sort_seg_c].out_base : nullptr;
+    if (blockIdx.x == 0)
+      seg_hist[((size_t)J.gseg * ALL_PASSES + NEST_PASS) * 256 + threadIdx.x] =
+          nested ? low_digit_total(J.sstart, J.nstrips) : threadIdx.x == 0 ? (uint32_t)len : 0u;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < len;
          r += (int64_t)gridDim.x * blockDim.x) {
-      if (nested) {
-        const int32_t w = vc[r] - J.seg_begin;
-        keys[out + r] = (uint64_t)((int64_t)inv[out + w] * J.nstrips / len);
-        vals[out + r] = w;
-      } else {
-        keys[out + r] = 0;
-        vals[out + r] = (int32_t)r;
-      }
+      const int32_t w = nested ? vc[r] - J.seg_begin : (int32_t)r;
+      const uint64_t strip = nested ? (uint64_t)((int64_t)inv[out + w] * J.nstrips / len) : 0u;
+      words[out + r] = strip << 32 | (uint32_t)w;
     }
   }
 }
@@ -634,9 +462,7 @@ __global__ void nest_sub_kernel(const TaskDev* __restrict__ tasks,
                                 const JobDev* __restrict__ jobs,
                                 const int32_t* __restrict__ grid_jobs, int ngrid,
                                 const SortSeg* __restrict__ gsegs,
-                                const uint64_t* __restrict__ keys_sorted,
-                                const int32_t* __restrict__ vals_sorted,
-                                int32_t* __restrict__ sub) {
+                                const uint64_t* __restrict__ words, int32_t* __restrict__ sub) {
   for (int g = blockIdx.y; g < ngrid; g += gridDim.y) {
     const JobDev& J = jobs[grid_jobs[g]];
     if (J.nsub <= 0) continue;
@@ -646,8 +472,9 @@ __global__ void nest_sub_kernel(const TaskDev* __restrict__ tasks,
     const double* z = t.col[J.sp.cols[2]] + J.seg_begin;
     for (int64_t p2 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p2 < J.len;
          p2 += (int64_t)gridDim.x * blockDim.x) {
-      const int s1 = (int)keys_sorted[out + p2];
-      const int32_t w = vals_sorted[out + p2];
+      const uint64_t word = words[out + p2];
+      const int s1 = (int)(word >> 32);
+      const int32_t w = (int32_t)(uint32_t)word;
       const int32_t s0 = J.sstart[s1];
       const int32_t L = J.sstart[s1 + 1] - s0;
       const int c2 = (int)((p2 - s0) * nsub / L);
@@ -685,47 +512,30 @@ void launch_grid_inv(const JobDev* jobs_d, const int32_t* grid_jobs_d, int ngrid
 
 void launch_grid_key(const JobDev* jobs_d, const int32_t* grid_jobs_d, int ngrid,
                      const SortSeg* gsegs_d, const int32_t* sorted_vals, const SortSeg* segs_d,
-                     const int32_t* inv_scratch, const int32_t* sub, uint64_t* gkeys,
-                     int32_t* gvals, int64_t max_len, cudaStream_t st) {
+                     const int32_t* inv_scratch, const int32_t* sub, uint64_t* words, const Sweep& w,
+                     int64_t max_len, cudaStream_t st) {
   if (ngrid <= 0) return;
-  grid_key_kernel<<<grid_of(ngrid, max_len), 256, 0, st>>>(jobs_d, grid_jobs_d, ngrid, gsegs_d,
-                                                           sorted_vals, segs_d, inv_scratch, sub,
-                                                           gkeys, gvals);
+  grid_key_kernel<<<grid_of(ngrid, max_len), 256, 0, st>>>(jobs_d, grid_jobs_d, ngrid, gsegs_d, sorted_vals,
+                                                           segs_d, inv_scratch, sub, words, w.seg_hist);
   count_launch();
 }
 
 void launch_nest_key(const JobDev* jobs_d, const int32_t* grid_jobs_d, int ngrid,
                      const SortSeg* gsegs_d, const int32_t* sorted_vals, const SortSeg* segs_d,
-                     const int32_t* inv_scratch, uint64_t* keys, int32_t* vals, int64_t max_len,
+                     const int32_t* inv_scratch, uint64_t* words, const Sweep& w, int64_t max_len,
                      cudaStream_t st) {
   if (ngrid <= 0) return;
-  nest_key_kernel<<<grid_of(ngrid, max_len), 256, 0, st>>>(jobs_d, grid_jobs_d, ngrid, gsegs_d,
-                                                           sorted_vals, segs_d, inv_scratch, keys,
-                                                           vals);
+  nest_key_kernel<<<grid_of(ngrid, max_len), 256, 0, st>>>(jobs_d, grid_jobs_d, ngrid, gsegs_d, sorted_vals,
+                                                           segs_d, inv_scratch, words, w.seg_hist);
   count_launch();
 }
 
 void launch_nest_sub(const TaskDev* tasks_d, const JobDev* jobs_d, const int32_t* grid_jobs_d,
-                     int ngrid, const SortSeg* gsegs_d, const uint64_t* keys_sorted,
-                     const int32_t* vals_sorted, int32_t* sub, int64_t max_len, cudaStream_t st) {
+                     int ngrid, const SortSeg* gsegs_d, const uint64_t* words, int32_t* sub,
+                     int64_t max_len, cudaStream_t st) {
   if (ngrid <= 0) return;
-  nest_sub_kernel<<<grid_of(ngrid, max_len), 256, 0, st>>>(tasks_d, jobs_d, grid_jobs_d, ngrid,
-                                                           gsegs_d, keys_sorted, vals_sorted, sub);
-  count_launch();
-}
-
-size_t sort_scan_tmp_elems(int nblk) {
-  const int64_t n = (int64_t)256 * nblk;
-  return (size_t)((n + SCAN_CHUNK - 1) / SCAN_CHUNK) + 1;
-}
-
-static void excl_scan(uint32_t* data, int64_t n, uint32_t* tmp, cudaStream_t st) {
-  const int nchunks = (int)((n + SCAN_CHUNK - 1) / SCAN_CHUNK);
-  scan_reduce_kernel<<<nchunks, SCAN_THREADS, 0, st>>>(data, n, tmp);
-  count_launch();
-  scan_top_kernel<<<1, SCAN_THREADS, 0, st>>>(tmp, nchunks);
-  count_launch();
-  scan_down_kernel<<<nchunks, SCAN_THREADS, 0, st>>>(data, n, tmp);
+  nest_sub_kernel<<<grid_of(ngrid, max_len), 256, 0, st>>>(tasks_d, jobs_d, grid_jobs_d, ngrid, gsegs_d, words,
+                                                           sub);
   count_launch();
 }
 
@@ -779,18 +589,6 @@ void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg
     count_launch();
   }
   launch_samples(segs_d, blk_seg_d, nblk, gl, keys_a, ko, redo, nseg, st);
-}
-
-void launch_radix_pass(const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
-                       const uint64_t* kin, const int32_t* vin, uint64_t* kout, int32_t* vout,
-                       int shift, uint32_t* hist, uint32_t* scan_tmp, cudaStream_t st) {
-  if (nblk <= 0) return;
-  sort_hist_kernel<<<nblk, SORT_THREADS, 0, st>>>(segs_d, blk_seg_d, kin, shift, hist);
-  count_launch();
-  excl_scan(hist, (int64_t)256 * nblk, scan_tmp, st);
-  sort_scatter_kernel<<<nblk, SORT_THREADS, 0, st>>>(segs_d, blk_seg_d, kin, vin, shift, hist,
-                                                     kout, vout);
-  count_launch();
 }
 
 void launch_sorted_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njobs,

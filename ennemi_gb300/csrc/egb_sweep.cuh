@@ -9,6 +9,10 @@ namespace egb {
 constexpr int OS_PASSES = 8;        // digits of a 64-bit key
 constexpr int CODE_PASSES = 4;      // digits of a 32-bit code, numbered 8 .. 11
 constexpr int ALL_PASSES = OS_PASSES + CODE_PASSES;
+// passes over the strip keys of the grid layouts, in a sweep buffer of their
+// own: the two digits of a cell, the strip of a nested job's column-2 order
+constexpr int GRID_PASS = OS_PASSES;
+constexpr int NEST_PASS = OS_PASSES + 2;
 constexpr int OS_SPIN_LIMIT = 1 << 22;
 
 // The sweep buffer (zeroed before the sort): flag words, digit totals per
