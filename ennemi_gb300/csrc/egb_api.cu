@@ -1048,6 +1048,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     }
   }
   int64_t sort_total = 0, s1_total = 0, s2_total = 0;
+  for (const SortSeg& s : segs) sort_total += s.len;
+  const int os_tile = os_tile_for(sort_total, ctx->num_sms);
+  sort_total = 0;
   int nblk_sort = 0, nblk_os = 0;
   for (SortSeg& s : segs) {
     s.out_base = sort_total;
@@ -1058,7 +1061,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     s.blk0 = nblk_sort;
     s.nblk = (s.len + SORT_TILE - 1) / SORT_TILE;
     s.os_blk0 = nblk_os;
-    s.os_nblk = (s.len + OS_TILE - 1) / OS_TILE;
+    s.os_nblk = (s.len + os_tile - 1) / os_tile;
     sort_total += s.len;
     nblk_sort += s.nblk;
     nblk_os += s.os_nblk;
@@ -1286,17 +1289,20 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       SortSeg g{};
       g.out_base = gsort_total;
       g.len = (int32_t)len;
-      g.os_blk0 = nblk_grid;
-      g.os_nblk = (int32_t)((len + OS_TILE - 1) / OS_TILE);
       gsegs.push_back(g);
       grid_jobs.push_back((int32_t)j);
       gsort_total += len;
-      nblk_grid += g.os_nblk;
       max_glen = std::max(max_glen, len);
     }
   }
 
   // strip-key sort of the grid jobs: words, ping-pong
+  const int grid_tile = os_tile_for(gsort_total, ctx->num_sms);
+  for (SortSeg& g : gsegs) {
+    g.os_blk0 = nblk_grid;
+    g.os_nblk = (g.len + grid_tile - 1) / grid_tile;
+    nblk_grid += g.os_nblk;
+  }
   const size_t off_gkeys_a = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(gsort_total, 1));
   const size_t off_gkeys_b = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(gsort_total, 1));
   const size_t off_ginv = dl.take(sizeof(int32_t) * (size_t)std::max<int64_t>(gsort_total, 1));
@@ -2003,7 +2009,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   const KeyIndex kx{keys, ko.fkeys, ko.s1, ko.s2, ko.fs1, ko.fs2};
   launch_sort(slots_d, (const double*)(A + off_centers), (const SortSeg*)dtab(tab_segs),
               (const int32_t*)dtab(tab_blkseg), nblk_sort, (const int32_t*)dtab(tab_osblkseg), nblk_os,
-              (int)segs.size(), keys, (uint64_t*)(A + off_keys_b), vals, (int32_t*)(A + off_vals_b), ko,
+              os_tile, (int)segs.size(), keys, (uint64_t*)(A + off_keys_b), vals, (int32_t*)(A + off_vals_b), ko,
               A + off_sweep, sort_first, sort_codes, ctx->num_sms, err_d, st,
               timing ? ctx->kev + 12 : nullptr);
   // the rank-space matrices need only the sorted values: they build on the
@@ -2036,7 +2042,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     Sweep gw;
     sweep_layout(A + off_gsweep, nblk_grid, (int)gsegs.size(), &gw);
     auto pass = [&](const uint64_t* in, uint64_t* out, int digit, int id) {
-      launch_word_pass(gsegs_d, blkg_d, nblk_grid, in, out, digit, id, gw, err_d, st);
+      launch_word_pass(gsegs_d, blkg_d, nblk_grid, grid_tile, in, out, digit, id, gw, err_d, st);
     };
     int32_t* ginv = (int32_t*)(A + off_ginv);
     int32_t* gsub = any_nested ? (int32_t*)(A + off_gsub) : nullptr;

@@ -37,8 +37,6 @@ constexpr int LOAD_THREADS = 256;
 constexpr int UNPACK_THREADS = 512;
 constexpr int PASS_THREADS = 256;          // one per digit
 constexpr int PASS_NW = PASS_THREADS / 32;
-constexpr int PASS_CH = OS_TILE / PASS_NW;   // words per warp
-constexpr int PASS_R = PASS_CH / 32;         // rounds per warp
 constexpr int TIE_RUN = 32;
 
 __device__ __forceinline__ uint32_t code_of(double x, double c) {
@@ -76,22 +74,26 @@ code_load_kernel(const BatchCol* __restrict__ slots, const double* __restrict__ 
 
 // One digit of the codes: the single-sweep pass of egb_sort.cu on words.  A
 // tile's missing words read as the largest digit, behind all others.
+template <int TILE>
 struct PassSmem {
   uint32_t wcnt[PASS_NW][256];  // per-warp digit counts, then offsets
   uint32_t dstart[256];         // first tile slot of each digit
   uint32_t gbase[256];          // first output position of each digit, less dstart
   uint2 warp_sum[PASS_NW];      // of the two digit scans
   int tile;
-  uint64_t sk[OS_TILE];
+  uint64_t sk[TILE];
 };
 
+template <int TILE, int LOOK>
 __global__ void __launch_bounds__(PASS_THREADS, 5)
 code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ os_blk_seg,
                  const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int digit, int pass,
                  const uint32_t* __restrict__ seg_hist, unsigned long long* flags, int* tile_counter,
                  uint32_t* err) {
+  constexpr int PASS_CH = TILE / PASS_NW;  // words per warp
+  constexpr int PASS_R = PASS_CH / 32;     // rounds per warp
   extern __shared__ __align__(16) unsigned char raw[];
-  PassSmem& S = *reinterpret_cast<PassSmem*>(raw);
+  PassSmem<TILE>& S = *reinterpret_cast<PassSmem<TILE>*>(raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) S.tile = atomicAdd(tile_counter, 1);
   for (int i = tid; i < PASS_NW * 256; i += PASS_THREADS) (&S.wcnt[0][0])[i] = 0u;
@@ -100,8 +102,8 @@ code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ o
   const int si = os_blk_seg[b];
   const int64_t base = segs[si].out_base;
   const int len = segs[si].len, first = segs[si].os_blk0;
-  const int i0 = (b - first) * OS_TILE;
-  const int n = min(OS_TILE, len - i0);
+  const int i0 = (b - first) * TILE;
+  const int n = min(TILE, len - i0);
   const int shift = 8 * digit;
   const uint32_t lt = (1u << lane) - 1u;
   uint64_t key[PASS_R];
@@ -133,7 +135,7 @@ code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ o
     S.wcnt[w][tid] = cnt;
     cnt += c;
   }
-  if (tid == 255) cnt -= (uint32_t)(OS_TILE - n);
+  if (tid == 255) cnt -= (uint32_t)(TILE - n);
   // exclusive scans over the digits of the tile's counts and of the segment's
   const uint32_t tot = seg_hist[((size_t)si * ALL_PASSES + pass) * 256 + tid];
   uint2 sum = make_uint2(cnt, tot);
@@ -143,7 +145,7 @@ code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ o
     if (lane >= o) sum.x += a, sum.y += c;
   }
   if (lane == 31) S.warp_sum[warp] = sum;
-  const uint32_t excl = sweep_look_back(flags, b, first, tid, pass, cnt, err);
+  const uint32_t excl = sweep_look_back<LOOK>(flags, b, first, tid, pass, cnt, err);
   __syncthreads();
   for (int w = 0; w < warp; ++w) sum.x += S.warp_sum[w].x, sum.y += S.warp_sum[w].y;
   S.gbase[tid] = (sum.y - tot) + excl - (sum.x - cnt);
@@ -246,15 +248,20 @@ static_assert((SORT_TILE + 64) % 32 == 0 && TIE_RUN <= 32, "inversion words");
 }  // namespace
 
 int init_code_sort() {
-  return (int)cudaFuncSetAttribute(code_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(PassSmem));
+  return (int)cudaFuncSetAttribute(code_pass_kernel<OS_TILE, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(PassSmem<OS_TILE>));
 }
 
-void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, const uint64_t* in,
-                      uint64_t* out, int digit, int pass, const Sweep& w, uint32_t* err, cudaStream_t st) {
+void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, int os_tile,
+                      const uint64_t* in, uint64_t* out, int digit, int pass, const Sweep& w, uint32_t* err,
+                      cudaStream_t st) {
   if (os_nblk <= 0) return;
-  code_pass_kernel<<<os_nblk, PASS_THREADS, sizeof(PassSmem), st>>>(segs_d, os_blk_seg_d, in, out, digit, pass,
-                                                                    w.seg_hist, w.flags, w.counters + pass, err);
+  auto run = [&](auto kernel, size_t smem) {
+    kernel<<<os_nblk, PASS_THREADS, smem, st>>>(segs_d, os_blk_seg_d, in, out, digit, pass, w.seg_hist, w.flags,
+                                                w.counters + pass, err);
+  };
+  if (os_tile == OS_TILE) run(code_pass_kernel<OS_TILE, 1>, sizeof(PassSmem<OS_TILE>));
+  else run(code_pass_kernel<OS_TILE_SMALL, 4>, sizeof(PassSmem<OS_TILE_SMALL>));
   count_launch();
 }
 
@@ -268,7 +275,7 @@ void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const So
   uint64_t* in = words;  // an even number of passes: back in words
   uint64_t* out = keys;
   for (int d = 0; d < CODE_PASSES; ++d) {
-    launch_word_pass(segs_d, os_blk_seg_d, os_nblk, in, out, d, OS_PASSES + d, w, err, st);
+    launch_word_pass(segs_d, os_blk_seg_d, os_nblk, OS_TILE, in, out, d, OS_PASSES + d, w, err, st);
     uint64_t* t = in; in = out; out = t;
   }
   if (pass_events) cudaEventRecord(pass_events[1], st);

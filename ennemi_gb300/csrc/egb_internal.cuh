@@ -433,7 +433,7 @@ struct SortSeg {          // one segment of the batched radix sort
   int32_t nblk;
   int32_t slot;           // batch column
   int32_t src_begin;      // first working index of the segment
-  int32_t os_blk0;        // its first tile of the single-sweep passes (OS_TILE keys)
+  int32_t os_blk0;        // its first tile of the single-sweep passes
   int32_t os_nblk;
 };
 
@@ -523,7 +523,16 @@ void launch_combine(const TaskDev* tasks_d, const CombineJob* jobs_d, const int3
 
 // egb_sort.cu
 constexpr int SORT_TILE = 2048;
-constexpr int OS_TILE = 4096;   // keys per tile of the batch sort's single-sweep passes
+// Keys per tile of the single-sweep passes.  A sort that the small tile still
+// leaves at one tile per SM takes it: there a pass lasts as long as a tile does.
+// Six passes over 20,000 / 40,000 / 300,000 keys: 47 / 50 / 56 us on 4096, 38 / 40 /
+// 50 on 2048 (34 / 37 / 55 on 1024); over 600,000, 60 against 69; 142 million words
+// in four passes, 3.3 ms against 4.1.
+constexpr int OS_TILE = 4096;
+constexpr int OS_TILE_SMALL = 2048;
+inline int os_tile_for(int64_t keys, int num_sms) {
+  return keys <= (int64_t)OS_TILE_SMALL * num_sms ? OS_TILE_SMALL : OS_TILE;
+}
 // The batch's sorted keys and the arrays searched in their place: each
 // key's value rounded down to FP32 (exact comparisons against FP32 bounds in
 // half the bytes), and samples of both (egb_search.cuh), at each segment's
@@ -577,9 +586,10 @@ void launch_nest_sub(const TaskDev* tasks_d, const JobDev* jobs_d, const int32_t
                      int ngrid, const SortSeg* gsegs_d, const uint64_t* words, int32_t* sub,
                      int64_t max_len, cudaStream_t st);
 // One stable pass (egb_codesort.cu) over the digit (bits 8 digit ..) of the
-// words' upper halves, the segments' OS_TILE tiles given.
-void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, const uint64_t* in,
-                      uint64_t* out, int digit, int pass, const Sweep& w, uint32_t* err, cudaStream_t st);
+// words' upper halves, the segments' tiles of os_tile words given.
+void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, int os_tile,
+                      const uint64_t* in, uint64_t* out, int digit, int pass, const Sweep& w, uint32_t* err,
+                      cudaStream_t st);
 // The batch sort: single-sweep LSD passes over the 8-bit digits first..7 of
 // the keys (first = 0: all; first = 2: the high 48 bits, then a repair of
 // the rare runs tied there, which sets DERR_SORT_TIES when one is too long);
@@ -587,7 +597,8 @@ void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os
 // flags, digit totals and tile counters.  `first` is even: the result is in
 // keys_a / vals_a.
 // blk_seg_d / nblk: the segments' SORT_TILE tiles (load and repair
-// kernels); os_blk_seg_d / os_nblk: their OS_TILE tiles (the passes).
+// kernels); os_blk_seg_d / os_nblk: their tiles of os_tile keys (the
+// passes).
 size_t sort_sweep_bytes(int os_nblk, int nseg);
 // Once per context, on its device: lets the passes use their shared memory
 // (above the 48 KB default); returns the cudaError_t.
@@ -602,7 +613,7 @@ int init_sort_kernels();
 constexpr int64_t SORT_CODES_MIN = 1 << 20;
 void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
                  const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
-                 int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
+                 int os_tile, int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
                  const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
                  uint32_t* err, cudaStream_t st,
                  cudaEvent_t* pass_events = nullptr);  // recorded around the passes alone

@@ -82,31 +82,33 @@ onesweep_load_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restri
   }
 }
 
-// A pass tile is OS_TILE keys on OS_THREADS threads (eight keys a thread);
+// A pass tile is TILE keys on OS_THREADS threads (four or eight keys a thread);
 // its staging arrays exceed the 48 KB of static shared memory.
 constexpr int OS_THREADS = 512;
 constexpr int OS_NW = OS_THREADS / 32;
+template <int TILE>
 struct OsSmem {
   uint32_t wcnt[OS_NW][256];  // per-warp digit counts, then offsets
   uint32_t dstart[256];       // first tile slot of each digit
   uint32_t gbase[256];        // first output position of each digit
   uint32_t ws[8];             // digit-scan scratch
   int tile;
-  uint64_t sk[OS_TILE];
-  int32_t sv[OS_TILE];
+  uint64_t sk[TILE];
+  int32_t sv[TILE];
 };
-static_assert(OS_TILE % OS_NW == 0 && (OS_TILE / OS_NW) % 32 == 0, "whole warp rounds");
 
+template <int TILE>
 __global__ void __launch_bounds__(OS_THREADS)
 onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ os_blk_seg, int nblk,
                      const uint64_t* __restrict__ kin, const int32_t* __restrict__ vin,
                      uint64_t* __restrict__ kout, int32_t* __restrict__ vout, int pass,
                      const uint32_t* __restrict__ seg_hist, unsigned long long* flags,
                      int* tile_counter, uint32_t* err, const uint32_t* __restrict__ redo, int nseg) {
-  constexpr int CH = OS_TILE / OS_NW;  // keys per warp
+  constexpr int CH = TILE / OS_NW;  // keys per warp
   constexpr int R = CH / 32;           // rounds per warp
+  static_assert(TILE % OS_NW == 0 && CH % 32 == 0, "whole warp rounds");
   extern __shared__ __align__(16) unsigned char os_raw[];
-  OsSmem& S = *reinterpret_cast<OsSmem*>(os_raw);
+  OsSmem<TILE>& S = *reinterpret_cast<OsSmem<TILE>*>(os_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (redo && !redo[nseg]) return;
   for (bool more = true; more; more = redo != nullptr) {
@@ -121,8 +123,8 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
     const SortSeg s = segs[si];
     const int lb = b - s.os_blk0;
     const int shift = 8 * pass;
-    const int i0 = lb * OS_TILE;
-    const int n = min(OS_TILE, s.len - i0);
+    const int i0 = lb * TILE;
+    const int n = min(TILE, s.len - i0);
     const uint32_t lt = (1u << lane) - 1u;
     uint64_t key[R];
     int32_t val[R];
@@ -159,7 +161,7 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
     }
     // publish this tile's count of digit tid, then look back for the count of
     // digit tid in the segment's earlier tiles
-    const uint32_t excl = tid < 256 ? sweep_look_back(flags, b, s.os_blk0, tid, pass, cnt, err) : 0u;
+    const uint32_t excl = tid < 256 ? sweep_look_back<8>(flags, b, s.os_blk0, tid, pass, cnt, err) : 0u;
     // digit tid of the whole segment starts after the smaller digits
     const uint32_t seg_tot = tid < 256 ? seg_hist[((size_t)si * ALL_PASSES + pass) * 256 + tid] : 0u;
     const uint32_t seg_off = digit_excl_scan(seg_tot, S.ws);
@@ -542,15 +544,15 @@ void launch_nest_sub(const TaskDev* tasks_d, const JobDev* jobs_d, const int32_t
 int init_sort_kernels() {
   const int rc = init_code_sort();
   if (rc) return rc;
-  return (int)cudaFuncSetAttribute(onesweep_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(OsSmem));
+  return (int)cudaFuncSetAttribute(onesweep_pass_kernel<OS_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(OsSmem<OS_TILE>));
 }
 
 size_t sort_sweep_bytes(int os_nblk, int nseg) { return sweep_layout(nullptr, os_nblk, nseg, nullptr) + 64; }
 
 void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
                  const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
-                 int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
+                 int os_tile, int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
                  const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
                  uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
   if (nblk <= 0 || os_nblk <= 0) {
@@ -574,9 +576,12 @@ void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg
   int32_t* vout = vals_b;
   if (pass_events && !codes) cudaEventRecord(pass_events[0], st);
   for (int pass = first; pass < OS_PASSES; ++pass) {
-    onesweep_pass_kernel<<<gp, OS_THREADS, sizeof(OsSmem), st>>>(segs_d, os_blk_seg_d, os_nblk, kin, vin,
-                                                                 kout, vout, pass, w.seg_hist, w.flags,
-                                                                 w.counters + pass, err, redo, nseg);
+    auto run = [&](auto kernel, size_t smem) {
+      kernel<<<gp, OS_THREADS, smem, st>>>(segs_d, os_blk_seg_d, os_nblk, kin, vin, kout, vout, pass, w.seg_hist,
+                                           w.flags, w.counters + pass, err, redo, nseg);
+    };
+    if (os_tile == OS_TILE) run(onesweep_pass_kernel<OS_TILE>, sizeof(OsSmem<OS_TILE>));
+    else run(onesweep_pass_kernel<OS_TILE_SMALL>, sizeof(OsSmem<OS_TILE_SMALL>));
     count_launch();
     uint64_t* tk = kin; kin = kout; kout = tk;
     int32_t* tv = vin; vin = vout; vout = tv;

@@ -44,6 +44,7 @@ __device__ __forceinline__ uint64_t key_of_bits(uint64_t u) {
 
 // Publishes the count of one digit in tile b and returns its count in the
 // segment's earlier tiles (first: the segment's first tile).
+template <int LOOK>
 __device__ __forceinline__ uint32_t sweep_look_back(unsigned long long* flags, int b, int first, int digit,
                                                     int pass, uint32_t cnt, uint32_t* err) {
   const unsigned long long tag = (unsigned long long)(pass + 1) << 56;
@@ -56,21 +57,25 @@ __device__ __forceinline__ uint32_t sweep_look_back(unsigned long long* flags, i
   atomicExch(mine, tag | cnt);
   uint32_t excl = 0;
   int pb = b - 1;
-  for (;;) {
-    const volatile unsigned long long* f = flags + (size_t)pb * 256 + digit;
-    unsigned long long w = *f;
-    int spins = 0;
-    while ((w >> 56) != (unsigned long long)(pass + 1)) {
-      if (++spins > OS_SPIN_LIMIT) {
-        atomicOr(err, DERR_WAIT_TIMEOUT);
-        w = tag | INCL;
-        break;
+  for (bool more = true; more; pb -= LOOK) {  // LOOK tiles at once: one latency
+    unsigned long long w[LOOK];
+#pragma unroll
+    for (int i = 0; i < LOOK; ++i) w[i] = *(volatile unsigned long long*)(flags + (size_t)max(pb - i, first) * 256 + digit);
+#pragma unroll
+    for (int i = 0; i < LOOK; ++i) {
+      if (!more) break;
+      int spins = 0;
+      while ((w[i] >> 56) != (unsigned long long)(pass + 1)) {
+        if (++spins > OS_SPIN_LIMIT) {
+          atomicOr(err, DERR_WAIT_TIMEOUT);
+          w[i] = tag | INCL;
+          break;
+        }
+        w[i] = *(volatile unsigned long long*)(flags + (size_t)(pb - i) * 256 + digit);
       }
-      w = *f;
+      excl += (uint32_t)w[i];
+      more = !(w[i] & INCL) && pb - i > first;
     }
-    excl += (uint32_t)w;
-    if ((w & INCL) || pb <= first) break;
-    --pb;
   }
   atomicExch(mine, tag | INCL | (excl + cnt));
   return excl;
