@@ -1200,7 +1200,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     if (m.mode >= 2) {
       J.c64g = (double*)(uintptr_t)dl.take(sizeof(double) * (size_t)(d * J.lds));
       // by point where the walks and the warp lists of two and three columns read it
-      J.aos = (m.mode == 3 && m.is_knn && !plain && d <= 3) ? 1 : 0;
+      J.aos = (m.mode == 3 && m.is_knn && !plain && d <= 4) ? 1 : 0;
       J.c32g = (float*)(uintptr_t)dl.take(sizeof(float) * (size_t)((J.aos ? grid_aos(d) : d) * J.lds));
       J.idxg = (int32_t*)(uintptr_t)dl.take(sizeof(int32_t) * (size_t)J.lds);
       // (read by the deferred queries of the CTA grid only)

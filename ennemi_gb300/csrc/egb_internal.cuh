@@ -308,7 +308,7 @@ struct JobDev {
   // equal-count strips by their rank in column 1, each strip sorted by
   // column 0 -- with, per position, its position in the column-0 order
   double* c64g;
-  float* c32g;            // [d][lds], or by point for the kNN kernels of d = 2, 3
+  float* c32g;            // [d][lds], or by point for the kNN kernels of d = 2 to 4
                           // (aos): grid_aos(d) floats each
   int32_t* idxg;
   int32_t* posg;
@@ -351,7 +351,8 @@ __host__ __device__ __forceinline__ int32_t cell_start(int32_t s0, int32_t L, in
   return s0 + strip_start(c2, L, nsub);
 }
 constexpr int NEST_CELL_3D = 384;     // points per nested-grid cell, kNN jobs of d = 3
-constexpr int NEST_CELL_4D = 512;     // d >= 4 (200,000 4-D points, K = 4: 1.83 ms on 256, 1.46 on 512)
+constexpr int NEST_CELL_4D = 512;     // d >= 4 (120 sets of 20,000 4-D points, K = 4: 5.04 ms on 512,
+                                      // 5.16 on 384; 200,000: 1.83 ms on 256, 1.46 on 512)
 // the FP64 comparator's kNN jobs of d >= 4, and its count jobs, which take at
 // least NEST_SIDE_C * len^(1/dj) cells per side (dj: see strips)
 constexpr int NEST_CELL_4D_FP64 = 256;

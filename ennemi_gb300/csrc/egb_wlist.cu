@@ -27,7 +27,11 @@
 // exact distances of the candidates within U (all candidates).
 //
 // What bounds it: instruction issue and the latency of a query's ranges in
-// turn.  20,000 points, K = 51, d = 2: 0.10 ms, against 25.4 ms for the select
+// turn (72 registers, seven blocks an SM: 6.3 -> 5.7 ms for 2.4 million 4-D
+// queries, K = 4, against six; eight blocks 5.8, ten 5.9).  First bounds from 128
+// neighbours and a bound renewed after two new candidates, against 32 and eight:
+// 5.7 -> 5.0 ms (256 neighbours 5.7); 100,000 6-D points, K = 6: 9.5 -> 4.1 ms; but
+// 100,000 3-D points, K = 13, 283 -> 324 us, so three columns keep 32 and eight.  20,000 points, K = 51, d = 2: 0.10 ms, against 25.4 ms for the select
 // over all points that served K > 32 before; K = 13: 65 us against 252 of the
 // CTA grid; d = 4, K = 4, 200,000 points: 1.04 ms against 1.66 of the walks.
 #include <algorithm>
@@ -49,12 +53,15 @@ using list_detail::radix_kth;
 constexpr int WL_WARPS = 4;
 
 template <int D, int R, bool GRID, bool NEST>
-__global__ void __launch_bounds__(WL_WARPS * 32)
+__global__ void __launch_bounds__(WL_WARPS * 32, 7)
 wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items, int nitems, int qb,
              int per, int* __restrict__ counter) {
   constexpr int DQ = D ? D : EGB_DMAX;
-  // two and three columns: grid copies by point (JobDev::aos)
-  constexpr int AOS = GRID && (D == 2 || D == 3) ? grid_aos(D) : 0;
+  // two to four columns: grid copies by point (JobDev::aos)
+  constexpr int AOS = GRID && D ? grid_aos(D) : 0;
+  // from four columns on a point's neighbours along column 0 are far in the
+  // others: more of them for the first bound, and the bound renewed sooner
+  constexpr bool DEEP = NEST && D != 3;
   __shared__ __align__(8) uint32_t store[WL_WARPS][CandidateList<R>::WORDS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int split = (qb + per - 1) / per;  // parts of `per` queries of an item
@@ -118,7 +125,8 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
               dd = fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1]));
             } else if constexpr (AOS == 4) {
               const float4 p = reinterpret_cast<const float4*>(g)[j];
-              dd = fmaxf(fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1])), fabsf(p.z - qv[D == 3 ? 2 : 0]));
+              dd = fmaxf(fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1])), fabsf(p.z - qv[D >= 3 ? 2 : 0]));
+              if constexpr (D == 4) dd = fmaxf(dd, fabsf(p.w - qv[D == 4 ? 3 : 0]));
             } else {
               dd = fabsf(g[j] - qv[0]);
 #pragma unroll
@@ -145,7 +153,7 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
           // first bound: the query's neighbours in its own strip or cell
           const int ha = NEST ? cst[sq * S2 + hc] : sst[sq];
           const int hb = NEST ? cst[sq * S2 + hc + 1] : sst[sq + 1];
-          const int w = (K + 31) / 32 * 16;
+          const int w = (K + 31) / 32 * (DEEP ? 64 : 16);
           e0 = max(ha, qp - w);
           e1 = min(hb, e0 + 2 * w);
           screen(e0, e1, 0, 0);
@@ -155,7 +163,7 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
           if (list.over) return;
           const int had = list.cnt;
           screen(a, b, e0, e1);
-          if (list.cnt >= K && (list.cnt - had >= 8 || !(list.thr < __builtin_huge_valf()))) list.tighten();
+          if (list.cnt >= K && (list.cnt - had >= (DEEP ? 2 : 8) || !(list.thr < __builtin_huge_valf()))) list.tighten();
         });
       }
       if (!unsafe && !list.over) {
