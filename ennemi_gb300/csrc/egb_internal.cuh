@@ -591,6 +591,18 @@ void launch_nest_sub(const TaskDev* tasks_d, const JobDev* jobs_d, const int32_t
 void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, int os_tile,
                       const uint64_t* in, uint64_t* out, int digit, int pass, const Sweep& w, uint32_t* err,
                       cudaStream_t st);
+// Class orders: perm[w] = the w-th sample by (label, sample), by one stable pass
+// per label byte over (label, sample) words.
+struct LabelJob {
+  const int32_t* labels;   // [n], each in [0, nclass)
+  const int32_t* starts;   // [nclass + 1] first place of each class
+  int32_t* perm;           // [n] out
+  int64_t out_base;        // of its words
+  int32_t n, nclass;
+};
+void launch_label_order(const LabelJob* jobs_d, int njobs, int max_classes, int64_t max_n,
+                        const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, int os_tile,
+                        uint64_t* words_a, uint64_t* words_b, const Sweep& w, uint32_t* err, cudaStream_t st);
 // The batch sort: single-sweep LSD passes over the 8-bit digits first..7 of
 // the keys (first = 0: all; first = 2: the high 48 bits, then a repair of
 // the rare runs tied there, which sets DERR_SORT_TIES when one is too long);

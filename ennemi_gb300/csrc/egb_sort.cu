@@ -404,6 +404,32 @@ __device__ __forceinline__ uint32_t high_digit_total(const int32_t* __restrict__
   return (uint32_t)(starts[min(k + 256, count)] - starts[min(k, count)]);
 }
 
+// words[out + i] = (label, i), with the digit totals from the class sizes.
+__global__ void __launch_bounds__(256)
+label_word_kernel(const LabelJob* __restrict__ jobs, int njobs, uint64_t* __restrict__ words,
+                  uint32_t* __restrict__ seg_hist) {
+  for (int g = blockIdx.y; g < njobs; g += gridDim.y) {
+    const LabelJob& J = jobs[g];
+    if (blockIdx.x == 0) {
+      uint32_t* h = seg_hist + ((size_t)g * ALL_PASSES + GRID_PASS) * 256 + threadIdx.x;
+      h[0] = low_digit_total(J.starts, J.nclass);
+      h[256] = high_digit_total(J.starts, J.nclass);
+    }
+    const int32_t* __restrict__ labels = J.labels;
+    uint64_t* __restrict__ out = words + J.out_base;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < J.n; i += gridDim.x * 256)
+      out[i] = (uint64_t)(uint32_t)labels[i] << 32 | (uint32_t)i;
+  }
+}
+__global__ void __launch_bounds__(256)
+label_perm_kernel(const LabelJob* __restrict__ jobs, int njobs, const uint64_t* __restrict__ words) {
+  for (int g = blockIdx.y; g < njobs; g += gridDim.y) {
+    const LabelJob& J = jobs[g];
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < J.n; i += gridDim.x * 256)
+      J.perm[i] = (int32_t)(uint32_t)words[J.out_base + i];
+  }
+}
+
 // words[out + p_A] = cell key of the point at column-0 position p_A, and p_A.
 // The first block of a job writes its digit totals: the sizes of the cells.
 __global__ void __launch_bounds__(256)
@@ -509,6 +535,22 @@ void launch_grid_inv(const JobDev* jobs_d, const int32_t* grid_jobs_d, int ngrid
   if (ngrid <= 0) return;
   grid_inv_kernel<<<grid_of(ngrid, max_len), 256, 0, st>>>(jobs_d, grid_jobs_d, ngrid, gsegs_d,
                                                            sorted_vals, segs_d, inv_scratch);
+  count_launch();
+}
+
+void launch_label_order(const LabelJob* jobs_d, int njobs, int max_classes, int64_t max_n,
+                        const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os_nblk, int os_tile,
+                        uint64_t* words_a, uint64_t* words_b, const Sweep& w, uint32_t* err, cudaStream_t st) {
+  if (njobs <= 0) return;
+  label_word_kernel<<<grid_of(njobs, max_n), 256, 0, st>>>(jobs_d, njobs, words_a, w.seg_hist);
+  count_launch();
+  launch_word_pass(segs_d, os_blk_seg_d, os_nblk, os_tile, words_a, words_b, 0, GRID_PASS, w, err, st);
+  uint64_t* sorted = words_b;
+  if (max_classes > 256) {
+    launch_word_pass(segs_d, os_blk_seg_d, os_nblk, os_tile, words_b, words_a, 1, GRID_PASS + 1, w, err, st);
+    sorted = words_a;
+  }
+  label_perm_kernel<<<grid_of(njobs, max_n), 256, 0, st>>>(jobs_d, njobs, sorted);
   count_launch();
 }
 

@@ -375,6 +375,28 @@ def test_small_batches_take_the_form_that_fits(count, n, data):
         assert np.array_equal(N.fetch(t, 0, n), e, equal_nan=True), t
 
 
+@pytest.mark.parametrize("nclass", [1, 2, 255, 256, 257, 900])
+@pytest.mark.parametrize("n", [19_999, 20_000, 20_480, 70_001])
+def test_class_order_on_the_device(n, nclass):
+    """Class orders built on the device (the sizes about where it starts; one
+    and two label bytes, empty classes) give what the host's order gives."""
+    rng = np.random.default_rng(n + nclass)
+    used = rng.permutation(nclass)[: max(1, nclass - nclass // 4)]
+    tasks = []
+    for kind in (N.SEMI, N.CSEMI, N.SEMI):
+        lab = np.sort(rng.choice(used, n)) if len(tasks) == 2 else rng.choice(used, n)
+        x = rng.normal(size=n) + 0.1 * lab / nclass
+        tasks.append(N.Task(kind, 3, [x], [], [rng.normal(size=n)] if kind == N.CSEMI else [],
+                            labels=lab.astype(np.int32), nclass=nclass, n=n))
+    host = N.run_tasks(tasks, flags=N.KEEP_INTERNALS)
+    for flags in (0, N.STAGE_HOST, N.TIMING):
+        assert np.array_equal(N.run_tasks(tasks, flags=flags), host, equal_nan=True), flags
+    bad = tasks[0].labels.copy()
+    bad[-1] = nclass
+    with pytest.raises(RuntimeError, match="label out of range"):
+        N.run_tasks([N.Task(N.SEMI, 3, [x], [], [], labels=bad, nclass=nclass, n=n)])
+
+
 @pytest.mark.parametrize("data", ["independent", "cubic", "square", "steps", "constant", "huge"])
 @pytest.mark.parametrize("n", [4096, 4099, 20_001])
 def test_strip_layouts(oracle, n, data):
