@@ -313,11 +313,9 @@ void launch_t(const JobDev* jobs, const WorkItem* items, int nitems, int* counte
 // are read instead
 bool count_keys_supported(int dclass) { return dclass == 2; }
 
-void launch_count_keys(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass,
+void launch_count_keys(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int /*dclass*/,
                        int* counter, int num_sms, cudaStream_t st) {
-  if (dclass == 2) launch_t<2>(jobs_d, items_d, nitems, counter, num_sms, st);
-  else if (dclass == 3) launch_t<3>(jobs_d, items_d, nitems, counter, num_sms, st);
-  else launch_t<4>(jobs_d, items_d, nitems, counter, num_sms, st);
+  launch_t<2>(jobs_d, items_d, nitems, counter, num_sms, st);
 }
 
 }  // namespace egb
