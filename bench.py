@@ -500,21 +500,23 @@ def main():
     max_mhz = clocks.get("sm_max_mhz") or peaks.get("sm_max_mhz") or 2070.0
     peak_ops = sms * 128 * max_mhz * 1e6
 
-    # The dominant kernel (largest share of the step in the ncu launch list)
-    # is the radix sort's pass, HBM-bound: per launch it reads and writes
-    # every key (8 B) and index (4 B) of the batch's sort once.  Its time per
-    # launch is the event-timed run of the batch's digit passes over their
-    # number.  DRAM traffic per launch from one ncu capture of this workload
-    # (cold cache, the six passes of one batch averaged): 137.6 MB read +
-    # 82.5 MB written.
+    # The kernel with the most bytes is the batch sort's pass, HBM-bound: per
+    # launch it reads and writes every point's word of the batch's sort (8 B;
+    # in batches below a million keys, which sort the keys' own digits, key and
+    # index, 12 B).  Its time per launch is the event-timed run of the passes
+    # over their number.  DRAM traffic per launch from one ncu capture of this
+    # workload (cold cache, the four passes of one batch averaged): 93.6 MB
+    # read + 67.0 MB written.
     keys = work_stats.get("sort_keys", 0)
     npass = work_stats.get("sort_passes", 0) or 8
+    codes = npass == 4
     pass_ms = phases.get("sort_passes", 0.0) / npass
-    pass_bytes = 24.0 * keys
+    pass_bytes = (16.0 if codes else 24.0) * keys
     pass_gbs = pass_bytes / (pass_ms / 1000.0) / 1e9 if pass_ms > 0 else 0.0
-    roofline = {"bound": "hbm", "kernel": "onesweep_pass_kernel (radix sort pass)",
+    roofline = {"bound": "hbm", "kernel": ("code_pass_kernel" if codes else "onesweep_pass_kernel")
+                + " (radix sort pass)",
                 "achieved": pass_gbs, "peak": hbm, "unit": "GB/s", "frac": pass_gbs / hbm,
-                "traffic": (137.61 + 82.46) * 1e6 if args.n == 1_000_000 else None,
+                "traffic": (93.6 + 67.0) * 1e6 if args.n == 1_000_000 else None,
                 "traffic_unit": "bytes per launch (ncu, cold cache)",
                 "algorithmic_bytes_per_launch": pass_bytes, "ms_per_launch": pass_ms,
                 "launches_per_step": npass, "peak_source": hbm_src}
@@ -533,31 +535,31 @@ def main():
             "achieved_gops": knn_ops / (knn_ms / 1000.0) / 1e9 if knn_ms > 0 else 0.0,
             "nominal_fp32_lane_gops": peak_ops / 1e9,
             "frac_of_nominal": (knn_ops / (knn_ms / 1000.0)) / peak_ops if knn_ms > 0 else 0.0,
-            "dram_traffic_per_launch": ((114.16 + 16.75) + (40.62 + 0.03)) / 2 * 1e6
+            "dram_traffic_per_launch": ((114.18 + 17.09) + (44.62 + 0.47)) / 2 * 1e6
             if args.n == 1_000_000 else None,
             "algorithmic_savings": {"bruteforce_ops": bf_ops, "counted_ops": knn_ops,
                                     "ratio": bf_ops / knn_ops if knn_ops else None}},
         "wm_count_kernel (rank-space counts, 2 x 2-D)": {
             "ms": cnt_ms, "queries": 2 * args.n,
             "ns_per_query": cnt_ms * 1e6 / (2 * args.n) if cnt_ms > 0 else None,
-            "dram_traffic_per_launch": (58.30 + 2.48) * 1e6 if args.n == 1_000_000 else None},
-        "sorted_jobs_kernel (1-D counts)": {
+            "dram_traffic_per_launch": (58.30 + 1.99) * 1e6 if args.n == 1_000_000 else None},
+        "ball_jobs_kernel (1-D counts)": {
             "ms": phases.get("count_1d", 0.0), "queries": sum(2 if kind == "mi" else 1
                                                               for kind, _ in work) * args.n,
-            "dram_traffic_per_launch": (186.65 + 37.53) * 1e6 if args.n == 1_000_000 else None},
+            "dram_traffic_per_launch": (187.84 + 32.19) * 1e6 if args.n == 1_000_000 else None},
     }
 
     # sort and 1-D search passes together, on the minimal byte count of a 1-D
     # marginal: 32 N (8 N keys read, 8 N sorted keys written, 8 N eps read,
     # 8 N counts written) over the radix sort's and the 1-D counts' event
-    # times -- a bound no multi-pass sort reaches (the sort moves 24 B per
+    # times -- a bound no multi-pass sort reaches (the sort moves 16 B per
     # key and pass, and sorts the grid-only columns too)
     n1d = sum(2 if kind == "mi" else 1 for kind, _ in work)
     sort_ms, c1_ms = phases.get("sort_radix", 0.0), phases.get("count_1d", 0.0)
     ss_bytes = 32.0 * args.n * n1d
     ss_gbs = ss_bytes / ((sort_ms + c1_ms) / 1000.0) / 1e9 if sort_ms + c1_ms > 0 else 0.0
     roofline_sort = {"bound": "hbm", "kernels": f"radix sort (load + {npass} single-sweep passes) + "
-                                                "sorted_jobs_kernel 1-D counts",
+                                                "ball_jobs_kernel 1-D counts",
                      "marginals_1d": n1d, "algorithmic_bytes": ss_bytes,
                      "sort_ms": sort_ms, "count_1d_ms": c1_ms,
                      "achieved": ss_gbs, "peak": hbm, "unit": "GB/s",
