@@ -7,7 +7,7 @@
 //               and the descriptor tables (one pinned copy)
 //   gather      -> per-task working FP64 columns (class-grouped for the
 //               semidiscrete estimators)
-//   prepare     column midranges (centres of the FP32 copies)
+//   centres     of the FP32 copies, a median of 32 values per job column
 //   sort        every 1-D space and the first column of every slab job, one
 //               segmented LSD radix sort for the whole batch
 //   materialise multi-D job blocks (FP64 + centred FP32, working or sorted)
@@ -1186,8 +1186,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   for (SlotPlan& sl : slots) sl.off = dl.take(sizeof(double) * (size_t)P[(size_t)sl.task].ld);
   for (TaskPlan& p : P)
     for (int sl : p.slot) p.off_col.push_back(slots[(size_t)sl].off);
-  const size_t off_centers = dl.take(sizeof(double) * (size_t)nslots);
-  const size_t off_minmax = dl.take(sizeof(unsigned long long) * 2 * (size_t)nslots);
   const size_t off_keys_a = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(sort_total, 1));
   const size_t off_keys_b = dl.take(sizeof(uint64_t) * (size_t)std::max<int64_t>(sort_total, 1));
   const size_t off_vals_a = dl.take(sizeof(int32_t) * (size_t)std::max<int64_t>(sort_total, 1));
@@ -1707,7 +1705,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   const size_t tab_tasks = tl.take(sizeof(TaskDev) * (size_t)ntasks);
   const size_t tab_slots = tl.take(sizeof(BatchCol) * (size_t)nslots);
   const size_t tab_colptr = tl.take(sizeof(double*) * (size_t)ncols_total);
-  const size_t tab_colslot = tl.take(sizeof(int32_t) * (size_t)ncols_total);
   const size_t tab_segs = tl.take(sizeof(SortSeg) * std::max<size_t>(segs.size(), 1));
   const size_t tab_blkseg = tl.take(sizeof(int32_t) * (size_t)std::max(nblk_sort, 1));
   const size_t tab_osblkseg = tl.take(sizeof(int32_t) * (size_t)std::max(nblk_os, 1));
@@ -1804,8 +1801,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     TaskDev& D = tdev[(size_t)t];
     std::memset(&D, 0, sizeof(D));
     D.col = (double* const*)(A + off_tab + tab_colptr) + p.center0;
-    D.slot = (const int32_t*)(A + off_tab + tab_colslot) + p.center0;
-    D.centers = (const double*)(A + off_centers);
     D.eps = (double*)devp(p.off_eps);
     D.rad = p.kind == KIND_COUNT_ONLY ? (double*)devp(p.off_rad) : D.eps;
     for (int s = 0; s < p.nslot; ++s) D.cnt[s] = (int32_t*)devp(p.off_cnt[s]);
@@ -1824,7 +1819,6 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       std::memcpy(H + p.tab_rad, count_radius, sizeof(double) * (size_t)p.n);
     for (int c = 0; c < p.ncol; ++c) {
       ((double**)(H + tab_colptr))[p.center0 + c] = (double*)devp(p.off_col[(size_t)c]);
-      ((int32_t*)(H + tab_colslot))[p.center0 + c] = p.slot[(size_t)c];
     }
   }
   for (int i = 0; i < nslots; ++i) {
@@ -2064,15 +2058,14 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
                        (uint64_t*)(A + off_owords_a), (uint64_t*)(A + off_owords_b), ow, err_d, st);
   }
   const BatchCol* slots_d = (const BatchCol*)dtab(tab_slots);
-  launch_gather(slots_d, nslots, max_ld, (unsigned long long*)(A + off_minmax), st);
+  launch_gather(slots_d, nslots, max_ld, st);
   if (!rcols.empty())
     launch_rescale(slots_d, (const RescaleStat*)dtab(tab_rstats), (int)rstats.size(),
                    (const RescaleCol*)dtab(tab_rcols), (int)rcols.size(),
                    (const PwTree*)dtab(tab_pwtrees), (const int2*)dtab(tab_pwnodes),
                    (const int32_t*)dtab(tab_pwlevels), (double*)(A + off_pw_scratch),
                    (double2*)(A + off_pw_ms), ctx->noise_d, (uint32_t*)(A + off_zr + zr_const), max_n, st);
-  launch_prepare(slots_d, nslots, max_n, tasks_d, (const JobDev*)dtab(tab_jobs), (int)jobs.size(),
-                 (unsigned long long*)(A + off_minmax), (double*)(A + off_centers), st);
+  launch_centres(tasks_d, (const JobDev*)dtab(tab_jobs), (int)jobs.size(), st);
   if (timing) EGB_CUDA(cudaEventRecord(ctx->ev[2], st));
 
   uint64_t* keys = (uint64_t*)(A + off_keys_a);
@@ -2081,7 +2074,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   const KeyIndexOut ko{(float*)(A + off_fk), (uint64_t*)(A + off_s1), (uint64_t*)(A + off_s2),
                        (float*)(A + off_fs1), (float*)(A + off_fs2)};
   const KeyIndex kx{keys, ko.fkeys, ko.s1, ko.s2, ko.fs1, ko.fs2};
-  launch_sort(slots_d, (const double*)(A + off_centers), (const SortSeg*)dtab(tab_segs),
+  launch_sort(slots_d, (const SortSeg*)dtab(tab_segs),
               (const int32_t*)dtab(tab_blkseg), nblk_sort, (const int32_t*)dtab(tab_osblkseg), nblk_os,
               os_tile, (int)segs.size(), keys, (uint64_t*)(A + off_keys_b), vals, (int32_t*)(A + off_vals_b), ko,
               A + off_sweep, sort_first, sort_codes, ctx->num_sms, err_d, st,

@@ -2,9 +2,12 @@
 // codes instead of six over 64-bit keys.
 //
 // A value's code is the order-preserving image of its FP32 distance from the
-// column's midrange, rounded to nearest.  Subtraction and rounding are
-// monotone, so codes never order two values wrongly; values that FP32 cannot
-// tell apart share one.  A pass moves one 8-byte word per point (code, working
+// median of 32 values of its segment, rounded to nearest.  Subtraction and
+// rounding are monotone, so codes never order two values wrongly, whatever the
+// centre; values that FP32 cannot tell apart share one.  A centre amid the
+// values gives the most of them distances of their own also in columns with an
+// offset or long tails (from the midrange, half of what one outlier reaches,
+// they would share few).  A pass moves one 8-byte word per point (code, working
 // index), 16 bytes of traffic against the 24 of key and index apart, and four
 // digits stand for six.  The last kernel reads each point's value through its
 // index (the column lies in L2), orders the runs of equal codes by the full
@@ -46,16 +49,21 @@ __device__ __forceinline__ uint32_t code_of(double x, double c) {
 }
 
 __global__ void __launch_bounds__(LOAD_THREADS)
-code_load_kernel(const BatchCol* __restrict__ slots, const double* __restrict__ centers,
-                 const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg,
-                 uint64_t* __restrict__ words, uint32_t* __restrict__ seg_hist) {
+code_load_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict__ segs,
+                 const int32_t* __restrict__ blk_seg, uint64_t* __restrict__ words,
+                 uint32_t* __restrict__ seg_hist) {
   __shared__ uint32_t h[CODE_PASSES * 256];
+  __shared__ double centre;
   const int si = blk_seg[blockIdx.x];
   const SortSeg& s = segs[si];
-  for (int i = threadIdx.x; i < CODE_PASSES * 256; i += LOAD_THREADS) h[i] = 0;
-  __syncthreads();
-  const double mid = centers[s.slot], c = isfinite(mid) ? mid : 0.0;
   const double* __restrict__ x = slots[s.slot].x + s.src_begin;
+  for (int i = threadIdx.x; i < CODE_PASSES * 256; i += LOAD_THREADS) h[i] = 0;
+  if (threadIdx.x < 32) {
+    const double m = centre_of(x, s.len);
+    if (threadIdx.x == 0) centre = m;
+  }
+  __syncthreads();
+  const double c = centre;
   uint64_t* __restrict__ out = words + s.out_base;
   const int i0 = ((int)blockIdx.x - s.blk0) * SORT_TILE;
   const int i1 = min(i0 + SORT_TILE, s.len);
@@ -265,11 +273,10 @@ void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os
   count_launch();
 }
 
-void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
-                      const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
-                      int nseg, uint64_t* keys, uint64_t* words, int32_t* vals, const KeyIndexOut& ko,
-                      const Sweep& w, uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
-  code_load_kernel<<<nblk, LOAD_THREADS, 0, st>>>(slots_d, centers_d, segs_d, blk_seg_d, words, w.seg_hist);
+void launch_code_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
+                      const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys, uint64_t* words,
+                      int32_t* vals, const KeyIndexOut& ko, const Sweep& w, uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
+  code_load_kernel<<<nblk, LOAD_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, words, w.seg_hist);
   count_launch();
   if (pass_events) cudaEventRecord(pass_events[0], st);
   uint64_t* in = words;  // an even number of passes: back in words

@@ -11,8 +11,8 @@
 //   * per sorted 1-D space: the order-preserving uint64 keys and the working
 //     index of each key, concatenated over all spaces of the batch;
 //   * per multi-D job: its columns copied into one SoA block (see JobDev),
-//     with an FP32 copy fl32(x - center_c) (center_c = the task column's
-//     midrange) read by the FP32 distance filters.
+//     with an FP32 copy fl32(x - center_c) (center_c = a value amid
+//     the column's, centre_of) read by the FP32 distance filters.
 // All distances are max-norm.  Every decision that fixes a neighbour count or
 // a k-th distance is taken on the exact FP64 distance max_c fl64(|a_c - b_c|)
 // -- the value scipy's cKDTree compares -- either directly or behind an FP32
@@ -249,13 +249,27 @@ __device__ __forceinline__ double radius_of(const double* rad, int given, int64_
   const double v = rad[w];
   return given ? v : v - 1e-12;
 }
+// A value amid x[0 .. len): the median of 32 of them at equal distances (0 if
+// it is not finite).  FP32 copies and codes hold distances from it, which FP32
+// resolves finely where most values are, whatever a column's offset or tails.
+// Whole warps; the same in every one that reads the same values.
+__device__ __forceinline__ double centre_of(const double* __restrict__ x, int64_t len) {
+  const int lane = threadIdx.x & 31;
+  const double v = x[(int64_t)lane * len / 32];
+  const uint64_t k = key_of(v);
+  int rank = 0;
+  for (int j = 0; j < 32; ++j) {
+    const uint64_t o = __shfl_sync(0xffffffffu, k, j);
+    rank += o < k || (o == k && j < lane);
+  }
+  const double m = __shfl_sync(0xffffffffu, v, __ffs(__ballot_sync(0xffffffffu, rank == 16)) - 1);
+  return isfinite(m) ? m : 0.0;
+}
 #endif
 
 // ------------------------------------------------------------ job structs --
 struct TaskDev {          // per-task device view
   double* const* col;     // [ncol] working FP64 columns (shared between tasks)
-  const int32_t* slot;    // [ncol] the batch column behind each
-  const double* centers;  // per batch column: its midrange (FP32 copies are x - it)
   double* eps;            // [ld]
   double* rad;            // [ld] caller radii (rad_given), else eps
   int32_t* cnt[4];        // count slots (working order)
@@ -504,11 +518,8 @@ void count_launch();
 // launches on `st` and never synchronises.
 
 // egb_prep.cu
-void launch_gather(const BatchCol* slots_d, int nslots, int64_t max_ld, unsigned long long* minmax_d,
-                   cudaStream_t st);
-void launch_prepare(const BatchCol* slots_d, int nslots, int64_t max_n, const TaskDev* tasks_d,
-                    const JobDev* jobs_d, int njobs, unsigned long long* minmax_d, double* centers_d,
-                    cudaStream_t st);
+void launch_gather(const BatchCol* slots_d, int nslots, int64_t max_ld, cudaStream_t st);
+void launch_centres(const TaskDev* tasks_d, const JobDev* jobs_d, int njobs, cudaStream_t st);
 void launch_materialize(const TaskDev* tasks_d, const JobDev* jobs_d, int njobs,
                         const int32_t* sorted_vals, const SortSeg* segs_d, int64_t max_lds,
                         cudaStream_t st);
@@ -624,17 +635,17 @@ int init_sort_kernels();
 // and 403, 425 and 416 (500,000); 2.2 million 841 and 801, 648 and 604; five
 // million 1639 and 1522, 1190 and 1076, 1201 and 1081.
 constexpr int64_t SORT_CODES_MIN = 1 << 20;
-void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
+void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d,
                  const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
                  int os_tile, int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
                  const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
                  uint32_t* err, cudaStream_t st,
                  cudaEvent_t* pass_events = nullptr);  // recorded around the passes alone
 int init_code_sort();
-void launch_code_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
-                      const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
-                      int nseg, uint64_t* keys, uint64_t* words, int32_t* vals, const KeyIndexOut& ko,
-                      const Sweep& w, uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events);
+void launch_code_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
+                      const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys, uint64_t* words,
+                      int32_t* vals, const KeyIndexOut& ko, const Sweep& w, uint32_t* err, cudaStream_t st,
+                      cudaEvent_t* pass_events);
 constexpr int SORTED_BLOCK = 128;
 void launch_sorted_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njobs,
                         int total_blocks, const KeyIndex& kx, const int32_t* perm, cudaStream_t st);

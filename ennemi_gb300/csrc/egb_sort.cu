@@ -592,7 +592,7 @@ int init_sort_kernels() {
 
 size_t sort_sweep_bytes(int os_nblk, int nseg) { return sweep_layout(nullptr, os_nblk, nseg, nullptr) + 64; }
 
-void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg* segs_d,
+void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d,
                  const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
                  int os_tile, int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
                  const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
@@ -604,8 +604,7 @@ void launch_sort(const BatchCol* slots_d, const double* centers_d, const SortSeg
   Sweep w;
   sweep_layout(sweep, os_nblk, nseg, &w);
   if (codes)
-    launch_code_sort(slots_d, centers_d, segs_d, blk_seg_d, nblk, os_blk_seg_d, os_nblk, nseg, keys_a,
-                     keys_b, vals_a, ko, w, err, st, pass_events);
+    launch_code_sort(slots_d, segs_d, blk_seg_d, nblk, os_blk_seg_d, os_nblk, nseg, keys_a, keys_b, vals_a, ko, w, err, st, pass_events);
   const uint32_t* redo = codes ? w.redo : nullptr;
   const int gl = codes ? std::min(nblk, 4 * num_sms) : nblk;
   const int gp = codes ? std::min(os_nblk, 2 * num_sms) : os_nblk;

@@ -302,13 +302,17 @@ def _code_columns(data, n, rng):
         x[::3] *= 1e300
     elif data == "tiny":
         x *= 1e-300
+    elif data == "cauchy":
+        x = rng.standard_cauchy(size=n)
+    elif data == "outlier":
+        x[n // 2] = 1e7
     elif data == "one_huge":  # everything else shares a code
         x[0] = 1e308
     return x
 
 
 @pytest.mark.parametrize("data", ["normal", "offset", "near", "levels", "zeros", "cluster", "twins", "huge",
-                                  "tiny", "one_huge"])
+                                  "tiny", "cauchy", "outlier", "one_huge"])
 def test_code_sort_equals_the_digit_sort(data):
     """A batch large enough for the code sort returns, for segments of one
     point up to several tiles, exactly what each of its tasks returns alone."""
