@@ -326,6 +326,8 @@ class Columns:
 
     def address(self, row, col=0):
         """Address of element (row, col); arrays of either give arrays."""
+        if np.asarray(row).dtype.kind not in "iu" or np.asarray(col).dtype.kind not in "iu":
+            raise TypeError("rows and columns must be integers")
         return self.ptr + row * self.row + col * self.col
 
 

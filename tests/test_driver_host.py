@@ -377,3 +377,39 @@ def test_kept_rows_are_the_rows_without_nans(n, share, threads):
             r = np.arange(n) if base is None else base
             want = r[~(np.isnan(u[r]) | np.isnan(v[r]))]
             assert counts[t] == len(want) and np.array_equal(rows[t, :counts[t]], want)
+
+
+@pytest.mark.parametrize("drop_nan", [False, True])
+@pytest.mark.parametrize("nvar", [1, 3])
+@pytest.mark.parametrize("lag,cond_lag", [([0, 0.5, 1.0, 1.5], 0), ([1.0, 2.0, 3.0, 4.0], 0), ([0.0] * 4, 0),
+                                          ([0, 1, 2, 3], 0.5), ([0, 1, 2, 3], [[0, 1.0]] * 4),
+                                          ([True, False, True, True], 0), ([[0, 1], [2, 3]], 0),
+                                          ([0.5], 0), ([1, 2], 0.5)])
+def test_lags_that_are_not_integers_are_refused(monkeypatch, lag, cond_lag, nvar, drop_nan):
+    """Lags that cannot slice raise a slice's TypeError however many tasks the
+    call has, and no address is handed to the library."""
+    rng = np.random.default_rng(5)
+    x, y, cond = rng.normal(size=(200, nvar)), rng.normal(size=200), rng.normal(size=(200, 2))
+    ran = []
+    monkeypatch.setattr(_native, "run_tasks", lambda tasks, **kw: ran.append(tasks) or np.zeros(len(tasks)))
+    with pytest.raises(TypeError):
+        eg.estimate_mi(y, x, lag=lag, cond=None if cond_lag == 0 else cond, cond_lag=cond_lag, drop_nan=drop_nan)
+    assert not ran
+
+
+@pytest.mark.parametrize("dtype", [np.int16, np.int64, np.uint32, object])
+def test_addresses_of_lagged_views(monkeypatch, dtype):
+    """Tasks handed over as addresses start where the lagged slices do, for any
+    integer type of the lags."""
+    rng = np.random.default_rng(6)
+    x, y = rng.normal(size=(300, 2)), rng.normal(size=600)[::2]
+    tables = []
+    monkeypatch.setattr(_native, "run_tasks", lambda tasks, **kw: tables.append(tasks) or np.zeros(len(tasks)))
+    lag = np.array([0, 120, 3, 7], dtype=dtype)
+    eg.estimate_mi(y, x, lag=lag)
+    t = tables[0]
+    assert isinstance(t, _native.TaskTable)
+    want = [[x[120 - int(lg):, c].ctypes.data, y[120:].ctypes.data] for lg in lag for c in range(2)]
+    assert t.ptr.tolist() == want and t.stride.tolist() == [[2, 2]] * 8
+    with pytest.raises(TypeError):
+        _native.Columns(y).address(1.5)
