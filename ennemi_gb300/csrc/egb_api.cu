@@ -784,7 +784,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
       return fail(ctx, EGB_ERR_ARG, who() + "column counts do not match the estimator kind");
     if (!T.cols) return fail(ctx, EGB_ERR_ARG, who() + "null column list");
     for (int c = 0; c < p.ncol; ++c)
-      if (!T.cols[c].data || T.cols[c].stride < 1)
+      if (!T.cols[c].data || T.cols[c].stride < 1 || (uintptr_t)T.cols[c].data % alignof(double))
         return fail(ctx, EGB_ERR_ARG, who() + "invalid column " + std::to_string(c));
     p.src_len = T.n;
     if (T.index) {

@@ -121,7 +121,8 @@ enum egb_flags {
                                   (tests; ignored with EGB_PLAIN_FP64)        */
 };
 
-/* One float64 column: sample i at data[i * stride] (stride in elements). */
+/* One float64 column: sample i at data[i * stride] (stride in elements; data
+ * aligned to 8 bytes). */
 typedef struct egb_column {
   const double* data;
   int64_t stride;

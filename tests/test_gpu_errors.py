@@ -76,3 +76,20 @@ def test_sort_tie_report_reruns_batch_with_full_sort():
     assert st["sort_passes"] == 8 and st["planned"] == 1 and st["graph"] == 0
     assert np.array_equal(base, again)
     assert np.array_equal(base_eps, N.fetch(0, 0, n))
+
+
+@pytest.mark.parametrize("n", [500, 6000])
+def test_misaligned_column_is_refused(n):
+    """A column that is not 8-byte aligned never reaches a kernel."""
+    import ctypes
+    rng = np.random.default_rng(n)
+    raw = np.zeros(8 * n + 8, dtype=np.uint8)
+    y = rng.normal(size=n)
+    cols = (N.EgbColumn * 2)(N.EgbColumn(raw.ctypes.data + 4, 1), N.EgbColumn(y.ctypes.data, 1))
+    task = N.EgbTask(kind=N.MI, k=3, n=n, dx=1, dy=1, dz=0, cols=cols)
+    res = N.EgbResult()
+    ctx = N.context(0)
+    with ctx.lock:
+        rc = ctx.lib.egb_run_batch(ctx.h, ctypes.byref(task), 1, 0, ctypes.byref(res))
+        with pytest.raises(RuntimeError, match="invalid column 0"):
+            ctx.check(rc, "egb_run_batch")
