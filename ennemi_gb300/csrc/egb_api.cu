@@ -101,6 +101,9 @@ double psi_int(double y) {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 int64_t round32(int64_t n) { return (n + 31) / 32 * 32; }
+// Whether the device may read a caller's int32 array where it is: the host takes
+// any address, a load on the device an aligned one.
+bool aligned_i32(const int32_t* p) { return (uintptr_t)p % alignof(int32_t) == 0; }
 
 struct Layout {
   size_t off = 0;
@@ -1145,7 +1148,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   };
 
   // class orders that the device builds (label_word_kernel)
-  const bool labels_in_place = ctx->host_direct && !(flags & EGB_STAGE_HOST);
+  auto labels_in_place = [&](const TaskPlan& p) {
+    return ctx->host_direct && !(flags & EGB_STAGE_HOST) && aligned_i32(p.dev_order);
+  };
   std::vector<SortSeg> order_segs;
   std::vector<int> order_tasks;
   int64_t order_total = 0;
@@ -1160,7 +1165,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     if (p.dev_order) {
       p.off_perm = dl.take(sizeof(int32_t) * (size_t)p.n);
       p.tab_classes = tl.take(sizeof(int32_t) * (size_t)(p.nclass + 1));
-      if (!labels_in_place) p.tab_perm = tl.take(sizeof(int32_t) * (size_t)p.n);
+      if (!labels_in_place(p)) p.tab_perm = tl.take(sizeof(int32_t) * (size_t)p.n);
       SortSeg g{};
       g.out_base = order_total;
       g.len = (int32_t)p.n;
@@ -1727,7 +1732,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   for (const TaskPlan& p : P)
     if (p.index) index_cols[p.index] += p.ncol;
   auto index_in_place = [&](const TaskPlan& p) {
-    return ctx->host_direct && !(flags & (EGB_STAGE_HOST | EGB_GRAPH)) && index_cols[p.index] <= 4;
+    return ctx->host_direct && !(flags & (EGB_STAGE_HOST | EGB_GRAPH)) && index_cols[p.index] <= 4 &&
+           aligned_i32(p.index);
   };
   for (TaskPlan& p : P) {
     if (!p.index || index_in_place(p)) continue;
@@ -1811,7 +1817,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     const std::vector<int32_t>& gp = p.gperm.empty() ? p.perm : p.gperm;
     if (!gp.empty()) std::memcpy(H + p.tab_perm, gp.data(), sizeof(int32_t) * gp.size());
     if (p.dev_order) {
-      if (!labels_in_place) std::memcpy(H + p.tab_perm, p.dev_order, sizeof(int32_t) * (size_t)p.n);
+      if (!labels_in_place(p)) std::memcpy(H + p.tab_perm, p.dev_order, sizeof(int32_t) * (size_t)p.n);
       for (int c = 0; c <= p.nclass; ++c)
         ((int32_t*)(H + p.tab_classes))[c] = (int32_t)p.cls_off[(size_t)c];
     }
@@ -1837,7 +1843,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   }
   for (size_t i = 0; i < order_tasks.size(); ++i) {
     const TaskPlan& p = P[(size_t)order_tasks[i]];
-    const LabelJob j{labels_in_place ? p.dev_order : (const int32_t*)(A + off_tab + p.tab_perm),
+    const LabelJob j{labels_in_place(p) ? p.dev_order : (const int32_t*)(A + off_tab + p.tab_perm),
                      (const int32_t*)(A + off_tab + p.tab_classes), (int32_t*)devp(p.off_perm),
                      order_segs[i].out_base, (int32_t)p.n, p.nclass};
     std::memcpy(H + tab_ojobs + sizeof(LabelJob) * i, &j, sizeof(j));

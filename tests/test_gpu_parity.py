@@ -335,6 +335,28 @@ def test_code_sort_equals_the_digit_sort(data):
             assert np.array_equal(N.fetch(0, w, n), kept[t][w], equal_nan=True), (n, w)
 
 
+def test_labels_and_index_at_any_address():
+    """int32 arrays that are not 4-byte aligned: never read where they are."""
+    rng = np.random.default_rng(8)
+    n = 24_001
+
+    def unaligned(a):
+        raw = np.zeros(a.nbytes + 4, dtype=np.uint8)
+        raw[1:1 + a.nbytes] = a.view(np.uint8)
+        return raw[1:1 + a.nbytes].view(np.int32)
+
+    lab = rng.integers(0, 5, n).astype(np.int32)
+    idx = np.sort(rng.choice(2 * n, n, replace=False)).astype(np.int32)
+    x, u, v = rng.normal(size=n), rng.normal(size=2 * n), rng.normal(size=2 * n)
+    for labels, index in ((lab, idx), (unaligned(lab), unaligned(idx))):
+        assert labels.flags.aligned == (labels is lab)
+        got = N.run_tasks([N.Task(N.SEMI, 3, [x], labels=labels, nclass=5, n=n),
+                           N.Task(N.MI, 3, [u], [v], n=n, index=index)])
+        if labels is lab:
+            want = got
+    assert np.array_equal(got, want)
+
+
 def _small_points(data, n, d, rng):
     x = rng.normal(size=(n, d))
     if data == "duplicates":
