@@ -139,13 +139,19 @@ __device__ __forceinline__ double raw_value(uint64_t k) {
   return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
 }
 
-// Raw keys [kl, kr] of the doubles x with fl64(|x - q|) <= r, for q and r
-// finite, r >= 0.  x -> fl64(x - q) is monotone (rounding is), so the set
+// Raw keys [kl, kr] of the doubles x with fl64(|x - q|) <= r, for a finite
+// r >= 0 (q not finite: none, an empty range; no step of the walks below would
+// satisfy the predicate, and they would not end).  x -> fl64(x - q) is monotone (rounding is), so the set
 // is one key range.  Its ends usually lie an ulp or two from fl64(q -+ r),
 // but where q -+ r is much smaller in magnitude than q many doubles share
 // one fl64 difference, so each end is found by galloping from there and
 // bisecting on the exact predicate (at most about 128 FP64 steps).
 __device__ __forceinline__ void ball_keys(double q, double r, uint64_t& kl, uint64_t& kr) {
+  if ((((uint64_t)__double_as_longlong(q) >> 52) & 0x7ffu) == 0x7ffu) {
+    kl = 1;
+    kr = 0;
+    return;
+  }
   // right end: largest k with value(k) - q <= r
   {
     uint64_t k = raw_key((uint64_t)__double_as_longlong(q + r));

@@ -335,6 +335,24 @@ def test_code_sort_equals_the_digit_sort(data):
             assert np.array_equal(N.fetch(0, w, n), kept[t][w], equal_nan=True), (n, w)
 
 
+@pytest.mark.parametrize("n", [300, 9001])
+@pytest.mark.parametrize("d", [1, 2, 3])
+def test_counts_about_points_that_are_not_finite(d, n):
+    """No point lies within a finite distance of an infinite or NaN one, itself
+    included; such points are in no finite ball."""
+    rng = np.random.default_rng(n + d)
+    pts = rng.normal(size=(n, d))
+    pts[[5, 6, 7, n // 2], d - 1] = [np.inf, -np.inf, np.nan, np.inf]
+    r = np.abs(rng.normal(0.3, 0.2, size=n))
+    r[9] = 0.0
+    for flags in (0, N.FORCE_BRUTE, N.FORCE_RANK if d == 2 else N.FORCE_GRID):
+        got = N.ball_count(pts, r, flags=flags)
+        for i in [*range(40), n // 2, n - 1]:
+            with np.errstate(invalid="ignore"):
+                dist = np.abs(pts - pts[i]).max(axis=1)
+            assert got[i] == np.count_nonzero(dist <= r[i]), (flags, i)
+
+
 def test_labels_and_index_at_any_address():
     """int32 arrays that are not 4-byte aligned: never read where they are."""
     rng = np.random.default_rng(8)
