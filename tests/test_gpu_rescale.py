@@ -110,6 +110,19 @@ def test_statistics_of_few_and_many_columns(n, tasks):
             assert np.array_equal(N.fetch(i, 16 + c, n).view(np.uint64), want.view(np.uint64)), (i, c)
 
 
+def test_more_columns_than_a_grid_has_rows():
+    """Over 65,535 distinct columns on the general path: every one is rescaled."""
+    n, tasks = 16, 32_800
+    rng = np.random.default_rng(1)
+    a, b = rng.normal(size=(2, tasks + n)) * 2.0 + 1.0
+    batch = [N.Task(N.MI, 3, [N.Col(a[i:i + n])], [N.Col(b[i:i + n])], n=n) for i in range(tasks)]
+    N.run_tasks(batch, flags=N.RESCALE | N.KEEP_INTERNALS | N.STAGE_HOST, noise=_noise)
+    for i in (0, 7, 32_766, 32_767, 32_768, tasks - 1):
+        for c, v in enumerate((a, b)):
+            want = _reference_rescale(v[i:i + n], c * n, n)
+            assert np.array_equal(N.fetch(i, 16 + c, n).view(np.uint64), want.view(np.uint64)), (i, c)
+
+
 def test_semidiscrete_columns_with_index():
     """Labels and an index together: the class order is applied on top of the
     index; the continuous column is rescaled from noise position 0."""
