@@ -343,7 +343,9 @@ int finish_batch(egb_ctx* ctx, const ReplayState& R, const char* H, int64_t laun
   }
   ctx->stats[13] = R.sort_passes;
   const uint32_t dev_err = *(const uint32_t*)(H + R.pin_zr + R.zr_err);
-  if (dev_err == DERR_SORT_TIES) return RC_SORT_RETRY;
+  // (with a tie report the searches did not run: what the later steps made of
+  // the arrays they would have written is not looked at)
+  if ((dev_err & DERR_SORT_TIES) && !(dev_err & DERR_WAIT_TIMEOUT)) return RC_SORT_RETRY;
   if (dev_err) {
     char buf[128];
     std::snprintf(buf, sizeof buf, "device error word 0x%x (%s)", dev_err,
@@ -2083,7 +2085,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
   launch_sort(slots_d, (const SortSeg*)dtab(tab_segs),
               (const int32_t*)dtab(tab_blkseg), nblk_sort, (const int32_t*)dtab(tab_osblkseg), nblk_os,
               os_tile, (int)segs.size(), keys, (uint64_t*)(A + off_keys_b), vals, (int32_t*)(A + off_vals_b), ko,
-              A + off_sweep, sort_first, sort_codes, ctx->num_sms, err_d, st,
+              A + off_sweep, sort_first, sort_codes, ctx->num_sms, err_d, counters, ncounters, st,
               timing ? ctx->kev + 12 : nullptr);
   // the rank-space matrices need only the sorted values: they build on the
   // side stream, joined back before their counts

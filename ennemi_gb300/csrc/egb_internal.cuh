@@ -628,7 +628,8 @@ void launch_label_order(const LabelJob* jobs_d, int njobs, int max_classes, int6
 // keys_a / vals_a.
 // blk_seg_d / nblk: the segments' SORT_TILE tiles (load and repair
 // kernels); os_blk_seg_d / os_nblk: their tiles of os_tile keys (the
-// passes).
+// passes).  counters: two per launch group of searches, its work counter first,
+// which a sort that reports DERR_SORT_TIES moves past the last item.
 size_t sort_sweep_bytes(int os_nblk, int nseg);
 // Once per context, on its device: lets the passes use their shared memory
 // (above the 48 KB default); returns the cudaError_t.
@@ -645,7 +646,7 @@ void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d,
                  const int32_t* blk_seg_d, int nblk, const int32_t* os_blk_seg_d, int os_nblk,
                  int os_tile, int nseg, uint64_t* keys_a, uint64_t* keys_b, int32_t* vals_a, int32_t* vals_b,
                  const KeyIndexOut& ko, void* sweep, int first, bool codes, int num_sms,
-                 uint32_t* err, cudaStream_t st,
+                 uint32_t* err, int* counters, int ncounters, cudaStream_t st,
                  cudaEvent_t* pass_events = nullptr);  // recorded around the passes alone
 int init_code_sort();
 void launch_code_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
