@@ -559,6 +559,7 @@ int run_direct(egb_ctx* ctx, const egb_task* tasks, std::vector<TaskPlan>& P, in
   const size_t tab_levels = tl.take(sizeof(int32_t) * levels.size());
   const size_t zr = tl.take(0);
   const size_t zr_zero = 0, zr_err = align_up(sizeof(uint32_t) * (size_t)ntasks, 16);
+  const size_t zr_crowded = zr_err + 4;
   const size_t zr_bytes = align_up(zr_err + 16, 256);
   const size_t tab_bytes = zr + zr_bytes;
   const size_t off_tab = dl.take(tab_bytes);
@@ -676,7 +677,7 @@ int run_direct(egb_ctx* ctx, const egb_task* tasks, std::vector<TaskPlan>& P, in
   for (const Run& r : runs) {
     const TaskPlan& p = P[(size_t)order[(size_t)r.first]];
     launch_direct_search(p.kind, p.ncol, (const DirectTask*)(T + tab_tasks) + r.first, r.count, r.kmax,
-                         r.part0, r.nparts, r.per, st);
+                         r.part0, r.nparts, r.per, (uint32_t*)(T + zr + zr_crowded), st);
   }
   launch_combine((const TaskDev*)(T + tab_tdev), (const CombineJob*)(T + tab_cjobs),
                  (const int32_t*)(T + tab_chunk), ntasks, ctx->psi_d, ctx->psi_len,
@@ -700,6 +701,7 @@ int run_direct(egb_ctx* ctx, const egb_task* tasks, std::vector<TaskPlan>& P, in
   R.zr_err = zr_err;
   R.pin_rb = pin_back + (off_partial - (off_tab + zr));
   const int rc_fin = finish_batch(ctx, R, H, (int64_t)(g_launches.load() - launches0), results);
+  ctx->stats[2] = *(const uint32_t*)(H + pin_back + zr_crowded);
   ctx->stats[11] = 1;
   ctx->stats[14] = plan_us;
   ctx->stats[15] = issue_us;

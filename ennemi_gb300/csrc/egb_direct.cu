@@ -6,7 +6,8 @@
 // the device).  When every task of a batch is small (run_direct in egb_api.cu
 // has the rule), the batch is
 //   direct_prep_kernel    one block per task column: gather, the reference's
-//                         rescale, midrange, FP32 copy
+//                         rescale, FP32 copy of the
+//                         distances from a value amid the column (centre_of)
 //   direct_search_kernel  one warp per query over all points of its task: the
 //                         exact (k+1)-NN distance, then every marginal count
 //                         of that query in one more sweep
@@ -14,7 +15,7 @@
 // The columns stay in L1 / L2; every decision is the exact one of the other
 // kernels: FP32 screen with the proven band, FP64 where it cannot settle.
 // Tasks with values that rule out the FP32 copy (not finite, or 1e37 from the
-// midrange) set DIRECT_REDO in their flag word, and the host runs the batch on
+// centre) set DIRECT_REDO in their flag word, and the host runs the batch on
 // the general path.
 #include <algorithm>
 
@@ -42,7 +43,6 @@ direct_prep_kernel(const DirectTask* __restrict__ tasks, const DirectCol* __rest
                    uint32_t* __restrict__ flags) {
   __shared__ double v[DIRECT_MAX_N + 1];
   __shared__ double sm[2 * DP_STAGE];   // node sums of the tree, or staged rows
-  __shared__ unsigned long long mm[2][DP_THREADS / 32];
   __shared__ double mean_s, sd_s, rsd_s, centre;
   const DirectCol dc = cols[blockIdx.x];
   const DirectTask& t = tasks[dc.task];
@@ -83,28 +83,9 @@ direct_prep_kernel(const DirectTask* __restrict__ tasks, const DirectCol* __rest
     }
     __syncthreads();
   }
-  unsigned long long lo = ~0ull, hi = 0ull;
-  for (int w = tid; w < n; w += DP_THREADS) {
-    const unsigned long long k = key_of(v[w]);
-    lo = min(lo, k);
-    hi = max(hi, k);
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    lo = min(lo, __shfl_xor_sync(FULL, lo, o));
-    hi = max(hi, __shfl_xor_sync(FULL, hi, o));
-  }
-  if ((tid & 31) == 0) {
-    mm[0][tid >> 5] = lo;
-    mm[1][tid >> 5] = hi;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < DP_THREADS / 32; ++w) {
-      lo = min(lo, mm[0][w]);
-      hi = max(hi, mm[1][w]);
-    }
-    centre = 0.5 * value_of(lo) + 0.5 * value_of(hi);
+  if (tid < 32) {
+    const double m = centre_of(v, n);
+    if (tid == 0) centre = m;
   }
   __syncthreads();
   const double c = centre;
@@ -147,7 +128,8 @@ struct Slots {
 
 template <int KIND, int D, int R>
 __global__ void __launch_bounds__(DS_WARPS * 32)
-direct_search_kernel(const DirectTask* __restrict__ tasks, int ntasks, int part_base, int nparts, int per) {
+direct_search_kernel(const DirectTask* __restrict__ tasks, int ntasks, int part_base, int nparts, int per,
+                     uint32_t* __restrict__ crowded) {
   using SL = Slots<KIND, D>;
   constexpr int NS = SL::N;
   constexpr float FINF = __builtin_huge_valf();
@@ -169,6 +151,7 @@ direct_search_kernel(const DirectTask* __restrict__ tasks, int ntasks, int part_
   for (int c = 0; c < D; ++c) gl[c] = g + c * ld + lane;
   const double* __restrict__ c64 = t.x64;
   const int q0 = (part - (t.part0 - part_base)) * per, q1 = min(q0 + per, n);
+  unsigned over = 0;
 
   for (int q = q0; q < q1; ++q) {
     float qv[D];
@@ -224,6 +207,7 @@ direct_search_kernel(const DirectTask* __restrict__ tasks, int ntasks, int part_
     if (!list.over) {
       kth = list.kth(exact_dist);
     } else if (b1 - b0 >= K) {  // more near ties than the list holds
+      ++over;
       kth = radix_kth(store[warp], K, [&](auto&& f) { f(b0, b1); }, exact_dist);
     }
     kth = __shfl_sync(FULL, kth, 0);
@@ -299,16 +283,19 @@ direct_search_kernel(const DirectTask* __restrict__ tasks, int ntasks, int part_
       }
     }
   }
+  if (lane == 0 && over) atomicAdd(crowded, over);
 }
 
 template <int KIND, int D>
 void launch_t(const DirectTask* tasks, int ntasks, int kmax, int part_base, int nparts, int per,
-              cudaStream_t st) {
+              uint32_t* crowded, cudaStream_t st) {
   const int grid = (nparts + DS_WARPS - 1) / DS_WARPS;
   if (kmax <= 16)
-    direct_search_kernel<KIND, D, 2><<<grid, DS_WARPS * 32, 0, st>>>(tasks, ntasks, part_base, nparts, per);
+    direct_search_kernel<KIND, D, 2><<<grid, DS_WARPS * 32, 0, st>>>(tasks, ntasks, part_base, nparts, per,
+                                                                      crowded);
   else
-    direct_search_kernel<KIND, D, 4><<<grid, DS_WARPS * 32, 0, st>>>(tasks, ntasks, part_base, nparts, per);
+    direct_search_kernel<KIND, D, 4><<<grid, DS_WARPS * 32, 0, st>>>(tasks, ntasks, part_base, nparts, per,
+                                                                      crowded);
   count_launch();
 }
 
@@ -336,11 +323,11 @@ void launch_direct_prep(const DirectTask* tasks_d, const DirectCol* cols_d, int 
 }
 
 void launch_direct_search(int kind, int d, const DirectTask* tasks_d, int ntasks, int kmax, int part_base,
-                          int nparts, int per, cudaStream_t st) {
+                          int nparts, int per, uint32_t* crowded, cudaStream_t st) {
   if (nparts <= 0) return;
 #define EGB_DIRECT(KIND, D)                                                         \
   case KIND * 8 + D:                                                                \
-    launch_t<KIND, D>(tasks_d, ntasks, kmax, part_base, nparts, per, st);           \
+    launch_t<KIND, D>(tasks_d, ntasks, kmax, part_base, nparts, per, crowded, st);  \
     break;
   switch (kind * 8 + d) {
     EGB_DIRECT(EGB_MI, 2)

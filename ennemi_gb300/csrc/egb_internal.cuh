@@ -798,7 +798,7 @@ constexpr double DIRECT_MAX_PAIRS = 4.5e8;
 constexpr uint32_t DIRECT_REDO = 1u << 30;  // flag word of a task: run the general path
 struct DirectTask {
   const double* x64;      // working columns, column c at + c * ld
-  const float* x32;       // the same less their midranges, in FP32
+  const float* x32;       // the same less their centres (centre_of), in FP32
   double* eps;
   int32_t* cnt[3];
   const int32_t* cls;     // class starts (nclass + 1), SEMI / CSEMI
@@ -822,8 +822,9 @@ bool direct_supported(int kind, int dx, int dy, int dz, int K);
 void launch_direct_prep(const DirectTask* tasks_d, const DirectCol* cols_d, int ncols, const PwTree* trees_d,
                         const int2* nodes_d, const int32_t* levels_d, const double* noise, uint32_t* flags,
                         cudaStream_t st);
+// crowded: += the queries with more near ties than their list holds
 void launch_direct_search(int kind, int d, const DirectTask* tasks_d, int ntasks, int kmax, int part_base,
-                          int nparts, int per, cudaStream_t st);
+                          int nparts, int per, uint32_t* crowded, cudaStream_t st);
 
 // egb_discrete.cu: exact group-by of the rows of one column subset of a
 // discrete task: the rows equal to each row, into count slot `slot`.

@@ -233,7 +233,8 @@ int egb_last_transfer(const egb_ctx* ctx, int64_t* h2d_bytes, int64_t* d2h_bytes
 
 /* Work counters of the last batch: [0] kNN candidate-query pairs screened by
  * tile work items, [1] kNN pairs screened for deferred queries, [2] kNN
- * queries deferred, [3..5] the same for the multi-D counts, [6] / [7]
+ * queries deferred, or searched again for near ties that a warp's list could
+ * not hold, [3..5] the same for the multi-D counts, [6] / [7]
  * algorithmic operations of the kNN / count tile kernels ((2d+1) per pair:
  * d differences, d max-of-abs, one compare), [8] kernels launched, [9] keys
  * and [10] segments of the batch's radix sort, [11] 1 if the batch was

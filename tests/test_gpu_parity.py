@@ -509,6 +509,29 @@ def test_small_batches_equal_the_general_path(n, k, data):
             assert np.array_equal(u.view(np.int64), w.view(np.int64))
 
 
+@pytest.mark.parametrize("data", ["outlier", "cauchy"])
+@pytest.mark.parametrize("n,k", [(40, 3), (1000, 3), (1000, 20), (4095, 3)])
+def test_small_batches_with_far_values(n, k, data):
+    """A value far from all others, and heavy tails: the general path's results
+    bit for bit, and few queries whose FP32 distances tie beyond the list."""
+    rng = np.random.default_rng(n + k)
+    c = rng.normal(size=(n, 4)) if data == "outlier" else rng.standard_cauchy(size=(n, 4))
+    if data == "outlier":
+        c[n // 2] = 1e6
+    col = [np.ascontiguousarray(v) for v in c.T]
+    lab = (np.arange(n) % 2).astype(np.int32)
+    tasks = [N.Task(N.MI, k, col[:1], col[1:2], n=n), N.Task(N.CMI, k, col[:1], col[1:2], col[2:], n=n),
+             N.Task(N.SEMI, k, col[:2], labels=lab, nclass=2, n=n), N.Task(N.ENTROPY, k, col[:3], n=n)]
+    want = N.run_tasks(tasks, flags=N.FORCE_BRUTE | N.KEEP_INTERNALS)
+    eps = [N.fetch(i, 0, n) for i in range(4)]
+    got = N.run_tasks(tasks, flags=N.KEEP_INTERNALS)
+    assert np.array_equal(got, want)
+    for i in range(4):
+        assert np.array_equal(N.fetch(i, 0, n), eps[i]), i
+    # the outlier's own query, and the few about as far out as heavy tails go
+    assert N.context(0).stats()["knn_deferred"] <= 4 * (1 if data == "outlier" else 0.01 * n)
+
+
 @pytest.mark.parametrize("n", [9, 129, 1000, 4095])
 def test_small_batches_rescale_and_index(n):
     """Strided views, a shared sample index, class orders and conditions of one
