@@ -29,7 +29,7 @@ namespace {
 
 using list_detail::CandidateList;
 using list_detail::FULL;
-using list_detail::radix_kth;
+using list_detail::ExactList;
 using list_detail::up_band32;
 
 constexpr int DP_THREADS = 256;
@@ -208,7 +208,21 @@ direct_search_kernel(const DirectTask* __restrict__ tasks, int ntasks, int part_
       kth = list.kth(exact_dist);
     } else if (b1 - b0 >= K) {  // more near ties than the list holds
       ++over;
-      kth = radix_kth(store[warp], K, [&](auto&& f) { f(b0, b1); }, exact_dist);
+      ExactList<R> exact(store[warp], K);
+      float sb = list.thr;  // the exact distances of the candidates within the bound
+      for (int j0 = b0; j0 < b1; j0 += 32) {
+        const int j = j0 + lane;
+        bool near = false;
+        if (j < b1) {
+          float dd = 0.0f;
+#pragma unroll
+          for (int c = 0; c < D; ++c) dd = fmaxf(dd, fabsf(g[c * ld + j] - qv[c]));
+          near = dd <= sb;
+        }
+        if (exact.push(near ? exact_dist(j) : ~0ull))
+          sb = fminf(sb, up_band32(f32_up_of_bits(exact.bound), mq));
+      }
+      kth = exact.kth();
     }
     kth = __shfl_sync(FULL, kth, 0);
     if (lane == 0) t.eps[q] = bits_to_double(kth);

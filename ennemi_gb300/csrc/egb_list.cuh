@@ -76,8 +76,7 @@ struct Entry {
 template <int R>
 struct CandidateList {
   static constexpr int CAP = 32 * R;
-  // 32-bit words of shared memory: the entries, or radix_kth's 256 counters
-  static constexpr int WORDS = 2 * CAP > 256 ? 2 * CAP : 256;
+  static constexpr int WORDS = 2 * CAP;  // 32-bit words of shared memory (an ExactList's too)
   Entry* list;
   int K;
   float mq;    // >= max_c |q_c - c|
@@ -187,58 +186,80 @@ struct CandidateList {
   }
 };
 
-// K-th smallest exact distance by radix select, 8 bits a pass; enumerate(f)
-// calls f(a, b) for ranges of candidates that hold the K nearest, each once.
-template <typename E, typename F>
-__device__ __forceinline__ uint64_t radix_kth(uint32_t* hist, int K, E&& enumerate, F&& exact) {
-  const int lane = threadIdx.x & 31;
-  uint64_t prefix = 0, mask = 0;
-  uint32_t rank = (uint32_t)K;
-  for (int shift = 56; shift >= 0; shift -= 8) {
-    __syncwarp();
-    for (int b = lane; b < 256; b += 32) hist[b] = 0u;
-    __syncwarp();
-    enumerate([&](int a, int b) {
-      for (int j = a + lane; j < b; j += 32) {
-        const uint64_t m = exact(j);
-        if ((m & mask) == prefix) atomicAdd(&hist[(m >> shift) & 255u], 1u);
-      }
-      __syncwarp();
-    });
-    __syncwarp();
-    uint32_t s = 0, loc[8];
+// The K smallest of a sequence of exact distances (FP64 bits), kept by one warp:
+// for queries whose near ties a CandidateList cannot hold.  Ties need no room
+// here: of the distances equal to the K-th, only as many as make K are kept.
+// (A radix select, used before, took eight sweeps of FP64 distances.)
+template <int R>
+struct ExactList {
+  static constexpr int CAP = 32 * R;
+  uint64_t* list;
+  int K;
+  int cnt;
+  uint64_t bound;  // the K-th of the distances seen at the last tightening
+
+  __device__ __forceinline__ ExactList(uint32_t* store, int K_)
+      : list(reinterpret_cast<uint64_t*>(store)), K(K_), cnt(0), bound(~0ull) {}
+
+  // The K-th smallest of the cnt >= K entries v (unused slots ~0).
+  __device__ __forceinline__ uint64_t select(const uint64_t (&v)[R]) const {
+    uint32_t w[R];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      loc[i] = hist[8 * lane + i];
-      s += loc[i];
-    }
-    uint32_t incl = s;
+    for (int r = 0; r < R; ++r) w[r] = (uint32_t)(v[r] >> 32);
+    const uint32_t h = kth_bits<R>(w, K);
+    int below = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += y;
+    for (int r = 0; r < R; ++r) {
+      below += __popc(__ballot_sync(FULL, w[r] < h));
+      w[r] = w[r] == h ? (uint32_t)v[r] : 0xffffffffu;
     }
-    const uint32_t excl = incl - s;
-    const unsigned hit = __ballot_sync(FULL, excl < rank && rank <= incl);
-    const int src = hit ? __ffs(hit) - 1 : 0;
-    uint32_t run = excl, digit = 255, before = excl;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {  // the bucket that reaches the rank
-      if (run < rank && rank <= run + loc[i]) {
-        digit = (uint32_t)(8 * lane + i);
-        before = run;
-      }
-      run += loc[i];
-    }
-    digit = __shfl_sync(FULL, digit, src);
-    before = __shfl_sync(FULL, before, src);
-    prefix |= (uint64_t)digit << shift;
-    mask |= 255ull << shift;
-    rank -= before;
+    return (uint64_t)h << 32 | kth_bits<R>(w, K - below);
   }
-  __syncwarp();
-  return prefix;
-}
+
+  __device__ __forceinline__ void load(uint64_t (&v)[R]) const {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = r * 32 + lane < cnt ? list[r * 32 + lane] : ~0ull;
+    __syncwarp();
+  }
+
+  // One distance per lane (~0: none); true if the bound was renewed.
+  __device__ __forceinline__ bool push(uint64_t e) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t m = __ballot_sync(FULL, e < bound);
+    if (!m) return false;
+    if (e < bound) list[cnt + __popc(m & lt)] = e;
+    cnt += __popc(m);
+    if (cnt <= CAP - 32) return false;
+    uint64_t v[R];
+    load(v);
+    bound = select(v);
+    int kept = 0;  // those below the K-th, then copies of it
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t k = __ballot_sync(FULL, v[r] < bound);
+      if (v[r] < bound) list[kept + __popc(k & lt)] = v[r];
+      kept += __popc(k);
+    }
+    for (int i = kept + lane; i < K; i += 32) list[i] = bound;
+    cnt = K;
+    return true;
+  }
+
+  // The K-th smallest of all, ~0 if there were fewer.
+  __device__ __forceinline__ uint64_t kth() const {
+    uint64_t res = ~0ull;
+    if (cnt >= K) {
+      uint64_t v[R];
+      load(v);
+      res = select(v);
+    }
+    __syncwarp();
+    return res;
+  }
+};
 
 }  // namespace list_detail
 }  // namespace egb

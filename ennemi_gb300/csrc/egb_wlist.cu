@@ -23,8 +23,11 @@
 //     K-th is the (K - nearer)-th smallest exact distance of the others --
 //     usually one candidate, one FP64 evaluation per query.
 // A query whose list cannot hold its near ties (rounded data) and the queries
-// of jobs whose centred values reach 1e37 take an 8-pass radix select on the
-// exact distances of the candidates within U (all candidates).
+// of jobs whose centred values reach 1e37 sweep the candidates within S (all of
+// them) once more, keep the K smallest exact distances and tighten S and U by
+// them.  20,000 points on 7 x 7 levels with 1e-10 of noise, K = 21: 0.23 ms,
+// against 3.2 with an 8-pass radix select (0.88 of the CTA grid); one far point among
+// 20,000: 0.13 against 1.6.
 //
 // What bounds it: instruction issue and the latency of a query's ranges in
 // turn (72 registers, seven blocks an SM: 6.3 -> 5.7 ms for 2.4 million 4-D
@@ -48,7 +51,9 @@ using leaf_detail::coord_below;
 using leaf_detail::query_ranges;
 using list_detail::CandidateList;
 using list_detail::FULL;
-using list_detail::radix_kth;
+using list_detail::ExactList;
+using list_detail::plan_margin;
+using list_detail::up_band32;
 
 constexpr int WL_WARPS = 4;
 
@@ -114,29 +119,30 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
         }
         return mm;
       };
+      auto dist32 = [&](int j) -> float {
+        float dd;
+        if constexpr (AOS == 2) {
+          const float2 p = reinterpret_cast<const float2*>(g)[j];
+          dd = fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1]));
+        } else if constexpr (AOS == 4) {
+          const float4 p = reinterpret_cast<const float4*>(g)[j];
+          dd = fmaxf(fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1])), fabsf(p.z - qv[D >= 3 ? 2 : 0]));
+          if constexpr (D == 4) dd = fmaxf(dd, fabsf(p.w - qv[D == 4 ? 3 : 0]));
+        } else {
+          dd = fabsf(g[j] - qv[0]);
+#pragma unroll
+          for (int c = 1; c < DQ; ++c) {
+            if (D == 0 && c >= d) break;
+            dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - qv[c]));
+          }
+        }
+        return dd;
+      };
       auto screen = [&](int a, int b, int ea, int eb) {  // [a, b) without [ea, eb)
         pairs += (unsigned)(b - a);
         for (int j0 = a; j0 < b && !list.over; j0 += 32) {
           const int j = j0 + lane;
-          float dd = __builtin_huge_valf();
-          if (j < b && !(j >= ea && j < eb)) {
-            if constexpr (AOS == 2) {
-              const float2 p = reinterpret_cast<const float2*>(g)[j];
-              dd = fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1]));
-            } else if constexpr (AOS == 4) {
-              const float4 p = reinterpret_cast<const float4*>(g)[j];
-              dd = fmaxf(fmaxf(fabsf(p.x - qv[0]), fabsf(p.y - qv[1])), fabsf(p.z - qv[D >= 3 ? 2 : 0]));
-              if constexpr (D == 4) dd = fmaxf(dd, fabsf(p.w - qv[D == 4 ? 3 : 0]));
-            } else {
-              dd = fabsf(g[j] - qv[0]);
-#pragma unroll
-              for (int c = 1; c < DQ; ++c) {
-                if (D == 0 && c >= d) break;
-                dd = fmaxf(dd, fabsf(g[(int64_t)c * lds + j] - qv[c]));
-              }
-            }
-          }
-          list.push(dd, j);
+          list.push(j < b && !(j >= ea && j < eb) ? dist32(j) : __builtin_huge_valf(), j);
         }
       };
       // every range of positions within the planning bound, nearest strips
@@ -169,10 +175,24 @@ wlist_kernel(const JobDev* __restrict__ jobs, const WorkItem* __restrict__ items
       if (!unsafe && !list.over) {
         kth = list.kth(exact_dist);
       } else if (len >= K) {
-        // the exact distances of the candidates within the bound (U was set
-        // from K listed candidates; none in a job with clamped values)
+        // the exact distances of the candidates within the bounds (set from K
+        // listed candidates; none in a job with clamped values)
         ++redone;
-        kth = radix_kth(store[warp], K, enumerate, exact_dist);
+        ExactList<R> exact(store[warp], K);
+        float sb = list.thr;
+        enumerate([&](int a, int b) {
+          pairs += (unsigned)(b - a);
+          for (int j0 = a; j0 < b; j0 += 32) {
+            const int j = j0 + lane;
+            const bool near = j < b && (unsafe || dist32(j) <= sb);
+            if (exact.push(near ? exact_dist(j) : ~0ull) && !unsafe) {
+              const float u = f32_up_of_bits(exact.bound);
+              sb = fminf(sb, up_band32(u, mq));
+              list.tb = fminf(list.tb, plan_margin(u));
+            }
+          }
+        });
+        kth = exact.kth();
         // distances of non-finite data, as the lists and the select rank them
         if (K <= EGB_KREG_MAX && kth > INF_BITS) kth = INF_BITS;
       }

@@ -217,6 +217,48 @@ def test_warp_list_knn(oracle, d, data):
         assert np.array_equal(N.knn_eps(few, k), oracle.knn_eps(few, k)), k
 
 
+def _noisy_levels(n, d, rng, step):
+    """Columns of a few levels with 1e-10 of noise: FP32 cannot tell a level's points apart."""
+    return np.round(rng.normal(size=(n, d)) / step) * step + 1e-10 * rng.normal(size=(n, d))
+
+
+@pytest.mark.parametrize("d", [2, 3, 4, 5])
+@pytest.mark.parametrize("n", [333, 2000, 5001])
+def test_crowded_queries(oracle, n, d):
+    """More near ties than a list holds, over all points and over grids, with
+    exact ties among them, at the edges of the list sizes."""
+    pts = _noisy_levels(n, d, np.random.default_rng(n + d), 0.8)
+    pts[1:-1:5] = pts[2::5][: len(pts[1:-1:5])]
+    crowded = 0
+    for k in [1, 3, 7, 8, 15, 16, 31, 32, 63, 64, 127]:
+        assert np.array_equal(N.knn_eps(pts, k), oracle.knn_eps(pts, k)), k
+        crowded += N.context(0).stats()["knn_deferred"]
+    assert crowded > n // 4
+
+
+@pytest.mark.parametrize("n,d,k", [(20_000, 2, 20), (20_000, 2, 50), (20_000, 3, 20)])
+def test_crowded_queries_cost_a_sweep_not_eight(n, d, k):
+    """The warp list's searches over noisy levels take no longer than those of
+    the tiles that it replaces (K <= 32), or eight times as long as over normal
+    data (device times)."""
+    rng = np.random.default_rng(n + k)
+    ctx = N.context(0)
+
+    def device_ms(pts, flags):
+        best = np.inf
+        for _ in range(4):
+            N.knn_eps(pts, k, flags=flags | N.TIMING)
+            best = min(best, ctx.timings()["knn"])
+        return best
+
+    crowded = device_ms(_noisy_levels(n, d, rng, 0.8), 0)
+    assert ctx.stats()["knn_deferred"] > n // 2
+    if k < 32:
+        assert crowded < device_ms(_noisy_levels(n, d, rng, 0.8), N.FORCE_CTA_GRID)
+    else:
+        assert crowded < 8 * device_ms(rng.normal(size=(n, d)), 0)
+
+
 @pytest.mark.parametrize("data", ["normal", "dyadic", "duplicates", "huge"])
 @pytest.mark.parametrize("d", [3, 4, 5])
 def test_leaf_counts(oracle, d, data):
