@@ -97,8 +97,13 @@ struct OsSmem {
   int32_t sv[TILE];
 };
 
-template <int TILE>
-__global__ void __launch_bounds__(OS_THREADS)
+// LOOK tiles at once shorten the passes of a sort with a tile per SM at most
+// (six over 400,000 keys: 74 us, 82 with one).  A larger one looks back one at a time,
+// which fits in 64 registers, and hides that behind a second block an SM:
+// eight passes over 18 million keys 1.32 ms, with 110 registers and one block 1.98.
+// REDO: after the code sort, a block takes tiles until none is left.
+template <int TILE, int LOOK, bool REDO>
+__global__ void __launch_bounds__(OS_THREADS, LOOK > 1 && TILE == OS_TILE ? 1 : 2)
 onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ os_blk_seg, int nblk,
                      const uint64_t* __restrict__ kin, const int32_t* __restrict__ vin,
                      uint64_t* __restrict__ kout, int32_t* __restrict__ vout, int pass,
@@ -110,16 +115,18 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
   extern __shared__ __align__(16) unsigned char os_raw[];
   OsSmem<TILE>& S = *reinterpret_cast<OsSmem<TILE>*>(os_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (redo && !redo[nseg]) return;
-  for (bool more = true; more; more = redo != nullptr) {
+  if (REDO && !redo[nseg]) return;
+  do {
     if (tid == 0) S.tile = atomicAdd(tile_counter, 1);
     for (int i = tid; i < OS_NW * 256; i += OS_THREADS) (&S.wcnt[0][0])[i] = 0u;
     __syncthreads();
     const int b = S.tile;
-    if (b >= nblk) break;
+    if (REDO && b >= nblk) break;
     const int si = os_blk_seg[b];
-    __syncthreads();  // S.tile is read before the next tile's id lands
-    if (redo && !redo[si]) continue;
+    if constexpr (REDO) {
+      __syncthreads();  // S.tile is read before the next tile's id lands
+      if (!redo[si]) continue;
+    }
     const SortSeg s = segs[si];
     const int lb = b - s.os_blk0;
     const int shift = 8 * pass;
@@ -161,7 +168,7 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
     }
     // publish this tile's count of digit tid, then look back for the count of
     // digit tid in the segment's earlier tiles
-    const uint32_t excl = tid < 256 ? sweep_look_back<8>(flags, b, s.os_blk0, tid, pass, cnt, err) : 0u;
+    const uint32_t excl = tid < 256 ? sweep_look_back<LOOK>(flags, b, s.os_blk0, tid, pass, cnt, err) : 0u;
     // digit tid of the whole segment starts after the smaller digits
     const uint32_t seg_tot = tid < 256 ? seg_hist[((size_t)si * ALL_PASSES + pass) * 256 + tid] : 0u;
     const uint32_t seg_off = digit_excl_scan(seg_tot, S.ws);
@@ -193,8 +200,8 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
         atomicOr(err, DERR_BAD_INDEX);
       }
     }
-    __syncthreads();
-  }
+    if (REDO) __syncthreads();
+  } while (REDO);
 }
 
 // ----------------------------------------------------------- tie repair --
@@ -592,10 +599,15 @@ void launch_nest_sub(const TaskDev* tasks_d, const JobDev* jobs_d, const int32_t
 }
 
 int init_sort_kernels() {
-  const int rc = init_code_sort();
-  if (rc) return rc;
-  return (int)cudaFuncSetAttribute(onesweep_pass_kernel<OS_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(OsSmem<OS_TILE>));
+  int rc = init_code_sort();
+  auto allow = [&](auto kernel) {
+    if (!rc)
+      rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OsSmem<OS_TILE>));
+  };
+  allow(onesweep_pass_kernel<OS_TILE, 1, false>);
+  allow(onesweep_pass_kernel<OS_TILE, 8, false>);
+  allow(onesweep_pass_kernel<OS_TILE, 1, true>);
+  return rc;
 }
 
 size_t sort_sweep_bytes(int os_nblk, int nseg) { return sweep_layout(nullptr, os_nblk, nseg, nullptr) + 64; }
@@ -629,8 +641,10 @@ void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d,
       kernel<<<gp, OS_THREADS, smem, st>>>(segs_d, os_blk_seg_d, os_nblk, kin, vin, kout, vout, pass, w.seg_hist,
                                            w.flags, w.counters + pass, err, redo, nseg);
     };
-    if (os_tile == OS_TILE) run(onesweep_pass_kernel<OS_TILE>, sizeof(OsSmem<OS_TILE>));
-    else run(onesweep_pass_kernel<OS_TILE_SMALL>, sizeof(OsSmem<OS_TILE_SMALL>));
+    if (codes) run(onesweep_pass_kernel<OS_TILE, 1, true>, sizeof(OsSmem<OS_TILE>));
+    else if (os_tile != OS_TILE) run(onesweep_pass_kernel<OS_TILE_SMALL, 8, false>, sizeof(OsSmem<OS_TILE_SMALL>));
+    else if (os_nblk <= num_sms) run(onesweep_pass_kernel<OS_TILE, 8, false>, sizeof(OsSmem<OS_TILE>));
+    else run(onesweep_pass_kernel<OS_TILE, 1, false>, sizeof(OsSmem<OS_TILE>));
     count_launch();
     uint64_t* tk = kin; kin = kout; kout = tk;
     int32_t* tv = vin; vin = vout; vout = tv;

@@ -104,6 +104,28 @@ def test_a_batch_to_be_rerun_stops_at_its_sort(levels, order):
     assert best < 8 * device, (best, device)
 
 
+def test_digit_passes_of_a_large_sort_keep_pace():
+    """The eight passes of the full sort move 24 bytes a key each, the four over
+    codes 16: three times the bytes, and no more than 3.45 times the time."""
+    n = 180_000
+    rng = np.random.default_rng(2)
+    cols = [rng.normal(size=n) for _ in range(60)]
+    tasks = [N.Task(N.MI, 3, [cols[i]], [cols[i + 1]], n=n) for i in range(0, 60, 2)]
+    ctx = N.context(0)
+
+    def passes_ms(word, want):
+        best = np.inf
+        for _ in range(4):
+            if word:
+                ctx.inject_device_error(word)
+            N.run_tasks(tasks, flags=N.TIMING)
+            assert ctx.stats()["sort_passes"] == want
+            best = min(best, ctx.timings()["sort_passes"])
+        return best
+
+    assert passes_ms(4, 8) < 3.45 * passes_ms(0, 4)
+
+
 @pytest.mark.parametrize("n", [500, 6000])
 def test_misaligned_column_is_refused(n):
     """A column that is not 8-byte aligned never reaches a kernel."""
