@@ -14,11 +14,18 @@
 // key, and writes keys, indices and the samples of the searches
 // (egb_search.cuh): the stable order of the full keys, exactly.
 //
-// A run of more than TIE_RUN equal codes that is out of order, and any pair
-// that is (NaNs), marks its segment in Sweep::redo, and the passes over the
-// keys' own digits (egb_sort.cu) run for the marked segments.  They are
-// launched always and return at once when nothing is marked, so nothing waits
-// for the host.  Exact duplicates are in order as they come and mark nothing.
+// A run of more than TIE_RUN equal codes that is out of order (rounded values,
+// which the noise of 1e-10 sets apart in FP64 alone: every level is one; a value
+// repeated in a column) marks its segment in Sweep::redo with REDO_RUNS, and
+// run_fix_kernel sorts the segment's long runs, up to RUN_CAP points, by their high
+// 48 key bits in shared memory.  Longer ones, and any other pair out of order
+// (NaNs), mark it with REDO_DIGITS, and the passes over the keys' own digits
+// (egb_sort.cu) run for it.  Either way the tie repair and the samples of egb_sort.cu
+// follow for the segment.  All of these are launched always and return at once
+// when nothing is marked, so nothing waits for the host.  Exact duplicates are in
+// order as they come and mark nothing.  100 columns of 180,000 normals (0.77 ms)
+// rounded to 0.001: 1.37 ms, 3.01 when all of them took the digits after the codes,
+// 1.30 with digits alone; 0.1 % of each column one value: 0.94, 2.55 and 1.20.
 //
 // 785 segments of 180,000 keys: load, passes, repair and samples 0.54 + 7.60 +
 // 0.35 + 0.28 ms with the keys' digits; here load, passes and unpack 0.57 + 3.23
@@ -28,6 +35,9 @@
 // 256 threads, one per digit and sixteen words each, five to an SM (with a few
 // spills): 3.23 ms; four 3.27; 512 threads, three to an SM: 3.65; two: 4.48.
 // The unpack is bound by its gathers from L2: 512 threads 1.19 ms, 256 1.30.
+#include <algorithm>
+#include <type_traits>
+
 #include "egb_internal.cuh"
 #include "egb_search.cuh"
 #include "egb_sweep.cuh"
@@ -41,6 +51,10 @@ constexpr int UNPACK_THREADS = 512;
 constexpr int PASS_THREADS = 256;          // one per digit
 constexpr int PASS_NW = PASS_THREADS / 32;
 constexpr int TIE_RUN = 32;
+constexpr int RUN_CAP = 2048;              // its places take 16 bits beside 48 of the key
+constexpr int RUN_THREADS = 256;
+constexpr int RUN_WARP = RUN_CAP / (RUN_THREADS / 32);  // longest run that one warp sorts
+constexpr int RUN_COUNT = 128;             // and ranks by counting
 
 __device__ __forceinline__ uint32_t code_of(double x, double c) {
   uint32_t b = __float_as_uint(f32_nearest(x - c));
@@ -179,7 +193,7 @@ code_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ o
 // Sorted words -> keys, indices and samples.  A block takes SORT_TILE
 // positions and 32 to either side: enough to see all of a run of TIE_RUN.
 // Warps with no inversion in sight write their positions as they are.
-__global__ void __launch_bounds__(UNPACK_THREADS)
+__global__ void __launch_bounds__(UNPACK_THREADS, 4)
 code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict__ segs,
                    const int32_t* __restrict__ blk_seg, const uint64_t* __restrict__ words,
                    uint64_t* __restrict__ keys, int32_t* __restrict__ vals, KeyIndexOut ko,
@@ -188,6 +202,7 @@ code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict
   __shared__ uint64_t sk[SPAN];
   __shared__ uint32_t sc[SPAN];
   __shared__ uint32_t inv[SPAN / 32];  // bit: below its predecessor
+  __shared__ uint32_t brk[SPAN / 32];  // bit: of another code, or the segment's end
   const int si = blk_seg[blockIdx.x];
   const SortSeg& s = segs[si];
   const int len = s.len;
@@ -213,13 +228,18 @@ code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict
     }
   }
   __syncthreads();
-  bool bad = false;
+  bool bad = false, runs = false;
   for (int u = threadIdx.x; u < SPAN; u += UNPACK_THREADS) {
     const int p = i0 - 32 + u;
     const bool below = u > 0 && p > 0 && p < len && sk[u] < sk[u - 1];
     bad |= below && sc[u] != sc[u - 1];
-    const uint32_t m = __ballot_sync(__activemask(), below);
-    if (lane == 0) inv[u / 32] = m;
+    const bool ends = p <= 0 || p >= len || sc[u] != sc[u - 1];
+    const uint32_t m = __ballot_sync(0xffffffffu, below);
+    const uint32_t e = __ballot_sync(0xffffffffu, ends);
+    if (lane == 0) {
+      inv[u / 32] = m;
+      brk[u / 32] = e;
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -230,28 +250,173 @@ code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict
     const uint64_t k = sk[u];
     int pos = p;
     if (inv[u / 32 - 1] | inv[u / 32] | inv[u / 32 + 1]) {
-      const uint32_t c = sc[u];
-      const int ml = min(TIE_RUN, p), mr = min(TIE_RUN, len - 1 - p);
-      int l = 0, g = 0;
-      while (l < ml && sc[u - 1 - l] == c) ++l;
-      while (g < mr && sc[u + 1 + g] == c) ++g;
+      // points of the run before and after this one (32: that many, or more):
+      // the breaks at u - 31 .. u from the top, at u + 1 .. u + 32 from the bottom
+      const uint32_t b = brk[u / 32];
+      const uint32_t before = __funnelshift_rc(brk[u / 32 - 1], b, u % 32 + 1);
+      const uint32_t after = __funnelshift_rc(b, brk[u / 32 + 1], u % 32 + 1);
+      const int l = __clz((int)before), g = after ? __ffs((int)after) - 1 : TIE_RUN;
       if (l + g + 1 <= TIE_RUN) {  // the rank among the run
         int below = 0;
         for (int j = u - l; j < u; ++j) below += sk[j] <= k;
         for (int j = u + 1; j <= u + g; ++j) below += sk[j] < k;
         pos = p - l + below;
       } else {
-        bad |= l > 0 && k < sk[u - 1];
+        runs |= l > 0 && k < sk[u - 1];
       }
     }
     keys[base + pos] = k;
     vals[base + pos] = (int32_t)idx[r];
     put_samples(ko, s, pos, k);
   }
-  if (bad) redo[si] = redo[nseg] = 1u;
+  const uint32_t mark = (bad ? REDO_DIGITS : 0u) | (runs ? REDO_RUNS : 0u);
+  if (mark && (*(volatile uint32_t*)(redo + si) & mark) != mark) {
+    atomicOr(redo + si, mark);
+    atomicOr(redo + nseg, mark);
+  }
+}
+
+// The m words of buf (a power of two) in order, by the threads i0, i0 + step, ...
+// of a warp or a block that sync() joins.
+template <typename F>
+__device__ __forceinline__ void bitonic_words(uint64_t* buf, int m, int i0, int step, F&& sync) {
+  for (int k = 2; k <= m; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int i = i0; i < m / 2; i += step) {
+        const int a = ((i & ~(j - 1)) << 1) | (i & (j - 1)), b = a | j;
+        const uint64_t u = buf[a], v = buf[b];
+        if ((u > v) == ((a & k) == 0)) {
+          buf[a] = v;
+          buf[b] = u;
+        }
+      }
+      sync();
+    }
+}
+
+// The runs of more than TIE_RUN equal codes that start in a tile, each stably by
+// the high 48 bits of its keys: a word is those and the point's place in the run.
+// Runs of up to RUN_WARP points take a warp each -- up to RUN_COUNT, the place is
+// the number of smaller words, each read by all lanes at once; sorting networks there
+// are bound by their shared-memory accesses (18 million points in runs of 50: the
+// sort takes 1.88 ms with them, 1.37 so) -- and then the block takes the longer ones.
+__global__ void __launch_bounds__(RUN_THREADS, 6)
+run_fix_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict__ blk_seg, int nblk,
+               const uint64_t* __restrict__ words, uint64_t* keys, int32_t* vals, uint32_t* redo, int nseg) {
+  constexpr int NW = RUN_THREADS / 32;
+  __shared__ uint64_t word[RUN_CAP];
+  __shared__ int32_t idx[RUN_CAP];     // of the run's points, in the order they came
+  __shared__ uint16_t low[RUN_CAP];    // and the low bits of their keys
+  __shared__ int starts[SORT_TILE / TIE_RUN], lens[SORT_TILE / TIE_RUN];
+  __shared__ int nrun;
+  if (!(redo[nseg] & REDO_RUNS)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    const int si = blk_seg[b];
+    if (threadIdx.x == 0) nrun = 0;
+    // REDO_RUNS is not written any more; a segment with REDO_DIGITS is sorted anew
+    if (!(*(volatile uint32_t*)(redo + si) & REDO_RUNS)) continue;
+    __syncthreads();
+    const SortSeg& s = segs[si];
+    const int len = s.len, i0 = (b - s.blk0) * SORT_TILE;
+    const uint64_t* __restrict__ w = words + s.out_base;
+    uint64_t* key = keys + s.out_base;
+    int32_t* val = vals + s.out_base;
+    auto code = [&](int p) { return (uint32_t)(__ldg(w + p) >> 32); };
+    for (int p = i0 + (int)threadIdx.x; p < min(i0 + SORT_TILE, len); p += RUN_THREADS) {
+      const uint32_t c = code(p);
+      if (p + TIE_RUN < len && code(p + TIE_RUN) == c && (p == 0 || code(p - 1) != c)) starts[atomicAdd(&nrun, 1)] = p;
+    }
+    __syncthreads();
+    const int n = nrun;
+    if ((int)threadIdx.x < n) {
+      const int p = starts[threadIdx.x];
+      const uint32_t c = code(p);
+      int lo = p + TIE_RUN, hi = lo + 1;  // codes ascend: code(lo) == c; steps that double, then halves
+      for (int step = TIE_RUN; hi < len && hi <= p + RUN_CAP && code(hi) == c; step <<= 1) {
+        lo = hi;
+        hi = min(hi + step, len);
+      }
+      while (hi - lo > 1) {
+        const int m = (lo + hi) >> 1;
+        if (code(m) == c) lo = m; else hi = m;
+      }
+      lens[threadIdx.x] = hi - p;
+      if (hi - p > RUN_CAP) {
+        atomicOr(redo + si, REDO_DIGITS);
+        atomicOr(redo + nseg, REDO_DIGITS);
+      }
+    }
+    __syncthreads();
+    // n points from p on, staged from slot o on, by threads t, t + step, ...
+    auto sort_run = [&](int o, int p, int n, int t, int step, auto&& sync) {
+      int m = 64;
+      while (m < n) m <<= 1;
+      for (int i = t; i < m; i += step) {
+        const uint64_t k = i < n ? key[p + i] : 0ull;
+        word[o + i] = i < n ? (k & ~0xffffull) | (uint32_t)i : ~0ull;
+        if (i < n) {
+          idx[o + i] = val[p + i];
+          low[o + i] = (uint16_t)k;
+        }
+      }
+      sync();
+      bitonic_words(word + o, m, t, step, sync);
+      for (int i = t; i < n; i += step) {
+        const uint64_t k = word[o + i];
+        const int from = o + (int)(k & 0xffffull);
+        key[p + i] = (k & ~0xffffull) | low[from];
+        val[p + i] = idx[from];
+      }
+      sync();
+    };
+    auto count_run = [&](auto words_a_lane, int o, int p, int n) {
+      constexpr int R = decltype(words_a_lane)::value;
+      uint64_t w[R];
+      int32_t v[R];
+      uint32_t lo[R];
+      int place[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int i = r * 32 + lane;
+        const uint64_t k = i < n ? key[p + i] : ~0ull;
+        v[r] = i < n ? val[p + i] : 0;
+        w[r] = (k & ~0xffffull) | (uint32_t)i;
+        lo[r] = (uint32_t)k & 0xffffu;
+        place[r] = 0;
+        if (i < n) word[o + i] = w[r];
+      }
+      __syncwarp();
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const uint64_t x = word[o + j];
+#pragma unroll
+        for (int r = 0; r < R; ++r) place[r] += x < w[r];
+      }
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r * 32 + lane < n) {
+          key[p + place[r]] = (w[r] & ~0xffffull) | lo[r];
+          val[p + place[r]] = v[r];
+        }
+    };
+    for (int r = warp; r < n; r += NW)
+      if (lens[r] <= RUN_COUNT / 2)
+        count_run(std::integral_constant<int, RUN_COUNT / 64>{}, warp * RUN_WARP, starts[r], lens[r]);
+      else if (lens[r] <= RUN_COUNT)
+        count_run(std::integral_constant<int, RUN_COUNT / 32>{}, warp * RUN_WARP, starts[r], lens[r]);
+      else if (lens[r] <= RUN_WARP)
+        sort_run(warp * RUN_WARP, starts[r], lens[r], lane, 32, [] { __syncwarp(); });
+    __syncthreads();
+    for (int r = 0; r < n; ++r)
+      if (lens[r] > RUN_WARP && lens[r] <= RUN_CAP)
+        sort_run(0, starts[r], lens[r], (int)threadIdx.x, RUN_THREADS, [] { __syncthreads(); });
+    __syncthreads();
+  }
 }
 static_assert(PASS_THREADS == 256, "one thread per digit");
-static_assert((SORT_TILE + 64) % 32 == 0 && TIE_RUN <= 32, "inversion words");
+static_assert((SORT_TILE + 64) % 32 == 0 && TIE_RUN == 32, "words of bits");
 
 }  // namespace
 
@@ -275,7 +440,8 @@ void launch_word_pass(const SortSeg* segs_d, const int32_t* os_blk_seg_d, int os
 
 void launch_code_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
                       const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys, uint64_t* words,
-                      int32_t* vals, const KeyIndexOut& ko, const Sweep& w, uint32_t* err, cudaStream_t st, cudaEvent_t* pass_events) {
+                      int32_t* vals, const KeyIndexOut& ko, const Sweep& w, int num_sms, uint32_t* err, cudaStream_t st,
+                      cudaEvent_t* pass_events) {
   code_load_kernel<<<nblk, LOAD_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, words, w.seg_hist);
   count_launch();
   if (pass_events) cudaEventRecord(pass_events[0], st);
@@ -288,6 +454,9 @@ void launch_code_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int3
   if (pass_events) cudaEventRecord(pass_events[1], st);
   code_unpack_kernel<<<nblk, UNPACK_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, words, keys, vals, ko, w.redo,
                                                    nseg);
+  count_launch();
+  run_fix_kernel<<<std::min(nblk, 6 * num_sms), RUN_THREADS, 0, st>>>(segs_d, blk_seg_d, nblk, words, keys, vals, w.redo,
+                                                                     nseg);
   count_launch();
 }
 

@@ -636,8 +636,8 @@ size_t sort_sweep_bytes(int os_nblk, int nseg);
 int init_sort_kernels();
 // codes: the code sort (egb_codesort.cu) does the work, and the passes run for
 // the segments it leaves over.  Writes the samples (ko) too.  Taken for large
-// batches, where it is faster in spite of the nine launches that then usually
-// find nothing to do.  Whole calls, digits and codes: 600,000 keys 383 and 388
+// batches, where it is faster in spite of the ten launches that find
+// nothing to do but in rounded columns.  Whole calls, digits and codes: 600,000 keys 383 and 388
 // us (segments of 20,000), 329 and 336 (100,000); a million 504 and 497, 405
 // and 403, 425 and 416 (500,000); 2.2 million 841 and 801, 648 and 604; five
 // million 1639 and 1522, 1190 and 1076, 1201 and 1081.
@@ -651,7 +651,7 @@ void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d,
 int init_code_sort();
 void launch_code_sort(const BatchCol* slots_d, const SortSeg* segs_d, const int32_t* blk_seg_d, int nblk,
                       const int32_t* os_blk_seg_d, int os_nblk, int nseg, uint64_t* keys, uint64_t* words,
-                      int32_t* vals, const KeyIndexOut& ko, const Sweep& w, uint32_t* err, cudaStream_t st,
+                      int32_t* vals, const KeyIndexOut& ko, const Sweep& w, int num_sms, uint32_t* err, cudaStream_t st,
                       cudaEvent_t* pass_events);
 constexpr int SORTED_BLOCK = 128;
 void launch_sorted_jobs(const TaskDev* tasks_d, const SortedJob* jobs_d, int njobs,

@@ -48,7 +48,7 @@ constexpr int SORTED_THREADS = SORTED_BLOCK;
 // reports EGB_ERR_DEVICE) and goes on.
 //
 // redo (else null): the kernels run after the code sort (egb_codesort.cu), for
-// the segments marked there alone -- usually none, so a launch has few blocks
+// the segments marked REDO_DIGITS there alone -- usually none, so a launch has few blocks
 // and each takes many tiles.
 __global__ void __launch_bounds__(SORT_THREADS)
 onesweep_load_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict__ segs,
@@ -56,10 +56,10 @@ onesweep_load_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restri
                      int32_t* __restrict__ vals, uint32_t* __restrict__ seg_hist, int first,
                      const uint32_t* __restrict__ redo, int nseg) {
   __shared__ uint32_t h[OS_PASSES * 256];
-  if (redo && !redo[nseg]) return;
+  if (redo && !(redo[nseg] & REDO_DIGITS)) return;
   for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
     const int si = blk_seg[b];
-    if (redo && !redo[si]) continue;
+    if (redo && !(redo[si] & REDO_DIGITS)) continue;
     const SortSeg s = segs[si];
     for (int i = threadIdx.x; i < OS_PASSES * 256; i += SORT_THREADS) h[i] = 0;
     __syncthreads();
@@ -115,7 +115,7 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
   extern __shared__ __align__(16) unsigned char os_raw[];
   OsSmem<TILE>& S = *reinterpret_cast<OsSmem<TILE>*>(os_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (REDO && !redo[nseg]) return;
+  if (REDO && !(redo[nseg] & REDO_DIGITS)) return;
   do {
     if (tid == 0) S.tile = atomicAdd(tile_counter, 1);
     for (int i = tid; i < OS_NW * 256; i += OS_THREADS) (&S.wcnt[0][0])[i] = 0u;
@@ -125,7 +125,7 @@ onesweep_pass_kernel(const SortSeg* __restrict__ segs, const int32_t* __restrict
     const int si = os_blk_seg[b];
     if constexpr (REDO) {
       __syncthreads();  // S.tile is read before the next tile's id lands
-      if (!redo[si]) continue;
+      if (!(redo[si] & REDO_DIGITS)) continue;
     }
     const SortSeg s = segs[si];
     const int lb = b - s.os_blk0;
@@ -624,9 +624,10 @@ void launch_sort(const BatchCol* slots_d, const SortSeg* segs_d,
   Sweep w;
   sweep_layout(sweep, os_nblk, nseg, &w);
   if (codes)
-    launch_code_sort(slots_d, segs_d, blk_seg_d, nblk, os_blk_seg_d, os_nblk, nseg, keys_a, keys_b, vals_a, ko, w, err, st, pass_events);
+    launch_code_sort(slots_d, segs_d, blk_seg_d, nblk, os_blk_seg_d, os_nblk, nseg, keys_a, keys_b, vals_a, ko, w, num_sms, err,
+                     st, pass_events);
   const uint32_t* redo = codes ? w.redo : nullptr;
-  const int gl = codes ? std::min(nblk, 4 * num_sms) : nblk;
+  const int gl = codes ? std::min(nblk, 8 * num_sms) : nblk;
   const int gp = codes ? std::min(os_nblk, 2 * num_sms) : os_nblk;
   onesweep_load_kernel<<<gl, SORT_THREADS, 0, st>>>(slots_d, segs_d, blk_seg_d, nblk, keys_a, vals_a,
                                                    w.seg_hist, first, redo, nseg);

@@ -17,7 +17,9 @@ constexpr int OS_SPIN_LIMIT = 1 << 22;
 
 // The sweep buffer (zeroed before the sort): flag words, digit totals per
 // segment and pass, a tile counter per pass, and per segment (then for all
-// of them) whether the code sort left it to the full sort.
+// of them) what the code sort left to do.
+constexpr uint32_t REDO_DIGITS = 1u;  // the passes over the keys' digits
+constexpr uint32_t REDO_RUNS = 2u;    // long runs of equal codes to be put in order
 struct Sweep {
   unsigned long long* flags;  // [256 tiles]
   uint32_t* seg_hist;         // [nseg][ALL_PASSES][256]
