@@ -261,7 +261,13 @@ __device__ __forceinline__ void ball_positions_at(const SegView& v, const float*
     lo = p + (b - at);
     const bool out1 = a > at + HALF && hi < v.len, out0 = b == at - HALF && lo > 0;
     bool more1 = out1 || !(win[a] > b1), more0 = out0 || !(win[b] > b0);
-    if (more1 || more0) {
+    // a bracket that holds more than BALL_SCAN values is not walked through first
+    // (8 columns of 180,000 on levels of 0.1: 293 -> 131 us; 156 with the searches
+    // before the windows, which walked through one end's)
+    if ((!out1 && a + BALL_SCAN <= at + HALF && !(win[a + BALL_SCAN] > b1)) ||
+        (!out0 && !(win[b + BALL_SCAN] > b0))) {
+      ok = false;
+    } else if (more1 || more0) {
       if (out1) hi = sampled_bound_from<float, false>(v.fk, v.fs1, v.len, a1, hi);
       if (out0) lo = sampled_bound_from<float, false>(v.fk, v.fs1, v.len, a0, lo);
       const double q = value_of(__ldg(v.keys + p));
