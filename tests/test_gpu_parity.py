@@ -662,6 +662,23 @@ def test_small_batches_with_far_values(n, k, data):
     assert N.context(0).stats()["knn_deferred"] <= 4 * (1 if data == "outlier" else 0.01 * n)
 
 
+@pytest.mark.parametrize("shift", [1e6, -1e6])
+def test_two_far_clusters_are_centred_between(shift):
+    """FP32 steps are 1/32 in either of two clusters 1e6 apart about the middle,
+    and 1/16 in the far one about the other's median, whose queries then have four times
+    the near ties: 6 % of all pairs are screened, not 11."""
+    n = 100_000
+    rng = np.random.default_rng(6)
+    x = rng.normal(size=(n, 2))
+    x[:, 1] = 0.6 * x[:, 0] + 0.8 * x[:, 1]
+    pts = x + shift * rng.integers(0, 2, n)[:, None]
+    eps = N.knn_eps(pts, 3)
+    assert N.context(0).stats()["knn_tile_pairs"] < 0.085 * n * n
+    rows = rng.integers(0, n, 50)
+    for i in rows:
+        assert eps[i] == np.partition(np.abs(pts - pts[i]).max(axis=1), 3)[3]
+
+
 @pytest.mark.parametrize("n", [9, 129, 1000, 4095])
 def test_small_batches_rescale_and_index(n):
     """Strided views, a shared sample index, class orders and conditions of one
