@@ -1014,6 +1014,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     else if (force_grid || cta_grid) mode = 3;
     else {
       mode = ctx->policy[egb_policy_index(is_knn ? 0 : 1, s.sp.d, s.K, len)];
+      // beyond K = 32 only the warp grid is a layout of its own: an entry for
+      // another one, which speaks of the K up to 32 in its class, says nothing
+      if (is_knn && s.K > EGB_KREG_MAX && mode != EGB_MODE_WARP_GRID) mode = EGB_MODE_AUTO;
       if (mode == EGB_MODE_AUTO) mode = (is_knn && len < SLAB_MIN ? small_grid(s.sp.d, len) : len >= SLAB_MIN) ? (rank_ok ? 4 : 3) : 0;
     }
     if (mode == 4 && !rank_ok) mode = 3;

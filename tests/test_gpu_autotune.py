@@ -101,3 +101,21 @@ def test_policy_change_replans_a_replayed_batch():
         assert np.array_equal(a, b) and np.array_equal(a, c)
     finally:
         ctx.set_policy(None)
+
+
+@pytest.mark.parametrize("mode", [N.MODE_BRUTE, N.MODE_SLAB, N.MODE_GRID, N.MODE_WARP_GRID])
+def test_policy_entries_of_small_k_leave_large_k_its_grid(mode):
+    """One K class holds all K > 16 and is measured at 32: what it names beside the
+    warp grid has no form for K > 32, whose searches keep the rule's (a list over
+    all points would screen n^2 pairs)."""
+    ctx = N.context()
+    n = 20_000
+    pts = np.random.default_rng(5).normal(size=(n, 2))
+    ctx.set_policy(None)
+    base = N.knn_eps(pts, 50)
+    try:
+        ctx.set_policy(np.full(N.POLICY_ENTRIES, mode, dtype=np.int8))
+        assert np.array_equal(N.knn_eps(pts, 50), base)
+        assert ctx.stats()["knn_tile_pairs"] < n * n // 16
+    finally:
+        ctx.set_policy(None)
