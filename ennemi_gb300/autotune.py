@@ -26,6 +26,7 @@ from __future__ import annotations
 import json
 import os
 from typing import Dict, Iterable, List, Optional, Sequence, Tuple
+from warnings import warn
 
 import numpy as np
 
@@ -36,6 +37,10 @@ MODE_NAMES = {N.MODE_AUTO: "auto", N.MODE_BRUTE: "brute", N.MODE_SLAB: "slab",
               N.MODE_GRID: "grid", N.MODE_WARP_GRID: "warp_grid", N.MODE_RANK: "rank"}
 K_OF_CLASS = (4, 8, 16, 32)   # K = k + 1 measured for each kNN K class
 CACHE_ENV = "ENNEMI_GB300_POLICY"
+# Which kernels the modes stand for: raised when that changes, so that tables
+# measured on other kernels are not installed by themselves.  1 (not written to
+# files): warp grids for K <= 8 only, any-K select beyond 32; 2: warp lists.
+REVISION = 2
 
 # (search, d, K) -> list of (size class, mode)
 Key = Tuple[int, int, int]
@@ -205,21 +210,26 @@ def cache_path(device: int = 0) -> str:
 
 def save(table: np.ndarray, path: str, meta: Optional[dict] = None) -> None:
     os.makedirs(os.path.dirname(os.path.abspath(path)), exist_ok=True)
-    doc = {"entries": N.POLICY_ENTRIES, "modes": [int(m) for m in table], "meta": meta or {}}
+    doc = {"entries": N.POLICY_ENTRIES, "revision": REVISION, "modes": [int(m) for m in table], "meta": meta or {}}
     tmp = path + ".tmp"
     with open(tmp, "w") as f:
         json.dump(doc, f)
     os.replace(tmp, path)
 
 
-def load(path: str) -> Optional[np.ndarray]:
-    """The table saved at `path`, or None if absent or of another layout."""
+def load(path: str, current: bool = False) -> Optional[np.ndarray]:
+    """The table saved at `path`, or None if absent or of another layout;
+    current: also None, with a warning, if tuned under another REVISION."""
     try:
         with open(path) as f:
             doc = json.load(f)
     except (OSError, ValueError):
         return None
     if doc.get("entries") != N.POLICY_ENTRIES or len(doc.get("modes", ())) != N.POLICY_ENTRIES:
+        return None
+    if current and doc.get("revision", 1) != REVISION:
+        warn(f"layout policy {path} was tuned for other kernels and is not installed; "
+             "run ennemi_gb300.autotune.autotune() again, or set it with Context.set_policy(load(path))")
         return None
     table = np.array(doc["modes"], dtype=np.int8)
     if table.min() < N.MODE_AUTO or table.max() > N.MODE_RANK:
@@ -231,7 +241,7 @@ def load_cached(ctx: N.Context) -> bool:
     env = os.environ.get(CACHE_ENV)
     tag = "".join(c if c.isalnum() else "_" for c in ctx.device_name())
     path = env or os.path.join(os.path.expanduser("~"), ".cache", "ennemi_gb300", f"policy_{tag}.json")
-    table = load(path)
+    table = load(path, current=True)
     if table is None:
         return False
     ctx.set_policy(table)

@@ -4,6 +4,7 @@ batch plans, filling of unmeasured size classes, and the policy file."""
 import json
 
 import numpy as np
+import pytest
 
 from ennemi_gb300 import _native as N
 from ennemi_gb300 import autotune as A
@@ -51,3 +52,21 @@ def test_policy_file_round_trip_and_rejects(tmp_path):
 def test_cache_path_honours_environment(monkeypatch, tmp_path):
     monkeypatch.setenv(A.CACHE_ENV, str(tmp_path / "x.json"))
     assert A.cache_path(0) == str(tmp_path / "x.json")
+
+
+def test_tables_of_another_revision_are_not_installed_by_themselves(tmp_path):
+    """A file without a revision, as saved before there was one, or with another:
+    load() still gives its table to a caller who asks for it."""
+    table = np.full(N.POLICY_ENTRIES, N.MODE_SLAB, dtype=np.int8)
+    path = str(tmp_path / "p.json")
+    A.save(table, path)
+    assert np.array_equal(A.load(path, current=True), table)
+    for revision in (None, A.REVISION - 1, A.REVISION + 1):
+        doc = json.load(open(path))
+        doc.pop("revision", None)
+        if revision is not None:
+            doc["revision"] = revision
+        json.dump(doc, open(path, "w"))
+        with pytest.warns(UserWarning, match="other kernels"):
+            assert A.load(path, current=True) is None
+        assert np.array_equal(A.load(path), table)
