@@ -32,10 +32,14 @@ import numpy as np
 
 from . import _native as N
 
-MODES = (N.MODE_BRUTE, N.MODE_SLAB, N.MODE_GRID, N.MODE_WARP_GRID, N.MODE_RANK)
+MODES = (N.MODE_AUTO, N.MODE_BRUTE, N.MODE_SLAB, N.MODE_GRID, N.MODE_WARP_GRID, N.MODE_RANK)
 MODE_NAMES = {N.MODE_AUTO: "auto", N.MODE_BRUTE: "brute", N.MODE_SLAB: "slab",
               N.MODE_GRID: "grid", N.MODE_WARP_GRID: "warp_grid", N.MODE_RANK: "rank"}
 K_OF_CLASS = (4, 8, 16, 32)   # K = k + 1 measured for each kNN K class
+# An entry is left to the built-in rule unless a layout is faster than the rule's
+# by more than this.  An entry says which layout to take, and batches of small
+# tasks, which the rule serves without any (egb_direct.cu), get one then.
+RULE_MARGIN = 0.05
 CACHE_ENV = "ENNEMI_GB300_POLICY"
 # Which kernels the modes stand for: raised when that changes, so that tables
 # measured on other kernels are not installed by themselves.  1 (not written to
@@ -81,6 +85,13 @@ def _measure(ctx: N.Context, search: int, d: int, K: int, n: int, mode: int,
     return best
 
 
+def _choose(times: Dict[int, float]) -> int:
+    """The mode of an entry, from the times of the modes measured."""
+    best = min(times, key=times.get)
+    auto = times.get(N.MODE_AUTO, np.inf)
+    return N.MODE_AUTO if auto <= times[best] * (1.0 + RULE_MARGIN) else best
+
+
 def _tune_key(ctx, key: Key, size_classes: Sequence[int], repeats: int,
               prune: float, log) -> Dict[int, Tuple[int, Dict[int, float]]]:
     search, d, K = key
@@ -93,13 +104,13 @@ def _tune_key(ctx, key: Key, size_classes: Sequence[int], repeats: int,
         if n <= K:
             continue
         times = {m: _measure(ctx, search, d, K, n, m, repeats, 1000 + sc) for m in alive}
-        best_mode = min(times, key=times.get)
+        best_mode = _choose(times)
         out[sc] = (best_mode, times)
         if log:
             log(f"search={'knn' if search == 0 else 'count'} d={d} K={K} n={n}: " +
                 " ".join(f"{MODE_NAMES[m]}={t:.3f}ms" for m, t in times.items()) +
                 f" -> {MODE_NAMES[best_mode]}")
-        alive = [m for m in alive if times[m] <= prune * times[best_mode]]
+        alive = [m for m in alive if m == N.MODE_AUTO or times[m] <= prune * min(times.values())]
     return out
 
 

@@ -70,3 +70,12 @@ def test_tables_of_another_revision_are_not_installed_by_themselves(tmp_path):
         with pytest.warns(UserWarning, match="other kernels"):
             assert A.load(path, current=True) is None
         assert np.array_equal(A.load(path), table)
+
+
+def test_entries_that_gain_nothing_stay_with_the_rule():
+    """Batches of small tasks take no layout at all under the rule, and one under
+    any other entry."""
+    assert A._choose({N.MODE_AUTO: 1.0, N.MODE_BRUTE: 0.97, N.MODE_SLAB: 2.0}) == N.MODE_AUTO
+    assert A._choose({N.MODE_AUTO: 1.0, N.MODE_BRUTE: 0.9, N.MODE_SLAB: 2.0}) == N.MODE_BRUTE
+    assert A._choose({N.MODE_BRUTE: 3.0, N.MODE_SLAB: 2.0}) == N.MODE_SLAB
+    assert N.MODE_AUTO in A.MODES

@@ -119,3 +119,22 @@ def test_policy_entries_of_small_k_leave_large_k_its_grid(mode):
         assert ctx.stats()["knn_tile_pairs"] < n * n // 16
     finally:
         ctx.set_policy(None)
+
+
+def test_a_tuned_context_keeps_small_batches_without_layouts(monkeypatch):
+    """Tuned for a pair of 1,000 samples, all layouts as fast as the rule, the pair
+    still runs in three launches."""
+    ctx = N.context()
+    rng = np.random.default_rng(6)
+    x = rng.normal(size=(2, 1000))
+    task = [N.Task(N.MI, 3, [x[0]], [x[0] + x[1]])]
+    ctx.set_policy(None)
+    base = N.run_tasks(task)
+    launches = ctx.stats()["kernel_launches"]
+    try:
+        monkeypatch.setattr(A, "_measure", lambda *a: 1.0)
+        A.autotune(tasks=task, save_to=None)
+        assert np.array_equal(N.run_tasks(task), base)
+        assert ctx.stats()["kernel_launches"] == launches == 3
+    finally:
+        ctx.set_policy(None)
