@@ -374,7 +374,7 @@ def _estimate_mi(y: FloatArray, x: FloatArray, lag: FloatArray, k: int,
             if dz:
                 ptr[:, :, 2:] = zc.address(z_rows, np.arange(dz)[None, :])[:, None, :]
                 stride[:, :, 2:] = zc.row // 8
-            return ptr.reshape(nlag * nvar, -1), stride.reshape(nlag * nvar, -1)
+            return ptr.reshape(nlag * nvar, 2 + dz), stride.reshape(nlag * nvar, 2 + dz)
 
         def spec(t):
             li, vi = divmod(t, nvar)

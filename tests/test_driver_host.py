@@ -413,3 +413,11 @@ def test_addresses_of_lagged_views(monkeypatch, dtype):
     assert t.ptr.tolist() == want and t.stride.tolist() == [[2, 2]] * 8
     with pytest.raises(TypeError):
         _native.Columns(y).address(1.5)
+
+
+@pytest.mark.parametrize("drop_nan", [False, True])
+@pytest.mark.parametrize("lag", [0, [0, 1, 2, 3, 4]])
+def test_no_variables_give_no_estimates(lag, drop_nan):
+    y = np.random.default_rng(0).normal(size=100)
+    r = eg.estimate_mi(y, np.empty((100, 0)), lag=lag, drop_nan=drop_nan, cond=y[:, None])
+    assert r.shape == (len(np.atleast_1d(lag)), 0)
