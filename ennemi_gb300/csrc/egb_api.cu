@@ -1236,8 +1236,8 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     J.seg_begin = (int32_t)m.s.b;
     J.len = (int32_t)len;
     J.K = m.is_knn ? m.s.K : 0;
-    // FP32-path warp-grid counts of d = 2, 3 run on keys (egb_wcount.cu)
-    J.kform = (m.mode == 3 && !m.is_knn && !plain && count_keys_supported(m.s.sp.d)) ? 1 : 0;
+    // FP32-path warp-grid counts of two columns run on keys (egb_wcount.cu)
+    J.kform = (m.mode == 3 && !m.is_knn && !plain && m.s.sp.d == 2) ? 1 : 0;
     J.slab = m.slab;
     J.sort_seg = m.sort_seg;
     J.sp = m.s.sp;
@@ -2236,9 +2236,9 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     Group& G = groups[g];
     if (G.is_knn || G.nitems == 0) continue;
     if (G.mode == 3) {
-      if (!plain && count_keys_supported(G.dclass))
-        launch_count_keys((const JobDev*)dtab(tab_jobs), items_of(G),
-                          (int)G.nitems, G.dclass, counters + 2 * g, ctx->num_sms, st);
+      if (!plain && G.dclass == 2)
+        launch_count_keys((const JobDev*)dtab(tab_jobs), items_of(G), (int)G.nitems, counters + 2 * g,
+                          ctx->num_sms, st);
       else if (G.boxed)
         launch_count_leaf((const JobDev*)dtab(tab_jobs), items_of(G), (int)G.nitems,
                           (const float*)(A + G.off_box), G.dclass, counters + 2 * g, ctx->num_sms, st);

@@ -723,9 +723,8 @@ void launch_knn_walk(const JobDev* jobs_d, const WorkItem* items_d, int nitems, 
                      int dclass, int* counter, int num_sms, cudaStream_t st);
 // egb_wcount.cu: exact key-range ball counts of d = 2 warp-grid jobs (FP32
 // path; the FP64 comparator keeps launch_count_wgrid)
-bool count_keys_supported(int dclass);
-void launch_count_keys(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass,
-                       int* counter, int num_sms, cudaStream_t st);
+void launch_count_keys(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int* counter, int num_sms,
+                       cudaStream_t st);
 void launch_count_wgrid(const JobDev* jobs_d, const WorkItem* items_d, int nitems, int dclass, int dmax,
                         int* counter, int num_sms, cudaStream_t st);
 
