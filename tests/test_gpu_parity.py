@@ -449,6 +449,24 @@ def test_labels_and_index_at_any_address():
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("n,k,data", [(270_000, 127, "normal"), (270_000, 127, "levels"), (270_000, 127, "huge"),
+                                      (650_000, 52, "normal"), (4_300_000, 3, "normal")])
+def test_strips_longer_than_a_block_orders(n, k, data):
+    """Two-column grids whose strips exceed 4096 points are laid out by sorted
+    strip keys: lists from n K = 3.3e7 on, walks from 4.2 million points."""
+    rng = np.random.default_rng(k)
+    pts = rng.normal(size=(n, 2))
+    if data == "levels":
+        pts = np.round(pts, 2) + 1e-10 * rng.normal(size=(n, 2))
+    elif data == "huge":
+        pts[:, 1] *= 1e300
+    eps = N.knn_eps(pts, k)
+    assert N.context(0).stats()["knn_tile_pairs"] < n * (n // 8) or data == "huge"
+    far = np.argsort(np.abs(pts[:, 0]))[-3:]
+    for i in [0, n - 1, *far, *rng.integers(0, n, 40 if n < 10 ** 6 else 10)]:
+        assert eps[i] == np.partition(np.abs(pts - pts[i]).max(axis=1), k)[k], i
+
+
 def _long_runs(n, lengths, rng):
     """Normal values, and runs of them 2^-40 apart: equal codes, out of order."""
     x = rng.normal(size=n)
