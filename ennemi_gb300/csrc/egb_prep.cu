@@ -202,46 +202,43 @@ rescale_stats_kernel(const BatchCol* __restrict__ slots, const RescaleStat* __re
   if (threadIdx.x == 0 && blockIdx.x % CL == 0) ms[stat] = make_double2(mean, __dsqrt_rn(__ddiv_rn(q, n)));
 }
 
-// x = RN(RN(RN(x - mean) / sd) + noise) per sample of a batch column (a y-row
-// of blocks per column and on, four samples in flight per thread)
+// x = RN(RN(RN(x - mean) / sd) + noise) per sample of a task column (one
+// y-row of blocks per column, four samples in flight per thread)
 __global__ void __launch_bounds__(PREP_THREADS)
-rescale_apply_kernel(const BatchCol* __restrict__ slots, const RescaleCol* __restrict__ cols, int ncols,
+rescale_apply_kernel(const BatchCol* __restrict__ slots, const RescaleCol* __restrict__ cols,
                      const double2* __restrict__ ms, const double* __restrict__ noise,
                      uint32_t* __restrict__ const_flags) {
-  __shared__ double rsd_s;  // RN(1 / sd), once per block and column
-  for (int g = blockIdx.y; g < ncols; g += gridDim.y) {
-    const RescaleCol rc = cols[g];
-    const int n = slots[rc.slot].n;
-    double* x = slots[rc.slot].x;
-    const double2 m = ms[rc.stat];
-    const double mean = m.x, sd = m.y;
-    if (fabs(sd) < 1e-20) {  // np.abs(std) < 1e-20: the reference warns and keeps x
-      if (blockIdx.x == 0 && threadIdx.x == 0) const_flags[rc.slot] = 1u;
-      continue;
-    }
-    __syncthreads();  // the last column's value has been read
-    if (threadIdx.x == 0) rsd_s = __ddiv_rn(1.0, sd);
-    __syncthreads();
-    const double rsd = rsd_s;
-    const double* nz = noise + rc.noise_pos;
-    const int64_t step = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
-      int w[4];
-      double v[4], z[4];
+  const RescaleCol rc = cols[blockIdx.y];
+  const int n = slots[rc.slot].n;
+  double* x = slots[rc.slot].x;
+  const double2 m = ms[rc.stat];
+  const double mean = m.x, sd = m.y;
+  if (fabs(sd) < 1e-20) {  // np.abs(std) < 1e-20: the reference warns and keeps x
+    if (blockIdx.x == 0 && threadIdx.x == 0) const_flags[rc.slot] = 1u;
+    return;
+  }
+  __shared__ double rsd_s;  // RN(1 / sd), once per block
+  if (threadIdx.x == 0) rsd_s = __ddiv_rn(1.0, sd);
+  __syncthreads();
+  const double rsd = rsd_s;
+  const double* nz = noise + rc.noise_pos;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * step) {
+    int w[4];
+    double v[4], z[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {  // sample i0 + u * step
-        const int64_t i = i0 + u * step;
-        w[u] = -1;
-        if (i < n) {
-          w[u] = rc.inv ? rc.inv[i] : (int)i;
-          v[u] = x[w[u]];
-          z[u] = nz[i * rc.group];
-        }
+    for (int u = 0; u < 4; ++u) {  // sample i0 + u * step
+      const int64_t i = i0 + u * step;
+      w[u] = -1;
+      if (i < n) {
+        w[u] = rc.inv ? rc.inv[i] : (int)i;
+        v[u] = x[w[u]];
+        z[u] = nz[i * rc.group];
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (w[u] >= 0) x[w[u]] = __dadd_rn(div_rn(__dsub_rn(v[u], mean), sd, rsd), z[u]);
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (w[u] >= 0) x[w[u]] = __dadd_rn(div_rn(__dsub_rn(v[u], mean), sd, rsd), z[u]);
   }
 }
 
@@ -542,9 +539,11 @@ void launch_rescale(const BatchCol* slots_d, const RescaleStat* stats_d, int nst
   // 16 us on two blocks each
   const int gx = std::min(grid_x_for((max_n + 3) / 4),
                           std::max(grid_x_for((max_n + 31) / 32), 2048 / std::min(ncols, 2048)));
-  const dim3 agrid(gx, grid_y_for(ncols));
-  rescale_apply_kernel<<<agrid, PREP_THREADS, 0, st>>>(slots_d, cols_d, ncols, ms, noise, const_flags);
-  count_launch();
+  for (int c0 = 0; c0 < ncols; c0 += 65535) {  // as many columns as a grid has rows
+    const dim3 agrid(gx, grid_y_for(ncols - c0));
+    rescale_apply_kernel<<<agrid, PREP_THREADS, 0, st>>>(slots_d, cols_d + c0, ms, noise, const_flags);
+    count_launch();
+  }
 }
 
 void launch_divide(const double* a_d, const double* b_d, int64_t n, double* out_d, cudaStream_t st) {
