@@ -236,7 +236,12 @@ __device__ __forceinline__ void ball_positions(const SegView& v, double q, doubl
 // next float, r in rd and below the next one, rn.  The 8-byte key of p is
 // read, and FP64 arithmetic done, only for ends with values inside a bracket;
 // one loop serves both ends, so a warp pays for the longer of its lanes'
-// checks rather than for each end in turn.
+// checks rather than for each end in turn, and for BALL_WALK values at most before
+// the exact search.  Rounded columns have hundreds in a bracket: 100 of 180,000,
+// rounded to 0.001, 2.70 ms with 32, 1.75 with 16, 1.33 with 8 (2.59 before the
+// windows); a million normals about 100, which have eight or so at either end, 145,
+// 162 and 197 us; at unit scale up to 16 million points none of them matters.
+constexpr int BALL_WALK = 16;
 template <int HALF>
 __device__ __forceinline__ void ball_positions_at(const SegView& v, const float* win, int at, int p,
                                                   double r, int& lo, int& hi) {
@@ -261,13 +266,7 @@ __device__ __forceinline__ void ball_positions_at(const SegView& v, const float*
     lo = p + (b - at);
     const bool out1 = a > at + HALF && hi < v.len, out0 = b == at - HALF && lo > 0;
     bool more1 = out1 || !(win[a] > b1), more0 = out0 || !(win[b] > b0);
-    // a bracket that holds more than BALL_SCAN values is not walked through first
-    // (8 columns of 180,000 on levels of 0.1: 293 -> 131 us; 156 with the searches
-    // before the windows, which walked through one end's)
-    if ((!out1 && a + BALL_SCAN <= at + HALF && !(win[a + BALL_SCAN] > b1)) ||
-        (!out0 && !(win[b + BALL_SCAN] > b0))) {
-      ok = false;
-    } else if (more1 || more0) {
+    if (more1 || more0) {
       if (out1) hi = sampled_bound_from<float, false>(v.fk, v.fs1, v.len, a1, hi);
       if (out0) lo = sampled_bound_from<float, false>(v.fk, v.fs1, v.len, a0, lo);
       const double q = value_of(__ldg(v.keys + p));
@@ -284,7 +283,7 @@ __device__ __forceinline__ void ball_positions_at(const SegView& v, const float*
           } else {
             if (in) more0 = false; else ++lo;
           }
-          ok = ++n < 2 * BALL_SCAN;
+          ok = ++n < BALL_WALK;
         }
       } while (ok && (more1 || more0));
     }

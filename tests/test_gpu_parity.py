@@ -339,7 +339,8 @@ def test_window_counts_on_noisy_levels(n):
 
 def test_window_counts_on_noisy_levels_keep_pace():
     """Device times of the 1-D counts, against those of continuous columns: the
-    exact search of each end (2.6 times) and no walk before it (5.7)."""
+    exact search of each end and a short walk before it (3.6 times; with a long
+    one 5.7)."""
     rng = np.random.default_rng(4)
     ctx = N.context(0)
 
@@ -354,7 +355,7 @@ def test_window_counts_on_noisy_levels_keep_pace():
             best = min(best, ctx.timings()["count_1d"])
         return best
 
-    assert counts_ms(0.1) < 4.0 * counts_ms(0.0)
+    assert counts_ms(0.1) < 4.5 * counts_ms(0.0)
 
 
 def _code_columns(data, n, rng):
