@@ -202,7 +202,6 @@ code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict
   __shared__ uint64_t sk[SPAN];
   __shared__ uint32_t sc[SPAN];
   __shared__ uint32_t inv[SPAN / 32];  // bit: below its predecessor
-  __shared__ uint32_t brk[SPAN / 32];  // bit: of another code, or the segment's end
   const int si = blk_seg[blockIdx.x];
   const SortSeg& s = segs[si];
   const int len = s.len;
@@ -233,30 +232,31 @@ code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict
     const int p = i0 - 32 + u;
     const bool below = u > 0 && p > 0 && p < len && sk[u] < sk[u - 1];
     bad |= below && sc[u] != sc[u - 1];
-    const bool ends = p <= 0 || p >= len || sc[u] != sc[u - 1];
     const uint32_t m = __ballot_sync(0xffffffffu, below);
-    const uint32_t e = __ballot_sync(0xffffffffu, ends);
-    if (lane == 0) {
-      inv[u / 32] = m;
-      brk[u / 32] = e;
-    }
+    if (lane == 0) inv[u / 32] = m;
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int u = 32 + r * UNPACK_THREADS + (int)threadIdx.x;
     const int p = i0 - 32 + u;
-    if (p >= len) break;
     const uint64_t k = sk[u];
     int pos = p;
-    if (inv[u / 32 - 1] | inv[u / 32] | inv[u / 32 + 1]) {
-      // points of the run before and after this one (32: that many, or more):
-      // the breaks at u - 31 .. u from the top, at u + 1 .. u + 32 from the bottom
-      const uint32_t b = brk[u / 32];
-      const uint32_t before = __funnelshift_rc(brk[u / 32 - 1], b, u % 32 + 1);
-      const uint32_t after = __funnelshift_rc(b, brk[u / 32 + 1], u % 32 + 1);
+    if (inv[u / 32 - 1] | inv[u / 32] | inv[u / 32 + 1]) {  // the same for the whole warp
+      // points of the run before and after this one (32: that many, or more), from
+      // the positions that start another run: those at u - 31 .. u from the top, at
+      // u + 1 .. u + 32 from the bottom
+      auto starts = [&](int w) {
+        const int q = i0 - 32 + w;
+        return w > 0 && (q <= 0 || q >= len || sc[w] != sc[w - 1]);
+      };
+      const uint32_t b0 = __ballot_sync(0xffffffffu, starts(u - 32));
+      const uint32_t b1 = __ballot_sync(0xffffffffu, starts(u));
+      const uint32_t b2 = __ballot_sync(0xffffffffu, starts(u + 32));
+      const uint32_t before = __funnelshift_rc(b0, b1, lane + 1), after = __funnelshift_rc(b1, b2, lane + 1);
       const int l = __clz((int)before), g = after ? __ffs((int)after) - 1 : TIE_RUN;
-      if (l + g + 1 <= TIE_RUN) {  // the rank among the run
+      if (p >= len) {
+      } else if (l + g + 1 <= TIE_RUN) {  // the rank among the run
         int below = 0;
         for (int j = u - l; j < u; ++j) below += sk[j] <= k;
         for (int j = u + 1; j <= u + g; ++j) below += sk[j] < k;
@@ -265,9 +265,11 @@ code_unpack_kernel(const BatchCol* __restrict__ slots, const SortSeg* __restrict
         runs |= l > 0 && k < sk[u - 1];
       }
     }
-    keys[base + pos] = k;
-    vals[base + pos] = (int32_t)idx[r];
-    put_samples(ko, s, pos, k);
+    if (p < len) {
+      keys[base + pos] = k;
+      vals[base + pos] = (int32_t)idx[r];
+      put_samples(ko, s, pos, k);
+    }
   }
   const uint32_t mark = (bad ? REDO_DIGITS : 0u) | (runs ? REDO_RUNS : 0u);
   if (mark && (*(volatile uint32_t*)(redo + si) & mark) != mark) {
