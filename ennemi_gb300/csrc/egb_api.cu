@@ -11,10 +11,12 @@
 //   sort        every 1-D space and the first column of every slab job, one
 //               segmented LSD radix sort for the whole batch
 //   materialise multi-D job blocks (FP64 + centred FP32, working or sorted)
-//   kNN         1-D: merge on sorted keys; multi-D: tile kernels (brute force
-//               or slab), any-K select for k + 1 > 32
-//   radius      rad = eps - 1e-12
-//   counts      1-D: windows of the sorted values; multi-D: tile kernels
+//   kNN         1-D: merge on sorted keys; multi-D: walks or warp lists on grid
+//               copies, lists over all points or tiles for small sets; K = k + 1
+//               > 128 (the all-FP64 comparator: > 32): select over all points
+//   counts      (radius fl64(eps - 1e-12), formed as it is read)  1-D: windows of
+//               the sorted values; two columns: rank space; more: leaf boxes;
+//               small sets: tiles
 //   combine     per-task term sums (psi table / log) + zero flags
 //   download    partial sums, flags, device error word
 //
@@ -1259,7 +1261,7 @@ int run_batch_sorted(egb_ctx* ctx, const egb_task* tasks, int ntasks, int flags,
     }
     if (m.mode >= 2) {
       J.c64g = (double*)(uintptr_t)dl.take(sizeof(double) * (size_t)(d * J.lds));
-      // by point where the walks and the warp lists of two and three columns read it
+      // by point where the walks and the warp lists of two to four columns read it
       J.aos = (m.mode == 3 && m.is_knn && !plain && d <= 4) ? 1 : 0;
       J.c32g = (float*)(uintptr_t)dl.take(sizeof(float) * (size_t)((J.aos ? grid_aos(d) : d) * J.lds));
       J.idxg = (int32_t*)(uintptr_t)dl.take(sizeof(int32_t) * (size_t)J.lds);

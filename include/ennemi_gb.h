@@ -253,7 +253,8 @@ int egb_last_stats(const egb_ctx* ctx, int64_t* out, int32_t max);
  * reference, whose cKDTree has a single layout).  Every multi-dimensional
  * search job of a batch -- a kNN search or a ball count over d >= 2 columns --
  * runs in one of five layouts:
- *   EGB_MODE_BRUTE      tiles of all points against all points
+ *   EGB_MODE_BRUTE      all points against all points: tiles, or for kNN a
+ *                       warp per query where that is faster
  *   EGB_MODE_SLAB       points sorted by column 0, tiles from a window
  *   EGB_MODE_GRID       equal-count strips, 128-query CTA work items
  *   EGB_MODE_WARP_GRID  equal-count strips, 32-query warp work items
@@ -265,10 +266,14 @@ int egb_last_stats(const egb_ctx* ctx, int64_t* out, int32_t max);
  * Each layout gives the same results bit for bit; only speed differs.  The
  * planner reads the context's table at egb_policy_index(search, d, K, len);
  * EGB_MODE_AUTO (every entry of a new context) selects the built-in rule:
- * brute force below 4096 points, otherwise the rank-space counts for d = 2
- * ball counts and the warp grid for the rest (CTA grid for kNN with
- * 9 <= K <= 32).  K > 32 kNN always uses the select kernel, and the
- * EGB_FORCE_* flags override the table.
+ * below 4096 points brute force, but the warp grid for kNN of 1024 points and
+ * more where a batch holds many of them; otherwise the rank-space counts for
+ * d = 2 ball counts and the warp grid for the rest (the all-FP64 comparator:
+ * CTA grid for 9 <= K <= 32).  For K of 33 to 128 an entry other than
+ * EGB_MODE_WARP_GRID leaves the rule in force (the comparator, and K > 128:
+ * the select kernel over all points).  A batch of small tasks whose entries are all
+ * EGB_MODE_AUTO runs without any layout, in three launches.  The EGB_FORCE_*
+ * flags override the table.
  */
 #define EGB_MODE_AUTO (-1)
 #define EGB_MODE_BRUTE 0
