@@ -355,9 +355,6 @@ def _estimate_mi(y: FloatArray, x: FloatArray, lag: FloatArray, k: int,
     if _device_prep_ok((x, y) + (() if cond is None else (cond,)), cond, preprocess, drop_nan,
                        discrete_x or discrete_y, nan_rows_ok=True):
         lo, hi = min(min_lag, 0), max(max_lag, 0)
-        y_row = operator.index(hi)
-        x_rows = _first_rows(y_row, lag, 1)
-        z_rows = None if cond is None else _first_rows(y_row, cond_lag, 2)
         n0 = len(y) - hi + lo
         xc, yc = _native.Columns(x), _native.Columns(y)
         zc = None if cond is None else _native.Columns(cond)
@@ -366,12 +363,15 @@ def _estimate_mi(y: FloatArray, x: FloatArray, lag: FloatArray, k: int,
         def addresses():
             # the lagged views: task (li, vi) starts at row hi - lag of x, hi of
             # y and hi - cond_lag of each condition column
+            y_row = operator.index(hi)
+            x_rows = _first_rows(y_row, lag, 1)
             ptr = np.empty((nlag, nvar, 2 + dz), dtype=np.uint64)
             stride = np.empty((nlag, nvar, 2 + dz), dtype=np.int64)
             ptr[:, :, 0] = xc.address(x_rows[:, None], np.arange(nvar)[None, :])
             ptr[:, :, 1] = yc.address(y_row)
             stride[:, :, 0], stride[:, :, 1] = xc.row // 8, yc.row // 8
             if dz:
+                z_rows = _first_rows(y_row, cond_lag, 2)
                 ptr[:, :, 2:] = zc.address(z_rows, np.arange(dz)[None, :])[:, None, :]
                 stride[:, :, 2:] = zc.row // 8
             return ptr.reshape(nlag * nvar, 2 + dz), stride.reshape(nlag * nvar, 2 + dz)
@@ -379,8 +379,8 @@ def _estimate_mi(y: FloatArray, x: FloatArray, lag: FloatArray, k: int,
         def spec(t):
             li, vi = divmod(t, nvar)
             xv = xc.array if x.ndim == 1 else xc.array[:, vi]
-            return (_native.Col(xv[x_rows[li]:]), _native.Col(yc.array[y_row:]),
-                    [_native.Col(zc.array[z_rows[li, c]:, c]) for c in range(dz)] if dz else None)
+            return (_native.Col(xv[hi - lag[li]:]), _native.Col(yc.array[hi:]),
+                    [_native.Col(zc.array[hi - cond_lag[li][c]:, c]) for c in range(dz)] if dz else None)
 
         values = _run_device_prep(nlag * nvar, 2 + dz, addresses, spec, n0, k, prep.idx, job, max_threads,
                                   drop_nan, (xc, yc, zc))
@@ -644,12 +644,13 @@ def _first_rows(hi: int, lags, ndim: int) -> np.ndarray:
     """hi - lags, the first rows of lagged views, as int64.  Lags that a slice
     does not take (floats, whatever their value, bools, arrays) raise its
     TypeError."""
-    lags = np.asarray(lags)
-    if lags.ndim != ndim:
-        raise TypeError("lags must be integers")
-    if lags.dtype.kind not in "iu":
-        lags = np.array([operator.index(v) for v in lags.ravel()], dtype=np.int64).reshape(lags.shape)
-    return hi - lags.astype(np.int64)
+    if lags.dtype != np.int64 or lags.ndim != ndim:
+        if lags.ndim != ndim:
+            raise TypeError("lags must be integers")
+        if lags.dtype.kind not in "iu":
+            lags = np.array([operator.index(v) for v in lags.ravel()]).reshape(lags.shape)
+        lags = lags.astype(np.int64)
+    return hi - lags
 
 
 def _run_device_prep(nt: int, nc: int, addresses, spec, n0: int, k: int, idx, job, max_threads,
